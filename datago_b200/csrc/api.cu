@@ -96,7 +96,6 @@ struct Block {
     void* ptr = nullptr;
     size_t size = 0;
     bool busy = false;
-    size_t zero_prefix = 0;  // scratch blocks: leading bytes known to be zero (the coefficient region, see dg_batch_run)
 };
 
 // Grow-only cache: a batch borrows blocks and hands them back; nothing is freed before the ctx goes away, so steady
@@ -105,7 +104,7 @@ struct BlockCache {
     bool pinned;
     std::vector<Block> blocks;
     explicit BlockCache(bool p) : pinned(p) {}
-    int acquire(size_t size, int* index, bool keep_zero_prefix = false) {
+    int acquire(size_t size, int* index) {
         if (size == 0) size = 256;
         int best = -1;
         for (size_t i = 0; i < blocks.size(); ++i)
@@ -130,7 +129,6 @@ struct BlockCache {
             else { blocks.push_back(nb); best = (int)blocks.size() - 1; }
         }
         blocks[best].busy = true;
-        if (!keep_zero_prefix) blocks[best].zero_prefix = 0;
         *index = best;
         return DG_OK;
     }
@@ -151,7 +149,7 @@ struct dg_ctx {
     cudaStream_t stream2 = nullptr;  // odd waves of a batch run here, concurrently with the even ones
     cudaStream_t aux[2] = {nullptr, nullptr};  // per lane: the restart-interval decoder runs beside the speculative one
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    cudaEvent_t ev_aux_go[2] = {nullptr, nullptr}, ev_aux_done[2] = {nullptr, nullptr};
+    cudaEvent_t ev_aux_go[2] = {nullptr, nullptr}, ev_aux_huge[2] = {nullptr, nullptr}, ev_aux_done[2] = {nullptr, nullptr};
     bool own_stream = false;
     bool has_tfm = false;
     dg_image_config cfg{};
@@ -226,6 +224,8 @@ static int ctx_create(int device, const dg_image_config* cfg, void* stream, bool
         cudaStreamCreateWithFlags(&c->aux[1], cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_aux_go[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_aux_go[1], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_aux_huge[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_aux_huge[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_aux_done[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_aux_done[1], cudaEventDisableTiming) != cudaSuccess) {
         delete c;
@@ -258,6 +258,7 @@ extern "C" void dg_ctx_destroy(dg_ctx* c) {
     for (int i = 0; i < 2; ++i) {
         cudaStreamSynchronize(c->aux[i]);
         cudaEventDestroy(c->ev_aux_go[i]);
+        cudaEventDestroy(c->ev_aux_huge[i]);
         cudaEventDestroy(c->ev_aux_done[i]);
         cudaStreamDestroy(c->aux[i]);
     }
@@ -397,7 +398,8 @@ struct ItemPlan {
 struct WavePlan {
     int first_item = 0, last_item = 0;  // [first, last)
     std::vector<JpegDesc> descs;
-    std::vector<uint32_t> spec_list, restart_list, restart_first, block_first, color_first;
+    std::vector<uint32_t> tile_first, spec_list, write_first, dc_first, restart_list, restart_first, block_first, color_first;
+    uint32_t max_tables = 2;  // most distinct Huffman tables of one image (DC and AC counted apart)
     std::vector<std::array<uint32_t, 4>> groups;  // (first block, block count, first colour tile, tile count) per L2 group
     // descs [fused_first, descs.size()) take the fused 4:2:0 path: prefix sums of their chroma blocks and tiles, and
     // their own launch groups (first chroma block, count, first tile, count)
@@ -416,11 +418,11 @@ struct WavePlan {
     std::vector<AlphaJob> alpha[4];
     std::vector<uint32_t> alpha_first[4];
     // scratch layout (bytes from the wave scratch base)
-    size_t us_bytes = 0, coef_blocks = 0, plane_bytes = 0, decoded_bytes = 0, mid_bytes = 0, nseg = 0;
-    size_t off_us = 0, off_uslen = 0, off_segstart = 0, off_segfound = 0, off_coef = 0, off_planes = 0, off_decoded = 0, off_mid = 0, total = 0;
+    size_t us_bytes = 0, coef_blocks = 0, plane_bytes = 0, decoded_bytes = 0, mid_bytes = 0, nseg = 0, cells = 0;
+    size_t off_us = 0, off_uslen = 0, off_segstart = 0, off_segfound = 0, off_tiles = 0, off_cells = 0, off_diff = 0, off_info = 0, off_coef = 0, off_planes = 0, off_decoded = 0, off_mid = 0, total = 0;
     // meta offsets
     size_t m_descs = 0, m_spec = 0, m_restart_list = 0, m_passes[4] = {0, 0, 0, 0}, m_copies = 0, m_torgbs = 0, m_alphas[4] = {0, 0, 0, 0};
-    OwnerMapOff m_restart, m_blocks, m_color, m_fchroma, m_ftile, m_pass[4], m_copy, m_torgb, m_alpha[4];
+    OwnerMapOff m_tiles, m_write, m_dc, m_restart, m_blocks, m_color, m_fchroma, m_ftile, m_pass[4], m_copy, m_torgb, m_alpha[4];
 };
 
 struct StageEvent { int stage; cudaEvent_t a, b; };
@@ -454,7 +456,6 @@ struct dg_batch {
     size_t off_meta = 0, off_status = 0, off_blob = 0, off_rawin = 0, off_out = 0, persist_bytes = 0;
     size_t blob_bytes = 0, rawin_bytes = 0, out_bytes = 0, pin_bytes = 0;
     size_t arena_bytes = 0;  // out_bytes plus the pre-conversion images of DG_ITEM_TO_RGB8 items (never downloaded)
-    uint32_t n_huff = 0;
     size_t m_huff = 0, m_qt = 0, m_tables = 0, meta_total = 0;  // meta_total: meta.bytes plus the filter tables behind it
     std::vector<const uint8_t*> raw_src;  // caller memory of raw items (used inside dg_batch_create only)
     uint64_t h2d = 0, d2h = 0;
@@ -851,6 +852,9 @@ static size_t resize_mid_bound(const dg_plan& p, uint32_t C) {
     return align_up(a, 256) + 2 * align_up(b, 256);
 }
 
+// cells of a restart-free stream, at most (the unstuffed stream is no longer than the raw one)
+static uint32_t stream_cells(uint32_t raw_len) { return (uint32_t)(((uint64_t)raw_len * 8 + kCellBits - 1) / kCellBits); }
+
 // Runs fn(0..n-1) on the process-wide host pool; small counts stay on the calling thread.
 template <typename F> static void parallel_items(int n, F&& fn) {
     HostPool::get().run((size_t)std::max(n, 0), [&fn](size_t i) { fn((int)i); }, 64);
@@ -1016,7 +1020,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
     // ---- pass 3: per-wave scratch layout and JPEG descriptors ------------------------------------------------------
     size_t scratch_max = 0, blob_off = 0;
     for (WavePlan& wv : b->waves) {
-        size_t us = 0, planes = 0, decoded = 0, mids = 0, blocks = 0, segs = 0;
+        size_t us = 0, planes = 0, decoded = 0, mids = 0, blocks = 0, segs = 0, cells = 0;
         // Descriptors are built in item order, then arranged so that the images of the general path come first and those
         // of the fused 4:2:0 path after them: each class then owns one contiguous range of the coefficient array.
         std::vector<JpegDesc> built;
@@ -1042,7 +1046,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             if (it.status) continue;  // nothing has been laid out for this image yet
             d.raw_off = blob_off; d.raw_len = (uint32_t)h.scan_len;
             blob_off += align_up(h.scan_len, 16) + 16;
-            d.us_off = us; us += align_up(h.scan_len + 32, 16);
+            d.us_off = us; us += align_up(h.scan_len + kStreamPad, 16);
             d.nblocks = it.nblocks;
             d.width = h.width; d.height = h.height; d.mcux = h.mcux; d.mcuy = h.mcuy;
             d.ncomp = h.ncomp; d.hs = h.hs; d.vs = h.vs; d.bpm = h.ncomp == 1 ? 1 : h.hs * h.vs + 2;
@@ -1074,6 +1078,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         wv.ftile_first.push_back(0);
         wv.fgroups.push_back({0, 0, 0, 0});
         wv.restart_first.push_back(0);
+        wv.tile_first.push_back(0);
         wv.fused_first = (uint32_t)built.size();
         for (size_t k : order) {
             JpegDesc d = built[k];
@@ -1081,12 +1086,29 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             const bool fused = ctx->fused_path && fused_decode(d.ncomp, d.hs, d.vs, d.width);
             d.block_off = blocks;
             it.coef_off_blocks = blocks;
-            blocks += it.nblocks;
+            const uint32_t padded_blocks = (uint32_t)align_up(it.nblocks, 8);  // images start at multiples of eight blocks (32 bytes of info[])
+            blocks += padded_blocks;
             // the fused path keeps no luma plane
             for (uint32_t c = fused ? 1 : 0; c < d.ncomp; ++c) { d.plane_off[c] = planes; planes += align_up((size_t)d.plane_pitch[c] * d.plane_rows[c], 256); }
             it.wave_local = (int)wv.descs.size();
-            if (d.restart) { wv.restart_list.push_back((uint32_t)wv.descs.size()); restart_total += d.nseg; wv.restart_first.push_back(restart_total); }
-            else wv.spec_list.push_back((uint32_t)wv.descs.size());
+            if (d.restart) {
+                wv.restart_list.push_back((uint32_t)wv.descs.size());
+                restart_total += (d.nseg + kSegsPerCta - 1) / kSegsPerCta;
+                wv.restart_first.push_back(restart_total);
+            } else {
+                wv.spec_list.push_back((uint32_t)wv.descs.size());
+                d.cell_off = cells;
+                cells += stream_cells(d.raw_len) + 1;
+            }
+            wv.tile_first.push_back(wv.tile_first.back() + std::max(1u, (d.raw_len + kUnstuffTile - 1) / kUnstuffTile));
+            {
+                uint32_t distinct = 2;
+                for (int c = 1; c < 3; ++c) {
+                    distinct += d.dc_tab[c] != d.dc_tab[0] && (c == 1 || d.dc_tab[c] != d.dc_tab[1]);
+                    distinct += d.ac_tab[c] != d.ac_tab[0] && (c == 1 || d.ac_tab[c] != d.ac_tab[1]);
+                }
+                wv.max_tables = std::max(wv.max_tables, distinct);
+            }
             if (fused && wv.fused_first == (uint32_t)built.size()) wv.fused_first = (uint32_t)wv.descs.size();
             wv.descs.push_back(d);
             // images whose planes fit the L2 budget together share one IDCT launch and one colour launch
@@ -1097,11 +1119,11 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
                 wv.color_first.push_back(color_total);
                 const size_t pbytes = (size_t)it.nblocks * 64;
                 if (wv.groups.back()[1] && group_bytes + pbytes > ctx->l2_group_bytes) {
-                    wv.groups.push_back({(uint32_t)(blocks - it.nblocks), 0, color_total - ntiles, 0});
+                    wv.groups.push_back({(uint32_t)(blocks - padded_blocks), 0, color_total - ntiles, 0});
                     group_bytes = 0;
                 }
                 group_bytes += pbytes;
-                wv.groups.back()[1] += it.nblocks;
+                wv.groups.back()[1] += padded_blocks;
                 wv.groups.back()[3] += ntiles;
             } else {
                 const uint32_t nchroma = 2 * d.mcux * d.mcuy, ntiles = fused_tiles(d.width, d.mcuy);
@@ -1122,12 +1144,23 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         // longest streams first: one CTA decodes one image, and the launch ends with its slowest CTA
         std::stable_sort(wv.spec_list.begin(), wv.spec_list.end(),
                          [&](uint32_t a, uint32_t c) { return wv.descs[a].raw_len > wv.descs[c].raw_len; });
+        wv.write_first.assign(1, 0);
+        wv.dc_first.assign(1, 0);
+        for (uint32_t k : wv.spec_list) {
+            const JpegDesc& d = wv.descs[k];
+            wv.write_first.push_back(wv.write_first.back() + (stream_cells(d.raw_len) + kCellsPerCta - 1) / kCellsPerCta);
+            wv.dc_first.push_back(wv.dc_first.back() + (d.mcux * d.mcuy + kDcMcus - 1) / kDcMcus);
+        }
         wv.n_huge = 0;
         // (at most kSpecHugeMax of them: one such CTA fills an SM, so they trade throughput for a shorter critical path)
         while (wv.n_huge < wv.spec_list.size() && wv.n_huge < kSpecHugeMax && wv.descs[wv.spec_list[wv.n_huge]].raw_len > kSpecHugeBytes) ++wv.n_huge;
-        wv.us_bytes = us; wv.coef_blocks = blocks; wv.plane_bytes = planes; wv.decoded_bytes = decoded; wv.mid_bytes = mids; wv.nseg = segs;
+        wv.us_bytes = us; wv.coef_blocks = blocks; wv.plane_bytes = planes; wv.decoded_bytes = decoded; wv.mid_bytes = mids; wv.nseg = segs; wv.cells = cells;
         size_t o = 0;
-        wv.off_coef = o; o += align_up(blocks * 128, 256);  // first: the zero prefix of a scratch block is tracked from offset 0
+        wv.off_coef = o; o += align_up(blocks * 128, 256);
+        wv.off_diff = o; o += align_up(blocks * 4, 256);
+        wv.off_info = o; o += align_up(blocks * 4, 256);
+        wv.off_cells = o; o += align_up(cells * 8, 256);
+        wv.off_tiles = o; o += align_up((size_t)wv.tile_first.back() * 4, 256);
         wv.off_us = o; o += align_up(us, 256);
         wv.off_uslen = o; o += align_up(wv.descs.size() * 4, 256);
         wv.off_segfound = o; o += align_up(wv.descs.size() * 4, 256);
@@ -1142,12 +1175,12 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
     // ---- device and pinned blocks (addresses are needed by the resize descriptors) ------------------------------------
     // persistent layout: [status | blob | raw inputs | outputs | meta]; meta size is known only after planning the
     // resize passes, so it gets a bound: descriptors + tables are small next to the pixel buffers.
-    int rc = ctx->dev.acquire(std::max<size_t>(scratch_max, 256), &b->blk_scratch, true);
+    int rc = ctx->dev.acquire(std::max<size_t>(scratch_max, 256), &b->blk_scratch);
     if (rc) return abandon(b, rc);
     b->d_scratch = (uint8_t*)ctx->dev.blocks[b->blk_scratch].ptr;
     b->d_scratch2 = b->d_scratch;
     if (b->waves.size() > 1) {
-        rc = ctx->dev.acquire(std::max<size_t>(scratch_max, 256), &b->blk_scratch2, true);
+        rc = ctx->dev.acquire(std::max<size_t>(scratch_max, 256), &b->blk_scratch2);
         if (rc) return abandon(b, rc);
         b->d_scratch2 = (uint8_t*)ctx->dev.blocks[b->blk_scratch2].ptr;
     }
@@ -1267,12 +1300,14 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         Meta& m = b->meta;
         m.bytes.clear();
         b->m_huff = m.put(pl.huff_pool, 16);
-        b->n_huff = (uint32_t)pl.huff_pool.size();
         b->m_qt = m.put(pl.qt_pool, 16);
         for (WavePlan& wv : b->waves) {
             wv.m_descs = m.put(wv.descs, 16);
             wv.m_spec = m.put(wv.spec_list);
             wv.m_restart_list = m.put(wv.restart_list);
+            wv.m_tiles = put_owner_map(m, wv.tile_first);
+            wv.m_write = put_owner_map(m, wv.write_first);
+            wv.m_dc = put_owner_map(m, wv.dc_first);
             wv.m_restart = put_owner_map(m, wv.restart_first);
             wv.m_blocks = put_owner_map(m, wv.block_first);
             wv.m_color = put_owner_map(m, wv.color_first);
@@ -1407,12 +1442,7 @@ extern "C" int dg_batch_run(dg_batch* b) {
     if (!b->uploaded) return fail(DG_E_INVALID, "dg_batch_run before dg_batch_upload");
     dg_ctx* ctx = b->ctx;
     std::lock_guard<std::mutex> lock(ctx->mu);
-    const int rc = batch_run_locked(b);
-    if (rc != DG_OK) {  // a pass that stopped half-way leaves no guarantee about the scratch contents
-        if (b->blk_scratch >= 0) ctx->dev.blocks[b->blk_scratch].zero_prefix = 0;
-        if (b->blk_scratch2 >= 0) ctx->dev.blocks[b->blk_scratch2].zero_prefix = 0;
-    }
-    return rc;
+    return batch_run_locked(b);
 }
 
 static int batch_run_locked(dg_batch* b) {
@@ -1451,10 +1481,6 @@ static int batch_run_locked(dg_batch* b) {
     for (size_t wi = 0; wi < b->waves.size(); ++wi) {
         WavePlan& wv = b->waves[wi];
         uint8_t* sc = (wi & 1) ? b->d_scratch2 : b->d_scratch;
-        // everything of the scratch block beyond this wave's coefficient region is about to be overwritten
-        const size_t coef_bytes = wv.coef_blocks * 128;
-        Block& scratch_blk = ctx->dev.blocks[(wi & 1) ? b->blk_scratch2 : b->blk_scratch];
-        if (scratch_blk.zero_prefix > coef_bytes) scratch_blk.zero_prefix = coef_bytes;
         // the scratch block belongs to the lane, so in one-stream mode an odd wave must wait for nothing extra:
         // stream order already serialises the waves
         s = (two_lanes && (wi & 1)) ? ctx->stream2 : ctx->stream;
@@ -1464,22 +1490,29 @@ static int batch_run_locked(dg_batch* b) {
             w.descs = (const JpegDesc*)(meta + wv.m_descs);
             w.n = (uint32_t)wv.descs.size();
             w.raw = b->d_persist + b->off_blob;
+            w.us_tiles = resolve(b, wv.m_tiles);
+            w.tile_info = (uint32_t*)(sc + wv.off_tiles);
             w.us = sc + wv.off_us;
             w.us_len = (uint32_t*)(sc + wv.off_uslen);
             w.seg_start = (uint32_t*)(sc + wv.off_segstart);
             w.seg_found = (uint32_t*)(sc + wv.off_segfound);
+            w.cells = (uint2*)(sc + wv.off_cells);
             w.coef = (int16_t*)(sc + wv.off_coef);
+            w.diff = (uint32_t*)(sc + wv.off_diff);
+            w.info = (uint32_t*)(sc + wv.off_info);
             w.planes = sc + wv.off_planes;
             w.out = transform ? sc + wv.off_decoded : b->d_persist + b->off_out;
             w.status = (uint32_t*)(b->d_persist + b->off_status);
             w.spec_stats = (unsigned long long*)(b->d_persist + b->off_status + align_up((size_t)b->n * 4, 8));
             w.huff = (const HuffTable*)(meta + b->m_huff);
-            w.n_huff = b->n_huff;
+            w.max_tables = wv.max_tables;
             w.qt32 = (const uint32_t*)(meta + b->m_qt);
             w.spec_list = (const uint32_t*)(meta + wv.m_spec);
             w.n_spec = (uint32_t)wv.spec_list.size();
             w.restart_list = (const uint32_t*)(meta + wv.m_restart_list);
-            w.restart_segs = resolve(b, wv.m_restart);
+            w.restart_ctas = resolve(b, wv.m_restart);
+            w.write_ctas = resolve(b, wv.m_write);
+            w.dc_ctas = resolve(b, wv.m_dc);
             w.blocks = resolve(b, wv.m_blocks);
             w.color_tiles = resolve(b, wv.m_color);
             w.fused_first = wv.fused_first;
@@ -1487,24 +1520,14 @@ static int batch_run_locked(dg_batch* b) {
             w.fused_tiles = resolve(b, wv.m_ftile);
             CU(mark(DG_STAGE_UNSTUFF, true));
             launch_unstuff(w, s);
-            ++b->launches;
+            b->launches += 2;
             CU(mark(DG_STAGE_UNSTUFF, false));
-            // The entropy decoders write only non-zero coefficients, so the coefficient region must be zero beforehand.
-            // The IDCT zeroes the rows it found non-zero after reading them, which keeps the region zero from one wave
-            // to the next on the same scratch block; only a part that was not a coefficient region before is cleared.
-            const bool rezero = !(b->flags & DG_BATCH_KEEP_COEFFICIENTS);
-            CU(mark(DG_STAGE_COEF_CLEAR, true));
-            if (coef_bytes > scratch_blk.zero_prefix)
-                CU(cudaMemsetAsync((uint8_t*)w.coef + scratch_blk.zero_prefix, 0, coef_bytes - scratch_blk.zero_prefix, s));
-            scratch_blk.zero_prefix = rezero ? coef_bytes : 0;
-            CU(mark(DG_STAGE_COEF_CLEAR, false));
-            // The two entropy kernels work on disjoint images and are both latency bound: outside timing mode they run
-            // side by side, the restart-interval one on the lane's auxiliary stream.
-            // The auxiliary stream of the lane takes what can run beside the speculative decoder: the restart-interval
-            // decoder, and the speculative decoder's widest CTAs for the few longest images of the wave.
+            // The auxiliary stream of the lane takes what can run beside the speculative decoder: its widest CTAs for the few
+            // longest images of the wave (also in a timing batch: the two launches are one stage), and outside timing mode
+            // the restart-interval decoder, which works on other images.
             const uint32_t n_huge = wv.n_huge;
-            const bool aux_restart = !timing && w.restart_segs.total && w.n_spec;
-            const bool aux_huge = n_huge && w.n_spec > n_huge;  // also in a timing batch: the two launches are one stage
+            const bool aux_restart = !timing && w.restart_ctas.total && w.n_spec;
+            const bool aux_huge = n_huge && w.n_spec > n_huge;
             const int lane = (int)(wi & 1);
             cudaStream_t aux = ctx->aux[lane];
             if (w.n_spec) {  // the longest images first: they decide when the stage ends
@@ -1513,28 +1536,41 @@ static int batch_run_locked(dg_batch* b) {
                     CU(cudaEventRecord(ctx->ev_aux_go[lane], s));
                     CU(cudaStreamWaitEvent(aux, ctx->ev_aux_go[lane], 0));
                 }
-                launch_huff_spec(w, n_huge, s, aux_huge ? aux : s);
-                b->launches += (n_huge ? 1 : 0) + (w.n_spec > n_huge ? 1 : 0);
-                if (timing && aux_huge) {  // the stage ends when both launches have
-                    CU(cudaEventRecord(ctx->ev_aux_done[lane], aux));
-                    CU(cudaStreamWaitEvent(s, ctx->ev_aux_done[lane], 0));
+                auto cells_of = [&](uint32_t k) { return stream_cells(wv.descs[wv.spec_list[k]].raw_len); };
+                if (n_huge) {
+                    launch_huff_sync(w, 0, n_huge, cells_of(0), true, aux_huge ? aux : s);
+                    ++b->launches;
+                    if (aux_huge) CU(cudaEventRecord(ctx->ev_aux_huge[lane], aux));
                 }
+                if (w.n_spec > n_huge) {
+                    launch_huff_sync(w, n_huge, w.n_spec - n_huge, cells_of(n_huge), false, s);
+                    ++b->launches;
+                }
+                if (aux_restart) {
+                    launch_huff_restart(w, aux);
+                    ++b->launches;
+                    CU(cudaEventRecord(ctx->ev_aux_done[lane], aux));
+                }
+                if (aux_huge) CU(cudaStreamWaitEvent(s, ctx->ev_aux_huge[lane], 0));
+                launch_huff_write(w, s);
+                b->launches += 2;
                 CU(mark(DG_STAGE_HUFF_SPEC, false));
+                if (aux_restart) CU(cudaStreamWaitEvent(s, ctx->ev_aux_done[lane], 0));
             }
-            if (w.restart_segs.total) {
+            if (w.restart_ctas.total && !aux_restart) {
                 CU(mark(DG_STAGE_HUFF_RESTART, true));
-                launch_huff_restart(w, aux_restart ? aux : s);
+                launch_huff_restart(w, s);
                 ++b->launches;
                 CU(mark(DG_STAGE_HUFF_RESTART, false));
             }
-            if (!timing && (aux_restart || aux_huge)) {
-                CU(cudaEventRecord(ctx->ev_aux_done[lane], aux));
-                CU(cudaStreamWaitEvent(s, ctx->ev_aux_done[lane], 0));
+            if (b->flags & DG_BATCH_KEEP_COEFFICIENTS) {
+                launch_whole_blocks(w, (uint32_t)wv.coef_blocks, s);
+                ++b->launches;
             }
             for (const auto& g : wv.groups) {
                 if (!g[1]) continue;
                 CU(mark(DG_STAGE_IDCT, true));
-                launch_idct(w, g[0], g[1], rezero, s);
+                launch_idct(w, g[0], g[1], s);
                 ++b->launches;
                 CU(mark(DG_STAGE_IDCT, false));
                 CU(mark(DG_STAGE_COLOR, true));
@@ -1545,11 +1581,11 @@ static int batch_run_locked(dg_batch* b) {
             for (const auto& g : wv.fgroups) {  // 4:2:0: chroma planes first, then luma IDCT + upsampling + colour in one kernel
                 if (!g[1]) continue;
                 CU(mark(DG_STAGE_IDCT, true));
-                launch_idct_chroma(w, g[0], g[1], rezero, s);
+                launch_idct_chroma(w, g[0], g[1], s);
                 ++b->launches;
                 CU(mark(DG_STAGE_IDCT, false));
                 CU(mark(DG_STAGE_COLOR, true));
-                launch_luma_color(w, g[2], g[3], rezero, s);
+                launch_luma_color(w, g[2], g[3], s);
                 ++b->launches;
                 CU(mark(DG_STAGE_COLOR, false));
             }

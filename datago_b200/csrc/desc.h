@@ -42,8 +42,9 @@ enum : uint32_t {
 // One baseline JPEG of a wave.
 struct JpegDesc {
     uint64_t raw_off;       // entropy-coded segment inside the raw blob (16-byte aligned)
-    uint64_t us_off;        // this image's slice of the unstuffed buffer (16-byte aligned, capacity raw_len + 32)
-    uint64_t block_off;     // first 8x8 block in the coefficient buffer
+    uint64_t us_off;        // this image's slice of the unstuffed buffer (16-byte aligned, capacity raw_len + kStreamPad)
+    uint64_t block_off;     // first 8x8 block in the coefficient buffer (a multiple of 8)
+    uint64_t cell_off;      // first entry in the cell array
     uint64_t plane_off[3];  // byte offset of each component plane (MCU-padded, pitch = plane_pitch)
     uint64_t out_off;       // byte offset of the decoded image (tightly packed HWC) in the decode target buffer
     uint32_t raw_len;

@@ -14,25 +14,48 @@ struct OwnerMap {
     uint32_t n, shift, total;
 };
 
+// ---- entropy decoding: work splits (see kernels_huff.cu) ------------------------------------------------------------------
+constexpr uint32_t kUnstuffTile = 4096;  // bytes of an entropy-coded segment per CTA of the unstuffing kernels
+constexpr uint32_t kCellBits = 1024;     // bits of an unstuffed stream per thread of the value decoder
+constexpr uint32_t kCellsPerCta = 128, kSegsPerCta = 128;
+constexpr uint32_t kDcMcus = 8192;       // MCUs per CTA of the DC prediction
+constexpr uint32_t kStreamPad = 512;     // bytes behind an image's unstuffed stream that the bit readers may touch
+
+// How much of a block is non-zero decides how much of the inverse DCT is needed: everything, the top-left 4x4 or 2x2
+// coefficients, the DC term alone.
+enum : int { kClsFull = 0, kCls4x4 = 1, kCls2x2 = 2, kClsDc = 3 };
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline uint32_t class_rows(int cls) { return cls == kClsFull ? 8u : cls == kCls4x4 ? 4u : cls == kCls2x2 ? 2u : 0u; }  // rows of coef[] it covers
+
 struct JpegWave {
     const JpegDesc* descs;   // device, n images
     uint32_t n;
     const uint8_t* raw;      // compressed blob
-    uint8_t* us;             // unstuffed streams
+    OwnerMap us_tiles;       // kUnstuffTile-byte pieces of the images' entropy-coded segments; owner = image
+    uint32_t* tile_info;     // [us_tiles.total] what each tile keeps
+    uint8_t* us;             // unstuffed streams, as big-endian 32-bit words
     uint32_t* us_len;        // [n] bytes of each unstuffed stream
     uint32_t* seg_start;     // restart-segment starts (bytes into the image's unstuffed stream)
     uint32_t* seg_found;     // [n] segments actually present
-    int16_t* coef;           // [blocks][64], scan order, natural order inside a block
+    uint2* cells;            // per cell of a restart-free stream: bit position of its first block, index of that block
+    int16_t* coef;           // [blocks][64], scan order, natural order inside a block; AC terms, rows the class covers
+    uint32_t* diff;          // [blocks] restart-free images: DC difference | class << 16
+    uint32_t* info;          // [blocks] DC coefficient (low half) | class << 16
     uint8_t* planes;         // component planes after the IDCT
     uint8_t* out;            // decoded images
     uint32_t* status;        // [items of the batch]
-    unsigned long long* spec_stats;  // [0] chunks, [1] synchronisation rounds, [2] subsequence decodes (all passes)
+    unsigned long long* spec_stats;  // [0] stretches of 256 cells, [1] synchronisation rounds, [2] decodes of a thread's run
     const HuffTable* huff;   // table pool
-    uint32_t n_huff;         // tables in the pool
+    uint32_t max_tables;     // most distinct tables (DC and AC counted apart) one image of the wave uses
     const uint32_t* qt32;    // quantisation pool, 32 words per table: word i holds q[2i] in byte 0 and q[2i+1] in byte 3
-    // speculative (no restart marker) images and restart-interval images of this wave
+    // restart-free images of this wave, longest first; CTAs of the value decoder and of the DC prediction: owner = index
+    // into spec_list
     const uint32_t* spec_list; uint32_t n_spec;
-    OwnerMap restart_segs;   // owner = index into restart_list
+    OwnerMap write_ctas, dc_ctas;
+    // restart-interval images: kSegsPerCta segments per CTA, owner = index into restart_list
+    OwnerMap restart_ctas;
     const uint32_t* restart_list;
     OwnerMap blocks;         // owner = image
     OwnerMap color_tiles;    // owner = image
@@ -46,19 +69,19 @@ struct JpegWave {
 
 void launch_unstuff(const JpegWave& w, cudaStream_t s);
 void launch_huff_restart(const JpegWave& w, cudaStream_t s);
-// the first n_huge images of spec_list (longest first) have more than kSpecHugeBytes of entropy-coded data: they get the
-// widest CTAs, on huge_stream, beside the others on s
+// images [first, first + count) of spec_list.  The leading ones with more than kSpecHugeBytes of entropy-coded data get the
+// widest CTAs, beside the others on another stream.
 constexpr uint32_t kSpecHugeBytes = 1024 * 2048 / 8, kSpecHugeMax = 64;
-void launch_huff_spec(const JpegWave& w, uint32_t n_huge, cudaStream_t s, cudaStream_t huge_stream);
+void launch_huff_sync(const JpegWave& w, uint32_t first, uint32_t count, uint32_t longest_cells, bool widest, cudaStream_t s);
+void launch_huff_write(const JpegWave& w, cudaStream_t s);  // all restart-free images, once launch_huff_sync has covered them
+void launch_whole_blocks(const JpegWave& w, uint32_t nblocks, cudaStream_t s);
 // blocks [first, first + count) of the wave / colour tiles [first, first + count): callers may launch them in groups of
 // images (the planes written by the IDCT are then still in L2 when the colour kernel reads them) or once per wave
-// rezero: the kernel writes zeros back over every coefficient row it found non-zero, which leaves the coefficient
-// buffer all-zero again for the next wave that uses it (the entropy decoders only write non-zero coefficients)
-void launch_idct(const JpegWave& w, uint32_t first, uint32_t count, bool rezero, cudaStream_t s);
+void launch_idct(const JpegWave& w, uint32_t first, uint32_t count, cudaStream_t s);
 void launch_color(const JpegWave& w, uint32_t first_tile, uint32_t count, cudaStream_t s);
 // the fused path: chroma blocks [first, first + count) of fused_chroma, tiles [first, first + count) of fused_tiles
-void launch_idct_chroma(const JpegWave& w, uint32_t first, uint32_t count, bool rezero, cudaStream_t s);
-void launch_luma_color(const JpegWave& w, uint32_t first_tile, uint32_t count, bool rezero, cudaStream_t s);
+void launch_idct_chroma(const JpegWave& w, uint32_t first, uint32_t count, cudaStream_t s);
+void launch_luma_color(const JpegWave& w, uint32_t first_tile, uint32_t count, cudaStream_t s);
 // whether an image takes the fused path
 inline bool fused_decode(uint32_t ncomp, uint32_t hs, uint32_t vs, uint32_t width) { return ncomp == 3 && hs == 2 && vs == 2 && width >= 5; }
 
