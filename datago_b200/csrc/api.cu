@@ -399,7 +399,16 @@ struct WavePlan {
     int first_item = 0, last_item = 0;  // [first, last)
     std::vector<JpegDesc> descs;
     std::vector<uint32_t> tile_first, spec_list, write_first, dc_first, restart_list, restart_first, block_first, color_first;
-    uint32_t max_tables = 2;  // most distinct Huffman tables of one image (DC and AC counted apart)
+    std::vector<std::array<uint32_t, 2>> pairs;  // (DC, AC) pairs of Huffman tables in use
+    std::map<std::array<uint32_t, 2>, uint32_t> pair_ids;
+    uint32_t max_pairs = 1;                      // most distinct ones in one image
+    uint32_t pair_id(uint32_t dc, uint32_t ac) {
+        const std::array<uint32_t, 2> key{dc, ac};
+        if (!pairs.empty() && pairs.back() == key) return (uint32_t)pairs.size() - 1;
+        const auto it = pair_ids.emplace(key, (uint32_t)pairs.size());
+        if (it.second) pairs.push_back(key);
+        return it.first->second;
+    }
     std::vector<std::array<uint32_t, 4>> groups;  // (first block, block count, first colour tile, tile count) per L2 group
     // descs [fused_first, descs.size()) take the fused 4:2:0 path: prefix sums of their chroma blocks and tiles, and
     // their own launch groups (first chroma block, count, first tile, count)
@@ -419,9 +428,9 @@ struct WavePlan {
     std::vector<uint32_t> alpha_first[4];
     // scratch layout (bytes from the wave scratch base)
     size_t us_bytes = 0, coef_blocks = 0, plane_bytes = 0, decoded_bytes = 0, mid_bytes = 0, nseg = 0, cells = 0;
-    size_t off_us = 0, off_uslen = 0, off_segstart = 0, off_segfound = 0, off_tiles = 0, off_cells = 0, off_diff = 0, off_info = 0, off_coef = 0, off_planes = 0, off_decoded = 0, off_mid = 0, total = 0;
+    size_t off_us = 0, off_uslen = 0, off_segstart = 0, off_segfound = 0, off_tiles = 0, off_codes = 0, off_cells = 0, off_diff = 0, off_info = 0, off_coef = 0, off_planes = 0, off_decoded = 0, off_mid = 0, total = 0;
     // meta offsets
-    size_t m_descs = 0, m_spec = 0, m_restart_list = 0, m_passes[4] = {0, 0, 0, 0}, m_copies = 0, m_torgbs = 0, m_alphas[4] = {0, 0, 0, 0};
+    size_t m_descs = 0, m_pairs = 0, m_spec = 0, m_restart_list = 0, m_passes[4] = {0, 0, 0, 0}, m_copies = 0, m_torgbs = 0, m_alphas[4] = {0, 0, 0, 0};
     OwnerMapOff m_tiles, m_write, m_dc, m_restart, m_blocks, m_color, m_fchroma, m_ftile, m_pass[4], m_copy, m_torgb, m_alpha[4];
 };
 
@@ -1039,9 +1048,11 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
                     if (h.qt[h.comp_tq[cc]][k] > 255) it.status = DG_E_UNSUPPORTED;
                 if (it.status) break;
                 d.qt[c] = pl.qt_id(h.qt[h.comp_tq[cc]]);
-                int rc = pl.huff_id(h.dc[h.comp_td[cc]], &d.dc_tab[c]);
-                if (!rc) rc = pl.huff_id(h.ac[h.comp_ta[cc]], &d.ac_tab[c]);
+                uint32_t dc_id = 0, ac_id = 0;
+                int rc = pl.huff_id(h.dc[h.comp_td[cc]], &dc_id);
+                if (!rc) rc = pl.huff_id(h.ac[h.comp_ta[cc]], &ac_id);
                 if (rc) it.status = rc;
+                else d.pair[c] = wv.pair_id(dc_id, ac_id);
             }
             if (it.status) continue;  // nothing has been laid out for this image yet
             d.raw_off = blob_off; d.raw_len = (uint32_t)h.scan_len;
@@ -1102,12 +1113,8 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             }
             wv.tile_first.push_back(wv.tile_first.back() + std::max(1u, (d.raw_len + kUnstuffTile - 1) / kUnstuffTile));
             {
-                uint32_t distinct = 2;
-                for (int c = 1; c < 3; ++c) {
-                    distinct += d.dc_tab[c] != d.dc_tab[0] && (c == 1 || d.dc_tab[c] != d.dc_tab[1]);
-                    distinct += d.ac_tab[c] != d.ac_tab[0] && (c == 1 || d.ac_tab[c] != d.ac_tab[1]);
-                }
-                wv.max_tables = std::max(wv.max_tables, distinct);
+                const uint32_t distinct = 1 + (d.pair[1] != d.pair[0]) + (d.pair[2] != d.pair[0] && d.pair[2] != d.pair[1]);
+                wv.max_pairs = std::max(wv.max_pairs, distinct);
             }
             if (fused && wv.fused_first == (uint32_t)built.size()) wv.fused_first = (uint32_t)wv.descs.size();
             wv.descs.push_back(d);
@@ -1159,6 +1166,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         wv.off_coef = o; o += align_up(blocks * 128, 256);
         wv.off_diff = o; o += align_up(blocks * 4, 256);
         wv.off_info = o; o += align_up(blocks * 4, 256);
+        wv.off_codes = o; o += align_up(wv.pairs.size() * kCodeTablesBytes, 256);
         wv.off_cells = o; o += align_up(cells * 8, 256);
         wv.off_tiles = o; o += align_up((size_t)wv.tile_first.back() * 4, 256);
         wv.off_us = o; o += align_up(us, 256);
@@ -1303,6 +1311,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         b->m_qt = m.put(pl.qt_pool, 16);
         for (WavePlan& wv : b->waves) {
             wv.m_descs = m.put(wv.descs, 16);
+            wv.m_pairs = m.put(wv.pairs);
             wv.m_spec = m.put(wv.spec_list);
             wv.m_restart_list = m.put(wv.restart_list);
             wv.m_tiles = put_owner_map(m, wv.tile_first);
@@ -1505,7 +1514,10 @@ static int batch_run_locked(dg_batch* b) {
             w.status = (uint32_t*)(b->d_persist + b->off_status);
             w.spec_stats = (unsigned long long*)(b->d_persist + b->off_status + align_up((size_t)b->n * 4, 8));
             w.huff = (const HuffTable*)(meta + b->m_huff);
-            w.max_tables = wv.max_tables;
+            w.table_pairs = (const uint2*)(meta + wv.m_pairs);
+            w.n_pairs = (uint32_t)wv.pairs.size();
+            w.codes = sc + wv.off_codes;
+            w.max_pairs = wv.max_pairs;
             w.qt32 = (const uint32_t*)(meta + b->m_qt);
             w.spec_list = (const uint32_t*)(meta + wv.m_spec);
             w.n_spec = (uint32_t)wv.spec_list.size();

@@ -52,7 +52,7 @@ struct JpegDesc {
     uint32_t mcux, mcuy;
     uint32_t ncomp, hs, vs, bpm;  // components, luma sampling factors, blocks per MCU
     uint32_t qt[3];               // quantisation table pool index per component
-    uint32_t dc_tab[3], ac_tab[3];  // Huffman table pool index per component
+    uint32_t pair[3];             // index of the component's (DC, AC) pair of Huffman tables in the wave's list
     uint32_t restart;             // MCUs per restart interval, 0 = none
     uint32_t nseg;                // restart segments expected (1 when restart == 0)
     uint32_t seg_off;             // first entry of this image in the segment-start array

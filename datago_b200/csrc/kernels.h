@@ -19,6 +19,7 @@ constexpr uint32_t kUnstuffTile = 4096;  // bytes of an entropy-coded segment pe
 constexpr uint32_t kCellBits = 1024;     // bits of an unstuffed stream per thread of the value decoder
 constexpr uint32_t kCellsPerCta = 128, kSegsPerCta = 128;
 constexpr uint32_t kDcMcus = 8192;       // MCUs per CTA of the DC prediction
+constexpr uint32_t kCodeTablesBytes = 20544;  // look-up tables of one (DC, AC) pair of Huffman tables
 constexpr uint32_t kStreamPad = 512;     // bytes behind an image's unstuffed stream that the bit readers may touch
 
 // How much of a block is non-zero decides how much of the inverse DCT is needed: everything, the top-left 4x4 or 2x2
@@ -48,7 +49,9 @@ struct JpegWave {
     uint32_t* status;        // [items of the batch]
     unsigned long long* spec_stats;  // [0] stretches of 256 cells, [1] synchronisation rounds, [2] decodes of a thread's run
     const HuffTable* huff;   // table pool
-    uint32_t max_tables;     // most distinct tables (DC and AC counted apart) one image of the wave uses
+    const uint2* table_pairs; uint32_t n_pairs;  // the (DC, AC) pairs of tables the images of the wave use
+    uint8_t* codes;          // [n_pairs] look-up tables made from them, kCodeTablesBytes each
+    uint32_t max_pairs;      // most distinct pairs one image of the wave uses
     const uint32_t* qt32;    // quantisation pool, 32 words per table: word i holds q[2i] in byte 0 and q[2i+1] in byte 3
     // restart-free images of this wave, longest first; CTAs of the value decoder and of the DC prediction: owner = index
     // into spec_list

@@ -10,6 +10,7 @@
 // to be zeroed before or after.
 #include <cooperative_groups.h>
 
+#include <cstddef>
 #include <cstdint>
 #include <mutex>
 
@@ -50,6 +51,119 @@ __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_gr
 template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+}  // namespace
+
+// ---- code tables ---------------------------------------------------------------------------------------------------------
+namespace {
+
+constexpr uint32_t kNoState = 0xFFFFFFFFu;  // "the stream has ended" in place of a bit position
+
+// Codes longer than the fast part of the host's table.  No search: the code length follows from six comparisons against
+// the table's left-aligned limits, the symbol from the canonical offset of that length.  v: the next 16 bits.
+// Returns length | symbol << 8; 16 with bit 31 set when no code matches.
+__device__ __forceinline__ uint32_t long_code(const HuffTable* t, uint32_t v) {
+    const uint4 la = __ldg(reinterpret_cast<const uint4*>(&t->limit[0])), lb = __ldg(reinterpret_cast<const uint4*>(&t->limit[4]));
+    const uint32_t len = 10u + (v >= la.x) + (v >= la.y) + (v >= la.z) + (v >= la.w) + (v >= lb.x) + (v >= lb.y);
+    if (v >= lb.z) return 16u | 0x80000000u;
+    return len | ((uint32_t)__ldg(t->vals + (int32_t)(v >> (16u - len)) + __ldg(t->valoff + len)) << 8);
+}
+// any code at the head of the 16 bits v, same result
+__device__ __forceinline__ uint32_t code_at(const HuffTable* t, uint32_t v) {
+    const uint32_t e = __ldg(t->lut + (v >> (16 - kLutBits)));
+    if (!e) return long_code(t, v);
+    return ((e >> 6) & 31u) | ((e >> 11) & 255u) << 8;
+}
+__device__ __forceinline__ uint32_t advance_of(uint32_t symbol, bool is_ac) {  // slots a symbol advances
+    const uint32_t s = symbol & 15u, r = symbol >> 4;
+    return !is_ac ? 1u : (s || r == 15u) ? r + 1u : 64u;  // coefficient after a run, ZRL, or end of block
+}
+
+// Look-up tables of the two decoders for one (DC, AC) pair of Huffman tables, made on the device (k_unstuff_count), because
+// they are several times the size of what the host sends.  Codes longer than the index: entry 0, and far[] takes over --
+// canonical codes grow with their length, so all of them lie above far_base, and the 16-bit windows from there on are few
+// (190 to 640 for the tables most files carry).  Windows behind the end of far[] go to the host's table.
+constexpr int kSyncBits = 10, kValueBits = 9;
+// Synchronising decoder: as many whole symbols as the index shows.  bits 0-4 / 5-11: bits consumed and slots advanced by the
+// first symbol alone, 12-16 / 17-23: by all of them, 24-29: slots before the last one (the last counts only if that many do
+// not end the block).  64 slots or more end the block.  A DC symbol is followed by AC symbols of the same component.
+struct SyncTab {
+    uint32_t lut[1 << kSyncBits];
+    uint32_t far[384];
+    uint32_t far_base, huff, is_ac, pad;
+};
+// Value decoder: bits 0-4 code and extra bits together, 5-9 code length, 10-13 extra bits s, 24 no such code, 25-31 slots
+// advanced (the coefficient sits in the last of them; 64: end of block).
+struct ValueTab {
+    uint32_t lut[1 << kValueBits];
+    uint32_t far[640];
+    uint32_t far_base, huff, is_ac, pad;
+};
+struct CodeTables { SyncTab sync[2]; ValueTab value[2]; };  // [0] DC, [1] AC
+static_assert(sizeof(SyncTab) % 16 == 0 && sizeof(ValueTab) % 16 == 0 && sizeof(CodeTables) == kCodeTablesBytes, "tables are copied in 16-byte pieces");
+
+__device__ __forceinline__ uint32_t sync_entry(uint32_t u, uint32_t a) { return u | a << 5 | u << 12 | a << 17; }
+__device__ __forceinline__ uint32_t value_entry(uint32_t code, bool is_ac) {
+    const uint32_t len = code & 31u, s = (code >> 8) & 15u;
+    return (len + s) | len << 5 | s << 10 | (code >> 31) << 24 | advance_of((code >> 8) & 255u, is_ac) << 25;
+}
+
+__device__ void build_tables(CodeTables& out, const HuffTable* pool, uint32_t dc_id, uint32_t ac_id, int tid, int nthreads) {
+    const HuffTable* const ac = pool + ac_id;
+    for (int side = 0; side < 2; ++side) {
+        const HuffTable* const t = pool + (side ? ac_id : dc_id);
+        SyncTab& st = out.sync[side];
+        ValueTab& vt = out.value[side];
+        for (uint32_t i = tid; i < (1u << kSyncBits); i += nthreads) {
+            const uint32_t window = i << (16 - kSyncBits);
+            uint32_t c = code_at(t, window), e = 0;
+            if ((c & 31u) <= (uint32_t)kSyncBits) {
+                uint32_t u = (c & 31u) + ((c >> 8) & 15u), a = advance_of((c >> 8) & 255u, side != 0), pre = 0;
+                const uint32_t first = u | a << 5;
+                while (u < (uint32_t)kSyncBits && a < 64u) {
+                    c = code_at(ac, (window << u) & 0xFFFFu);
+                    const uint32_t len = c & 31u;
+                    if (u + len > (uint32_t)kSyncBits) break;
+                    pre = a;
+                    u += len + ((c >> 8) & 15u);
+                    a += advance_of((c >> 8) & 255u, true);
+                }
+                e = first | u << 12 | a << 17 | pre << 24;
+            }
+            st.lut[i] = e;
+        }
+        // the windows from the first one that no code of at most kLutBits / kSyncBits bits covers
+        uint32_t covered = 0;
+        for (int k = 0; k < (1 << kLutBits); k += 32) covered += __popc(__ballot_sync(0xFFFFFFFFu, __ldg(t->lut + k + (tid & 31)) != 0u));
+        const uint32_t vbase = covered << (16 - kLutBits), sbase = __ldg(t->limit + 0);
+        static_assert(kValueBits == kLutBits && kSyncBits == 10, "limit[0] covers ten bits");
+        for (uint32_t i = tid; i < sizeof(st.far) / 4; i += nthreads) {
+            const uint32_t c = code_at(t, min(sbase + i, 0xFFFFu));
+            st.far[i] = sync_entry((c & 31u) + ((c >> 8) & 15u), advance_of((c >> 8) & 255u, side != 0));
+        }
+        for (uint32_t i = tid; i < (1u << kValueBits); i += nthreads) {
+            const uint32_t c = code_at(t, i << (16 - kValueBits));
+            vt.lut[i] = (c & 31u) <= (uint32_t)kValueBits ? value_entry(c, side != 0) : 0u;
+        }
+        for (uint32_t i = tid; i < sizeof(vt.far) / 4; i += nthreads) vt.far[i] = value_entry(code_at(t, min(vbase + i, 0xFFFFu)), side != 0);
+        if (tid == 0) {
+            st.far_base = sbase; vt.far_base = vbase;
+            st.huff = vt.huff = side ? ac_id : dc_id;
+            st.is_ac = vt.is_ac = side;
+        }
+    }
+}
+
+// the entry of a code longer than the index; `tab`: shared-memory address of the table
+template <class Tab>
+__device__ __forceinline__ uint32_t far_entry(uint32_t tab, uint32_t top, const HuffTable* pool) {
+    const uint32_t v = top >> 16, i = v - lds32(tab + (uint32_t)offsetof(Tab, far_base));
+    if (i < (uint32_t)(sizeof(Tab::far) / 4)) return lds32(tab + (uint32_t)offsetof(Tab, far) + i * 4);
+    const uint32_t c = long_code(pool + lds32(tab + (uint32_t)offsetof(Tab, huff)), v);
+    const bool is_ac = lds32(tab + (uint32_t)offsetof(Tab, is_ac)) != 0;
+    if (sizeof(Tab) == sizeof(SyncTab)) return sync_entry((c & 31u) + ((c >> 8) & 15u), advance_of((c >> 8) & 255u, is_ac));
+    return value_entry(c, is_ac);
+}
 
 }  // namespace
 
@@ -100,7 +214,15 @@ __device__ __forceinline__ Unit classify(const uint8_t* in, uint32_t i0, uint32_
 
 }  // namespace
 
+// (The CTAs behind the last tile make the code tables of the wave: work of the same length, for which a launch of its own
+// would be too much.)
 __global__ void __launch_bounds__(kUnstuffThreads) k_unstuff_count(JpegWave w) {
+    if (blockIdx.x >= w.us_tiles.total) {
+        const uint32_t k = blockIdx.x - w.us_tiles.total;
+        const uint2 ids = w.table_pairs[k];
+        build_tables(reinterpret_cast<CodeTables*>(w.codes)[k], w.huff, ids.x, ids.y, threadIdx.x, kUnstuffThreads);
+        return;
+    }
     const uint32_t o = owner_of(w.us_tiles, blockIdx.x);
     const JpegDesc& d = w.descs[o];
     const uint32_t tile = blockIdx.x - __ldg(w.us_tiles.first + o);
@@ -209,7 +331,7 @@ __global__ void __launch_bounds__(kUnstuffThreads) k_unstuff_write(JpegWave w) {
 
 void launch_unstuff(const JpegWave& w, cudaStream_t s) {
     if (!w.n) return;
-    k_unstuff_count<<<w.us_tiles.total, kUnstuffThreads, 0, s>>>(w);
+    k_unstuff_count<<<w.us_tiles.total + w.n_pairs, kUnstuffThreads, 0, s>>>(w);
     k_unstuff_write<<<w.us_tiles.total, kUnstuffThreads, 0, s>>>(w);
 }
 
@@ -237,75 +359,116 @@ void launch_unstuff(const JpegWave& w, cudaStream_t s) {
 // ---------------------------------------------------------------------------------------------------------------
 namespace {
 
-constexpr int kPairBits = 10;       // table index of the symbol-pair look-up
-constexpr uint32_t kNoState = 0xFFFFFFFFu;  // "the stream has ended" in place of a bit position
-
-// What follows the fast table: codes longer than it (see HuffTable::limit).
-struct LongCodes {
-    uint32_t limit[8];
-    int32_t valoff[20];  // 17 used
-    uint8_t vals[256];
-};
-__device__ __forceinline__ void load_long_codes(LongCodes& t, const HuffTable* src, int tid, int nthreads) {
-    for (int i = tid; i < 8; i += nthreads) t.limit[i] = __ldg(src->limit + i);
-    for (int i = tid; i < 17; i += nthreads) t.valoff[i] = __ldg(src->valoff + i);
-    for (int i = tid; i < 64; i += nthreads) reinterpret_cast<uint32_t*>(t.vals)[i] = __ldg(reinterpret_cast<const uint32_t*>(src->vals) + i);
+// Where a decoder stands inside the MCU: the tables of the current block as shared-memory addresses, and the entry of the
+// block after it.  One 16-byte read per block instead of arithmetic on indices.
+struct McuBlock { uint32_t dc, ac, next, index; };
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
 }
-// No search: the code length follows from six comparisons against the table's left-aligned limits, the symbol from the
-// canonical offset of that length.  Returns length | symbol << 8; 16 with bit 31 set when no code matches.
-__device__ __forceinline__ uint32_t long_code(const LongCodes* t, uint32_t top) {
-    const uint32_t v = top >> 16;
-    const uint4 la = *reinterpret_cast<const uint4*>(&t->limit[0]);
-    const uint4 lb = *reinterpret_cast<const uint4*>(&t->limit[4]);
-    const uint32_t len = 10u + (v >= la.x) + (v >= la.y) + (v >= la.z) + (v >= la.w) + (v >= lb.x) + (v >= lb.y);
-    if (v >= lb.z) return 16u | 0x80000000u;
-    return len | ((uint32_t)t->vals[(int32_t)(v >> (16u - len)) + t->valoff[len]] << 8);
-}
-
-// The image's tables, each distinct one once: slot of the DC / AC table of component i.
-struct TableSlots {
-    uint32_t id[6], n;
-    uint8_t dc[3], ac[3];
-};
-__device__ __forceinline__ TableSlots table_slots(const JpegDesc& d) {
-    TableSlots t;
-    t.n = 0;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        int same = -1;
-#pragma unroll
-        for (int j = 0; j < k; ++j) if (same < 0 && d.dc_tab[j] == d.dc_tab[k]) same = j;
-        if (same >= 0) t.dc[k] = t.dc[same]; else { t.dc[k] = (uint8_t)t.n; t.id[t.n++] = d.dc_tab[k]; }
+// The image's tables into shared memory, each distinct pair once.  Tab: SyncTab or ValueTab; which: offset of its [2] array
+// inside CodeTables.
+template <class Tab>
+__device__ __forceinline__ void load_tables(const JpegWave& w, const JpegDesc& d, McuBlock* mcu, unsigned char* tab0, uint32_t which, int tid, int nthreads) {
+    const uint32_t p0 = d.pair[0], p1 = d.pair[1], p2 = d.pair[2];
+    const uint32_t slot1 = p1 == p0 ? 0u : 1u, slot2 = p2 == p0 ? 0u : p2 == p1 ? slot1 : slot1 + 1u;
+    constexpr uint32_t kPieces = 2 * sizeof(Tab) / 16;
+    const uint32_t nslot = max(slot1, slot2) + 1u;
+    for (uint32_t k = 0; k < nslot; ++k) {
+        const uint32_t id = k == 0 ? p0 : k == slot1 ? p1 : p2;
+        const uint4* src = reinterpret_cast<const uint4*>(w.codes + (size_t)id * kCodeTablesBytes + which);
+        const uint32_t dst = smem_addr(tab0) + k * 2 * (uint32_t)sizeof(Tab);
+        for (uint32_t i = tid; i < kPieces; i += nthreads) copy16(dst + i * 16, src + i);
     }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        int same = -1;
-#pragma unroll
-        for (int j = 0; j < k; ++j) if (same < 0 && d.ac_tab[j] == d.ac_tab[k]) same = j;
-        if (same >= 0) t.ac[k] = t.ac[same]; else { t.ac[k] = (uint8_t)t.n; t.id[t.n++] = d.ac_tab[k] | 0x80000000u; }
+    if ((uint32_t)tid < d.bpm) {
+        const uint32_t luma = d.hs * d.vs, slot = (uint32_t)tid < luma ? 0u : (uint32_t)tid == luma ? slot1 : slot2;
+        const uint32_t at = smem_addr(tab0) + slot * 2 * (uint32_t)sizeof(Tab);
+        mcu[tid] = McuBlock{at, at + (uint32_t)sizeof(Tab), smem_addr(&mcu[(uint32_t)tid + 1 == d.bpm ? 0 : tid + 1]), (uint32_t)tid};
     }
-    return t;
 }
 
-// One table of the synchronising decoder: index = next kPairBits bits.  Low half: the first symbol alone, high half: the
-// first two when the second one's code lies inside the index (else the first again).  A half is bits consumed | slots
-// advanced << 5; 64 slots or more end the block.  0: the first code is longer than the fast table.
-struct SyncTab {
-    uint32_t pair[1 << kPairBits];
-    LongCodes lc;
+// Window of two stream words (w0 holds the current bit): when bit position `was` -> `now` crosses a word boundary (one at
+// most: symbols have 31 bits at most), w0 takes w1 and w1 the word behind the one at address `word`.  Predicated by hand:
+// some lane of a warp crosses in nearly every step.
+__device__ __forceinline__ void advance_window(uint32_t& w0, uint32_t& w1, uint32_t was, uint32_t now, uint32_t word) {
+    asm volatile("{\n .reg .pred q;\n setp.ge.u32 q, %2, 32;\n @q mov.u32 %0, %1;\n @q ld.shared.u32 %1, [%3+4];\n}" : "+r"(w0), "+r"(w1) : "r"(was ^ now), "r"(word));
+}
+// Streams in shared memory: at(p) is the address of the word that holds bit p; the word behind it follows.
+template <class Address>
+struct SharedSource {
+    Address at;
+    __device__ __forceinline__ void start(uint32_t& w0, uint32_t& w1, uint32_t p) const { w0 = lds32(at(p)); w1 = lds32(at(p) + 4); }
+    __device__ __forceinline__ void advance(uint32_t& w0, uint32_t& w1, uint32_t was, uint32_t now) const { advance_window(w0, w1, was, now, at(now)); }
 };
-static_assert(sizeof(SyncTab) % 16 == 0, "tables follow one another in shared memory");
+template <class Address> __device__ __forceinline__ SharedSource<Address> shared_source(Address at) { return SharedSource<Address>{at}; }
+// ... and in global memory
+struct GlobalSource {
+    const uint32_t* words;
+    uint32_t n;
+    __device__ __forceinline__ uint32_t word(uint32_t i) const { return i < n ? __ldg(words + i) : 0u; }
+    __device__ __forceinline__ void start(uint32_t& w0, uint32_t& w1, uint32_t p) const { w0 = word(p >> 5); w1 = word((p >> 5) + 1); }
+    __device__ __forceinline__ void advance(uint32_t& w0, uint32_t& w1, uint32_t was, uint32_t now) const {
+        if ((was ^ now) >= 32u) { w0 = w1; w1 = word((now >> 5) + 1); }
+    }
+};
 
-constexpr int kRingPitch = 144;  // bytes per thread: eight 16-byte pieces of its stream, padded against bank conflicts
+// A lane of a synchronising decoder.
+struct SyncLane {
+    uint32_t p, z, nb;   // bit position, slot inside the block, blocks ended since nb was last set to zero
+    uint32_t w0, w1, tab;
+    uint4 mb;            // McuBlock of the current block
+    template <class Source>
+    __device__ __forceinline__ void start(const Source& src, uint32_t mcu0, uint32_t bit, uint32_t slot, uint32_t c) {
+        p = bit; z = slot; nb = 0;
+        src.start(w0, w1, p);
+        mb = lds128(mcu0 + c * (uint32_t)sizeof(McuBlock));
+        tab = z ? mb.y : mb.x;
+    }
+    // Lanes with `live` decode to the first block start at p >= stop.  Called by whole warps: the loop has one exit, taken by
+    // all lanes together, and no other jump out of it -- with returns from inside, the lanes of a warp never met again
+    // after their first different turn and went on alone.  turn(): called every four steps (124 bits at most) by all.
+    template <class Source, class Turn>
+    __device__ __forceinline__ void run_to(bool live, uint32_t stop, const Source& src, const HuffTable* pool, Turn&& turn) {
+        while (__any_sync(0xFFFFFFFFu, live)) {
+            turn(live);
+#pragma unroll
+            for (int step = 0; step < 4; ++step) {
+                if (live) {
+                    const uint32_t top = __funnelshift_l(w1, w0, p);
+                    uint32_t e = lds32(tab + ((top >> (32 - kSyncBits)) << 2));
+                    if (e == 0) e = far_entry<SyncTab>(tab, top, pool);
+                    const uint32_t h = z + (e >> 24) >= 64u ? e : e >> 12;
+                    const uint32_t was = p;
+                    p += h & 31u;
+                    z += (h >> 5) & 127u;
+                    tab = mb.y;
+                    src.advance(w0, w1, was, p);
+                    if (z >= 64u) {
+                        z = 0;
+                        ++nb;
+                        mb = lds128(mb.z);
+                        tab = mb.x;
+                        live = p < stop;
+                    }
+                }
+            }
+        }
+    }
+};
+
+constexpr int kRingPitch = 144;  // bytes per thread: eight 16-byte pieces of its stream, and the first of them once more behind them
 
 template <int T>
 struct SyncMisc {
     uint2 exit[T];         // state each thread hands to its right neighbour
-    uint32_t tabs[8];      // per block of the MCU: byte offset of its DC table | AC table << 16
+    McuBlock mcu[6];
     uint32_t warp[32];
     uint32_t flag[3];      // cluster: some thread still differs (by round, modulo 3)
     uint32_t total;        // blocks found by this CTA's threads
+    uint32_t pad[3];
 };
+static_assert(sizeof(SyncMisc<256>) % 16 == 0, "tables follow in shared memory");
 
 }  // namespace
 
@@ -320,39 +483,10 @@ __global__ void __launch_bounds__(T) k_huff_sync(JpegWave w, uint32_t first) {
     if (CLUSTER) { rank = cg::this_cluster().block_rank(); nrank = cg::this_cluster().num_blocks(); }
     const uint32_t img = w.spec_list[first + blockIdx.x / nrank];
     const JpegDesc& d = w.descs[img];
-
-    const uint32_t bpm = d.bpm;
-    {
-        const TableSlots ts = table_slots(d);
-        for (uint32_t t = 0; t < ts.n; ++t) {
-            const HuffTable* src = w.huff + (ts.id[t] & 0x7FFFFFFFu);
-            const bool is_ac = (ts.id[t] >> 31) != 0;
-            SyncTab& dst = *reinterpret_cast<SyncTab*>(tab0 + t * sizeof(SyncTab));
-            for (uint32_t i = tid; i < (1u << kPairBits); i += T) {
-                const uint32_t e1 = __ldg(src->lut + (i >> (kPairBits - kLutBits)));
-                uint32_t one = 0, two = 0;
-                if (e1) {
-                    const uint32_t u1 = e1 & 63u, s1 = (e1 >> 11) & 15u, r1 = (e1 >> 15) & 15u;
-                    const uint32_t a1 = !is_ac ? 1u : (s1 || r1 == 15u) ? r1 + 1u : 64u;
-                    one = two = u1 | a1 << 5;
-                    if (is_ac && a1 < 64u && u1 < (uint32_t)kPairBits) {
-                        const uint32_t e2 = __ldg(src->lut + (((i << u1) & ((1u << kPairBits) - 1u)) >> (kPairBits - kLutBits)));
-                        if (e2 && ((e2 >> 6) & 31u) <= kPairBits - u1) {
-                            const uint32_t s2 = (e2 >> 11) & 15u, r2 = (e2 >> 15) & 15u;
-                            two = (u1 + (e2 & 63u)) | (a1 + ((s2 || r2 == 15u) ? r2 + 1u : 64u)) << 5;
-                        }
-                    }
-                }
-                dst.pair[i] = one | two << 16;
-            }
-            load_long_codes(dst.lc, src, tid, T);
-        }
-        if ((uint32_t)tid < bpm) {
-            const uint32_t luma = d.hs * d.vs, comp = (uint32_t)tid < luma ? 0u : tid - luma + 1u;
-            sh.tabs[tid] = (uint32_t)(ts.dc[comp] * sizeof(SyncTab)) | (uint32_t)(ts.ac[comp] * sizeof(SyncTab)) << 16;
-        }
-        if (tid < 3) sh.flag[tid] = 0;
-    }
+    load_tables<SyncTab>(w, d, sh.mcu, tab0, (uint32_t)offsetof(CodeTables, sync), tid, T);
+    copy_commit();
+    if (tid < 3) sh.flag[tid] = 0;
+    copy_wait<0>();
     __syncthreads();
 
     const uint32_t total = w.us_len[img] * 8u;
@@ -363,89 +497,65 @@ __global__ void __launch_bounds__(T) k_huff_sync(JpegWave w, uint32_t first) {
     const uint32_t run = (ncell + nthread - 1) / nthread;
     const uint32_t kbeg = min(gt * run, ncell), kend = min(kbeg + run, ncell);
     const bool active = kbeg < kend;
-    const uint32_t ring = smem_addr(ring0) + tid * kRingPitch, tabs = smem_addr(sh.tabs), tbase = smem_addr(tab0);
+    const uint32_t ring = smem_addr(ring0) + tid * kRingPitch, mcu0 = smem_addr(&sh.mcu[0]);
 
     uint32_t found = 0;                       // blocks that start in this thread's cells
     uint2 entry = make_uint2(0, 0), exit = make_uint2(kNoState, 0);
 
-    // Decodes from (p, z, c) to the first block start at or behind the end of the run.  Redoing (REDO), it stops as soon as
-    // it meets the state recorded for one of the cells.
-    auto decode = [&](uint32_t p, uint32_t z, uint32_t c, bool redo) {
-        uint32_t k = kbeg, bound = kbeg * kCellBits;  // the next cell to enter, and where it begins
-        uint32_t nb = 0, old_n = 0;                   // blocks since the open cell's entry; what the cell counted before
-        bool open = false;
-        uint2 at = make_uint2(0, 0);                  // entry state of the open cell
-        // a block start at p >= bound, or behind the end of the stream: true when the run is done
-        auto enter = [&]() -> bool {
-            if (p > total) {  // the block that ended here is not whole
-                if (p != kNoState && nb) --nb;
-                p = kNoState; c = 0;
-            }
-            while (p >= bound) {
-                uint32_t had_n = 0;
-                bool met = false;
-                if (k < kend && redo) {
-                    const uint2 had = recs[k];
-                    had_n = had.y & 0x0FFFFFFFu;
-                    met = open && had.x == p && (had.y >> 28) == c;
-                }
-                if (open) { recs[k - 1] = make_uint2(at.x, at.y << 28 | nb); found += nb - old_n; }
-                if (met) return true;
-                if (k == kend) { exit = make_uint2(p, c); return true; }
-                if (k == kbeg) entry = make_uint2(p, c);
-                nb = 0; old_n = had_n; at = make_uint2(p, c); open = true;
-                ++k; bound += kCellBits;
-            }
-            return false;
+    // Decodes the thread's cells from (p, z, c).  Redoing, it stops as soon as it meets the state recorded for one of them.
+    auto decode = [&](bool live, uint32_t p, uint32_t z, uint32_t c, bool redo) {
+        // the stream in pieces of 16 bytes through this thread's ring
+        const bool ended = p == kNoState;
+        uint32_t wr = ended ? 0u : p >> 7;
+        SyncLane L;
+        auto fetch = [&]() {
+            copy16(ring + (wr & 7u) * 16, us + (size_t)wr * 16);
+            if ((wr & 7u) == 0) copy16(ring + 128, us + (size_t)wr * 16);
+            ++wr;
         };
-        if (z == 0 && enter()) return;
-        // the stream in pieces of 16 bytes through this thread's ring; a window of three words in registers
-        uint32_t wr = p >> 7, wi = p >> 5;
-#pragma unroll
-        for (int i = 0; i < 8; ++i, ++wr) copy16(ring + (wr & 7u) * 16, us + (size_t)wr * 16);
+        if (live && !ended) {
+            for (int i = 0; i < 8; ++i) fetch();
+        }
         copy_commit();
         copy_wait<0>();
-        auto word = [&](uint32_t i) { return lds32(ring + ((i << 2) & 124u)); };
-        uint32_t w0 = word(wi), w1 = word(wi + 1), w2 = word(wi + 2);
-        uint32_t tb = lds32(tabs + c * 4);
-        uint32_t tab = tbase + (z ? tb >> 16 : tb & 0xFFFFu);
-        for (;;) {
-            // A step consumes at most 31 bits, so four of them cross at most one piece and one copy per turn keeps the
-            // ring full.  The copies of the last four turns may still be under way: they are at least three pieces ahead.
-            if (wr < (p >> 7) + 8) { copy16(ring + (wr & 7u) * 16, us + (size_t)wr * 16); ++wr; }
+        const auto source = shared_source([&](uint32_t bit) { return ring + ((bit >> 3) & 124u); });
+        // A step consumes at most 31 bits, so four of them cross at most one piece and one copy per turn keeps the ring
+        // full.  The copies of the last four turns may still be under way: they are at least three pieces ahead.
+        auto turn = [&](bool on) {
+            if (on && wr < (L.p >> 7) + 8) fetch();
             copy_commit();
             copy_wait<4>();
-#pragma unroll
-            for (int step = 0; step < 4; ++step) {
-                const uint32_t top = __funnelshift_l(w1, w0, p);
-                uint32_t e = lds32(tab + ((top >> (32 - kPairBits)) << 2));
-                if (e == 0) {
-                    const uint32_t lc = long_code(reinterpret_cast<const LongCodes*>(__cvta_shared_to_generic(tab + (sizeof(uint32_t) << kPairBits))), top);
-                    const uint32_t s = (lc >> 8) & 15u, r = (lc >> 12) & 15u;
-                    const uint32_t adv = z == 0 ? 1u : (s || r == 15u) ? r + 1u : 64u;
-                    e = ((lc & 31u) + s) | adv << 5;
-                    e |= e << 16;
+        };
+        L.start(source, mcu0, p, z, c);
+        if (!redo) L.run_to(live && z != 0, kbeg * kCellBits, source, w.huff, turn);  // the guess: to the first block start it meets
+        for (uint32_t i = 0; i < run; ++i) {
+            const uint32_t k = kbeg + i, bound = (k + 1) * kCellBits;
+            bool on = live && k < kend;
+            if (L.p > total) { L.p = kNoState; L.mb.w = 0; }  // the block that ended here is not whole
+            const uint2 at = make_uint2(L.p, L.mb.w);
+            uint32_t old_n = 0;
+            if (on) {
+                if (redo) {
+                    const uint2 had = recs[k];
+                    old_n = had.y & 0x0FFFFFFFu;
+                    if (i && had.x == at.x && (had.y >> 28) == at.y) on = live = false;  // met
                 }
-                // the second symbol belongs to this block only if the first one does not end it
-                const uint32_t h = z + ((e >> 5) & 127u) >= 64u ? e & 0xFFFFu : e >> 16;
-                p += h & 31u;
-                z += h >> 5;
-                tab = tbase + (tb >> 16);
-                if (z >= 64u) {
-                    z = 0;
-                    c = c + 1 == bpm ? 0u : c + 1;
-                    tb = lds32(tabs + c * 4);
-                    tab = tbase + (tb & 0xFFFFu);
-                    ++nb;
-                    if (p >= bound || p > total) { if (enter()) return; }
-                }
-                const uint32_t nwi = p >> 5;
-                if (nwi != wi) { w0 = w1; w1 = w2; w2 = word(nwi + 2); wi = nwi; }
+                if (!redo && i == 0) entry = at;
+            }
+            if (!__any_sync(0xFFFFFFFFu, on)) break;
+            L.nb = 0;
+            L.run_to(on && L.p < bound, min(bound, total + 1), source, w.huff, turn);
+            if (on) {
+                if (L.p > total && L.p != kNoState) --L.nb;
+                recs[k] = make_uint2(at.x, at.y << 28 | L.nb);
+                found += L.nb - old_n;
             }
         }
+        if (L.p > total) { L.p = kNoState; L.mb.w = 0; }
+        if (live) exit = make_uint2(L.p, L.mb.w);
     };
 
-    if (active) decode(gt ? kbeg * kCellBits : 0u, gt ? 1u : 0u, 0u, false);
+    decode(active, gt ? kbeg * kCellBits : 0u, gt ? 1u : 0u, 0u, false);
     sh.exit[tid] = exit;
     uint32_t decodes = active ? 1u : 0u, rounds = 1;
     if (CLUSTER) cg::this_cluster().sync(); else __syncthreads();
@@ -463,9 +573,10 @@ __global__ void __launch_bounds__(T) k_huff_sync(JpegWave w, uint32_t first) {
             if (rank == 0 && tid == 0) sh.flag[(round + 2) % 3] = 0;
         }
         if (!any) break;
-        if (need) {
-            ++decodes;
-            decode(prev.x, 0, prev.y, true);
+        if (__any_sync(0xFFFFFFFFu, need)) {
+            decodes += need;
+            if (need) entry = prev;
+            decode(need, need ? prev.x : kNoState, 0, prev.y, true);
             sh.exit[tid] = exit;
         }
         ++rounds;
@@ -504,13 +615,6 @@ __global__ void __launch_bounds__(T) k_huff_sync(JpegWave w, uint32_t first) {
 // ---- blocks with their values --------------------------------------------------------------------------------------
 namespace {
 
-// One table of the value decoder: HuffTable::lut as it is, and the codes beyond it.
-struct ValueTab {
-    uint32_t lut[1 << kLutBits];
-    LongCodes lc;
-};
-static_assert(sizeof(ValueTab) % 16 == 0, "tables follow one another in shared memory");
-
 constexpr uint32_t kNotDc = 1u << 28, kNot2x2 = 1u << 29, kNot4x4 = 1u << 30;
 
 // Zig-zag position -> byte offset of the coefficient in a lane's block buffer (row r of the lane's block sits at
@@ -518,118 +622,114 @@ constexpr uint32_t kNotDc = 1u << 28, kNot2x2 = 1u << 29, kNot4x4 = 1u << 30;
 template <int T>
 __device__ __forceinline__ uint32_t place_of(uint32_t zz) {
     const uint32_t nat = kNatural[zz], r = nat >> 3, c = nat & 7u;
-    return r * (T * 16) + c * 2 | kNotDc | (r > 1 || c > 1 ? kNot2x2 : 0u) | (r > 3 || c > 3 ? kNot4x4 : 0u);
+    return r * (T * 16) + c * 2 | (zz ? kNotDc : 0u) | (r > 1 || c > 1 ? kNot2x2 : 0u) | (r > 3 || c > 3 ? kNot4x4 : 0u);
 }
 
 template <int T>
 struct ValueMisc {
     uint4 block[8 * T];    // the lanes' current blocks
     uint32_t place[64];
-    uint32_t tabs[8];      // per block of the MCU: byte offset of its DC table | AC table << 16
+    McuBlock mcu[6];
+    uint32_t pad[8];
 };
 
-// Shared memory of the value decoder: [ValueMisc | tables]; returns the base address of the tables.
+// Shared memory of the value decoder: [ValueMisc | ... | tables].  The caller waits for the copies and the barrier.
 template <int T>
 __device__ __forceinline__ void value_setup(const JpegWave& w, const JpegDesc& d, ValueMisc<T>& sh, unsigned char* tab0) {
     const int tid = threadIdx.x;
-    const TableSlots ts = table_slots(d);
-    for (uint32_t t = 0; t < ts.n; ++t) {
-        const HuffTable* src = w.huff + (ts.id[t] & 0x7FFFFFFFu);
-        ValueTab& dst = *reinterpret_cast<ValueTab*>(tab0 + t * sizeof(ValueTab));
-        for (int i = tid; i < (1 << kLutBits) / 4; i += T) reinterpret_cast<uint4*>(dst.lut)[i] = __ldg(reinterpret_cast<const uint4*>(src->lut) + i);
-        load_long_codes(dst.lc, src, tid, T);
-    }
-    if ((uint32_t)tid < d.bpm) {
-        const uint32_t luma = d.hs * d.vs, comp = (uint32_t)tid < luma ? 0u : tid - luma + 1u;
-        sh.tabs[tid] = (uint32_t)(ts.dc[comp] * sizeof(ValueTab)) | (uint32_t)(ts.ac[comp] * sizeof(ValueTab)) << 16;
-    }
+    load_tables<ValueTab>(w, d, sh.mcu, tab0, (uint32_t)offsetof(CodeTables, value), tid, T);
+    copy_commit();
     if (tid < 64) sh.place[tid] = place_of<T>(tid);
 #pragma unroll
     for (int r = 0; r < 8; ++r) sh.block[r * T + tid] = make_uint4(0, 0, 0, 0);
 }
 
-// Decodes blocks [blk, end) of an image from bit p on.  word(i): the i-th big-endian word of the image's stream.
-// limit: blocks that reach beyond this bit are not whole -- decoding stops there.  ABSOLUTE: the DC predictors start at
-// zero here (a restart segment) and info[] receives the DC terms themselves instead of their differences.
-// Returns the blocks decoded.  One code path for DC and AC symbols: the lanes of a warp are at unrelated places.
-template <int T, bool ABSOLUTE, class Word>
-__device__ __forceinline__ uint32_t decode_blocks(Word&& word, uint32_t p, uint32_t blk, const uint32_t end, const uint32_t limit, uint32_t c,
-                                                  const uint32_t bpm, const uint32_t luma, ValueMisc<T>& sh, const unsigned char* tab0, int16_t* __restrict__ coef,
+// Decodes blocks [blk, end) of an image from bit p on.  src: the image's stream, see SharedSource.
+// limit: blocks that reach beyond this bit are not whole -- decoding stops there; so it does at a block that starts at or
+// behind `stop`.  ABSOLUTE: the DC predictors start at zero here (a restart segment) and info[] receives the DC terms
+// themselves instead of their differences.  Returns the blocks decoded.  Called by whole warps.
+//
+// One code path for DC and AC symbols, the DC difference going to slot 0 of the block buffer like any coefficient: the lanes
+// of a warp are at unrelated places.  For the same reason a lane whose block is complete waits until kFlushLanes lanes
+// have one (or no lane has anything else to do): writing a block out takes more instructions than decoding a symbol,
+// and they cost the same whether two lanes execute them or ten.
+constexpr int kFlushLanes = 8;
+
+template <int T, bool ABSOLUTE, class Source>
+__device__ __forceinline__ uint32_t decode_blocks(const Source& src, uint32_t p, uint32_t blk, const uint32_t end, const uint32_t limit, const uint32_t stop,
+                                                  uint32_t c, const uint32_t luma, ValueMisc<T>& sh, const HuffTable* pool, int16_t* __restrict__ coef,
                                                   uint32_t* __restrict__ info, uint32_t& err) {
     const uint32_t first = blk;
-    if (blk >= end) return 0;
-    uint32_t wi = p >> 5;
-    uint32_t w0 = word(wi), w1 = word(wi + 1), w2 = word(wi + 2);
-    const uint32_t tabs = smem_addr(sh.tabs), tbase = smem_addr(tab0), place = smem_addr(sh.place), buf = smem_addr(&sh.block[threadIdx.x]);
-    uint32_t tb = lds32(tabs + c * 4);
-    uint32_t tab = tbase + (tb & 0xFFFFu);
-    uint32_t z = 0, seen = 0;
-    int32_t dc = 0, pred0 = 0, pred1 = 0, pred2 = 0;
+    bool live = blk < end;
+    uint32_t w0, w1;
+    src.start(w0, w1, p);
+    const uint32_t place = smem_addr(sh.place) - 4, buf = smem_addr(&sh.block[threadIdx.x]);
+    uint4 mb = lds128(smem_addr(&sh.mcu[0]) + c * sizeof(McuBlock));
+    uint32_t tab = mb.x, z = 0, seen = 0;
+    int32_t pred0 = 0, pred1 = 0, pred2 = 0;
     for (;;) {
-        const uint32_t top = __funnelshift_l(w1, w0, p);
-        uint32_t e = lds32(tab + ((top >> (32 - kLutBits)) << 2));
-        if (e == 0) {
-            const uint32_t lc = long_code(reinterpret_cast<const LongCodes*>(__cvta_shared_to_generic(tab + (sizeof(uint32_t) << kLutBits))), top);
-            if ((lc >> 31) && p < limit) err |= kStBadCode;
-            e = huff_pack(lc & 31u, (lc >> 8) & 255u);
-        }
-        const uint32_t used = e & 63u, len = (e >> 6) & 31u, s = (e >> 11) & 15u, r = (e >> 15) & 15u;
-        // the s extra bits (T.81 EXTEND): a leading 1 means the value itself, a leading 0 the complement of its magnitude
-        const uint32_t bits = top << len;
-        const int32_t neg = ~((int32_t)bits >> 31);
-        const int32_t v = (int32_t)(shr_clamp(bits ^ (uint32_t)neg, 32u - s) ^ (uint32_t)neg) - neg;
-        p += used;
-        if (z == 0) {
-            dc = v;
-            z = 1;
-            tab = tbase + (tb >> 16);
-        } else if (s) {
-            const uint32_t at = z + r;
-            if (at > 63u) { if (p <= limit) err |= kStCoefRange; }
-            else {
-                const uint32_t pl = lds32(place + at * 4);
+        const uint32_t alive = __ballot_sync(0xFFFFFFFFu, live);
+        if (!alive) break;  // one exit for the whole warp, see k_huff_sync
+        if (live && z < 64u) {
+            const uint32_t top = __funnelshift_l(w1, w0, p);
+            uint32_t e = lds32(tab + ((top >> (32 - kValueBits)) << 2));
+            if (e == 0) {
+                e = far_entry<ValueTab>(tab, top, pool);
+                if (((e >> 24) & 1u) && p < limit) err |= kStBadCode;
+            }
+            const uint32_t was = p, s = (e >> 10) & 15u;
+            // the s extra bits (T.81 EXTEND): a leading 1 means the value itself, a leading 0 the complement of its magnitude
+            const uint32_t bits = top << ((e >> 5) & 31u);
+            const int32_t neg = ~((int32_t)bits >> 31);
+            const int32_t v = (int32_t)(shr_clamp(bits ^ (uint32_t)neg, 32u - s) ^ (uint32_t)neg) - neg;
+            p += e & 31u;
+            z += e >> 25;
+            src.advance(w0, w1, was, p);
+            if (s && z <= 64u) {
+                const uint32_t pl = lds32(place + z * 4);
                 asm volatile("st.shared.u16 [%0], %1;" ::"r"(buf + (pl & 0xFFFFu)), "h"((uint16_t)v) : "memory");
                 seen |= pl;
             }
-            z = at + 1;
-        } else {
-            z = r == 15u ? z + 16u : 64u;
+            if (s && z > 64u && p <= limit) err |= kStCoefRange;
+            tab = mb.y;
         }
-        if (z >= 64u) {
-            if (p > limit) {  // (what the buffer holds is of no use, and neither is the rest of the span)
-                break;
-            }
-            if (ABSOLUTE) {
-                if (c < luma) dc = pred0 += dc;
-                else if (c == luma) dc = pred1 += dc;
-                else dc = pred2 += dc;
-            }
-            const uint32_t cls = seen & kNot4x4 ? (uint32_t)kClsFull : seen & kNot2x2 ? (uint32_t)kCls4x4 : seen & kNotDc ? (uint32_t)kCls2x2 : (uint32_t)kClsDc;
-            info[blk] = ((uint32_t)dc & 0xFFFFu) | cls << 16;
-            uint4* const rows = reinterpret_cast<uint4*>(coef) + (size_t)blk * 8;
-            const uint4 zero = make_uint4(0, 0, 0, 0);
-            uint4* const b = sh.block + threadIdx.x;
-            if (cls <= kCls2x2) {
-                rows[0] = b[0]; rows[1] = b[T];
-                b[0] = zero; b[T] = zero;
-                if (cls <= kCls4x4) {
-                    rows[2] = b[2 * T]; rows[3] = b[3 * T];
-                    b[2 * T] = zero; b[3 * T] = zero;
+        const uint32_t done = __ballot_sync(0xFFFFFFFFu, live && z >= 64u);
+        if (__popc(done) >= kFlushLanes || done == alive) {
+            if (live && z >= 64u) {
+                if (p > limit) live = false;  // (what the buffer holds is of no use, and neither is the rest of the span)
+                else {
+                    uint4* const b = sh.block + threadIdx.x;
+                    uint4* const rows = reinterpret_cast<uint4*>(coef) + (size_t)blk * 8;
+                    const uint4 zero = make_uint4(0, 0, 0, 0), q0 = b[0];
+                    int32_t dc = (int16_t)(q0.x & 0xFFFFu);
+                    if (ABSOLUTE) {
+                        if (mb.w < luma) dc = pred0 += dc;
+                        else if (mb.w == luma) dc = pred1 += dc;
+                        else dc = pred2 += dc;
+                    }
+                    const uint32_t cls = seen & kNot4x4 ? (uint32_t)kClsFull : seen & kNot2x2 ? (uint32_t)kCls4x4 : seen & kNotDc ? (uint32_t)kCls2x2 : (uint32_t)kClsDc;
+                    info[blk] = ((uint32_t)dc & 0xFFFFu) | cls << 16;
+                    b[0] = zero;
+                    if (cls <= kCls2x2) {
+                        rows[0] = q0; rows[1] = b[T];
+                        b[T] = zero;
+                    }
+                    if (cls <= kCls4x4) {
+                        rows[2] = b[2 * T]; rows[3] = b[3 * T];
+                        b[2 * T] = zero; b[3 * T] = zero;
+                    }
                     if (cls == kClsFull) {
 #pragma unroll
                         for (int q = 4; q < 8; ++q) { rows[q] = b[q * T]; b[q * T] = zero; }
                     }
+                    ++blk;
+                    live = blk < end && p < stop;
+                    z = 0; seen = 0;
+                    mb = lds128(mb.z);
+                    tab = mb.x;
                 }
             }
-            ++blk;
-            if (blk >= end) break;
-            z = 0; seen = 0;
-            c = c + 1 == bpm ? 0u : c + 1;
-            tb = lds32(tabs + c * 4);
-            tab = tbase + (tb & 0xFFFFu);
         }
-        const uint32_t nwi = p >> 5;
-        if (nwi != wi) { w0 = w1; w1 = w2; w2 = word(nwi + 2); wi = nwi; }  // a symbol has at most 31 bits: one boundary at a time
     }
     return blk - first;
 }
@@ -638,8 +738,9 @@ __device__ __forceinline__ uint32_t decode_blocks(Word&& word, uint32_t p, uint3
 
 // ---- restart-free images: one thread per cell -----------------------------------------------------------------------
 constexpr int kWriteThreads = (int)kCellsPerCta;
-// The CTA's cells are consecutive: their 16 KB of stream are staged in shared memory, a cell per row, rows padded against
-// bank conflicts; a block may run 1984 bits (64 symbols of 31 bits) into what follows.
+// The CTA's cells are consecutive: their 16 KB of stream are staged in shared memory, a cell per row and the first 16 bytes
+// of the next cell behind it (which spreads the rows over the banks and makes the word behind any word its neighbour); a
+// block may run 1984 bits (64 symbols of 31 bits) into what follows.
 constexpr int kStageRows = kWriteThreads + 3, kStagePitch = (int)kCellBits / 8 + 16;
 
 __global__ void __launch_bounds__(kWriteThreads) k_huff_write(JpegWave w) {
@@ -656,12 +757,12 @@ __global__ void __launch_bounds__(kWriteThreads) k_huff_write(JpegWave w) {
     if (cell0 >= ncell) return;
     const int tid = threadIdx.x;
     {
-        constexpr int kPieces = (int)kCellBits / 128;  // 16-byte pieces per row
+        constexpr int kPieces = (int)kCellBits / 128 + 1;  // 16-byte pieces per row
         const uint8_t* src = w.us + d.us_off + (size_t)cell0 * (kCellBits / 8);
         const uint32_t dst = smem_addr(stage);
         // no further than the stream and its padding reach
         const int rows = (int)min((uint32_t)kStageRows, ncell - cell0 + 2);
-        for (int i = tid; i < rows * kPieces; i += kWriteThreads) copy16(dst + (i / kPieces) * kStagePitch + (i % kPieces) * 16, src + (size_t)i * 16);
+        for (int i = tid; i < rows * kPieces; i += kWriteThreads) copy16(dst + i * 16, src + (i / kPieces) * (kCellBits / 8) + (i % kPieces) * 16);
         copy_commit();
     }
     value_setup<kWriteThreads>(w, d, sh, tab0);
@@ -675,14 +776,11 @@ __global__ void __launch_bounds__(kWriteThreads) k_huff_write(JpegWave w) {
     }
     copy_wait<0>();
     __syncthreads();
-    if (k >= ncell || a.y >= b1) return;
     uint32_t err = 0;
-    const uint32_t sbase = smem_addr(stage), word0 = cell0 * (kCellBits / 32);
-    auto word = [&](uint32_t i) {
-        const uint32_t l = min(i - word0, kStageRows * (kCellBits / 32) - 1u);  // (consistent cells never reach past the stage)
-        return lds32(sbase + (l + (l / (kCellBits / 32)) * 4) * 4);
-    };
-    decode_blocks<kWriteThreads, false>(word, a.x, a.y, b1, total, a.y % d.bpm, d.bpm, d.hs * d.vs, sh, tab0,
+    const uint32_t sbase = smem_addr(stage) - cell0 * kStagePitch;
+    const auto source = shared_source([&](uint32_t p) { return sbase + ((p >> 3) & ~3u) + (p / kCellBits) * 16; });
+    const uint32_t p0 = a.y < b1 ? a.x : cell0 * kCellBits;
+    decode_blocks<kWriteThreads, false>(source, p0, a.y, b1, total, (cell0 + kCellsPerCta) * kCellBits, a.y % d.bpm, d.hs * d.vs, sh, w.huff,
                                         w.coef + d.block_off * 64, w.diff + d.block_off, err);
     if (err) atomicOr(w.status + d.item, err);
 }
@@ -721,23 +819,21 @@ __global__ void __launch_bounds__(kRestartThreads) k_huff_restart(JpegWave w) {
     value_setup<kRestartThreads>(w, d, sh, tab0);
     copy_wait<0>();
     __syncthreads();
-    if (k >= have) return;
-    const uint32_t b0 = seg[k], b1 = k + 1 < have ? seg[k + 1] : us_len;
+    const bool mine = k < have;
+    const uint32_t b0 = mine ? seg[k] : lo, b1 = k + 1 < have ? seg[k + 1] : us_len;
     const uint32_t mcus = d.mcux * d.mcuy;
-    const uint32_t m0 = k * d.restart, m1 = min(m0 + d.restart, mcus);
+    const uint32_t m0 = mine ? k * d.restart : 0u, m1 = mine ? min(m0 + d.restart, mcus) : 0u;
     const uint32_t blk0 = m0 * d.bpm, blk1 = m1 * d.bpm;
     int16_t* coef = w.coef + d.block_off * 64;
     uint32_t* info = w.info + d.block_off;
     uint32_t err = 0, n;
     if (staged) {
         const uint32_t sbase = smem_addr(stage) - lo;
-        n = decode_blocks<kRestartThreads, true>([&](uint32_t i) { return lds32(sbase + i * 4); }, b0 * 8u, blk0, blk1, b1 * 8u, 0u, d.bpm,
-                                                 d.hs * d.vs, sh, tab0, coef, info, err);
+        n = decode_blocks<kRestartThreads, true>(shared_source([&](uint32_t p) { return sbase + ((p >> 3) & ~3u); }), b0 * 8u, blk0, blk1, b1 * 8u, b1 * 8u, 0u,
+                                                 d.hs * d.vs, sh, w.huff, coef, info, err);
     } else {
-        const uint32_t* words = reinterpret_cast<const uint32_t*>(us);
-        const uint32_t nwords = (us_len + 3) / 4 + 2;
-        n = decode_blocks<kRestartThreads, true>([&](uint32_t i) { return i < nwords ? __ldg(words + i) : 0u; }, b0 * 8u, blk0, blk1, b1 * 8u, 0u,
-                                                 d.bpm, d.hs * d.vs, sh, tab0, coef, info, err);
+        const GlobalSource source{reinterpret_cast<const uint32_t*>(us), (us_len + 3) / 4 + 2};
+        n = decode_blocks<kRestartThreads, true>(source, b0 * 8u, blk0, blk1, b1 * 8u, b1 * 8u, 0u, d.hs * d.vs, sh, w.huff, coef, info, err);
     }
     if (n < blk1 - blk0) err |= kStTruncated;
     if (err) atomicOr(w.status + d.item, err);
@@ -900,7 +996,7 @@ void launch_sync(const JpegWave& w, uint32_t first, uint32_t count, uint32_t clu
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(count * cluster);
     cfg.blockDim = dim3(T);
-    cfg.dynamicSmemBytes = (size_t)T * kRingPitch + sizeof(SyncMisc<T>) + w.max_tables * sizeof(SyncTab);
+    cfg.dynamicSmemBytes = (size_t)T * kRingPitch + sizeof(SyncMisc<T>) + w.max_pairs * 2 * sizeof(SyncTab);
     cfg.stream = s;
     cudaLaunchAttribute attr;
     if (CLUSTER) {
@@ -934,7 +1030,7 @@ void launch_huff_sync(const JpegWave& w, uint32_t first, uint32_t count, uint32_
 void launch_huff_write(const JpegWave& w, cudaStream_t s) {
     if (!w.write_ctas.total) return;
     configure_once();
-    const size_t smem = sizeof(ValueMisc<kWriteThreads>) + (size_t)kStageRows * kStagePitch + w.max_tables * sizeof(ValueTab);
+    const size_t smem = sizeof(ValueMisc<kWriteThreads>) + (size_t)kStageRows * kStagePitch + w.max_pairs * 2 * sizeof(ValueTab);
     k_huff_write<<<w.write_ctas.total, kWriteThreads, smem, s>>>(w);
     k_dc<<<w.dc_ctas.total, kDcThreads, 0, s>>>(w);
 }
@@ -942,7 +1038,7 @@ void launch_huff_write(const JpegWave& w, cudaStream_t s) {
 void launch_huff_restart(const JpegWave& w, cudaStream_t s) {
     if (!w.restart_ctas.total) return;
     configure_once();
-    const size_t smem = sizeof(ValueMisc<kRestartThreads>) + kRestartStage + w.max_tables * sizeof(ValueTab);
+    const size_t smem = sizeof(ValueMisc<kRestartThreads>) + kRestartStage + w.max_pairs * 2 * sizeof(ValueTab);
     k_huff_restart<<<w.restart_ctas.total, kRestartThreads, smem, s>>>(w);
 }
 
