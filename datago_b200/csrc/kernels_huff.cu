@@ -551,6 +551,8 @@ __global__ void __launch_bounds__(T) k_huff_sync(JpegWave w, uint32_t first) {
                 found += L.nb - old_n;
             }
         }
+        // Nothing may be on its way into the ring when it is filled anew: of two copies to one place the older may land last.
+        copy_wait<0>();
         if (L.p > total) { L.p = kNoState; L.mb.w = 0; }
         if (live) exit = make_uint2(L.p, L.mb.w);
     };
