@@ -186,6 +186,7 @@ extern "C" {
     pub fn dg_batch_packed_bytes(b: *const dg_batch) -> u64;
     pub fn dg_batch_sync(b: *mut dg_batch) -> c_int;
     pub fn dg_batch_result(b: *const dg_batch, i: c_int, out: *mut dg_result) -> c_int;
+    pub fn dg_batch_results(b: *const dg_batch, out: *mut dg_result) -> c_int;
     pub fn dg_batch_bucket_count(b: *const dg_batch) -> c_int;
     pub fn dg_batch_bucket(b: *const dg_batch, k: c_int, out: *mut dg_bucket) -> c_int;
     pub fn dg_batch_stage_ms(b: *const dg_batch, ms: *mut f32) -> c_int;
@@ -201,11 +202,14 @@ extern "C" {
     pub fn dg_wait(f: *mut dg_feeder, ticket: dg_ticket, timeout_ns: u64, out: *mut dg_result) -> c_int;
     pub fn dg_fetch(f: *mut dg_feeder, ticket: dg_ticket, host_out: *mut u8, capacity: u64) -> c_int;
     pub fn dg_peek(f: *mut dg_feeder, ticket: dg_ticket, host_data: *mut *const u8) -> c_int;
+    pub fn dg_fetch_view(f: *mut dg_feeder, ticket: dg_ticket, host_data: *mut *const u8, block: *mut *mut c_void) -> c_int;
     pub fn dg_release(f: *mut dg_feeder, ticket: dg_ticket) -> c_int;
     pub fn dg_feeder_get_stats(f: *mut dg_feeder, out: *mut dg_feeder_stats) -> c_int;
     pub fn dg_feeder_destroy(f: *mut dg_feeder);
 
     pub fn dg_resize_device_static(ctx: *mut dg_ctx, device_src: *const u8, w: u32, h: u32, channels: u32, forced_key: *const c_char,
                                    device_dst: *mut u8, plan_out: *mut dg_plan) -> c_int;
+    pub fn dg_host_alloc(nbytes: u64, out: *mut *mut c_void) -> c_int;
+    pub fn dg_host_release(block: *mut c_void);
     pub fn dg_copy_to_host(ctx: *mut dg_ctx, dst: *mut c_void, device_src: *const c_void, nbytes: u64) -> c_int;
 }

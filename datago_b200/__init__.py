@@ -23,6 +23,7 @@ STAGES = ("unstuff", "coef_clear", "huff_restart", "huff_spec", "idct", "color",
           "to_rgb8")
 STATUS_NAMES = {0: "ok", 1: "invalid", 2: "cuda", 3: "truncated", 4: "bad_marker", 5: "unsupported", 6: "bad_table",
                 7: "bad_code", 8: "unknown_key", 9: "no_transform", 10: "sync_limit", 11: "too_large", 12: "timeout"}
+E_TOO_LARGE = 11
 E_TIMEOUT = 12
 
 
@@ -115,6 +116,28 @@ class DeviceArray:
         return {"shape": self.shape, "typestr": "|u1", "data": (self.ptr, False), "version": 3, "strides": None}
 
 
+class _HostBlock:
+    """A page-locked block of the library's pool, or a part of one: numpy arrays made from it (np.asarray) keep it alive, and
+    the block goes back to the pool with the last of them."""
+
+    def __init__(self, ptr, nbytes, block):
+        self._block = block
+        self.__array_interface__ = {"shape": (nbytes,), "typestr": "|u1", "data": (ptr, False), "version": 3}
+
+    def __del__(self):
+        if _lib is not None:
+            _lib.dg_host_release(self._block)
+
+
+def host_block(nbytes):
+    """A writable uint8 array of nbytes in page-locked memory (what Batch.download_packed wants), or None while so much of
+    it is in use that ordinary memory has to do."""
+    ptr = C.c_void_p()
+    if nbytes == 0 or lib().dg_host_alloc(nbytes, C.byref(ptr)):
+        return None
+    return np.asarray(_HostBlock(ptr.value, nbytes, ptr))
+
+
 _lib = None
 
 
@@ -158,6 +181,7 @@ def lib():
         "dg_batch_packed_bytes": (C.c_uint64, [vp]),
         "dg_batch_sync": (C.c_int, [vp]),
         "dg_batch_result": (C.c_int, [vp, C.c_int, C.POINTER(Result)]),
+        "dg_batch_results": (C.c_int, [vp, C.POINTER(Result)]),
         "dg_batch_bucket_count": (C.c_int, [vp]),
         "dg_batch_bucket": (C.c_int, [vp, C.c_int, C.POINTER(Bucket)]),
         "dg_batch_stage_ms": (C.c_int, [vp, C.POINTER(C.c_float)]),
@@ -173,7 +197,10 @@ def lib():
         "dg_wait": (C.c_int, [vp, C.c_uint64, C.c_uint64, C.POINTER(Result)]),
         "dg_fetch": (C.c_int, [vp, C.c_uint64, vp, C.c_uint64]),
         "dg_peek": (C.c_int, [vp, C.c_uint64, C.POINTER(vp)]),
+        "dg_fetch_view": (C.c_int, [vp, C.c_uint64, C.POINTER(vp), C.POINTER(vp)]),
         "dg_release": (C.c_int, [vp, C.c_uint64]),
+        "dg_host_alloc": (C.c_int, [C.c_uint64, C.POINTER(vp)]),
+        "dg_host_release": (None, [vp]),
         "dg_feeder_get_stats": (C.c_int, [vp, C.POINTER(FeederStats)]),
         "dg_feeder_destroy": (None, [vp]),
         "dg_resize_device_static": (C.c_int, [vp, vp, C.c_uint32, C.c_uint32, C.c_uint32, C.c_char_p, vp, C.POINTER(Plan)]),
@@ -190,8 +217,8 @@ EXPORTS = ("dg_set_log_callback dg_ctx_get_counters dg_last_error dg_version dg_
            "dg_bucket_table dg_closest_aspect_ratio dg_aspect_ratio_to_str dg_plan_geometry dg_jpeg_probe dg_rank_slice "
            "dg_key_hash dg_key_rank dg_batch_create dg_batch_upload dg_batch_run dg_batch_download dg_batch_sync "
            "dg_batch_download_packed dg_batch_packed_bytes dg_batch_bucket_count dg_batch_bucket "
-           "dg_batch_result dg_batch_stage_ms dg_batch_counters dg_batch_huffman_stats dg_batch_debug dg_batch_destroy dg_process "
-           "dg_copy_to_host dg_resize_device_static dg_feeder_create dg_feeder_ctx dg_submit dg_wait dg_fetch dg_peek dg_release "
+           "dg_batch_result dg_batch_results dg_batch_stage_ms dg_batch_counters dg_batch_huffman_stats dg_batch_debug dg_batch_destroy dg_process "
+           "dg_copy_to_host dg_resize_device_static dg_feeder_create dg_feeder_ctx dg_submit dg_wait dg_fetch dg_peek dg_fetch_view dg_release dg_host_alloc dg_host_release "
            "dg_feeder_get_stats dg_feeder_destroy").split()
 
 
@@ -348,7 +375,7 @@ class Context:
             b.run()
             outs = b.download()
             b.sync()
-            res = [b.result(i) for i in range(len(b))]
+            res = b.results()
         return [(r.status, o if r.status == 0 else None, r) for r, o in zip(res, outs)]
 
     def resize_device_static(self, src_ptr, w, h, channels, dst_ptr, forced_key=None):
@@ -448,20 +475,24 @@ class Batch:
         _check(lib().dg_batch_result(self._h, i, C.byref(r)))
         return r
 
+    def results(self):
+        """Every item's Result."""
+        out = (Result * max(1, self._n))()
+        _check(lib().dg_batch_results(self._h, out))
+        return out[:self._n]
+
     def host_buffers(self):
         """numpy arrays shaped like each ok payload (None for failed items)."""
-        outs = []
-        for i in range(self._n):
-            r = self.result(i)
-            if r.status:
-                outs.append(None)
-            else:
-                outs.append(np.empty(_shape(r), np.uint8))
-        return outs
+        return [None if r.status else np.empty(_shape(r), np.uint8) for r in self.results()]
 
     def download(self, outs=None):
-        """Queue device->host copies into `outs` (from host_buffers()); valid after sync()."""
+        """Queue device->host copies into `outs` (from host_buffers()); valid after sync().  Without `outs` the payloads arrive in
+        one copy in page-locked memory, and the arrays returned are views of it (which lives as long as any of them)."""
         if outs is None:
+            block = host_block(self.packed_bytes())
+            if block is not None:
+                self.download_packed(block)
+                return [None if r.status else block[r.packed_offset:r.packed_offset + r.nbytes].reshape(_shape(r)) for r in self.results()]
             outs = self.host_buffers()
         ptrs = (C.c_void_p * max(1, self._n))(*[o.ctypes.data if o is not None else None for o in outs])
         self._outs = outs
@@ -587,7 +618,16 @@ class Feeder:
         return r
 
     def fetch(self, ticket, result):
-        """The payload of a finished ticket as a numpy array (H x W x 3, or H x W for one channel)."""
+        """The payload of a finished ticket as a numpy array (H x W x 3, or H x W for one channel): a view of the page-locked
+        memory it arrived in (kept alive by the array), or a copy when it is small or too much is held already."""
+        nbytes = int(result.nbytes)
+        if nbytes >= 1 << 15:
+            ptr, block = C.c_void_p(), C.c_void_p()
+            rc = lib().dg_fetch_view(self._h, ticket, C.byref(ptr), C.byref(block))
+            if rc == 0:
+                return np.asarray(_HostBlock(ptr.value, nbytes, block)).reshape(_shape(result))
+            if rc != E_TOO_LARGE:
+                _check(rc)
         out = np.empty(_shape(result), np.uint8)
         _check(lib().dg_fetch(self._h, ticket, out.ctypes.data, out.nbytes))
         return out

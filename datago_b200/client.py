@@ -28,7 +28,7 @@ import threading
 
 import numpy as np
 
-from . import BATCH_DECODE_ONLY, Context, DatagoB200Error, aspect_ratio_to_str, jpeg_probe, key_rank, rank_slice
+from . import BATCH_DECODE_ONLY, Context, DatagoB200Error, aspect_ratio_to_str, host_block, jpeg_probe, key_rank, rank_slice
 
 log = logging.getLogger("datago_b200")
 
@@ -36,19 +36,32 @@ IMG_TYPES = ("jpg", "jpeg", "png")          # src/worker_wds.rs:11
 TEXT_TYPES = ("cls", "json", "txt")         # src/worker_wds.rs:10
 FILE_EXTENSIONS = ("jpg", "jpeg", "png", "bmp", "gif", "webp")  # src/generator_files.rs:50
 TIMEOUT_S = 300                             # src/client.rs:12
+READ_UNITS = 8                              # samples the reader thread hands over at a time
+FIRST_UNITS = 16                            # samples that are worth a batch
 
 
 class ImagePayload:
     """The fields of datago's ImagePayload; `data` is host bytes, or empty when the payload stayed on the device."""
 
     def __init__(self, data=b"", original_height=0, original_width=0, height=0, width=0, channels=0, bit_depth=0,
-                 is_encoded=False, device_ptr=0, keepalive=None):
-        self.data = data
+                 is_encoded=False, device_ptr=0, keepalive=None, view=None):
+        self._data = data
+        self._view = view  # the pixels where the download left them (a read-only uint8 array); bytes are made when asked for
         self.original_height, self.original_width = original_height, original_width
         self.height, self.width, self.channels, self.bit_depth = height, width, channels, bit_depth
         self.is_encoded = is_encoded
         self._device_ptr = device_ptr
         self._keepalive = keepalive  # the batch that owns the device memory
+
+    @property
+    def data(self):
+        if self._view is not None:
+            self._data, self._view = self._view.tobytes(), None
+        return self._data
+
+    @data.setter
+    def data(self, value):
+        self._data, self._view = value, None
 
     def _shape(self):
         return (self.height, self.width, self.channels) if self.channels > 1 else (self.height, self.width)
@@ -59,6 +72,8 @@ class ImagePayload:
             import io
             from PIL import Image
             return np.asarray(Image.open(io.BytesIO(self.data)).convert("RGB"))
+        if self._view is not None:
+            return self._view.reshape(self._shape())
         if self._device_ptr and not len(self.data):
             return self._keepalive.ctx.copy_to_host(self._device_ptr, self.height * self.width * self.channels).reshape(self._shape())
         return np.frombuffer(self.data, np.uint8).reshape(self._shape())
@@ -394,27 +409,40 @@ class DatagoClient:
         """The engine: a reader thread walks files / shards ahead of this thread (datago's generator task), and this
         thread keeps one batch on the GPU while it plans the next (datago's worker pool): a batch is launched -- host
         planning, upload, kernels and the packed download queued on the context's stream -- before the previous one is
-        waited for and turned into samples.  Samples leave in source order."""
+        waited for and turned into samples.  A batch does not wait until it is full: it takes what the reader has at hand,
+        FIRST_UNITS samples at least, so the GPU starts early and batches grow while it is busy.  Samples leave in source
+        order."""
         produced = 0
-        units_q = queue.Queue(maxsize=max(4 * self.batch_size, 16))
+        units_q = queue.Queue(maxsize=max(4 * self.batch_size // READ_UNITS, 4))
         reader = threading.Thread(target=self._read_ahead, args=(units_q,), daemon=True)
         reader.start()
         in_flight, flight_units = None, 0
         try:
-            pending, lane, eof = [], 0, False
+            pending, backlog, lane, eof = [], [], 0, False
             while not self._stop.is_set():
                 room = self.limit - produced - flight_units - len(pending)
+                enough = min(self.batch_size, FIRST_UNITS)
                 if not eof and room > 0 and len(pending) < self.batch_size:
-                    try:
-                        unit = units_q.get(timeout=0.1)
-                    except queue.Empty:  # the reader is still at work (or the client is being stopped)
+                    if not backlog:
+                        try:
+                            # waiting only when there is nothing else to do: neither a batch to launch nor one to finish
+                            backlog = units_q.get(block=in_flight is None and len(pending) < enough, timeout=0.1)
+                        except queue.Empty:  # the reader is still at work (or the client is being stopped)
+                            if len(pending) < enough:
+                                if in_flight is not None:
+                                    produced += self._finish(in_flight)
+                                    in_flight, flight_units = None, 0
+                                continue
+                            backlog = []
+                    if backlog is None:
+                        eof, backlog = True, []
                         continue
-                    if unit is None:
-                        eof = True
-                    else:
-                        pending.append(unit)
-                    continue
-                if pending:  # a full batch, the last units below the limit, or the end of the source
+                    if backlog:
+                        take = min(room, self.batch_size - len(pending))
+                        pending += backlog[:take]
+                        backlog = backlog[take:]
+                        continue
+                if pending:  # enough for a batch, the last units below the limit, or the end of the source
                     launched = self._launch(pending, lane)
                     lane ^= 1
                     if in_flight is not None:
@@ -445,16 +473,25 @@ class DatagoClient:
             self._put(None)
 
     def _read_ahead(self, units_q):
+        def hand_over(units):
+            while not (self._stop.is_set() or self._reader_stop.is_set()):
+                try:
+                    units_q.put(units, timeout=0.1)
+                    return True
+                except queue.Full:
+                    continue
+            return False
+
         try:
+            units = []  # handed over a few at a time: every hand-over is a switch of threads
             for unit in self._units():
-                while not (self._stop.is_set() or self._reader_stop.is_set()):
-                    try:
-                        units_q.put(unit, timeout=0.1)
-                        break
-                    except queue.Full:
-                        continue
-                else:
-                    return
+                units.append(unit)
+                if len(units) == READ_UNITS:
+                    if not hand_over(units):
+                        return
+                    units = []
+            if units:
+                hand_over(units)
         except Exception:  # noqa: BLE001
             log.exception("datago_b200 reader failed")
         finally:
@@ -525,20 +562,26 @@ class DatagoClient:
         batch = self.ctx.batch(inputs, keys, 0 if has_tfm else BATCH_DECODE_ONLY, to_rgb8=to_rgb8)
         batch.upload()
         batch.run()
-        buf = None
+        buf, views = None, False
         if not self.device_payloads and len(batch):
-            buf = self._host_buffer(lane, batch.packed_bytes())
+            buf = None if self.pre_encode else host_block(batch.packed_bytes())  # samples keep views of it
+            views = buf is not None
+            if not views:
+                buf = self._host_buffer(lane, batch.packed_bytes())
             batch.download_packed(buf)  # one copy; payload i lands at result(i).packed_offset
-        return batch, units, slots, buf
+        return batch, units, slots, buf, views
 
     def _finish(self, launched):
         """Waits for a launched batch and puts its samples on the queue; returns how many it made."""
-        batch, units, slots, buf = launched
+        batch, units, slots, buf, views = launched
         batch.sync()
+        if views:
+            buf.flags.writeable = False  # payloads are read-only, as bytes are
+        results = batch.results()
         made = 0
         payloads = {}
         for i, (ui, name) in enumerate(slots):
-            r = batch.result(i)
+            r = results[i]
             if r.status != 0:
                 log.error("decode failed for %s (status %d)", name, r.status)
                 continue
@@ -548,7 +591,8 @@ class DatagoClient:
                                   original_height=r.original_height, original_width=r.original_width, height=r.height,
                                   width=r.width, channels=-1, bit_depth=8, is_encoded=True)
             else:
-                pl = ImagePayload(data=b"" if self.device_payloads else buf[r.packed_offset:r.packed_offset + r.nbytes].tobytes(), original_height=r.original_height,
+                px = None if self.device_payloads else buf[r.packed_offset:r.packed_offset + r.nbytes]
+                pl = ImagePayload(data=b"" if px is None or views else px.tobytes(), view=px if views else None, original_height=r.original_height,
                                   original_width=r.original_width, height=r.height, width=r.width, channels=r.channels,
                                   bit_depth=8, is_encoded=False, device_ptr=r.device_data if self.device_payloads else 0,
                                   keepalive=batch if self.device_payloads else None)

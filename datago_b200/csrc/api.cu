@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "host.h"
+#include "host_blocks.h"
 #include "host_pool.h"
 #include "kernels.h"
 
@@ -98,35 +99,54 @@ struct Block {
     bool busy = false;
 };
 
-// Grow-only cache: a batch borrows blocks and hands them back; nothing is freed before the ctx goes away, so steady
-// state makes no allocation calls.
+// Cache of blocks: a batch borrows them and hands them back; nothing is freed in the steady state, so it makes no allocation
+// calls.  A request takes the smallest idle block that fits and is not far too large for it (a large block lent to a small
+// request is missing when the next large one comes, and then the cache allocates on every batch).
 struct BlockCache {
     bool pinned;
     std::vector<Block> blocks;
     explicit BlockCache(bool p) : pinned(p) {}
-    int acquire(size_t size, int* index) {
-        if (size == 0) size = 256;
+    void give_back(Block& b) {
+        if (b.ptr) { if (pinned) cudaFreeHost(b.ptr); else cudaFree(b.ptr); }
+        b = Block();
+    }
+    int smallest_fit(size_t size, size_t most) const {
         int best = -1;
         for (size_t i = 0; i < blocks.size(); ++i)
-            if (!blocks[i].busy && blocks[i].size >= size && (best < 0 || blocks[i].size < blocks[best].size)) best = (int)i;
+            if (!blocks[i].busy && blocks[i].size >= size && blocks[i].size <= most && (best < 0 || blocks[i].size < blocks[best].size)) best = (int)i;
+        return best;
+    }
+    int acquire(size_t size, int* index) {
+        if (size == 0) size = 256;
+        int best = smallest_fit(size, 2 * size + ((size_t)4 << 20));
         if (best < 0) {
-            // replace the largest idle block that is too small, so the cache does not pile up stale sizes
+            // the largest idle block that is too small makes room, so that the cache does not pile up stale sizes
             int victim = -1;
             for (size_t i = 0; i < blocks.size(); ++i)
-                if (!blocks[i].busy && (victim < 0 || blocks[i].size > blocks[victim].size)) victim = (int)i;
+                if (!blocks[i].busy && blocks[i].size < size && (victim < 0 || blocks[i].size > blocks[victim].size)) victim = (int)i;
+            // ... once the idle ones add up to something, and not a much smaller one, which serves other requests
+            size_t idle = 0;
+            for (const Block& b : blocks) idle += b.busy ? 0 : b.size;
+            if (victim >= 0 && (blocks[victim].size < size / 2 || idle < ((size_t)1 << 30))) victim = -1;
+            if (victim < 0) { blocks.emplace_back(); victim = (int)blocks.size() - 1; }
+            give_back(blocks[victim]);
             Block nb;
             nb.size = size + size / 8 + 4096;
-            if (victim >= 0) {
-                if (pinned) cudaFreeHost(blocks[victim].ptr); else cudaFree(blocks[victim].ptr);
-                blocks[victim] = Block();
-            }
-            cudaError_t e = pinned ? cudaHostAlloc(&nb.ptr, nb.size, cudaHostAllocDefault) : cudaMalloc(&nb.ptr, nb.size);
-            if (e != cudaSuccess) {
+            auto allocate = [&] { return pinned ? cudaHostAlloc(&nb.ptr, nb.size, cudaHostAllocDefault) : cudaMalloc(&nb.ptr, nb.size); };
+            cudaError_t e = allocate();
+            if (e != cudaSuccess) {  // out of memory: whatever fits, else without the idle blocks
                 cudaGetLastError();  // a failed allocation must not surface again as the next healthy batch's error
-                return fail(DG_E_CUDA, "%s of %zu bytes: %s", pinned ? "cudaHostAlloc" : "cudaMalloc", nb.size, cudaGetErrorString(e));
+                best = smallest_fit(size, ~(size_t)0);
+                if (best < 0) {
+                    for (Block& b : blocks) if (!b.busy) give_back(b);
+                    e = allocate();
+                    if (e != cudaSuccess) {
+                        cudaGetLastError();
+                        return fail(DG_E_CUDA, "%s of %zu bytes: %s", pinned ? "cudaHostAlloc" : "cudaMalloc", nb.size, cudaGetErrorString(e));
+                    }
+                }
             }
-            if (victim >= 0) { blocks[victim] = nb; best = victim; }
-            else { blocks.push_back(nb); best = (int)blocks.size() - 1; }
+            if (best < 0) { blocks[victim] = nb; best = victim; }
         }
         blocks[best].busy = true;
         *index = best;
@@ -238,6 +258,7 @@ static int ctx_create(int device, const dg_image_config* cfg, void* stream, bool
     if (!encode_tiled_fn()) c->hmma = false;  // a driver without tensor maps: every horizontal pass takes the dp2a kernel
     if (const char* mb = getenv("DATAGO_B200_MAX_IMAGE_MB")) { long v = atol(mb); if (v >= 1) c->max_image_bytes = (uint64_t)v << 20; }
     if (const char* mb = getenv("DATAGO_B200_WAVE_MB")) { long v = atol(mb); if (v >= 16) c->wave_bytes = (size_t)v << 20; }
+    host_blocks_context(+1);
     *out = c;
     return DG_OK;
 }
@@ -265,6 +286,7 @@ extern "C" void dg_ctx_destroy(dg_ctx* c) {
     cudaStreamDestroy(c->stream2);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
+    host_blocks_context(-1);
 }
 
 extern "C" void* dg_ctx_stream(dg_ctx* c) { return c ? (void*)c->stream : nullptr; }
@@ -455,15 +477,17 @@ struct dg_batch {
     std::vector<WavePlan> waves;
     std::vector<BucketPlan> buckets;
     Meta meta;
-    // persistent device block: [meta | status | blob | raw inputs | outputs]
-    int blk_persist = -1, blk_scratch = -1, blk_scratch2 = -1, blk_pin = -1, blk_pin_status = -1;
+    // device blocks that live as long as the batch: [status | blob | raw inputs | outputs], and the metadata
+    int blk_persist = -1, blk_meta = -1, blk_scratch = -1, blk_scratch2 = -1, blk_pin = -1, blk_pin_meta = -1, blk_pin_status = -1;
     uint8_t* d_persist = nullptr;
+    uint8_t* d_meta = nullptr;
     uint8_t* d_scratch = nullptr;   // scratch of the even waves
     uint8_t* d_scratch2 = nullptr;  // scratch of the odd waves (same block when the batch has one wave)
-    uint8_t* h_pin = nullptr;       // pinned image of [meta | status zeros | blob]
+    uint8_t* h_pin = nullptr;       // pinned image of [status zeros | blob | raw inputs]
+    uint8_t* h_meta = nullptr;      // ... and of the metadata
     uint32_t* h_status = nullptr;   // pinned, n words
-    size_t off_meta = 0, off_status = 0, off_blob = 0, off_rawin = 0, off_out = 0, persist_bytes = 0;
-    size_t blob_bytes = 0, rawin_bytes = 0, out_bytes = 0, pin_bytes = 0;
+    size_t off_status = 0, off_blob = 0, off_rawin = 0, off_out = 0;
+    size_t blob_bytes = 0, rawin_bytes = 0, out_bytes = 0;
     size_t arena_bytes = 0;  // out_bytes plus the pre-conversion images of DG_ITEM_TO_RGB8 items (never downloaded)
     size_t m_huff = 0, m_qt = 0, m_tables = 0, meta_total = 0;  // meta_total: meta.bytes plus the filter tables behind it
     std::vector<const uint8_t*> raw_src;  // caller memory of raw items (used inside dg_batch_create only)
@@ -481,7 +505,6 @@ namespace {
 struct Planner {
     dg_ctx* ctx;
     dg_batch* b;
-    bool final_round = true;   // device addresses are final: tensor maps are encoded (the sizing round skips them)
     std::atomic<bool> tmap_failed{false};  // a tensor map could not be encoded (items are planned on several threads)
     std::unordered_map<std::string, uint32_t> huff_ids, qt_ids;
     std::vector<HuffTable> huff_pool;
@@ -785,7 +808,7 @@ static void plan_resize(Planner& pl, WavePlan& wv, const dg_plan& p, uint32_t C,
             if (guarded) { cp.guard_lo = src; cp.guard_hi = src + (size_t)w * h * C; }
             else if (pl.ctx->hmma && (((uintptr_t)s | spitch) & 15) == 0 && hmma_fits(*T, t0, out_w, C, origin, &cp.box_pieces)) {
                 cp.fast = 2;
-                if (pl.final_round && !encode_source_map(cp)) pl.tmap_failed = true;
+                if (!encode_source_map(cp)) pl.tmap_failed = true;
             }
         } else {
             const uintptr_t bits = (uintptr_t)s | (uintptr_t)d | spitch | dpitch;
@@ -796,7 +819,7 @@ static void plan_resize(Planner& pl, WavePlan& wv, const dg_plan& p, uint32_t C,
             uint32_t src_rows = 0;
             if (cp.fast && !guarded && pl.ctx->hmma && vmma_fits(*T, t0, out_h, origin, &cp.box_pieces, &src_rows)) {
                 cp.fast = 2;
-                if (pl.final_round && !encode_source_map_v(cp, src_rows)) pl.tmap_failed = true;
+                if (!encode_source_map_v(cp, src_rows)) pl.tmap_failed = true;
             }
         }
         cp.tiles_x = conv_tiles_x(cp, !horizontal);
@@ -866,15 +889,17 @@ static uint32_t stream_cells(uint32_t raw_len) { return (uint32_t)(((uint64_t)ra
 
 // Runs fn(0..n-1) on the process-wide host pool; small counts stay on the calling thread.
 template <typename F> static void parallel_items(int n, F&& fn) {
-    HostPool::get().run((size_t)std::max(n, 0), [&fn](size_t i) { fn((int)i); }, 64);
+    HostPool::get().run((size_t)std::max(n, 0), [&fn](size_t i) { fn((int)i); }, 16);
 }
 
 static int abandon(dg_batch* b, int rc) {
     dg_ctx* ctx = b->ctx;
     ctx->dev.release(b->blk_persist);
+    ctx->dev.release(b->blk_meta);
     ctx->dev.release(b->blk_scratch);
     ctx->dev.release(b->blk_scratch2);
     ctx->pin.release(b->blk_pin);
+    ctx->pin.release(b->blk_pin_meta);
     ctx->pin.release(b->blk_pin_status);
     delete b;
     return rc;
@@ -1180,9 +1205,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         scratch_max = std::max(scratch_max, o);
     }
 
-    // ---- device and pinned blocks (addresses are needed by the resize descriptors) ------------------------------------
-    // persistent layout: [status | blob | raw inputs | outputs | meta]; meta size is known only after planning the
-    // resize passes, so it gets a bound: descriptors + tables are small next to the pixel buffers.
+    // ---- device blocks (the resize descriptors hold addresses inside them) ---------------------------------------------
     int rc = ctx->dev.acquire(std::max<size_t>(scratch_max, 256), &b->blk_scratch);
     if (rc) return abandon(b, rc);
     b->d_scratch = (uint8_t*)ctx->dev.blocks[b->blk_scratch].ptr;
@@ -1192,32 +1215,26 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         if (rc) return abandon(b, rc);
         b->d_scratch2 = (uint8_t*)ctx->dev.blocks[b->blk_scratch2].ptr;
     }
-
     b->off_status = 0;  // n status words, then 4 counters of the speculative Huffman kernel
     b->off_blob = align_up((size_t)n * 4 + 32, 256);
     b->off_rawin = b->off_blob + align_up(blob, 256);
     b->off_out = b->off_rawin + align_up(rawin, 256);
-    const size_t fixed_bytes = b->off_out + align_up(b->arena_bytes, 256);
+    rc = ctx->dev.acquire(b->off_out + align_up(b->arena_bytes, 256), &b->blk_persist);
+    if (rc) return abandon(b, rc);
+    b->d_persist = (uint8_t*)ctx->dev.blocks[b->blk_persist].ptr;
 
-    // Resize descriptors hold device addresses inside the persistent block, whose size depends on the metadata that
-    // contains them.  So the passes are planned twice: once against a stand-in base to size the metadata (filter
-    // tables are cached, the second round is cheap), once with the real base address.
+    // ---- resize passes and the metadata image ----------------------------------------------------------------------------
     if (transform) {
         std::vector<const dg_plan*> plans;
         for (const ItemPlan& it : b->items)
             if (!it.status && it.wave >= 0) plans.push_back(&it.plan);
         pl.prebuild_tables(plans);
     }
-    for (int round = 0; round < 2; ++round) {
-        uint8_t* baseP = round == 0 ? b->d_scratch : b->d_persist;
-        pl.final_round = round == 1;
+    {
+        uint8_t* const baseP = b->d_persist;
         for (size_t wi = 0; wi < b->waves.size(); ++wi) {
             WavePlan& wv = b->waves[wi];
             uint8_t* const kBaseS = (wi & 1) ? b->d_scratch2 : b->d_scratch;
-            for (int s = 0; s < 4; ++s) { wv.passes[s].clear(); wv.pass_first[s].clear(); }
-            wv.copies.clear(); wv.copy_first.clear();
-            wv.torgb.clear(); wv.torgb_first.clear();
-            for (int a = 0; a < 4; ++a) { wv.alpha[a].clear(); wv.alpha_first[a].clear(); }
             // Every item is planned on its own (the filter tables are all there by now, so the planner is only read):
             // its intermediates get the slice of the wave's scratch that its worst-case bound reserves, and its passes
             // and jobs are appended to the wave's lists in item order afterwards.
@@ -1230,7 +1247,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             size_t mid_used = mid_at[n_wave_items];
             std::vector<WavePlan> parts((size_t)n_wave_items);
             std::atomic<bool> overflow{false};
-            parallel_items(n_wave_items, [&](int k) {
+            HostPool::get().run((size_t)n_wave_items, [&](size_t k) {
                 ItemPlan& it = b->items[wv.first_item + k];
                 if (it.status || it.wave < 0) return;
                 // encoding a tensor map is a driver call and wants a current context, which the pool's threads do not
@@ -1259,7 +1276,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
                     j.tile_first = 0; j.pad = 0;
                     part.torgb.push_back(j);
                 }
-            });
+            }, 4);
             if (overflow) mid_used = wv.mid_bytes + 1;
             for (const WavePlan& part : parts) {
                 for (int s = 0; s < 4; ++s) wv.passes[s].insert(wv.passes[s].end(), part.passes[s].begin(), part.passes[s].end());
@@ -1306,7 +1323,6 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         }
         // meta image
         Meta& m = b->meta;
-        m.bytes.clear();
         b->m_huff = m.put(pl.huff_pool, 16);
         b->m_qt = m.put(pl.qt_pool, 16);
         for (WavePlan& wv : b->waves) {
@@ -1342,78 +1358,72 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         // the filter tables follow the rest of the metadata; they are written into the staging buffer directly
         b->m_tables = align_up(m.bytes.size(), 256);
         b->meta_total = b->m_tables + pl.table_words_total * 4;
-        if (round == 0) {
-            b->off_meta = fixed_bytes;
-            b->persist_bytes = fixed_bytes + align_up(b->meta_total, 256);
-            rc = ctx->dev.acquire(b->persist_bytes, &b->blk_persist);
-            if (rc) return abandon(b, rc);
-            b->d_persist = (uint8_t*)ctx->dev.blocks[b->blk_persist].ptr;
-            bool pointers = transform;  // resize passes and copy jobs carry device pointers: lay them out again for real
-            for (const WavePlan& wv : b->waves) pointers = pointers || !wv.copies.empty() || !wv.torgb.empty();  // (alpha jobs only exist with a transform)
-            if (!pointers) break;
-        }
     }
     if (pl.tmap_failed) return abandon(b, fail(DG_E_CUDA, "cuTensorMapEncodeTiled rejected the source of a horizontal resize pass"));
 
-    // ---- pinned staging: [status zeros | blob | raw pixel inputs] + meta ------------------------------------------
+    // ---- page-locked staging -------------------------------------------------------------------------------------------
     // Raw inputs are staged too: a copy from pageable caller memory is serialised by the driver at a fraction of the
     // link rate, while host threads fill page-locked memory in parallel and the upload becomes one large transfer.
-    const size_t staged_head = b->off_rawin + align_up(rawin, 256);
-    b->pin_bytes = staged_head + align_up(b->meta_total, 256);
-    rc = ctx->pin.acquire(b->pin_bytes, &b->blk_pin);
+    rc = ctx->dev.acquire(b->meta_total, &b->blk_meta);
+    if (!rc) rc = ctx->pin.acquire(b->off_rawin + align_up(rawin, 256), &b->blk_pin);
+    if (!rc) rc = ctx->pin.acquire(b->meta_total, &b->blk_pin_meta);
     if (!rc) rc = ctx->pin.acquire(std::max<size_t>((size_t)n * 4, 256), &b->blk_pin_status);
     if (rc) return abandon(b, rc);
+    b->d_meta = (uint8_t*)ctx->dev.blocks[b->blk_meta].ptr;
     b->h_pin = (uint8_t*)ctx->pin.blocks[b->blk_pin].ptr;
+    b->h_meta = (uint8_t*)ctx->pin.blocks[b->blk_pin_meta].ptr;
     b->h_status = (uint32_t*)ctx->pin.blocks[b->blk_pin_status].ptr;
     memset(b->h_pin, 0, b->off_blob);
     {
-        std::vector<std::pair<int, size_t>> jobs;  // (item, offset in the blob): same order as the descriptors' raw_off
-        size_t off = 0;
+        // One list of copies for everything: pieces of about 128 KB, or one filter table each, so that a few large inputs
+        // spread over the host threads as well as many small ones.
+        constexpr size_t kPiece = (size_t)128 << 10;
+        struct Piece { uint8_t* dst; const uint8_t* src; size_t len; uint32_t rows, pitch; };  // rows == 0: one flat run of len bytes
+        std::vector<Piece> pieces;
+        size_t bytes = b->meta.bytes.size();
+        auto flat = [&](uint8_t* dst, const uint8_t* src, size_t len) {
+            bytes += len;
+            for (size_t o = 0; o < len; o += kPiece) pieces.push_back({dst + o, src + o, std::min(len - o, kPiece), 0, 0});
+        };
+        size_t off = 0;  // in the blob: same order as the descriptors' raw_off
         for (WavePlan& wv : b->waves)
             for (int i = wv.first_item; i < wv.last_item; ++i) {
                 const ItemPlan& it = b->items[i];
                 if (it.status || !it.is_jpeg || it.wave_local < 0) continue;
-                jobs.emplace_back(i, off);
-                off += align_up(it.hdr->scan_len, 16) + 16;
+                const JpegHeader& h = *it.hdr;
+                uint8_t* dst = b->h_pin + b->off_blob + off;
+                const size_t slot = align_up(h.scan_len, 16) + 16;
+                flat(dst, items[i].data + h.scan_off, h.scan_len);
+                memset(dst + h.scan_len, 0, slot - h.scan_len);
+                off += slot;
             }
-        parallel_items((int)jobs.size(), [&](int k) {
-            const int i = jobs[k].first;
-            const JpegHeader& h = *b->items[i].hdr;
-            uint8_t* dst = b->h_pin + b->off_blob + jobs[k].second;
-            memcpy(dst, items[i].data + h.scan_off, h.scan_len);
-            memset(dst + h.scan_len, 0, align_up(h.scan_len, 16) + 16 - h.scan_len);
-        });
-    }
-    if (rawin) {
-        struct Piece { uint8_t* dst; const uint8_t* src; size_t len; uint32_t rows, pitch; };  // rows == 0: one flat run of len bytes
-        std::vector<Piece> pieces;  // 4 MB pieces, so that a few large images still spread over the threads
-        for (int i = 0; i < n; ++i) {
+        for (int i = 0; i < n && rawin; ++i) {
             const ItemPlan& it = b->items[i];
             if (it.status || it.is_jpeg || !b->raw_src[i]) continue;
-            const size_t row = (size_t)it.w * it.c, bytes = row * it.h;
+            const size_t row = (size_t)it.w * it.c;
             uint8_t* dst = b->h_pin + b->off_rawin + it.raw_in_off;
-            if (it.src_pitch == row) {
-                for (size_t o = 0; o < bytes; o += (size_t)4 << 20)
-                    pieces.push_back({dst + o, b->raw_src[i] + o, std::min(bytes - o, (size_t)4 << 20), 0, 0});
-            } else {  // rows are re-pitched on the way: a piece is a run of whole rows
-                const size_t rows_per = std::max<size_t>(1, ((size_t)4 << 20) / row);
+            if (it.src_pitch == row) flat(dst, b->raw_src[i], row * it.h);
+            else {  // rows are re-pitched on the way: a piece is a run of whole rows
+                const size_t rows_per = std::max<size_t>(1, kPiece / row);
+                bytes += row * it.h;
                 for (size_t y = 0; y < it.h; y += rows_per)
                     pieces.push_back({dst + y * it.src_pitch, b->raw_src[i] + y * row, row, (uint32_t)std::min<size_t>(rows_per, it.h - y), it.src_pitch});
             }
         }
-        HostPool::get().run(pieces.size(), [&](size_t k) {
+        flat(b->h_meta, b->meta.bytes.data(), b->meta.bytes.size());
+        uint32_t* const pool = reinterpret_cast<uint32_t*>(b->h_meta + b->m_tables);
+        const auto& list = pl.table_list;
+        bytes += pl.table_words_total * 4;
+        const size_t np = pieces.size();
+        // below half a megabyte waking the other threads takes longer than the copies
+        HostPool::get().run(np + list.size(), [&](size_t k) {
+            if (k >= np) { list[k - np].second->pack(pool + list[k - np].first); return; }
             const Piece& pc = pieces[k];
             if (!pc.rows) { memcpy(pc.dst, pc.src, pc.len); return; }
             for (uint32_t y = 0; y < pc.rows; ++y) memcpy(pc.dst + (size_t)y * pc.pitch, pc.src + (size_t)y * pc.len, pc.len);
-        }, 1);
+        }, bytes < ((size_t)1 << 19) ? np + list.size() : 1);
     }
     b->raw_src.clear();  // caller memory is not needed after this call
-    memcpy(b->h_pin + staged_head, b->meta.bytes.data(), b->meta.bytes.size());
-    {
-        uint32_t* pool = reinterpret_cast<uint32_t*>(b->h_pin + staged_head + b->m_tables);
-        const auto& list = pl.table_list;
-        HostPool::get().run(list.size(), [&](size_t k) { list[k].second->pack(pool + list[k].first); }, 8);
-    }
     *out = b;
     return DG_OK;
 }
@@ -1429,7 +1439,7 @@ extern "C" int dg_batch_upload(dg_batch* b) {
     CU(cudaMemcpyAsync(b->d_persist, b->h_pin, head, cudaMemcpyHostToDevice, ctx->stream));
     b->h2d += head;
     // metadata
-    CU(cudaMemcpyAsync(b->d_persist + b->off_meta, b->h_pin + head, b->meta_total, cudaMemcpyHostToDevice, ctx->stream));
+    CU(cudaMemcpyAsync(b->d_meta, b->h_meta, b->meta_total, cudaMemcpyHostToDevice, ctx->stream));
     b->h2d += b->meta_total;
     b->uploaded = true;
     return DG_OK;
@@ -1437,7 +1447,7 @@ extern "C" int dg_batch_upload(dg_batch* b) {
 
 static OwnerMap resolve(const dg_batch* b, const OwnerMapOff& o) {
     OwnerMap m;
-    const uint8_t* base = b->d_persist + b->off_meta;
+    const uint8_t* base = b->d_meta;
     m.first = (const uint32_t*)(base + o.first);
     m.coarse = (const uint32_t*)(base + o.coarse);
     m.n = o.n; m.shift = o.shift; m.total = o.total;
@@ -1458,7 +1468,7 @@ static int batch_run_locked(dg_batch* b) {
     dg_ctx* ctx = b->ctx;
     CU(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
-    const uint8_t* meta = b->d_persist + b->off_meta;
+    const uint8_t* meta = b->d_meta;
     const bool timing = (b->flags & DG_BATCH_TIMING) != 0;
     // Waves alternate between two streams and two scratch blocks, so the serial, latency-bound entropy decoding of one
     // wave overlaps the bandwidth-hungry reconstruction of the other.  A timing batch stays on one stream: its stage
@@ -1744,6 +1754,12 @@ extern "C" int dg_batch_result(const dg_batch* b, int i, dg_result* out) {
     return DG_OK;
 }
 
+extern "C" int dg_batch_results(const dg_batch* b, dg_result* out) {
+    if (!b || !out) return fail(DG_E_INVALID, "NULL argument");
+    for (int i = 0; i < b->n; ++i) dg_batch_result(b, i, out + i);
+    return DG_OK;
+}
+
 extern "C" int dg_batch_bucket_count(const dg_batch* b) { return b ? (int)b->buckets.size() : 0; }
 
 extern "C" int dg_batch_bucket(const dg_batch* b, int k, dg_bucket* out) {
@@ -1805,9 +1821,11 @@ extern "C" void dg_batch_destroy(dg_batch* b) {
     cudaStreamSynchronize(ctx->stream);
     for (StageEvent& se : b->events) { cudaEventDestroy(se.a); cudaEventDestroy(se.b); }
     ctx->dev.release(b->blk_persist);
+    ctx->dev.release(b->blk_meta);
     ctx->dev.release(b->blk_scratch);
     ctx->dev.release(b->blk_scratch2);
     ctx->pin.release(b->blk_pin);
+    ctx->pin.release(b->blk_pin_meta);
     ctx->pin.release(b->blk_pin_status);
     delete b;
 }

@@ -23,6 +23,7 @@
 
 #include "../../include/datago_b200.h"
 #include "host.h"
+#include "host_blocks.h"
 
 namespace {
 
@@ -30,16 +31,14 @@ using Clock = std::chrono::steady_clock;
 
 struct Lane;
 
-// One finished batch: keeps the device payloads and their pinned host copy alive until the last ticket lets go.
+// One finished batch: keeps the device payloads and their page-locked host copy alive until the last ticket lets go (the
+// host copy longer, if somebody took a view of it).
 struct Flight {
     Lane* lane = nullptr;
     dg_batch* batch = nullptr;
-    int pinned_index = -1;
-    uint8_t* pinned = nullptr;
+    uint8_t* pinned = nullptr;  // a host block
     std::atomic<int> refs{0};
 };
-
-struct PinnedBuf { uint8_t* ptr = nullptr; size_t size = 0; bool busy = false; };
 
 struct Ticket {
     uint64_t id = 0;
@@ -58,7 +57,6 @@ struct Ticket {
 struct Lane {
     dg_ctx* ctx = nullptr;
     std::thread thread;
-    std::vector<PinnedBuf> pinned;     // touched by the lane thread only
     std::mutex dead_mu;
     std::vector<Flight*> dead;          // flights nobody references any more; the lane thread destroys them
 };
@@ -98,28 +96,9 @@ void bury(Lane& lane) {
     }
     for (Flight* f : dead) {
         if (f->batch) dg_batch_destroy(f->batch);
-        if (f->pinned_index >= 0) lane.pinned[f->pinned_index].busy = false;
+        dg::host_block_release(f->pinned);
         delete f;
     }
-}
-
-int pinned_acquire(Lane& lane, size_t size, int* index) {
-    if (size == 0) size = 256;
-    int best = -1;
-    for (size_t i = 0; i < lane.pinned.size(); ++i)
-        if (!lane.pinned[i].busy && lane.pinned[i].size >= size && (best < 0 || lane.pinned[i].size < lane.pinned[best].size)) best = (int)i;
-    if (best < 0) {
-        for (size_t i = 0; i < lane.pinned.size(); ++i)  // recycle an idle buffer that is too small
-            if (!lane.pinned[i].busy) { cudaFreeHost(lane.pinned[i].ptr); lane.pinned[i] = PinnedBuf(); best = (int)i; break; }
-        PinnedBuf nb;
-        nb.size = size + size / 4;
-        if (cudaHostAlloc((void**)&nb.ptr, nb.size, cudaHostAllocDefault) != cudaSuccess) return set_error(DG_E_CUDA, "feeder: pinned host allocation failed");
-        if (best >= 0) lane.pinned[best] = nb;
-        else { lane.pinned.push_back(nb); best = (int)lane.pinned.size() - 1; }
-    }
-    lane.pinned[best].busy = true;
-    *index = best;
-    return DG_OK;
 }
 
 // Finish a group of tickets with one status (batch-level failure).
@@ -174,18 +153,18 @@ void lane_main(dg_feeder* f, Lane* lane) {
         if (!rc) rc = dg_batch_upload(batch);
         for (Ticket* t : group) { std::vector<uint8_t>().swap(t->bytes); }  // staged: the copies are no longer needed
         if (!rc) rc = dg_batch_run(batch);
-        int pin = -1;
-        if (!rc) rc = pinned_acquire(*lane, dg_batch_packed_bytes(batch), &pin);
-        if (!rc) rc = dg_batch_download_packed(batch, lane->pinned[pin].ptr, lane->pinned[pin].size);
+        void* landing = nullptr;
+        if (!rc) rc = dg::host_block_acquire(dg_batch_packed_bytes(batch), false, &landing);
+        if (!rc) rc = dg_batch_download_packed(batch, (uint8_t*)landing, dg_batch_packed_bytes(batch));
         if (!rc) rc = dg_batch_sync(batch);
         if (rc) {
             if (batch) dg_batch_destroy(batch);
-            if (pin >= 0) lane->pinned[pin].busy = false;
+            dg::host_block_release(landing);
             fail_all(f, group, rc);
             continue;
         }
         Flight* fl = new Flight();
-        fl->lane = lane; fl->batch = batch; fl->pinned_index = pin; fl->pinned = lane->pinned[pin].ptr;
+        fl->lane = lane; fl->batch = batch; fl->pinned = (uint8_t*)landing;
         fl->refs.store(n + 1);  // one per ticket + this thread's own
         {
             std::lock_guard<std::mutex> lock(f->mu);
@@ -332,6 +311,19 @@ extern "C" int dg_peek(dg_feeder* f, dg_ticket id, const uint8_t** host_data) {
     return DG_OK;
 }
 
+extern "C" int dg_fetch_view(dg_feeder* f, dg_ticket id, const uint8_t** host_data, void** block) {
+    if (!block) return set_error(DG_E_INVALID, "NULL argument");
+    *block = nullptr;
+    const int rc = dg_peek(f, id, host_data);
+    if (rc) return rc;
+    std::lock_guard<std::mutex> lock(f->mu);
+    const Ticket* t = f->tickets.find(id)->second.get();  // (a ticket belongs to one thread: it is still there)
+    if (dg::host_blocks_scarce()) return set_error(DG_E_TOO_LARGE, "too much page-locked memory is held by views");
+    dg::host_block_retain(t->flight->pinned);
+    *block = t->flight->pinned;
+    return DG_OK;
+}
+
 extern "C" int dg_release(dg_feeder* f, dg_ticket id) {
     if (!f) return set_error(DG_E_INVALID, "NULL feeder");
     std::lock_guard<std::mutex> lock(f->mu);
@@ -381,7 +373,6 @@ extern "C" void dg_feeder_destroy(dg_feeder* f) {
     cudaSetDevice(f->device);
     for (auto& l : f->lanes) {
         bury(*l);
-        for (PinnedBuf& p : l->pinned) if (p.ptr) cudaFreeHost(p.ptr);
         dg_ctx_destroy(l->ctx);
     }
     delete f;

@@ -7,6 +7,7 @@
 // counts as one of them.  One job runs at a time: a caller that finds the pool busy does its work on its own thread.
 #pragma once
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <cstdlib>
 #include <functional>
@@ -25,6 +26,7 @@ public:
     int threads() const { return (int)workers_.size() + 1; }
 
     // Calls fn(i) for every i in [0, n); returns when all calls have returned.  grain: fewest items worth a hand-over.
+    // The caller works too and does not wait for workers that have not woken up by the time everything is taken.
     void run(size_t n, const std::function<void(size_t)>& fn, size_t grain = 64) {
         if (n == 0) return;
         if (workers_.empty() || n < 2 * grain || !job_mu_.try_lock()) {
@@ -38,15 +40,14 @@ public:
             total_ = n;
             chunk_ = (n + parts - 1) / parts;
             next_.store(0);
-            busy_ = (int)workers_.size();
-            ++generation_;
+            generation_.fetch_add(1);
         }
         cv_work_.notify_all();
-        drain();
+        drain(fn);
         {
             std::unique_lock<std::mutex> lock(mu_);
-            cv_done_.wait(lock, [&] { return busy_ == 0; });
-            fn_ = nullptr;
+            fn_ = nullptr;  // nobody joins any more
+            cv_done_.wait(lock, [&] { return inside_ == 0; });
         }
         job_mu_.unlock();
     }
@@ -64,26 +65,38 @@ private:
         for (int i = 1; i < std::min(want, 64); ++i) workers_.emplace_back([this] { loop(); });
         for (auto& t : workers_) t.detach();
     }
-    void drain() {
+    void drain(const std::function<void(size_t)>& fn) {
         for (;;) {
             const size_t a = next_.fetch_add(chunk_);
             if (a >= total_) return;
             const size_t b = std::min(total_, a + chunk_);
-            for (size_t i = a; i < b; ++i) (*fn_)(i);
+            for (size_t i = a; i < b; ++i) fn(i);
         }
     }
     void loop() {
         uint64_t seen = 0;
         for (;;) {
+            // The phases of planning a batch follow one another within tens of microseconds, and waking a sleeping thread
+            // takes as long as most of them: look out for the next one a little before going to sleep.
+            const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(60);
+            while (generation_.load(std::memory_order_relaxed) == seen && std::chrono::steady_clock::now() < until) {
+#if defined(__x86_64__)
+                __builtin_ia32_pause();
+#endif
+            }
+            const std::function<void(size_t)>* fn;
             {
                 std::unique_lock<std::mutex> lock(mu_);
-                cv_work_.wait(lock, [&] { return generation_ != seen; });
-                seen = generation_;
+                cv_work_.wait(lock, [&] { return generation_.load() != seen; });
+                seen = generation_.load();
+                fn = fn_;
+                if (!fn) continue;  // that one is over already
+                ++inside_;
             }
-            drain();
+            drain(*fn);
             {
-                std::lock_guard<std::mutex> lock(mu_);
-                if (--busy_ == 0) cv_done_.notify_all();
+                std::unique_lock<std::mutex> lock(mu_);
+                if (--inside_ == 0) cv_done_.notify_all();
             }
         }
     }
@@ -94,8 +107,8 @@ private:
     const std::function<void(size_t)>* fn_ = nullptr;
     std::atomic<size_t> next_{0};
     size_t total_ = 0, chunk_ = 1;
-    int busy_ = 0;
-    uint64_t generation_ = 0;
+    int inside_ = 0;  // workers at work on the current job
+    std::atomic<uint64_t> generation_{0};
 };
 
 }  // namespace dg

@@ -508,6 +508,7 @@ __global__ void __launch_bounds__(T) k_huff_sync(JpegWave w, uint32_t first) {
         const bool ended = p == kNoState;
         uint32_t wr = ended ? 0u : p >> 7;
         SyncLane L;
+        L.p = p;
         auto fetch = [&]() {
             copy16(ring + (wr & 7u) * 16, us + (size_t)wr * 16);
             if ((wr & 7u) == 0) copy16(ring + 128, us + (size_t)wr * 16);

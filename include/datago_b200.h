@@ -212,6 +212,7 @@ DG_API int dg_batch_download_packed(dg_batch* b, uint8_t* host_base, uint64_t ca
 DG_API uint64_t dg_batch_packed_bytes(const dg_batch* b);
 DG_API int dg_batch_sync(dg_batch* b);
 DG_API int dg_batch_result(const dg_batch* b, int i, dg_result* out);
+DG_API int dg_batch_results(const dg_batch* b, dg_result* out); /* all of them: out has room for the batch's n items */
 /* Buckets of a DG_BATCH_COLLATE batch, in order of first appearance.  Items that dg_batch_create rejected (bad header
  * or tables, unknown key, too large) belong to no bucket.  An item whose entropy-coded data turns out to be damaged is
  * only found on the device: it keeps its slot, the slot's pixels are undefined and its dg_result.status is non-zero
@@ -280,6 +281,10 @@ DG_API int dg_fetch(dg_feeder* f, dg_ticket ticket, uint8_t* host_out, uint64_t 
 /* The payload where the feeder's own device -> host copy left it (page-locked host memory of the library), valid until
  * dg_release: lets a caller consume the pixels without a second host copy. */
 DG_API int dg_peek(dg_feeder* f, dg_ticket ticket, const uint8_t** host_data);
+/* Like dg_peek, for a caller that keeps the pixels: *host_data stays valid after dg_release and after the feeder is gone, until
+ * the caller hands *block to dg_host_release.  DG_E_TOO_LARGE while too much page-locked memory is held this way (see
+ * dg_host_alloc): copy with dg_fetch instead. */
+DG_API int dg_fetch_view(dg_feeder* f, dg_ticket ticket, const uint8_t** host_data, void** block);
 DG_API int dg_release(dg_feeder* f, dg_ticket ticket);
 DG_API int dg_feeder_get_stats(dg_feeder* f, dg_feeder_stats* out);
 /* Stops the lanes, fails what is still queued, frees everything (device payloads of unreleased tickets included).
@@ -305,6 +310,13 @@ DG_API void dg_feeder_destroy(dg_feeder* f);
  * on one ctx are serialised and the function returns after its work has completed. */
 DG_API int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, uint32_t w, uint32_t h, uint32_t channels,
                             const char* forced_key, uint8_t* device_dst, dg_plan* plan_out);
+
+/* Page-locked host memory for dg_batch_download_packed (or any other use), from a pool the process shares: blocks that have
+ * been released are reused, because page-locking is slow and a fresh pageable buffer costs a page fault per 4 KB.  Idle
+ * blocks beyond DATAGO_B200_HOST_BLOCKS_MB (default 1024) are freed, and so are all of them with the last context.
+ * DG_E_TOO_LARGE while more than the same amount is in use: fall back to ordinary memory.  Thread-safe. */
+DG_API int dg_host_alloc(uint64_t nbytes, void** out);
+DG_API void dg_host_release(void* block);
 
 /* Device -> host copy helper for callers without a CUDA binding (tests). */
 DG_API int dg_copy_to_host(dg_ctx* ctx, void* dst, const void* device_src, uint64_t nbytes);
