@@ -822,7 +822,6 @@ static void plan_resize(Planner& pl, WavePlan& wv, const dg_plan& p, uint32_t C,
                 if (!encode_source_map_v(cp, src_rows)) pl.tmap_failed = true;
             }
         }
-        cp.tiles_x = conv_tiles_x(cp, !horizontal);
         wv.passes[stage].push_back(cp);
         ++done;
     };
@@ -1290,6 +1289,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
                 wv.pass_first[s].push_back(0);
                 std::stable_partition(wv.passes[s].begin(), wv.passes[s].end(), [](const ConvPass& cp) { return cp.fast == 2; });
                 wv.mma_tiles[s] = 0;
+                cut_pass_tiles(wv.passes[s].data(), wv.passes[s].size(), (s & 1) != 0);
                 for (ConvPass& cp : wv.passes[s]) {
                     cp.tile_first = t;
                     t += conv_tiles(cp, (s & 1) != 0);
@@ -1929,6 +1929,7 @@ extern "C" int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, u
     for (int s = 0; s < 4; ++s) {
         uint32_t t = 0;
         wv.pass_first[s].push_back(0);
+        cut_pass_tiles(wv.passes[s].data(), wv.passes[s].size(), (s & 1) != 0);
         for (ConvPass& cp : wv.passes[s]) {  // at most one pass per stage here, so the tensor-core passes trivially come first
             cp.tile_first = t;
             t += conv_tiles(cp, (s & 1) != 0);

@@ -82,6 +82,8 @@ struct ConvPass {
     uint32_t fast;                  // vertical: 1 = the vectorised path applies; 2 (both directions) = the tensor-core path (see kernels_resize.cu)
     uint32_t box_pieces;            // tensor-core path, horizontal: 16-byte pieces per staged source row (odd), the width of the tensor map's
                                     // box; vertical: rows of a box | boxes per chunk << 16
+    uint32_t cta_chunks;            // tensor-core path: chunks a CTA walks (horizontal: of 32 rows, vertical: of 64 bytes of a row)
+    uint32_t pad;
     // Set when `src` is memory the library does not own (no slack behind it): the horizontal pass then loads no byte
     // outside [guard_lo, guard_hi).  Both null for sources inside the library's own padded arenas.
     const uint8_t* guard_lo;

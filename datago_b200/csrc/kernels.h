@@ -108,22 +108,46 @@ constexpr uint32_t kConvTileW = 64, kConvTileH = 16;    // horizontal pass: outp
 constexpr uint32_t kVTileBytes = 256, kVTileH = 4;      // vertical pass, plain path: output bytes x rows per CTA
 constexpr uint32_t kVFastBytes = 1024, kVFastRows = 32; // vertical pass, vector path: 64 x 16-byte columns, 4 x 8 rows
 constexpr uint32_t kVFastMaxWindow = 128;
-// horizontal pass on the tensor cores (ConvPass::fast == 2): output bytes per strip x rows per CTA; limits of what a CTA
+// horizontal pass on the tensor cores (ConvPass::fast == 2): output bytes per strip x rows per chunk; limits of what a CTA
 // can stage -- source bytes under one 8-byte output tile, and under a whole strip
-constexpr uint32_t kHMmaStrip = 64, kHMmaRows = 2048, kHMmaMaxBand = 256, kHMmaMaxSpan = 1008;  // span: 63 pieces of 16 bytes = 252 words, inside the 256 elements a tensor-map box may have
-// vertical pass on the tensor cores (ConvPass::fast == 2): output rows x bytes of a row per CTA; limits of what a CTA can
+constexpr uint32_t kHMmaStrip = 64, kHMmaChunk = 32, kHMmaMaxBand = 256, kHMmaMaxSpan = 1008;  // span: 63 pieces of 16 bytes = 252 words, inside the 256 elements a tensor-map box may have
+// vertical pass on the tensor cores (ConvPass::fast == 2): output rows per CTA x bytes of a row per chunk; limits of what a CTA can
 // stage -- source rows under the eight output rows of one warp, and under all rows of the CTA
-constexpr uint32_t kVMmaRows = 64, kVMmaCols = 4096, kVMmaMaxBand = 256, kVMmaMaxSpan = 704;
+constexpr uint32_t kVMmaRows = 64, kVMmaChunk = 64, kVMmaMaxBand = 256, kVMmaMaxSpan = 704;
 inline uint32_t conv_tiles_x(const ConvPass& p, bool vertical) {
     if (!vertical && p.fast == 2) return (p.out_w * p.channels + kHMmaStrip - 1) / kHMmaStrip;
-    if (vertical && p.fast == 2) return (p.out_w * p.channels + kVMmaCols - 1) / kVMmaCols;
+    if (vertical && p.fast == 2) return (p.out_w * p.channels + p.cta_chunks * kVMmaChunk - 1) / (p.cta_chunks * kVMmaChunk);
     if (!vertical) return (p.out_w + kConvTileW - 1) / kConvTileW;
     const uint32_t row_bytes = p.out_w * p.channels;
     return p.fast ? (row_bytes + kVFastBytes - 1) / kVFastBytes : (row_bytes + kVTileBytes - 1) / kVTileBytes;
 }
 inline uint32_t conv_tiles(const ConvPass& p, bool vertical) {
-    const uint32_t rows = !vertical ? (p.fast == 2 ? kHMmaRows : kConvTileH) : p.fast == 2 ? kVMmaRows : p.fast ? kVFastRows : kVTileH;
+    const uint32_t rows = !vertical ? (p.fast == 2 ? p.cta_chunks * kHMmaChunk : kConvTileH) : p.fast == 2 ? kVMmaRows : p.fast ? kVFastRows : kVTileH;
     return conv_tiles_x(p, vertical) * ((p.out_h + rows - 1) / rows);
+}
+// Cuts the passes of one stage into CTA tiles.  A CTA of a tensor-core pass first gathers its weights and then walks
+// chunks: two CTAs per resident place of the chip keep its SMs evenly busy to the end, one per place is better where that
+// leaves a CTA only a few chunks, and two chunks are the least a CTA gets.  (One image of 1.5 Mpixel: horizontal pass 20.6 us
+// at four CTAs per place, 15.7 at two, 10.9 at one; 48 images of 5 Mpixel: 275, 253, 252 us, and 268 with CTAs of 2048 rows.)
+constexpr uint32_t kMmaMinChunks = 2, kMmaFewChunks = 4, kMmaMaxChunks = 64;
+inline void cut_pass_tiles(ConvPass* passes, size_t n, bool vertical) {
+    uint64_t work = 0;  // chunks of all CTAs together
+    auto rows_of_ctas = [&](const ConvPass& p) -> uint64_t { return vertical ? (p.out_h + kVMmaRows - 1) / kVMmaRows : (p.out_w * p.channels + kHMmaStrip - 1) / kHMmaStrip; };
+    auto chunks_of = [&](const ConvPass& p) -> uint64_t { return vertical ? (p.out_w * p.channels + kVMmaChunk - 1) / kVMmaChunk : (p.out_h + kHMmaChunk - 1) / kHMmaChunk; };
+    for (size_t i = 0; i < n; ++i)
+        if (passes[i].fast == 2) work += rows_of_ctas(passes[i]) * chunks_of(passes[i]);
+    const uint64_t places = 148 * (vertical ? 2 : 3), one = (work + places - 1) / places;
+    uint64_t chunks = (one + 1) / 2;
+    if (chunks < kMmaFewChunks) chunks = one < kMmaFewChunks ? one : kMmaFewChunks;
+    chunks = chunks < kMmaMinChunks ? kMmaMinChunks : chunks > kMmaMaxChunks ? kMmaMaxChunks : chunks;
+    for (size_t i = 0; i < n; ++i) {
+        ConvPass& p = passes[i];
+        if (p.fast == 2) {  // as few CTAs as that gives, as equal as they get
+            const uint64_t all = chunks_of(p), ctas = (all + chunks - 1) / chunks;
+            p.cta_chunks = (uint32_t)((all + ctas - 1) / ctas);
+        }
+        p.tiles_x = conv_tiles_x(p, vertical);
+    }
 }
 constexpr uint32_t kCopyTileBytes = 4096;
 

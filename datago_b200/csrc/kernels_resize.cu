@@ -143,7 +143,7 @@ __device__ __forceinline__ void conv_h_rows(const ConvPass& p, const Table& tb, 
 // pixel x when k % C == c and zero otherwise.  The 16-bit weights are split into a signed high and an unsigned low
 // byte, w = 256 hi + lo, so that the product runs on the 8-bit integer tensor-core path with 32-bit accumulation:
 // out = 256 (src x hi) + (src x lo), which is exact -- the result equals the dp2a kernel's bit for bit.
-//   CTA  = one strip of 64 output bytes x up to 2048 rows of one pass; warp q of the first eight owns output bytes
+//   CTA  = one strip of 64 output bytes x some chunks of 32 rows of one pass (see cut_pass_tiles); warp q of the first eight owns output bytes
 //          8q .. 8q+7 of the strip, one thread of a ninth warp issues the copies.
 //   B    = the warp's slice of Wt (source bytes under its eight outputs, at most 256), both limbs: every lane gathers its
 //          mma.m16n8k32 fragments from the filter table once and keeps them in registers for all rows of the CTA;
@@ -160,7 +160,6 @@ __device__ __forceinline__ void conv_h_rows(const ConvPass& p, const Table& tb, 
 constexpr int kHMmaConsumers = 256;   // eight warps multiply
 constexpr int kHMmaProducers = 32;    // one more warp, of which one thread issues the copies into the ring
 constexpr int kHMmaThreads = kHMmaConsumers + kHMmaProducers;
-constexpr int kHMmaChunk = 32;                       // rows per chunk (two mma row tiles)
 #ifndef DG_HMMA_CTAS
 #define DG_HMMA_CTAS 3
 #endif
@@ -235,7 +234,7 @@ __global__ void __launch_bounds__(kHMmaThreads, kHMmaCtasPerSm) k_conv_h_mma(con
     const uint32_t row_bytes = out_w * C;
     const uint32_t j0 = tx * kHMmaStrip;                          // first output byte of the strip
     const uint32_t jn0 = j0 + warp * 8;                           // ... of this warp's tile
-    const uint32_t y_first = ty * kHMmaRows, y_end = min(out_h, y_first + kHMmaRows);
+    const uint32_t cta_rows = pg.cta_chunks * kHMmaChunk, y_first = ty * cta_rows, y_end = min(out_h, y_first + cta_rows);
     // first source byte of the strip, from the start of a source row of the pass (a multiple of 16)
     const uint32_t xs0 = j0 / C;
     const int32_t strip_lo = ((__ldg(tb.start + t0 + xs0) - origin) * (int32_t)C) & ~15;
@@ -595,7 +594,7 @@ __device__ __forceinline__ void conv_v_vector(const ConvPass& p, const Table& tb
 // ---- vertical pass on the tensor cores --------------------------------------------------------------------------------
 // out[y][x] = sum_k w[y][k] * src[k][x] as a matrix product with the image's columns as the M dimension, the output rows
 // as N and the source rows as K, on the same 8-bit path with the weights split into two limbs as in the horizontal pass.
-//   CTA  = 64 output rows (warp q of the first eight owns rows 8q .. 8q+7) x up to 4096 bytes of the rows, walked in chunks
+//   CTA  = 64 output rows (warp q of the first eight owns rows 8q .. 8q+7) x some chunks (see cut_pass_tiles)
 //          of 64 bytes (four tiles of 16 columns); one thread of a ninth warp issues the copies.
 //   B    = the warp's weights (eight output rows x the source rows under them, at most 256), both limbs, gathered once
 //          into registers.
@@ -609,7 +608,6 @@ __device__ __forceinline__ void conv_v_vector(const ConvPass& p, const Table& tb
 //   D    = 16 columns x 8 rows per tile: merged, rounded, saturated, collected per warp as 8 rows x 64 bytes in shared
 //          memory and stored as 16 bytes per lane.
 constexpr int kVMmaConsumers = 256, kVMmaThreads = kVMmaConsumers + 32;
-constexpr int kVMmaChunk = 64;            // bytes of a row per chunk
 constexpr int kVMmaRing = 98304;          // bytes of the ring: two CTAs per SM
 constexpr int kVMmaRingSlack = 2048;      // a warp's last k step reads up to 31 rows past the staged ones (zero weights)
 constexpr int kVMmaMaxStages = 8;
@@ -636,7 +634,7 @@ __global__ void __launch_bounds__(kVMmaThreads, 2) k_conv_v_mma(const ConvPass* 
     const uint32_t ty = tile / tiles_x, tx = tile - ty * tiles_x;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t y0 = ty * kVMmaRows, yw = y0 + warp * 8;
-    const uint32_t x_first = tx * kVMmaCols, x_end = min(row_bytes, x_first + kVMmaCols);
+    const uint32_t cta_cols = pg.cta_chunks * kVMmaChunk, x_first = tx * cta_cols, x_end = min(row_bytes, x_first + cta_cols);
     const uint32_t nchunks = (x_end - x_first + kVMmaChunk - 1) / kVMmaChunk;
     // first source row under the CTA's output rows (row 0 = the first row of the pass's source)
     const int32_t r_lo = __ldg(tb.start + t0 + y0) - origin;
