@@ -169,7 +169,7 @@ struct dg_ctx {
     cudaStream_t stream2 = nullptr;  // odd waves of a batch run here, concurrently with the even ones
     cudaStream_t aux[2] = {nullptr, nullptr};  // per lane: the restart-interval decoder runs beside the speculative one
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    cudaEvent_t ev_aux_go[2] = {nullptr, nullptr}, ev_aux_huge[2] = {nullptr, nullptr}, ev_aux_done[2] = {nullptr, nullptr};
+    cudaEvent_t ev_aux_go[2] = {nullptr, nullptr}, ev_aux_done[2] = {nullptr, nullptr};
     bool own_stream = false;
     bool has_tfm = false;
     dg_image_config cfg{};
@@ -244,8 +244,6 @@ static int ctx_create(int device, const dg_image_config* cfg, void* stream, bool
         cudaStreamCreateWithFlags(&c->aux[1], cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_aux_go[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_aux_go[1], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_aux_huge[0], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_aux_huge[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_aux_done[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_aux_done[1], cudaEventDisableTiming) != cudaSuccess) {
         delete c;
@@ -279,7 +277,6 @@ extern "C" void dg_ctx_destroy(dg_ctx* c) {
     for (int i = 0; i < 2; ++i) {
         cudaStreamSynchronize(c->aux[i]);
         cudaEventDestroy(c->ev_aux_go[i]);
-        cudaEventDestroy(c->ev_aux_huge[i]);
         cudaEventDestroy(c->ev_aux_done[i]);
         cudaStreamDestroy(c->aux[i]);
     }
@@ -420,9 +417,10 @@ struct ItemPlan {
 struct WavePlan {
     int first_item = 0, last_item = 0;  // [first, last)
     std::vector<JpegDesc> descs;
-    std::vector<uint32_t> tile_first, spec_list, write_first, dc_first, restart_list, restart_first, block_first, color_first;
+    std::vector<uint32_t> tile_first, spec_list, guess_first, write_first, dc_first, restart_list, restart_first, block_first, color_first;
     std::vector<std::array<uint32_t, 2>> pairs;  // (DC, AC) pairs of Huffman tables in use
     std::map<std::array<uint32_t, 2>, uint32_t> pair_ids;
+    uint32_t guess_span = 1;                     // cells a thread of the synchronising decoder goes through
     uint32_t max_pairs = 1;                      // most distinct ones in one image
     uint32_t pair_id(uint32_t dc, uint32_t ac) {
         const std::array<uint32_t, 2> key{dc, ac};
@@ -435,7 +433,6 @@ struct WavePlan {
     // descs [fused_first, descs.size()) take the fused 4:2:0 path: prefix sums of their chroma blocks and tiles, and
     // their own launch groups (first chroma block, count, first tile, count)
     uint32_t fused_first = 0;
-    uint32_t n_huge = 0;  // leading entries of spec_list (sorted longest first) with more than kSpecHugeBytes of entropy-coded data
     std::vector<uint32_t> fchroma_first, ftile_first;
     std::vector<std::array<uint32_t, 4>> fgroups;
     std::vector<ConvPass> passes[4];    // H1, V1, H2, V2
@@ -450,10 +447,10 @@ struct WavePlan {
     std::vector<uint32_t> alpha_first[4];
     // scratch layout (bytes from the wave scratch base)
     size_t us_bytes = 0, coef_blocks = 0, plane_bytes = 0, decoded_bytes = 0, mid_bytes = 0, nseg = 0, cells = 0;
-    size_t off_us = 0, off_uslen = 0, off_segstart = 0, off_segfound = 0, off_tiles = 0, off_codes = 0, off_cells = 0, off_diff = 0, off_info = 0, off_coef = 0, off_planes = 0, off_decoded = 0, off_mid = 0, total = 0;
+    size_t off_us = 0, off_uslen = 0, off_segstart = 0, off_segfound = 0, off_tiles = 0, off_codes = 0, off_cells = 0, off_cand = 0, off_diff = 0, off_info = 0, off_coef = 0, off_planes = 0, off_decoded = 0, off_mid = 0, total = 0;
     // meta offsets
     size_t m_descs = 0, m_pairs = 0, m_spec = 0, m_restart_list = 0, m_passes[4] = {0, 0, 0, 0}, m_copies = 0, m_torgbs = 0, m_alphas[4] = {0, 0, 0, 0};
-    OwnerMapOff m_tiles, m_write, m_dc, m_restart, m_blocks, m_color, m_fchroma, m_ftile, m_pass[4], m_copy, m_torgb, m_alpha[4];
+    OwnerMapOff m_tiles, m_guess, m_write, m_dc, m_restart, m_blocks, m_color, m_fchroma, m_ftile, m_pass[4], m_copy, m_torgb, m_alpha[4];
 };
 
 struct StageEvent { int stage; cudaEvent_t a, b; };
@@ -1104,6 +1101,13 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         for (int pass = 0; pass < 2; ++pass)
             for (size_t k = 0; k < built.size(); ++k)
                 if ((int)(ctx->fused_path && fused_decode(built[k].ncomp, built[k].hs, built[k].vs, built[k].width)) == pass) order.push_back(k);
+        // With a thread per cell and block of the MCU the synchronising decoder's threads fit the chip at once: the shortest
+        // way for every thread.  Beyond that, less work in all counts more (256 files, 1.2 Gbit: 817 us with spans of four
+        // cells, 1005 with single ones; 8 files of 4:4:4, 34 Mbit: 94 and 52 us).
+        uint64_t guess_bits = 0;
+        for (const JpegDesc& d : built)
+            if (!d.restart) guess_bits += (uint64_t)d.raw_len * 8 * d.bpm;
+        wv.guess_span = guess_bits / kCellBits > kGuessSpanThreads ? kGuessSpan : 1;
         uint32_t color_total = 0, restart_total = 0, fchroma_total = 0, ftile_total = 0;
         size_t group_bytes = 0, fgroup_bytes = 0;
         wv.block_first.push_back(0);
@@ -1175,16 +1179,16 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         // longest streams first: one CTA decodes one image, and the launch ends with its slowest CTA
         std::stable_sort(wv.spec_list.begin(), wv.spec_list.end(),
                          [&](uint32_t a, uint32_t c) { return wv.descs[a].raw_len > wv.descs[c].raw_len; });
+        wv.guess_first.assign(1, 0);
         wv.write_first.assign(1, 0);
         wv.dc_first.assign(1, 0);
         for (uint32_t k : wv.spec_list) {
             const JpegDesc& d = wv.descs[k];
+            const uint32_t guess_step = guess_spans(d.bpm, wv.guess_span) * wv.guess_span;
+            wv.guess_first.push_back(wv.guess_first.back() + (stream_cells(d.raw_len) + guess_step - 1) / guess_step);
             wv.write_first.push_back(wv.write_first.back() + (stream_cells(d.raw_len) + kCellsPerCta - 1) / kCellsPerCta);
             wv.dc_first.push_back(wv.dc_first.back() + (d.mcux * d.mcuy + kDcMcus - 1) / kDcMcus);
         }
-        wv.n_huge = 0;
-        // (at most kSpecHugeMax of them: one such CTA fills an SM, so they trade throughput for a shorter critical path)
-        while (wv.n_huge < wv.spec_list.size() && wv.n_huge < kSpecHugeMax && wv.descs[wv.spec_list[wv.n_huge]].raw_len > kSpecHugeBytes) ++wv.n_huge;
         wv.us_bytes = us; wv.coef_blocks = blocks; wv.plane_bytes = planes; wv.decoded_bytes = decoded; wv.mid_bytes = mids; wv.nseg = segs; wv.cells = cells;
         size_t o = 0;
         wv.off_coef = o; o += align_up(blocks * 128, 256);
@@ -1200,6 +1204,8 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         wv.off_planes = o; o += align_up(planes, 256);
         wv.off_decoded = o; o += align_up(decoded, 256);
         wv.off_mid = o; o += align_up(mids, 256);
+        // the candidate states are gone before anything behind off_planes is written
+        wv.off_cand = wv.off_planes; o = std::max(o, wv.off_cand + align_up(cells * kCandidates * sizeof(uint2), 256));
         wv.total = o;
         scratch_max = std::max(scratch_max, o);
     }
@@ -1331,6 +1337,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             wv.m_spec = m.put(wv.spec_list);
             wv.m_restart_list = m.put(wv.restart_list);
             wv.m_tiles = put_owner_map(m, wv.tile_first);
+            wv.m_guess = put_owner_map(m, wv.guess_first);
             wv.m_write = put_owner_map(m, wv.write_first);
             wv.m_dc = put_owner_map(m, wv.dc_first);
             wv.m_restart = put_owner_map(m, wv.restart_first);
@@ -1516,6 +1523,7 @@ static int batch_run_locked(dg_batch* b) {
             w.seg_start = (uint32_t*)(sc + wv.off_segstart);
             w.seg_found = (uint32_t*)(sc + wv.off_segfound);
             w.cells = (uint2*)(sc + wv.off_cells);
+            w.cand = (uint2*)(sc + wv.off_cand);
             w.coef = (int16_t*)(sc + wv.off_coef);
             w.diff = (uint32_t*)(sc + wv.off_diff);
             w.info = (uint32_t*)(sc + wv.off_info);
@@ -1533,6 +1541,8 @@ static int batch_run_locked(dg_batch* b) {
             w.n_spec = (uint32_t)wv.spec_list.size();
             w.restart_list = (const uint32_t*)(meta + wv.m_restart_list);
             w.restart_ctas = resolve(b, wv.m_restart);
+            w.guess_span = wv.guess_span;
+            w.guess_ctas = resolve(b, wv.m_guess);
             w.write_ctas = resolve(b, wv.m_write);
             w.dc_ctas = resolve(b, wv.m_dc);
             w.blocks = resolve(b, wv.m_blocks);
@@ -1544,38 +1554,26 @@ static int batch_run_locked(dg_batch* b) {
             launch_unstuff(w, s);
             b->launches += 2;
             CU(mark(DG_STAGE_UNSTUFF, false));
-            // The auxiliary stream of the lane takes what can run beside the speculative decoder: its widest CTAs for the few
-            // longest images of the wave (also in a timing batch: the two launches are one stage), and outside timing mode
-            // the restart-interval decoder, which works on other images.
-            const uint32_t n_huge = wv.n_huge;
+            // The auxiliary stream of the lane takes the restart-interval decoder, which works on other images, beside the
+            // speculative one (not in a timing batch).
             const bool aux_restart = !timing && w.restart_ctas.total && w.n_spec;
-            const bool aux_huge = n_huge && w.n_spec > n_huge;
             const int lane = (int)(wi & 1);
             cudaStream_t aux = ctx->aux[lane];
-            if (w.n_spec) {  // the longest images first: they decide when the stage ends
+            if (w.n_spec) {
                 CU(mark(DG_STAGE_HUFF_SPEC, true));
-                if (aux_restart || aux_huge) {
+                if (aux_restart) {
                     CU(cudaEventRecord(ctx->ev_aux_go[lane], s));
                     CU(cudaStreamWaitEvent(aux, ctx->ev_aux_go[lane], 0));
                 }
-                auto cells_of = [&](uint32_t k) { return stream_cells(wv.descs[wv.spec_list[k]].raw_len); };
-                if (n_huge) {
-                    launch_huff_sync(w, 0, n_huge, cells_of(0), true, aux_huge ? aux : s);
-                    ++b->launches;
-                    if (aux_huge) CU(cudaEventRecord(ctx->ev_aux_huge[lane], aux));
-                }
-                if (w.n_spec > n_huge) {
-                    launch_huff_sync(w, n_huge, w.n_spec - n_huge, cells_of(n_huge), false, s);
-                    ++b->launches;
-                }
+                launch_huff_guess(w, s);
+                launch_huff_chain(w, s);
                 if (aux_restart) {
                     launch_huff_restart(w, aux);
                     ++b->launches;
                     CU(cudaEventRecord(ctx->ev_aux_done[lane], aux));
                 }
-                if (aux_huge) CU(cudaStreamWaitEvent(s, ctx->ev_aux_huge[lane], 0));
                 launch_huff_write(w, s);
-                b->launches += 2;
+                b->launches += 4;
                 CU(mark(DG_STAGE_HUFF_SPEC, false));
                 if (aux_restart) CU(cudaStreamWaitEvent(s, ctx->ev_aux_done[lane], 0));
             }

@@ -16,8 +16,20 @@ struct OwnerMap {
 
 // ---- entropy decoding: work splits (see kernels_huff.cu) ------------------------------------------------------------------
 constexpr uint32_t kUnstuffTile = 4096;  // bytes of an entropy-coded segment per CTA of the unstuffing kernels
-constexpr uint32_t kCellBits = 1024;     // bits of an unstuffed stream per thread of the value decoder
+constexpr int kCellBits = 1024;          // bits of an unstuffed stream per thread of the value decoder
 constexpr uint32_t kCellsPerCta = 128, kSegsPerCta = 128;
+// synchronising decoder: threads per CTA, the entries of the candidate array per cell, and the cells of a span once a thread
+// per cell and block of the MCU would be more than the chip holds at once
+constexpr uint32_t kGuessLanes = 384, kCandidates = 6, kGuessSpan = 4;
+constexpr uint64_t kGuessSpanThreads = 148 * 2048;
+// spans of cells a CTA takes, each with a thread per block of the MCU: what the threads allow, 256 staged cells at most
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline uint32_t guess_spans(uint32_t bpm, uint32_t span) {
+    const uint32_t lanes = kGuessLanes / bpm, stage = span == 1 ? 128u : 256u / span;
+    return lanes < stage ? lanes : stage;
+}
 constexpr uint32_t kDcMcus = 8192;       // MCUs per CTA of the DC prediction
 constexpr uint32_t kCodeTablesBytes = 20544;  // look-up tables of one (DC, AC) pair of Huffman tables
 constexpr uint32_t kStreamPad = 512;     // bytes behind an image's unstuffed stream that the bit readers may touch
@@ -41,6 +53,8 @@ struct JpegWave {
     uint32_t* seg_start;     // restart-segment starts (bytes into the image's unstuffed stream)
     uint32_t* seg_found;     // [n] segments actually present
     uint2* cells;            // per cell of a restart-free stream: bit position of its first block, index of that block
+    uint2* cand;             // [cells][kCandidates] entry state | exit state << 16, blocks that start in the cell (see k_huff_guess);
+                             // lies over what is written after the entropy stage
     int16_t* coef;           // [blocks][64], scan order, natural order inside a block; AC terms, rows the class covers
     uint32_t* diff;          // [blocks] restart-free images: DC difference | class << 16
     uint32_t* info;          // [blocks] DC coefficient (low half) | class << 16
@@ -53,10 +67,11 @@ struct JpegWave {
     uint8_t* codes;          // [n_pairs] look-up tables made from them, kCodeTablesBytes each
     uint32_t max_pairs;      // most distinct pairs one image of the wave uses
     const uint32_t* qt32;    // quantisation pool, 32 words per table: word i holds q[2i] in byte 0 and q[2i+1] in byte 3
-    // restart-free images of this wave, longest first; CTAs of the value decoder and of the DC prediction: owner = index
-    // into spec_list
+    // restart-free images of this wave, longest first; CTAs of the synchronising decoder, the value decoder and the DC
+    // prediction: owner = index into spec_list
     const uint32_t* spec_list; uint32_t n_spec;
-    OwnerMap write_ctas, dc_ctas;
+    OwnerMap guess_ctas, write_ctas, dc_ctas;
+    uint32_t guess_span;     // cells a thread of the synchronising decoder goes through
     // restart-interval images: kSegsPerCta segments per CTA, owner = index into restart_list
     OwnerMap restart_ctas;
     const uint32_t* restart_list;
@@ -72,11 +87,9 @@ struct JpegWave {
 
 void launch_unstuff(const JpegWave& w, cudaStream_t s);
 void launch_huff_restart(const JpegWave& w, cudaStream_t s);
-// images [first, first + count) of spec_list.  The leading ones with more than kSpecHugeBytes of entropy-coded data get the
-// widest CTAs, beside the others on another stream.
-constexpr uint32_t kSpecHugeBytes = 1024 * 2048 / 8, kSpecHugeMax = 64;
-void launch_huff_sync(const JpegWave& w, uint32_t first, uint32_t count, uint32_t longest_cells, bool widest, cudaStream_t s);
-void launch_huff_write(const JpegWave& w, cudaStream_t s);  // all restart-free images, once launch_huff_sync has covered them
+void launch_huff_guess(const JpegWave& w, cudaStream_t s);
+void launch_huff_chain(const JpegWave& w, cudaStream_t s);
+void launch_huff_write(const JpegWave& w, cudaStream_t s);  // all restart-free images, once launch_huff_chain has covered them
 void launch_whole_blocks(const JpegWave& w, uint32_t nblocks, cudaStream_t s);
 // blocks [first, first + count) of the wave / colour tiles [first, first + count): callers may launch them in groups of
 // images (the planes written by the IDCT are then still in L2 when the colour kernel reads them) or once per wave

@@ -8,15 +8,11 @@
 // qualities half of the blocks or more carry a handful of low-frequency coefficients or none, so keeping the DC terms
 // dense and skipping the rows that hold nothing is worth several times the memory traffic of whole blocks, and nothing has
 // to be zeroed before or after.
-#include <cooperative_groups.h>
-
 #include <cstddef>
 #include <cstdint>
 #include <mutex>
 
 #include "kernels.h"
-
-namespace cg = cooperative_groups;
 
 namespace dg {
 
@@ -82,7 +78,9 @@ __device__ __forceinline__ uint32_t advance_of(uint32_t symbol, bool is_ac) {  /
 // Look-up tables of the two decoders for one (DC, AC) pair of Huffman tables, made on the device (k_unstuff_count), because
 // they are several times the size of what the host sends.  Codes longer than the index: entry 0, and far[] takes over --
 // canonical codes grow with their length, so all of them lie above far_base, and the 16-bit windows from there on are few
-// (190 to 640 for the tables most files carry).  Windows behind the end of far[] go to the host's table.
+// (190 to 640 for the tables most files carry).  One comparison with far_base picks the array, so that a long code costs no
+// second look-up and no branch: some lane of a warp has one in nearly every step (see entry_at).  Windows behind the end
+// of far[], whose last entry is 0, go to the host's table.
 constexpr int kSyncBits = 10, kValueBits = 9;
 // Synchronising decoder: as many whole symbols as the index shows.  bits 0-4 / 5-11: bits consumed and slots advanced by the
 // first symbol alone, 12-16 / 17-23: by all of them, 24-29: slots before the last one (the last counts only if that many do
@@ -139,13 +137,13 @@ __device__ void build_tables(CodeTables& out, const HuffTable* pool, uint32_t dc
         static_assert(kValueBits == kLutBits && kSyncBits == 10, "limit[0] covers ten bits");
         for (uint32_t i = tid; i < sizeof(st.far) / 4; i += nthreads) {
             const uint32_t c = code_at(t, min(sbase + i, 0xFFFFu));
-            st.far[i] = sync_entry((c & 31u) + ((c >> 8) & 15u), advance_of((c >> 8) & 255u, side != 0));
+            st.far[i] = i + 1 < sizeof(st.far) / 4 ? sync_entry((c & 31u) + ((c >> 8) & 15u), advance_of((c >> 8) & 255u, side != 0)) : 0u;
         }
         for (uint32_t i = tid; i < (1u << kValueBits); i += nthreads) {
             const uint32_t c = code_at(t, i << (16 - kValueBits));
             vt.lut[i] = (c & 31u) <= (uint32_t)kValueBits ? value_entry(c, side != 0) : 0u;
         }
-        for (uint32_t i = tid; i < sizeof(vt.far) / 4; i += nthreads) vt.far[i] = value_entry(code_at(t, min(vbase + i, 0xFFFFu)), side != 0);
+        for (uint32_t i = tid; i < sizeof(vt.far) / 4; i += nthreads) vt.far[i] = i + 1 < sizeof(vt.far) / 4 ? value_entry(code_at(t, min(vbase + i, 0xFFFFu)), side != 0) : 0u;
         if (tid == 0) {
             st.far_base = sbase; vt.far_base = vbase;
             st.huff = vt.huff = side ? ac_id : dc_id;
@@ -154,12 +152,21 @@ __device__ void build_tables(CodeTables& out, const HuffTable* pool, uint32_t dc
     }
 }
 
-// the entry of a code longer than the index; `tab`: shared-memory address of the table
+// The entry of the code at the head of `top`, 0: see rare_entry.  tab: shared-memory address of the table, off: far_offset()
+// of it.
+template <class Tab> __device__ __forceinline__ uint32_t far_offset(uint32_t far_base) { return (uint32_t)(sizeof(Tab::lut) / 4) - far_base; }
 template <class Tab>
-__device__ __forceinline__ uint32_t far_entry(uint32_t tab, uint32_t top, const HuffTable* pool) {
-    const uint32_t v = top >> 16, i = v - lds32(tab + (uint32_t)offsetof(Tab, far_base));
-    if (i < (uint32_t)(sizeof(Tab::far) / 4)) return lds32(tab + (uint32_t)offsetof(Tab, far) + i * 4);
-    const uint32_t c = long_code(pool + lds32(tab + (uint32_t)offsetof(Tab, huff)), v);
+__device__ __forceinline__ uint32_t entry_at(uint32_t tab, uint32_t off, uint32_t top) {
+    constexpr int kNear = (int)(sizeof(Tab::lut) / 4), kBits = kNear == 1 << kSyncBits ? kSyncBits : kValueBits, kAll = kNear + (int)(sizeof(Tab::far) / 4);
+    static_assert(kNear == 1 << kBits && offsetof(Tab, far) == sizeof(Tab::lut), "far[] follows lut[]");
+    const int32_t behind = (int32_t)((top >> 16) + off);
+    const uint32_t i = behind >= kNear ? (uint32_t)min(behind, kAll - 1) : top >> (32 - kBits);
+    return lds32(tab + i * 4);
+}
+// ... of a code whose window lies behind the end of far[]
+template <class Tab>
+__device__ __noinline__ uint32_t rare_entry(uint32_t tab, uint32_t top, const HuffTable* pool) {
+    const uint32_t c = long_code(pool + lds32(tab + (uint32_t)offsetof(Tab, huff)), top >> 16);
     const bool is_ac = lds32(tab + (uint32_t)offsetof(Tab, is_ac)) != 0;
     if (sizeof(Tab) == sizeof(SyncTab)) return sync_entry((c & 31u) + ((c >> 8) & 15u), advance_of((c >> 8) & 255u, is_ac));
     return value_entry(c, is_ac);
@@ -342,26 +349,33 @@ void launch_unstuff(const JpegWave& w, cudaStream_t s) {
 // of the next symbol follow from it.  The stream is cut into cells of kCellBits (1024) bits; what the second kernel needs
 // is, for every cell, the state at the first block that starts in it and that block's index in the image.
 //
-//  k_huff_sync   finds those states.  Every thread owns a run of consecutive cells and decodes it from a guessed state
-//     (first AC symbol of a luma block at the run's first bit), noting the state at the first block start of each cell
-//     and of the next thread's run.  Huffman streams re-synchronise, so the state a thread hands over is usually right
-//     even though it started from a guess; each thread then compares what its left neighbour hands over with what it
-//     assumed, decodes again from the corrected state where they differ -- only until it meets the recorded state of
-//     a cell -- and this repeats until nothing changes (bounded: thread j is final after round j).  Nothing but code
-//     lengths matters here, so symbols are looked up two at a time where they fit the table index and no value is ever
-//     extracted.  Measured on 4:2:0 photographs the distance to synchronisation is 200 to 800 bits in the median and 3000
-//     to 5000 at the 99th percentile (the phase inside the MCU is what takes long: with the 4:4:4 pattern it is 70 and
-//     330), so runs of several cells lose little to the second decode; a short image gets short runs instead, because
-//     then the latency of one thread's run is what counts.
-//     One CTA, or one cluster of CTAs sharing the hand-over states through distributed shared memory, per image.
+//  k_huff_guess  Huffman streams re-synchronise: a decoder started at a wrong place soon stands where the right one does.
+//     What takes long on subsampled images is the phase c, because only code lengths tell the tables apart.  Measured on
+//     4:2:0 photographs (cells of 1024 bits): one decoder started 256 bits before a cell as if in block 0 of an MCU is
+//     right at the cell for 25 to 58 % of the cells, but of the decoders started there in each of the MCU's blocks one is
+//     right for 96 to 99 %.  So all of them run: one thread per cell and block of the MCU goes through the lead, states
+//     that have met are dropped, and the distinct ones (two to four of six) decode the cell, packed into as few warps as
+//     they fill.  Nothing but code lengths matters here, so symbols are looked up several at a time and no value is ever
+//     extracted.  Every cell's work is independent of every other's.
+//  k_huff_chain  links them: a cell's entry state is the exit state of the cell before it, and its own exit is what
+//     k_huff_guess found for that entry.  One CTA per image; a thread owns a run of consecutive cells, follows the
+//     candidates through it, then compares what its left neighbour hands over with what it assumed, and so on until
+//     nothing changes; states nobody guessed are then decoded, all at once, and it goes on.  Chains of wrong phases are 5
+//     to 15 cells long: resolving them by decoding, with one guess per cell, took 12 rounds of a cell each for a photo of
+//     2.7 Mbit (276 us in a cluster of eight CTAs; 28 + 54 us for these two kernels).
 //  k_huff_write  one thread per cell decodes the blocks that start in it, values included, collects a block in shared
 //     memory and writes it out whole: DC difference and class to diff[], the rows the class covers to coef[].
 // ---------------------------------------------------------------------------------------------------------------
 namespace {
 
 // Where a decoder stands inside the MCU: the tables of the current block as shared-memory addresses, and the entry of the
-// block after it.  One 16-byte read per block instead of arithmetic on indices.
-struct McuBlock { uint32_t dc, ac, next, index; };
+// block after it.  Two reads per block instead of arithmetic on indices.
+struct alignas(16) McuBlock { uint32_t dc, ac, next, index; uint32_t dc_off, ac_off, pad[2]; };
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
@@ -384,7 +398,9 @@ __device__ __forceinline__ void load_tables(const JpegWave& w, const JpegDesc& d
     if ((uint32_t)tid < d.bpm) {
         const uint32_t luma = d.hs * d.vs, slot = (uint32_t)tid < luma ? 0u : (uint32_t)tid == luma ? slot1 : slot2;
         const uint32_t at = smem_addr(tab0) + slot * 2 * (uint32_t)sizeof(Tab);
-        mcu[tid] = McuBlock{at, at + (uint32_t)sizeof(Tab), smem_addr(&mcu[(uint32_t)tid + 1 == d.bpm ? 0 : tid + 1]), (uint32_t)tid};
+        const Tab* const tabs = reinterpret_cast<const Tab*>(w.codes + (size_t)(slot == 0 ? p0 : slot == slot1 ? p1 : p2) * kCodeTablesBytes + which);
+        mcu[tid] = McuBlock{at, at + (uint32_t)sizeof(Tab), smem_addr(&mcu[(uint32_t)tid + 1 == d.bpm ? 0 : tid + 1]), (uint32_t)tid,
+                            far_offset<Tab>(__ldg(&tabs[0].far_base)), far_offset<Tab>(__ldg(&tabs[1].far_base)), {0, 0}};
     }
 }
 
@@ -416,39 +432,44 @@ struct GlobalSource {
 // A lane of a synchronising decoder.
 struct SyncLane {
     uint32_t p, z, nb;   // bit position, slot inside the block, blocks ended since nb was last set to zero
-    uint32_t w0, w1, tab;
+    uint32_t w0, w1, tab, off;
     uint4 mb;            // McuBlock of the current block
+    uint2 mo;
     template <class Source>
     __device__ __forceinline__ void start(const Source& src, uint32_t mcu0, uint32_t bit, uint32_t slot, uint32_t c) {
         p = bit; z = slot; nb = 0;
         src.start(w0, w1, p);
         mb = lds128(mcu0 + c * (uint32_t)sizeof(McuBlock));
+        mo = lds64(mcu0 + c * (uint32_t)sizeof(McuBlock) + 16);
         tab = z ? mb.y : mb.x;
+        off = z ? mo.y : mo.x;
     }
     // Lanes with `live` decode to the first block start at p >= stop.  Called by whole warps: the loop has one exit, taken by
     // all lanes together, and no other jump out of it -- with returns from inside, the lanes of a warp never met again
-    // after their first different turn and went on alone.  turn(): called every four steps (124 bits at most) by all.
-    template <class Source, class Turn>
-    __device__ __forceinline__ void run_to(bool live, uint32_t stop, const Source& src, const HuffTable* pool, Turn&& turn) {
+    // after their first different turn and went on alone.
+    template <class Source>
+    __device__ __forceinline__ void run_to(bool live, uint32_t stop, const Source& src, const HuffTable* pool) {
         while (__any_sync(0xFFFFFFFFu, live)) {
-            turn(live);
 #pragma unroll
             for (int step = 0; step < 4; ++step) {
                 if (live) {
                     const uint32_t top = __funnelshift_l(w1, w0, p);
-                    uint32_t e = lds32(tab + ((top >> (32 - kSyncBits)) << 2));
-                    if (e == 0) e = far_entry<SyncTab>(tab, top, pool);
+                    uint32_t e = entry_at<SyncTab>(tab, off, top);
+                    if (e == 0) e = rare_entry<SyncTab>(tab, top, pool);
                     const uint32_t h = z + (e >> 24) >= 64u ? e : e >> 12;
                     const uint32_t was = p;
                     p += h & 31u;
                     z += (h >> 5) & 127u;
                     tab = mb.y;
+                    off = mo.y;
                     src.advance(w0, w1, was, p);
                     if (z >= 64u) {
                         z = 0;
                         ++nb;
+                        mo = lds64(mb.z + 16);
                         mb = lds128(mb.z);
                         tab = mb.x;
+                        off = mo.x;
                         live = p < stop;
                     }
                 }
@@ -457,154 +478,242 @@ struct SyncLane {
     }
 };
 
-constexpr int kRingPitch = 144;  // bytes per thread: eight 16-byte pieces of its stream, and the first of them once more behind them
-
-template <int T>
-struct SyncMisc {
-    uint2 exit[T];         // state each thread hands to its right neighbour
-    McuBlock mcu[6];
-    uint32_t warp[32];
-    uint32_t flag[3];      // cluster: some thread still differs (by round, modulo 3)
-    uint32_t total;        // blocks found by this CTA's threads
-    uint32_t pad[3];
+// Streams staged in shared memory, a cell per row and the first 16 bytes of the next cell behind it (which spreads the rows
+// over the banks and makes the word behind any word its neighbour).  A block may run 1984 bits (64 symbols of 31 bits) into
+// what follows the last cell, and the padding of a stream covers that: kRowsBehind, kRowsPadded.
+template <int CELL>
+struct Staged {
+    static constexpr int kPitch = CELL / 8 + 16, kRowsBehind = 1984 / CELL + 2, kRowsPadded = 2048 / CELL;
+    // cells [row0, row0 + rows) of the stream `us`
+    static __device__ __forceinline__ void copy(unsigned char* stage, const uint8_t* us, uint32_t row0, int rows, int tid, int nthreads) {
+        constexpr int kPieces = CELL / 128 + 1;  // 16-byte pieces per row
+        const uint8_t* src = us + (size_t)row0 * (CELL / 8);
+        const uint32_t dst = smem_addr(stage);
+        for (int i = tid; i < rows * kPieces; i += nthreads) copy16(dst + i * 16, src + (i / kPieces) * (CELL / 8) + (i % kPieces) * 16);
+        copy_commit();
+    }
+    // shared-memory address of the word with bit p; base: address row 0 of the stream would have
+    static __device__ __forceinline__ uint32_t at(uint32_t base, uint32_t p) { return base + ((p >> 3) & ~3u) + (p / CELL) * 16; }
 };
-static_assert(sizeof(SyncMisc<256>) % 16 == 0, "tables follow in shared memory");
+static_assert(kStreamPad >= (2048 + 1024) / 8 + 16, "rows behind the end of a stream are copied");
+
+// A state at or behind the first bit of a cell, relative to it: bits 0-11 distance of the block start (less than 2048: a
+// block has 64 symbols of 31 bits at most), 12-14 its block c.
+constexpr uint32_t kStNone = 0xFFFFu, kStDropped = 0xFFFEu;  // the stream ends before; no candidate
+__device__ __forceinline__ uint32_t pack_state(uint32_t p, uint32_t cell_bit, uint32_t c, uint32_t total) { return p > total ? kStNone : (p - cell_bit) | c << 12; }
+
+constexpr uint32_t kLeadBits = 256;
+constexpr int kGuessThreads = (int)kGuessLanes;
 
 }  // namespace
 
-template <int T, bool CLUSTER>
-__global__ void __launch_bounds__(T) k_huff_sync(JpegWave w, uint32_t first) {
-    extern __shared__ __align__(16) unsigned char sync_smem[];
-    unsigned char* const ring0 = sync_smem;
-    SyncMisc<T>& sh = *reinterpret_cast<SyncMisc<T>*>(sync_smem + T * kRingPitch);
-    unsigned char* const tab0 = sync_smem + T * kRingPitch + sizeof(SyncMisc<T>);
+// A CTA takes guess_spans() spans of w.guess_span cells, a thread per span and block of the MCU.  Decoders that meet are one
+// from then on, so in a span of several cells the lead is run once and fewer decoders are left from cell to cell; with few
+// images a span is one cell, because then the length of a thread's way is what counts.
+template <int CELL>
+__global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
+    extern __shared__ __align__(16) unsigned char guess_smem[];
+    __shared__ McuBlock mcu[6];
+    __shared__ uint16_t s_state[kGuessThreads], s_list[kGuessThreads];
+    __shared__ uint32_t s_warp[kGuessThreads / 32];
+    const uint32_t o = owner_of(w.guess_ctas, blockIdx.x);
+    const uint32_t img = w.spec_list[o];
+    const JpegDesc& d = w.descs[img];
+    const uint32_t span = w.guess_span, bpm = d.bpm, nspans = guess_spans(bpm, span), cell0 = (blockIdx.x - __ldg(w.guess_ctas.first + o)) * nspans * span;
+    const uint32_t total = w.us_len[img] * 8u, ncell = (total + CELL - 1) / CELL;
+    if (cell0 >= ncell) return;
+    unsigned char* const tab0 = guess_smem;
+    unsigned char* const stage = tab0 + w.max_pairs * 2 * sizeof(SyncTab);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    uint32_t rank = 0, nrank = 1;
-    if (CLUSTER) { rank = cg::this_cluster().block_rank(); nrank = cg::this_cluster().num_blocks(); }
-    const uint32_t img = w.spec_list[first + blockIdx.x / nrank];
+    const uint32_t row0 = cell0 ? cell0 - 1 : 0, cell1 = min(cell0 + nspans * span, ncell);
+    Staged<CELL>::copy(stage, w.us + d.us_off, row0, (int)(min(cell0 + nspans * span + Staged<CELL>::kRowsBehind, ncell + Staged<CELL>::kRowsPadded) - row0), tid, kGuessThreads);
+    load_tables<SyncTab>(w, d, mcu, tab0, (uint32_t)offsetof(CodeTables, sync), tid, kGuessThreads);
+    copy_commit();
+    uint2* const cand = w.cand + (size_t)d.cell_off * kCandidates;
+    for (uint32_t i = cell0 * (kCandidates / 2) + tid; i < cell1 * (kCandidates / 2); i += kGuessThreads)
+        reinterpret_cast<uint4*>(cand)[i] = make_uint4(kStDropped, 0, kStDropped, 0);
+    copy_wait<0>();
+    __syncthreads();
+    const uint32_t sbase = smem_addr(stage) - row0 * Staged<CELL>::kPitch, mcu0 = smem_addr(&mcu[0]);
+    const auto source = shared_source([&](uint32_t p) { return Staged<CELL>::at(sbase, p); });
+
+    // ---- the lead: from its first bit on, as if inside each of the MCU's blocks
+    const uint32_t mine = cell0 + (uint32_t)tid / bpm * span, myh = (uint32_t)tid % bpm;  // first cell of this thread's span
+    const bool live = (uint32_t)tid < nspans * bpm && mine < ncell;
+    uint32_t k = live ? mine : cell0;
+    SyncLane L{};
+    L.start(source, mcu0, k ? k * CELL - kLeadBits : 0u, k ? 1u : 0u, live && k ? myh : 0u);
+    L.run_to(live && k, k * CELL, source, w.huff);
+    s_state[tid] = (uint16_t)(live ? pack_state(L.p, k * CELL, L.mb.w, total) : kStNone);
+    for (uint32_t step = 0; step < span; ++step) {
+        __syncthreads();
+        // ---- the distinct states, in as few warps as they fill
+        const uint32_t state = s_state[tid];
+        bool keep = state < kStDropped && mine + step < ncell;
+        for (uint32_t i = 1; keep && i <= myh; ++i) keep = s_state[tid - i] != state;
+        const uint32_t kept = __ballot_sync(0xFFFFFFFFu, keep);
+        if (lane == 0) s_warp[warp] = __popc(kept);
+        __syncthreads();
+        if (!keep) s_state[tid] = (uint16_t)kStDropped;
+        uint32_t before = 0, all = 0;
+#pragma unroll
+        for (int i = 0; i < kGuessThreads / 32; ++i) { const uint32_t n = s_warp[i]; if (i < warp) before += n; all += n; }
+        if (keep) s_list[before + __popc(kept & ((1u << lane) - 1u))] = (uint16_t)tid;
+        __syncthreads();
+        // ---- through their cell
+        if ((uint32_t)warp * 32u < all) {
+            const bool on = (uint32_t)tid < all;
+            const uint32_t t = s_list[on ? tid : warp * 32], entry = s_state[t];
+            k = cell0 + t / bpm * span + step;
+            const uint32_t bound = (k + 1) * CELL, p = k * CELL + (entry & 0xFFFu);
+            L.start(source, mcu0, p, 0, entry >> 12);
+            L.run_to(on && p < bound, min(bound, total + 1), source, w.huff);
+            __syncwarp();
+            if (on) {
+                const uint32_t exit = pack_state(L.p, bound, L.mb.w, total);
+                if (L.p > total) --L.nb;  // the block that ended here is not whole
+                cand[(size_t)k * kCandidates + t % bpm] = make_uint2(entry | exit << 16, L.nb);
+                s_state[t] = (uint16_t)exit;
+            }
+        }
+    }
+}
+
+namespace {
+
+template <int T>
+struct ChainMisc {
+    uint32_t exit[T];      // state each thread hands to its right neighbour
+    McuBlock mcu[6];
+    uint32_t warp[32];
+};
+static_assert(sizeof(ChainMisc<256>) % 16 == 0, "tables follow in shared memory");
+
+}  // namespace
+
+template <int T, int CELL>
+__global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
+    extern __shared__ __align__(16) unsigned char chain_smem[];
+    ChainMisc<T>& sh = *reinterpret_cast<ChainMisc<T>*>(chain_smem);
+    unsigned char* const tab0 = chain_smem + sizeof(ChainMisc<T>);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t img = w.spec_list[blockIdx.x];
     const JpegDesc& d = w.descs[img];
     load_tables<SyncTab>(w, d, sh.mcu, tab0, (uint32_t)offsetof(CodeTables, sync), tid, T);
     copy_commit();
-    if (tid < 3) sh.flag[tid] = 0;
+    const uint32_t us_len = w.us_len[img], total = us_len * 8u;
+    const uint32_t ncell = (total + CELL - 1) / CELL;
+    const GlobalSource source{reinterpret_cast<const uint32_t*>(w.us + d.us_off), (us_len + 3) / 4 + 2};
+    uint2* const recs = w.cells + d.cell_off;  // while linking: block start, state << 12 | blocks that start in the cell
+    const uint4* const cand = reinterpret_cast<const uint4*>(w.cand + (size_t)d.cell_off * kCandidates);
+    const uint32_t run = (ncell + T - 1) / T;
+    const uint32_t kbeg = min(tid * run, ncell), kend = min(kbeg + run, ncell);
+    const bool active = kbeg < kend;
+    const uint32_t mcu0 = smem_addr(&sh.mcu[0]);
+    uint32_t found = 0;  // blocks that start in this thread's cells
+    uint32_t exit = kStNone;
     copy_wait<0>();
     __syncthreads();
 
-    const uint32_t total = w.us_len[img] * 8u;
-    const uint32_t ncell = (total + kCellBits - 1) / kCellBits;
-    const uint8_t* const us = w.us + d.us_off;
-    uint2* const recs = w.cells + d.cell_off;
-    const uint32_t gt = rank * T + tid, nthread = nrank * T;
-    const uint32_t run = (ncell + nthread - 1) / nthread;
-    const uint32_t kbeg = min(gt * run, ncell), kend = min(kbeg + run, ncell);
-    const bool active = kbeg < kend;
-    const uint32_t ring = smem_addr(ring0) + tid * kRingPitch, mcu0 = smem_addr(&sh.mcu[0]);
-
-    uint32_t found = 0;                       // blocks that start in this thread's cells
-    uint2 entry = make_uint2(0, 0), exit = make_uint2(kNoState, 0);
-
-    // Decodes the thread's cells from (p, z, c).  Redoing, it stops as soon as it meets the state recorded for one of them.
-    auto decode = [&](bool live, uint32_t p, uint32_t z, uint32_t c, bool redo) {
-        // the stream in pieces of 16 bytes through this thread's ring
-        const bool ended = p == kNoState;
-        uint32_t wr = ended ? 0u : p >> 7;
-        SyncLane L;
-        L.p = p;
-        auto fetch = [&]() {
-            copy16(ring + (wr & 7u) * 16, us + (size_t)wr * 16);
-            if ((wr & 7u) == 0) copy16(ring + 128, us + (size_t)wr * 16);
-            ++wr;
-        };
-        if (live && !ended) {
-            for (int i = 0; i < 8; ++i) fetch();
-        }
-        copy_commit();
-        copy_wait<0>();
-        const auto source = shared_source([&](uint32_t bit) { return ring + ((bit >> 3) & 124u); });
-        // A step consumes at most 31 bits, so four of them cross at most one piece and one copy per turn keeps the ring
-        // full.  The copies of the last four turns may still be under way: they are at least three pieces ahead.
-        auto turn = [&](bool on) {
-            if (on && wr < (L.p >> 7) + 8) fetch();
-            copy_commit();
-            copy_wait<4>();
-        };
-        L.start(source, mcu0, p, z, c);
-        if (!redo) L.run_to(live && z != 0, kbeg * kCellBits, source, w.huff, turn);  // the guess: to the first block start it meets
-        for (uint32_t i = 0; i < run; ++i) {
-            const uint32_t k = kbeg + i, bound = (k + 1) * kCellBits;
-            bool on = live && k < kend;
-            if (L.p > total) { L.p = kNoState; L.mb.w = 0; }  // the block that ended here is not whole
-            const uint2 at = make_uint2(L.p, L.mb.w);
-            uint32_t old_n = 0;
-            if (on) {
-                if (redo) {
-                    const uint2 had = recs[k];
-                    old_n = had.y & 0x0FFFFFFFu;
-                    if (i && had.x == at.x && (had.y >> 28) == at.y) on = live = false;  // met
+    // Follows the candidates from `state` at cell `k` on.  Walking again (`redo`), it stops at a cell whose recorded state it
+    // meets, unless something behind that cell is still open.  A state that is no candidate of its cell is left open
+    // (open_at, open_state): the cells from there on keep what they have, on the first walk a chain of their own.
+    uint32_t open_at = ~0u, open_state = 0, last_open = 0;  // last_open: no cell from here on is open
+    auto follow = [&](bool live, uint32_t k, uint32_t state, bool redo) {
+        if (live) open_at = ~0u;
+        const bool on = live && k < kend;
+        uint32_t still_open = 0;
+        for (const uint32_t first = k; on; ++k) {
+            const uint32_t cell_bit = k * CELL;
+            uint32_t next = kStNone, n = 0;
+            uint2 had = make_uint2(0, 0);
+            if (redo) {
+                had = recs[k];
+                if (k != first && k >= last_open && (had.y >> 12) == state) break;  // met
+            }
+            if (state != kStNone) {
+                if ((state & 0xFFFu) >= (uint32_t)CELL) next = state - CELL;  // no block starts in this cell
+                else {
+                    const uint4* const c = cand + (size_t)k * (kCandidates / 2);
+                    const uint4 a = __ldg(c), b = __ldg(c + 1), e = __ldg(c + 2);
+                    bool known = false;
+                    auto look = [&](uint32_t x, uint32_t y) { if ((x & 0xFFFFu) == state) { next = x >> 16; n = y; known = true; } };
+                    look(a.x, a.y); look(a.z, a.w); look(b.x, b.y); look(b.z, b.w); look(e.x, e.y); look(e.z, e.w);
+                    if (!known) {
+                        if (open_at == ~0u) { open_at = k; open_state = state; }
+                        still_open = k + 1;
+                        if (redo) { still_open = max(still_open, last_open); break; }
+                        state = a.x & 0xFFFFu;
+                        if (state == kStDropped) state = kStNone;
+                        else { next = a.x >> 16; n = a.y; }
+                    }
                 }
-                if (!redo && i == 0) entry = at;
             }
-            if (!__any_sync(0xFFFFFFFFu, on)) break;
-            L.nb = 0;
-            L.run_to(on && L.p < bound, min(bound, total + 1), source, w.huff, turn);
-            if (on) {
-                if (L.p > total && L.p != kNoState) --L.nb;
-                recs[k] = make_uint2(at.x, at.y << 28 | L.nb);
-                found += L.nb - old_n;
-            }
+            recs[k] = make_uint2(state == kStNone ? kNoState : cell_bit + (state & 0xFFFu), state << 12 | n);
+            found += n - (had.y & 0xFFFu);
+            state = next;
+            if (k + 1 == kend) { exit = state; break; }
         }
-        // Nothing may be on its way into the ring when it is filled anew: of two copies to one place the older may land last.
-        copy_wait<0>();
-        if (L.p > total) { L.p = kNoState; L.mb.w = 0; }
-        if (live) exit = make_uint2(L.p, L.mb.w);
+        if (on) last_open = still_open;
     };
 
-    decode(active, gt ? kbeg * kCellBits : 0u, gt ? 1u : 0u, 0u, false);
+    uint32_t entry = 0;  // thread 0: bit 0, block 0
+    if (active && tid) {
+        entry = __ldg(&cand[(size_t)kbeg * (kCandidates / 2)].x) & 0xFFFFu;
+        if (entry == kStDropped) entry = kStNone;
+    }
+    follow(active, kbeg, entry, false);
     sh.exit[tid] = exit;
-    uint32_t decodes = active ? 1u : 0u, rounds = 1;
-    if (CLUSTER) cg::this_cluster().sync(); else __syncthreads();
-    const uint32_t limit = nthread + 1;
-    uint32_t round = 0;
+    uint32_t walks = active ? 1u : 0u, rounds = 1, round = 0;
+    __syncthreads();
+    // Look-ups until nothing changes any more; then what is open is decoded, one cell per thread; and again.  Opened cells have
+    // their turn in every eighth round in any case: of eight rounds, one settles the first thread that is not final yet or
+    // its next open cell, which bounds the rounds (a photo takes 10 to 30, one to three of them decoding).
+    const uint64_t limit = 8ull * (ncell + T) + 8;
     for (; round <= limit; ++round) {
-        uint2 prev = entry;
-        if (active && gt) prev = tid ? sh.exit[tid - 1] : *cg::this_cluster().map_shared_rank(&sh.exit[T - 1], rank - 1);
-        const bool need = active && (prev.x != entry.x || prev.y != entry.y);
-        bool any = __syncthreads_or(need);
-        if (CLUSTER) {
-            if (any && tid == 0) *cg::this_cluster().map_shared_rank(&sh.flag[round % 3], 0) = 1;
-            cg::this_cluster().sync();
-            any = *cg::this_cluster().map_shared_rank(&sh.flag[round % 3], 0) != 0;
-            if (rank == 0 && tid == 0) sh.flag[(round + 2) % 3] = 0;
-        }
-        if (!any) break;
-        if (__any_sync(0xFFFFFFFFu, need)) {
-            decodes += need;
+        const uint32_t prev = active && tid ? sh.exit[tid - 1] : entry;
+        const bool need = prev != entry, any_need = __syncthreads_or(need);
+        const bool decode = open_at != ~0u;
+        bool any_decode = false;
+        if (!any_need || (round & 7u) == 7u) any_decode = __syncthreads_or(decode);
+        if (!any_need && !any_decode) break;
+        if (!any_decode) {
+            walks += need;
             if (need) entry = prev;
-            decode(need, need ? prev.x : kNoState, 0, prev.y, true);
-            sh.exit[tid] = exit;
+            follow(need, kbeg, entry, true);
+        } else {
+            if (__any_sync(0xFFFFFFFFu, decode)) {
+                const uint32_t k = decode ? open_at : 0, bound = (k + 1) * CELL, p = k * CELL + (decode ? open_state & 0xFFFu : 0u);
+                SyncLane L;
+                L.start(source, mcu0, p, 0, decode ? open_state >> 12 : 0u);
+                L.run_to(decode, min(bound, total + 1), source, w.huff);
+                __syncwarp();
+                if (decode) {
+                    const uint32_t n = L.nb - (L.p > total ? 1u : 0u), next = pack_state(L.p, bound, L.mb.w, total);
+                    found += n - (recs[k].y & 0xFFFu);
+                    recs[k] = make_uint2(p, open_state << 12 | n);
+                    if (k + 1 == kend) { exit = next; open_at = ~0u; last_open = 0; }
+                    else follow(true, k + 1, next, true);
+                }
+            }
         }
+        sh.exit[tid] = exit;
         ++rounds;
-        if (CLUSTER) cg::this_cluster().sync(); else __syncthreads();
+        __syncthreads();
     }
     // index of the first block of every cell
     uint32_t inc = found;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, o); if (lane >= o) inc += t; }
     if (lane == 31) sh.warp[warp] = inc;
-    decodes = __reduce_add_sync(0xFFFFFFFFu, decodes);
-    if (lane == 0) atomicAdd(w.spec_stats + 2, (unsigned long long)decodes);
+    walks = __reduce_add_sync(0xFFFFFFFFu, walks);
+    if (lane == 0) atomicAdd(w.spec_stats + 2, (unsigned long long)walks);
     __syncthreads();
-    uint32_t before = 0, all = 0;
+    uint32_t base = inc - found;
 #pragma unroll
-    for (int i = 0; i < T / 32; ++i) { const uint32_t v = sh.warp[i]; if (i < warp) before += v; all += v; }
-    if (CLUSTER) {
-        if (tid == 0) sh.total = all;
-        cg::this_cluster().sync();
-        for (uint32_t r = 0; r < rank; ++r) before += *cg::this_cluster().map_shared_rank(&sh.total, r);
-        cg::this_cluster().sync();  // nobody's shared memory goes away while it is being read
-    }
-    uint32_t base = before + inc - found;
-    for (uint32_t k = kbeg; k < kend; ++k) { const uint32_t n = recs[k].y & 0x0FFFFFFFu; recs[k].y = base; base += n; }
-    if (rank + 1 == nrank && tid == T - 1) {
+    for (int i = 0; i < T / 32; ++i) if (i < warp) base += sh.warp[i];
+    for (uint32_t k = kbeg; k < kend; ++k) { const uint32_t n = recs[k].y & 0xFFFu; recs[k].y = base; base += n; }
+    if (tid == T - 1) {
         recs[ncell] = make_uint2(kNoState, base);
         uint32_t err = 0;
         if (base < d.nblocks) err |= kStTruncated;
@@ -668,18 +777,17 @@ __device__ __forceinline__ uint32_t decode_blocks(const Source& src, uint32_t p,
     src.start(w0, w1, p);
     const uint32_t place = smem_addr(sh.place) - 4, buf = smem_addr(&sh.block[threadIdx.x]);
     uint4 mb = lds128(smem_addr(&sh.mcu[0]) + c * sizeof(McuBlock));
-    uint32_t tab = mb.x, z = 0, seen = 0;
+    uint2 mo = lds64(smem_addr(&sh.mcu[0]) + c * sizeof(McuBlock) + 16);
+    uint32_t tab = mb.x, off = mo.x, z = 0, seen = 0;
     int32_t pred0 = 0, pred1 = 0, pred2 = 0;
     for (;;) {
         const uint32_t alive = __ballot_sync(0xFFFFFFFFu, live);
-        if (!alive) break;  // one exit for the whole warp, see k_huff_sync
+        if (!alive) break;  // one exit for the whole warp, see SyncLane::run_to
         if (live && z < 64u) {
             const uint32_t top = __funnelshift_l(w1, w0, p);
-            uint32_t e = lds32(tab + ((top >> (32 - kValueBits)) << 2));
-            if (e == 0) {
-                e = far_entry<ValueTab>(tab, top, pool);
-                if (((e >> 24) & 1u) && p < limit) err |= kStBadCode;
-            }
+            uint32_t e = entry_at<ValueTab>(tab, off, top);
+            if (e == 0) e = rare_entry<ValueTab>(tab, top, pool);
+            if (((e >> 24) & 1u) && p < limit) err |= kStBadCode;
             const uint32_t was = p, s = (e >> 10) & 15u;
             // the s extra bits (T.81 EXTEND): a leading 1 means the value itself, a leading 0 the complement of its magnitude
             const uint32_t bits = top << ((e >> 5) & 31u);
@@ -695,6 +803,7 @@ __device__ __forceinline__ uint32_t decode_blocks(const Source& src, uint32_t p,
             }
             if (s && z > 64u && p <= limit) err |= kStCoefRange;
             tab = mb.y;
+            off = mo.y;
         }
         const uint32_t done = __ballot_sync(0xFFFFFFFFu, live && z >= 64u);
         if (__popc(done) >= kFlushLanes || done == alive) {
@@ -728,8 +837,10 @@ __device__ __forceinline__ uint32_t decode_blocks(const Source& src, uint32_t p,
                     ++blk;
                     live = blk < end && p < stop;
                     z = 0; seen = 0;
+                    mo = lds64(mb.z + 16);
                     mb = lds128(mb.z);
                     tab = mb.x;
+                    off = mo.x;
                 }
             }
         }
@@ -741,33 +852,23 @@ __device__ __forceinline__ uint32_t decode_blocks(const Source& src, uint32_t p,
 
 // ---- restart-free images: one thread per cell -----------------------------------------------------------------------
 constexpr int kWriteThreads = (int)kCellsPerCta;
-// The CTA's cells are consecutive: their 16 KB of stream are staged in shared memory, a cell per row and the first 16 bytes
-// of the next cell behind it (which spreads the rows over the banks and makes the word behind any word its neighbour); a
-// block may run 1984 bits (64 symbols of 31 bits) into what follows.
-constexpr int kStageRows = kWriteThreads + 3, kStagePitch = (int)kCellBits / 8 + 16;
-
+// The CTA's cells are consecutive: their stream is staged in shared memory.
+template <int CELL>
 __global__ void __launch_bounds__(kWriteThreads) k_huff_write(JpegWave w) {
     extern __shared__ __align__(16) unsigned char write_smem[];
     ValueMisc<kWriteThreads>& sh = *reinterpret_cast<ValueMisc<kWriteThreads>*>(write_smem);
     unsigned char* const stage = write_smem + sizeof(ValueMisc<kWriteThreads>);
-    unsigned char* const tab0 = stage + kStageRows * kStagePitch;
+    unsigned char* const tab0 = stage + (kWriteThreads + Staged<CELL>::kRowsBehind) * Staged<CELL>::kPitch;
     const uint32_t o = owner_of(w.write_ctas, blockIdx.x);
     const uint32_t img = w.spec_list[o];
     const JpegDesc& d = w.descs[img];
     const uint32_t cell0 = (blockIdx.x - __ldg(w.write_ctas.first + o)) * kCellsPerCta;
     const uint32_t total = w.us_len[img] * 8u;
-    const uint32_t ncell = (total + kCellBits - 1) / kCellBits;
+    const uint32_t ncell = (total + CELL - 1) / CELL;
     if (cell0 >= ncell) return;
     const int tid = threadIdx.x;
-    {
-        constexpr int kPieces = (int)kCellBits / 128 + 1;  // 16-byte pieces per row
-        const uint8_t* src = w.us + d.us_off + (size_t)cell0 * (kCellBits / 8);
-        const uint32_t dst = smem_addr(stage);
-        // no further than the stream and its padding reach
-        const int rows = (int)min((uint32_t)kStageRows, ncell - cell0 + 2);
-        for (int i = tid; i < rows * kPieces; i += kWriteThreads) copy16(dst + i * 16, src + (i / kPieces) * (kCellBits / 8) + (i % kPieces) * 16);
-        copy_commit();
-    }
+    // (no further than the stream and its padding reach)
+    Staged<CELL>::copy(stage, w.us + d.us_off, cell0, (int)min((uint32_t)(kWriteThreads + Staged<CELL>::kRowsBehind), ncell - cell0 + Staged<CELL>::kRowsPadded), tid, kWriteThreads);
     value_setup<kWriteThreads>(w, d, sh, tab0);
     const uint32_t k = cell0 + tid;
     const uint2* recs = w.cells + d.cell_off;
@@ -780,10 +881,10 @@ __global__ void __launch_bounds__(kWriteThreads) k_huff_write(JpegWave w) {
     copy_wait<0>();
     __syncthreads();
     uint32_t err = 0;
-    const uint32_t sbase = smem_addr(stage) - cell0 * kStagePitch;
-    const auto source = shared_source([&](uint32_t p) { return sbase + ((p >> 3) & ~3u) + (p / kCellBits) * 16; });
-    const uint32_t p0 = a.y < b1 ? a.x : cell0 * kCellBits;
-    decode_blocks<kWriteThreads, false>(source, p0, a.y, b1, total, (cell0 + kCellsPerCta) * kCellBits, a.y % d.bpm, d.hs * d.vs, sh, w.huff,
+    const uint32_t sbase = smem_addr(stage) - cell0 * Staged<CELL>::kPitch;
+    const auto source = shared_source([&](uint32_t p) { return Staged<CELL>::at(sbase, p); });
+    const uint32_t p0 = a.y < b1 ? a.x : cell0 * CELL;
+    decode_blocks<kWriteThreads, false>(source, p0, a.y, b1, total, (cell0 + kCellsPerCta) * CELL, a.y % d.bpm, d.hs * d.vs, sh, w.huff,
                                         w.coef + d.block_off * 64, w.diff + d.block_off, err);
     if (err) atomicOr(w.status + d.item, err);
 }
@@ -985,56 +1086,54 @@ void configure_once() {
     if (dev < 0 || dev >= 64) dev = 0;
     std::call_once(done[dev], [] {
         const size_t most = 227 * 1024 - 1024;
-        allow_smem(k_huff_sync<256, false>, most);
-        allow_smem(k_huff_sync<512, false>, most);
-        allow_smem(k_huff_sync<1024, false>, most);
-        allow_smem(k_huff_sync<1024, true>, most);
-        allow_smem(k_huff_write, most);
+        allow_smem(k_huff_guess<kCellBits>, most - 4096);  // (it has static arrays as well)
+        allow_smem(k_huff_chain<256, kCellBits>, most);
+        allow_smem(k_huff_chain<1024, kCellBits>, most);
+        allow_smem(k_huff_write<kCellBits>, most);
         allow_smem(k_huff_restart, most);
     });
 }
 
-template <int T, bool CLUSTER>
-void launch_sync(const JpegWave& w, uint32_t first, uint32_t count, uint32_t cluster, cudaStream_t s) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(count * cluster);
-    cfg.blockDim = dim3(T);
-    cfg.dynamicSmemBytes = (size_t)T * kRingPitch + sizeof(SyncMisc<T>) + w.max_pairs * 2 * sizeof(SyncTab);
-    cfg.stream = s;
-    cudaLaunchAttribute attr;
-    if (CLUSTER) {
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = cluster;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-    }
-    cudaLaunchKernelEx(&cfg, k_huff_sync<T, CLUSTER>, w, first);
+template <int CELL>
+void launch_guess(const JpegWave& w, cudaStream_t s) {
+    // the cell before the first, the cells, and what a block may run over
+    const size_t rows = 1 + (size_t)guess_spans(1, w.guess_span) * w.guess_span + Staged<CELL>::kRowsBehind;
+    k_huff_guess<CELL><<<w.guess_ctas.total, kGuessThreads, rows * Staged<CELL>::kPitch + w.max_pairs * 2 * sizeof(SyncTab), s>>>(w);
+}
+
+// With hundreds of images in a launch they fill the GPU with 256 threads each; with fewer, an image gets 1024, so that its
+// threads' runs are short.
+template <int CELL>
+void launch_chain(const JpegWave& w, cudaStream_t s) {
+    const size_t tables = w.max_pairs * 2 * sizeof(SyncTab);
+    if (w.n_spec >= 2 * 148) k_huff_chain<256, CELL><<<w.n_spec, 256, sizeof(ChainMisc<256>) + tables, s>>>(w);
+    else k_huff_chain<1024, CELL><<<w.n_spec, 1024, sizeof(ChainMisc<1024>) + tables, s>>>(w);
+}
+
+template <int CELL>
+void launch_write(const JpegWave& w, cudaStream_t s) {
+    const size_t smem = sizeof(ValueMisc<kWriteThreads>) + (size_t)(kWriteThreads + Staged<CELL>::kRowsBehind) * Staged<CELL>::kPitch + w.max_pairs * 2 * sizeof(ValueTab);
+    k_huff_write<CELL><<<w.write_ctas.total, kWriteThreads, smem, s>>>(w);
 }
 
 }  // namespace
 
-// How many threads an image gets.  With hundreds of images in a launch the images fill the GPU by themselves and 256
-// threads each (runs of a dozen cells) waste the least on synchronisation; with fewer, an image gets more threads, so
-// that the launch does not last as long as one thread's run; with a few tens or less, a cluster of up to eight 1024-thread
-// CTAs.  longest_cells: cells of the longest image of the launch (more CTAs than it has cells for would idle).  widest: the
-// images are the few longest of a wave, launched beside the others: 1024 threads at least.
-void launch_huff_sync(const JpegWave& w, uint32_t first, uint32_t count, uint32_t longest_cells, bool widest, cudaStream_t s) {
-    if (!count) return;
+void launch_huff_guess(const JpegWave& w, cudaStream_t s) {
+    if (!w.guess_ctas.total) return;
     configure_once();
-    if (!widest && count >= 3 * 148) { launch_sync<256, false>(w, first, count, 1, s); return; }
-    if (!widest && count >= 120) { launch_sync<512, false>(w, first, count, 1, s); return; }
-    uint32_t cluster = 1;
-    while (cluster < 8 && 2 * cluster * count <= 148 && cluster * 1024 < longest_cells) cluster *= 2;
-    if (cluster == 1) launch_sync<1024, false>(w, first, count, 1, s);
-    else launch_sync<1024, true>(w, first, count, cluster, s);
+    launch_guess<kCellBits>(w, s);
+}
+
+void launch_huff_chain(const JpegWave& w, cudaStream_t s) {
+    if (!w.n_spec) return;
+    configure_once();
+    launch_chain<kCellBits>(w, s);
 }
 
 void launch_huff_write(const JpegWave& w, cudaStream_t s) {
     if (!w.write_ctas.total) return;
     configure_once();
-    const size_t smem = sizeof(ValueMisc<kWriteThreads>) + (size_t)kStageRows * kStagePitch + w.max_pairs * 2 * sizeof(ValueTab);
-    k_huff_write<<<w.write_ctas.total, kWriteThreads, smem, s>>>(w);
+    launch_write<kCellBits>(w, s);
     k_dc<<<w.dc_ctas.total, kDcThreads, 0, s>>>(w);
 }
 
