@@ -420,6 +420,7 @@ struct WavePlan {
     std::vector<uint32_t> tile_first, spec_list, guess_first, write_first, dc_first, restart_list, restart_first, block_first, color_first;
     std::vector<std::array<uint32_t, 2>> pairs;  // (DC, AC) pairs of Huffman tables in use
     std::map<std::array<uint32_t, 2>, uint32_t> pair_ids;
+    uint32_t cell_bits = kCellBits;              // of the wave's streams: bits per thread of the value decoder
     uint32_t guess_span = 1;                     // cells a thread of the synchronising decoder goes through
     uint32_t max_pairs = 1;                      // most distinct ones in one image
     uint32_t pair_id(uint32_t dc, uint32_t ac) {
@@ -881,7 +882,7 @@ static size_t resize_mid_bound(const dg_plan& p, uint32_t C) {
 }
 
 // cells of a restart-free stream, at most (the unstuffed stream is no longer than the raw one)
-static uint32_t stream_cells(uint32_t raw_len) { return (uint32_t)(((uint64_t)raw_len * 8 + kCellBits - 1) / kCellBits); }
+static uint32_t stream_cells(uint32_t raw_len, uint32_t cell_bits) { return (uint32_t)(((uint64_t)raw_len * 8 + cell_bits - 1) / cell_bits); }
 
 // Runs fn(0..n-1) on the process-wide host pool; small counts stay on the calling thread.
 template <typename F> static void parallel_items(int n, F&& fn) {
@@ -1101,12 +1102,15 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         for (int pass = 0; pass < 2; ++pass)
             for (size_t k = 0; k < built.size(); ++k)
                 if ((int)(ctx->fused_path && fused_decode(built[k].ncomp, built[k].hs, built[k].vs, built[k].width)) == pass) order.push_back(k);
-        // With a thread per cell and block of the MCU the synchronising decoder's threads fit the chip at once: the shortest
-        // way for every thread.  Beyond that, less work in all counts more (256 files, 1.2 Gbit: 817 us with spans of four
-        // cells, 1005 with single ones; 8 files of 4:4:4, 34 Mbit: 94 and 52 us).
+        // While a thread per cell of 512 bits and block of the MCU fits the chip at once, the length of a thread's way is what
+        // counts: short cells (synchronisation + values of one photo 173 us with cells of 1024 bits, 122 with 512; 32 web
+        // images 193 and 118).  Beyond that, less work in all counts more (8 files of 4:4:4, 75 Mbit: a pass 0.84 ms with
+        // 512, 0.80 with 1024), and with several times as many threads, spans of cells as well (256 files, 1.2 Gbit: 1005 us
+        // for single cells, 817 with four in a span; the 4:4:4 files: 52 and 94 us).
         uint64_t guess_bits = 0;
         for (const JpegDesc& d : built)
             if (!d.restart) guess_bits += (uint64_t)d.raw_len * 8 * d.bpm;
+        wv.cell_bits = guess_bits / kShortCellBits > kGuessSpanThreads ? kCellBits : kShortCellBits;
         wv.guess_span = guess_bits / kCellBits > kGuessSpanThreads ? kGuessSpan : 1;
         uint32_t color_total = 0, restart_total = 0, fchroma_total = 0, ftile_total = 0;
         size_t group_bytes = 0, fgroup_bytes = 0;
@@ -1137,7 +1141,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             } else {
                 wv.spec_list.push_back((uint32_t)wv.descs.size());
                 d.cell_off = cells;
-                cells += stream_cells(d.raw_len) + 1;
+                cells += stream_cells(d.raw_len, wv.cell_bits) + 1;
             }
             wv.tile_first.push_back(wv.tile_first.back() + std::max(1u, (d.raw_len + kUnstuffTile - 1) / kUnstuffTile));
             {
@@ -1185,8 +1189,8 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         for (uint32_t k : wv.spec_list) {
             const JpegDesc& d = wv.descs[k];
             const uint32_t guess_step = guess_spans(d.bpm, wv.guess_span) * wv.guess_span;
-            wv.guess_first.push_back(wv.guess_first.back() + (stream_cells(d.raw_len) + guess_step - 1) / guess_step);
-            wv.write_first.push_back(wv.write_first.back() + (stream_cells(d.raw_len) + kCellsPerCta - 1) / kCellsPerCta);
+            wv.guess_first.push_back(wv.guess_first.back() + (stream_cells(d.raw_len, wv.cell_bits) + guess_step - 1) / guess_step);
+            wv.write_first.push_back(wv.write_first.back() + (stream_cells(d.raw_len, wv.cell_bits) + kCellsPerCta - 1) / kCellsPerCta);
             wv.dc_first.push_back(wv.dc_first.back() + (d.mcux * d.mcuy + kDcMcus - 1) / kDcMcus);
         }
         wv.us_bytes = us; wv.coef_blocks = blocks; wv.plane_bytes = planes; wv.decoded_bytes = decoded; wv.mid_bytes = mids; wv.nseg = segs; wv.cells = cells;
@@ -1541,6 +1545,7 @@ static int batch_run_locked(dg_batch* b) {
             w.n_spec = (uint32_t)wv.spec_list.size();
             w.restart_list = (const uint32_t*)(meta + wv.m_restart_list);
             w.restart_ctas = resolve(b, wv.m_restart);
+            w.cell_bits = wv.cell_bits;
             w.guess_span = wv.guess_span;
             w.guess_ctas = resolve(b, wv.m_guess);
             w.write_ctas = resolve(b, wv.m_write);

@@ -16,7 +16,8 @@ struct OwnerMap {
 
 // ---- entropy decoding: work splits (see kernels_huff.cu) ------------------------------------------------------------------
 constexpr uint32_t kUnstuffTile = 4096;  // bytes of an entropy-coded segment per CTA of the unstuffing kernels
-constexpr int kCellBits = 1024;          // bits of an unstuffed stream per thread of the value decoder
+// bits of an unstuffed stream per thread of the value decoder; the short form while all threads are resident at once
+constexpr int kCellBits = 1024, kShortCellBits = 512;
 constexpr uint32_t kCellsPerCta = 128, kSegsPerCta = 128;
 // synchronising decoder: threads per CTA, the entries of the candidate array per cell, and the cells of a span once a thread
 // per cell and block of the MCU would be more than the chip holds at once
@@ -71,6 +72,7 @@ struct JpegWave {
     // prediction: owner = index into spec_list
     const uint32_t* spec_list; uint32_t n_spec;
     OwnerMap guess_ctas, write_ctas, dc_ctas;
+    uint32_t cell_bits;      // kCellBits or kShortCellBits
     uint32_t guess_span;     // cells a thread of the synchronising decoder goes through
     // restart-interval images: kSegsPerCta segments per CTA, owner = index into restart_list
     OwnerMap restart_ctas;

@@ -346,7 +346,7 @@ void launch_unstuff(const JpegWave& w, cudaStream_t s) {
 // K1  Huffman entropy decode of images without restart markers, in two kernels.
 //
 // The only decoder state between two blocks is (bit position p, block index c inside the MCU): the tables and the meaning
-// of the next symbol follow from it.  The stream is cut into cells of kCellBits (1024) bits; what the second kernel needs
+// of the next symbol follow from it.  The stream is cut into cells of CELL (1024 or 512) bits; what the second kernel needs
 // is, for every cell, the state at the first block that starts in it and that block's index in the image.
 //
 //  k_huff_guess  Huffman streams re-synchronise: a decoder started at a wrong place soon stands where the right one does.
@@ -1087,9 +1087,13 @@ void configure_once() {
     std::call_once(done[dev], [] {
         const size_t most = 227 * 1024 - 1024;
         allow_smem(k_huff_guess<kCellBits>, most - 4096);  // (it has static arrays as well)
+        allow_smem(k_huff_guess<kShortCellBits>, most - 4096);
         allow_smem(k_huff_chain<256, kCellBits>, most);
         allow_smem(k_huff_chain<1024, kCellBits>, most);
+        allow_smem(k_huff_chain<256, kShortCellBits>, most);
+        allow_smem(k_huff_chain<1024, kShortCellBits>, most);
         allow_smem(k_huff_write<kCellBits>, most);
+        allow_smem(k_huff_write<kShortCellBits>, most);
         allow_smem(k_huff_restart, most);
     });
 }
@@ -1101,12 +1105,13 @@ void launch_guess(const JpegWave& w, cudaStream_t s) {
     k_huff_guess<CELL><<<w.guess_ctas.total, kGuessThreads, rows * Staged<CELL>::kPitch + w.max_pairs * 2 * sizeof(SyncTab), s>>>(w);
 }
 
-// With hundreds of images in a launch they fill the GPU with 256 threads each; with fewer, an image gets 1024, so that its
-// threads' runs are short.
+// With an image per SM or more, 256 threads each leave the most room for other kernels beside them (1024 files of 0.4 Mbit:
+// 3.37 ms a pass against 3.48 with 1024 threads; 256 files of 5 Mbit: 4.29 against 4.30); with fewer, an image gets 1024, so
+// that its threads' runs are short.
 template <int CELL>
 void launch_chain(const JpegWave& w, cudaStream_t s) {
     const size_t tables = w.max_pairs * 2 * sizeof(SyncTab);
-    if (w.n_spec >= 2 * 148) k_huff_chain<256, CELL><<<w.n_spec, 256, sizeof(ChainMisc<256>) + tables, s>>>(w);
+    if (w.n_spec >= 120) k_huff_chain<256, CELL><<<w.n_spec, 256, sizeof(ChainMisc<256>) + tables, s>>>(w);
     else k_huff_chain<1024, CELL><<<w.n_spec, 1024, sizeof(ChainMisc<1024>) + tables, s>>>(w);
 }
 
@@ -1121,19 +1126,22 @@ void launch_write(const JpegWave& w, cudaStream_t s) {
 void launch_huff_guess(const JpegWave& w, cudaStream_t s) {
     if (!w.guess_ctas.total) return;
     configure_once();
-    launch_guess<kCellBits>(w, s);
+    if (w.cell_bits == (uint32_t)kCellBits) launch_guess<kCellBits>(w, s);
+    else launch_guess<kShortCellBits>(w, s);
 }
 
 void launch_huff_chain(const JpegWave& w, cudaStream_t s) {
     if (!w.n_spec) return;
     configure_once();
-    launch_chain<kCellBits>(w, s);
+    if (w.cell_bits == (uint32_t)kCellBits) launch_chain<kCellBits>(w, s);
+    else launch_chain<kShortCellBits>(w, s);
 }
 
 void launch_huff_write(const JpegWave& w, cudaStream_t s) {
     if (!w.write_ctas.total) return;
     configure_once();
-    launch_write<kCellBits>(w, s);
+    if (w.cell_bits == (uint32_t)kCellBits) launch_write<kCellBits>(w, s);
+    else launch_write<kShortCellBits>(w, s);
     k_dc<<<w.dc_ctas.total, kDcThreads, 0, s>>>(w);
 }
 
