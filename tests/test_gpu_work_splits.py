@@ -1,0 +1,95 @@
+"""Kernels whose split of the work depends on sizes, at the sizes where a split changes or a tile ends.  Everything is integer
+arithmetic on 8-bit samples, so results equal the oracle's exactly."""
+import io
+
+import numpy as np
+import pytest
+
+import datago_b200 as dg
+import oracle
+from datago_b200 import synth
+from gpu_common import assert_same, ctx, jpeg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("w", [3, 5, 6, 7, 8, 9, 15, 16, 17, 31, 33, 255, 256, 257, 263, 264])
+def test_horizontal_chroma_filter_at_the_edges(w):
+    # 4:2:2: eight pixels per thread; the last chroma column is replicated, also inside a word
+    rng = np.random.default_rng(300 + w)
+    datas = [synth.encode_jpeg(rng.integers(0, 256, (h, w, 3), dtype=np.uint8), 92, "4:2:2", 0) for h in (1, 9, 40)]
+    for data, (st, out, _) in zip(datas, ctx().process(datas)):
+        assert st == 0
+        assert_same(out, oracle.jpeg_decode(data), str(w))
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (1, 3, 3), (5, 3, 3), (7, 11), (37, 41, 3), (64, 64, 4), (127, 129, 3)])
+def test_raw_pixels_handed_through_at_every_alignment(shape):
+    # collated payloads lie back to back, so those of an odd size start at every byte alignment
+    rng = np.random.default_rng(310)
+    items = [rng.integers(0, 256, shape, dtype=np.uint8) for _ in range(20)]
+    with ctx().batch(items, None, dg.BATCH_COLLATE) as b:
+        b.upload(); b.run()
+        host = np.empty(max(1, b.packed_bytes()), np.uint8)
+        b.download_packed(host); b.sync()
+        k, = b.buckets()
+        got = host[k["packed_offset"]:k["packed_offset"] + k["nbytes"]].reshape(len(items), -1)
+        for i, x in enumerate(items):
+            assert np.array_equal(got[i], x.reshape(-1)), i
+
+
+def test_integral_crop_of_a_pitched_source():
+    # an aspect ratio between two buckets at the bucket's own scale: rows of the source are cut, nothing is filtered
+    cfg = dict(crop_and_resize=True, default_image_size=224, downsampling_ratio=16, min_aspect_ratio=0.5, max_aspect_ratio=2.0)
+    rng = np.random.default_rng(311)
+    base = ctx(cfg).plan_geometry(224, 224, 3)
+    for dw in (2, 6, 8):
+        x = rng.integers(0, 256, (base.target_h, base.target_w + dw, 3), dtype=np.uint8)
+        (st, out, _), = ctx(cfg).process([x])
+        want, _ = oracle.crop_and_resize(cfg, x)
+        assert st == 0
+        assert_same(out, want, str(dw))
+
+
+def _noisy(rng, w, h, sub, q, optimize=False):
+    b = io.BytesIO()
+    from PIL import Image, ImageFile
+    ImageFile.MAXBLOCK = 1 << 24  # the encoder's buffer: it cannot suspend while it optimises its tables
+    a = rng.integers(0, 256, (h, w, 3), dtype=np.uint8)
+    a[: h // 3] //= 8  # a quieter part: other code lengths, more blocks per cell
+    if sub is None:
+        Image.fromarray(a[:, :, 0]).save(b, "JPEG", quality=q, optimize=optimize)
+    else:
+        Image.fromarray(a).save(b, "JPEG", quality=q, subsampling=sub, optimize=optimize)
+    return b.getvalue()
+
+
+@pytest.mark.parametrize("copies", [1, 6, 30, 130])
+def test_entropy_cells_and_spans(copies):
+    # one file per sampling, with the standard and with its own code tables; more of them pass through short cells, long
+    # cells, spans of cells and the smaller linking CTAs
+    rng = np.random.default_rng(320)
+    distinct = [_noisy(rng, w, h, sub, q, opt) for (w, h, sub, q, opt) in
+                [(700, 500, "4:2:0", 95, False), (640, 640, "4:2:0", 75, True), (500, 301, "4:4:4", 98, True), (400, 333, "4:2:2", 90, False),
+                 (611, 400, None, 97, True), (33, 17, "4:2:0", 90, False)]]
+    distinct.append(jpeg(rng, 512, 480, q=40, noise=0.0))  # many blocks per cell
+    want = [oracle.jpeg_decode(d) for d in distinct]
+    with ctx().batch(distinct * copies) as b:
+        b.upload(); b.run()
+        outs = b.download(); b.sync()
+        for i, out in enumerate(outs):
+            assert b.result(i).status == 0, i
+            assert_same(out, want[i % len(distinct)], str(i))
+
+
+@pytest.mark.parametrize("h", [1, 40, 700, 2300])
+def test_resize_pass_cuts(h):
+    # one image (CTAs of two chunks) and forty (longer ones), as tall and as flat as a pass gets
+    cfg = dict(crop_and_resize=True, default_image_size=512, downsampling_ratio=16, min_aspect_ratio=0.5, max_aspect_ratio=2.0)
+    rng = np.random.default_rng(330 + h)
+    x = rng.integers(0, 256, (h, 600, 3), dtype=np.uint8)
+    want, _ = oracle.crop_and_resize(cfg, x)
+    for n in (1, 40):
+        for st, out, _ in ctx(cfg).process([x] * n):
+            assert st == 0
+            assert_same(out, want, str((h, n)))
