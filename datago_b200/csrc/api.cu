@@ -1180,7 +1180,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
                 wv.fgroups.back()[3] += ntiles;
             }
         }
-        // longest streams first: one CTA decodes one image, and the launch ends with its slowest CTA
+        // longest streams first: one CTA links the cells of an image, and the launch ends with its slowest CTA
         std::stable_sort(wv.spec_list.begin(), wv.spec_list.end(),
                          [&](uint32_t a, uint32_t c) { return wv.descs[a].raw_len > wv.descs[c].raw_len; });
         wv.guess_first.assign(1, 0);
@@ -1311,7 +1311,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             wv.copy_first.push_back(0);
             for (CopyJob& j : wv.copies) {
                 j.tile_first = t;
-                t += (uint32_t)(((uint64_t)j.row_bytes * j.rows + kCopyTileBytes - 1) / kCopyTileBytes);
+                t += copy_tiles(j);
                 wv.copy_first.push_back(t);
             }
             for (int a = 0; a < 4; ++a) {
@@ -1947,7 +1947,7 @@ extern "C" int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, u
         wv.copy_first.push_back(0);
         for (CopyJob& j : wv.copies) {
             j.tile_first = t;
-            t += (uint32_t)(((uint64_t)j.row_bytes * j.rows + kCopyTileBytes - 1) / kCopyTileBytes);
+            t += copy_tiles(j);
             wv.copy_first.push_back(t);
         }
     }

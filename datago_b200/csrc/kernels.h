@@ -165,6 +165,9 @@ inline void cut_pass_tiles(ConvPass* passes, size_t n, bool vertical) {
     }
 }
 constexpr uint32_t kCopyTileBytes = 4096;
+inline uint32_t copy_tiles(const CopyJob& j) {  // tiles start at multiples of 16 of the destination's address
+    return (uint32_t)(((uint64_t)j.row_bytes * j.rows + 15 + kCopyTileBytes - 1) / kCopyTileBytes);
+}
 
 // the passes that take the tensor-core kernel (fast == 2) come first in `passes` and own tiles [0, mma_tiles)
 void launch_conv_h(const ConvPass* passes, OwnerMap map, const uint32_t* tables, uint32_t mma_tiles, cudaStream_t s);

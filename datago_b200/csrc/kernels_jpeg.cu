@@ -246,6 +246,7 @@ void launch_idct(const JpegWave& w, uint32_t first, uint32_t count, cudaStream_t
 //              neighbourhood -- one dp4a on bytes gathered from a shared-memory tile (1-sample halo, clamped to the
 //              real plane extent, which is what the edge rules of the filter amount to);
 //       4:4:4  and grayscale: straight from the planes;
+//       4:2:2  triangle filter along the row, from the planes;
 //       other samplings and chroma planes at most two samples wide: a plain per-pixel path.
 //     The +128 offsets and the rounding term are folded into one constant per channel; the luma byte is added with a
 //     one-hot dp4a; results are saturated and packed four at a time.
@@ -499,7 +500,46 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
         }
         return;
     }
-    // remaining samplings (4:2:2, 4:4:0, chroma planes at most two samples wide): one pixel at a time
+    if (hs == 2 && vs == 1 && dw > 2) {
+        // 4:2:2: (3 near + far + 1 or 2) >> 2 along the row.  A thread's eight pixels read four chroma samples (one aligned
+        // word) and their two neighbours; samples behind the real extent are the last real one, which makes the general
+        // form give the edge rules (3 t + t + 1 or 2) >> 2 = t.
+        const int c0 = x >> 1;
+        const bool inner = c0 + 4 < dw;
+#pragma unroll 2
+        for (int k = 0; k < nsteps; ++k) {
+            const int y = y_base + rowi + 8 * k;
+            if (y >= H) break;
+            int32_t cbv[8], crv[8];
+#pragma unroll
+            for (int comp = 1; comp <= 2; ++comp) {
+                const uint8_t* row = w.planes + d.plane_off[comp] + (size_t)y * d.plane_pitch[comp];
+                const uint32_t q = __ldg(reinterpret_cast<const uint32_t*>(row + c0));
+                int32_t t[6];
+                t[0] = __ldg(row + max(c0 - 1, 0));
+#pragma unroll
+                for (int i = 0; i < 4; ++i) t[i + 1] = (int32_t)((q >> (8 * i)) & 255u);
+                if (inner) t[5] = __ldg(row + c0 + 4);
+                else {
+                    const int32_t last = __ldg(row + dw - 1);
+#pragma unroll
+                    for (int i = 1; i < 6; ++i) if (c0 + i - 1 >= dw) t[i] = last;
+                }
+                int32_t (&v)[8] = comp == 1 ? cbv : crv;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    v[2 * i] = ((3 * t[i + 1] + t[i] + 1) >> 2) - 128;
+                    v[2 * i + 1] = ((3 * t[i + 1] + t[i + 2] + 2) >> 2) - 128;
+                }
+            }
+            const uint2 yv = __ldg(reinterpret_cast<const uint2*>(yp + (size_t)y * ypitch + x));
+            uint32_t px[6];
+            ycc_to_rgb8(yv.x, yv.y, cbv, crv, px);
+            store_rgb8(out + (size_t)y * d.out_pitch + x * 3, px, npx);
+        }
+        return;
+    }
+    // remaining samplings (4:4:0, chroma planes at most two samples wide): one pixel at a time
     const ChromaPlane cbp{w.planes + d.plane_off[1], d.plane_pitch[1], dw, dh, hs, vs};
     const ChromaPlane crp{w.planes + d.plane_off[2], d.plane_pitch[2], dw, dh, hs, vs};
 #pragma unroll 1
@@ -529,7 +569,7 @@ void launch_color(const JpegWave& w, uint32_t first_tile, uint32_t count, cudaSt
 //                  staged with asynchronous copies, the chroma tile (with its halo, which is why chroma cannot be
 //                  reconstructed tile by tile) loaded from the planes meanwhile, luma IDCT into shared memory, then
 //                  upsampling and colour conversion from shared memory, RGB out.
-// Traffic per pixel: 1 + 0.5 (chroma) + 2 + 0.5 + 3 (fused kernel) plus the zero write-back, against
+// Traffic per pixel, at most (all rows of all blocks): 1 + 0.5 (chroma) + 2 + 0.5 + 3 (fused kernel), against
 // 3 + 1.5 + 1.5 + 3 for the two general kernels.
 // ---------------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kIdctThreads, DG_IDCT_MIN_CTAS) k_idct_chroma(JpegWave w, uint32_t first, uint32_t count) {

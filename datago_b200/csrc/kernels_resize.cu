@@ -807,17 +807,42 @@ void launch_conv_v(const ConvPass* passes, OwnerMap map, const uint32_t* tables,
     if (map.total > mma_tiles) k_conv_v<<<map.total - mma_tiles, kConvVThreads, 0, s>>>(passes, map, tables, mma_tiles);
 }
 
-// ---- plain copies (identity payloads, integral crops without any filtering) ----------------------------------------
+// ---- plain copies (identity payloads, integral crops without any filtering, raw pixels handed through) ----------------
+// The destination is contiguous.  A thread moves 16 bytes that are aligned there: the source words under them, realigned
+// with funnel shifts (payloads of odd sizes start anywhere), one division per 16 bytes.  Pieces that cross a source row go
+// byte by byte, and so do the first and the last ones of a job, whose aligned words may reach outside the source.
 __global__ void __launch_bounds__(256) k_copy(const CopyJob* jobs, OwnerMap map) {
     const uint32_t ji = owner_of_tile(map, blockIdx.x);
     const CopyJob& j = jobs[ji];
+    uint8_t* const dst = j.dst;
+    const uint8_t* const src = j.src;
+    const bool flat = j.src_pitch == j.row_bytes;
     const uint64_t total = (uint64_t)j.row_bytes * j.rows;
-    const uint64_t base = (uint64_t)(blockIdx.x - j.tile_first) * kCopyTileBytes;
-    for (uint32_t i = threadIdx.x; i < kCopyTileBytes; i += 256) {
-        const uint64_t b = base + i;
-        if (b >= total) break;
-        const uint32_t y = (uint32_t)(b / j.row_bytes), x = (uint32_t)(b - (uint64_t)y * j.row_bytes);
-        j.dst[b] = __ldg(j.src + (size_t)y * j.src_pitch + x);
+    const uint32_t lead = (uint32_t)(reinterpret_cast<uintptr_t>(dst) & 15u);  // pieces start at multiples of 16 of the address
+    static_assert(kCopyTileBytes == 256 * 16, "one piece per thread");
+    const uint64_t at = (uint64_t)(blockIdx.x - j.tile_first) * kCopyTileBytes + threadIdx.x * 16;  // bytes [at - lead, at - lead + 16) of the payload
+    if (at >= total + lead) return;
+    if (at >= lead + 4u && at - lead + 20 <= total) {
+        const uint64_t b = at - lead;
+        const uint64_t y = flat ? 0 : (b >> 32) ? b / j.row_bytes : (uint32_t)b / j.row_bytes, x = b - y * j.row_bytes;
+        if (flat || x + 16 <= j.row_bytes) {
+            const uint8_t* s = src + y * j.src_pitch + x;
+            const uint32_t m = (uint32_t)(reinterpret_cast<uintptr_t>(s) & 15u);
+            uint4 v;
+            if (m == 0) v = __ldg(reinterpret_cast<const uint4*>(s));
+            else {
+                const uint32_t* w = reinterpret_cast<const uint32_t*>(s - (m & 3u));
+                const uint32_t sh = (m & 3u) * 8;
+                const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3), w4 = sh ? __ldg(w + 4) : 0u;
+                v = make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), __funnelshift_r(w2, w3, sh), __funnelshift_r(w3, w4, sh));
+            }
+            *reinterpret_cast<uint4*>(dst + b) = v;
+            return;
+        }
+    }
+    for (uint64_t b = at < lead ? 0 : at - lead; b < total && b + lead < at + 16; ++b) {
+        const uint64_t y = b / j.row_bytes, x = b - y * j.row_bytes;
+        dst[b] = __ldg(src + y * j.src_pitch + x);
     }
 }
 
@@ -831,12 +856,25 @@ void launch_copy(const CopyJob* jobs, OwnerMap map, cudaStream_t s) {
 __global__ void __launch_bounds__(256) k_alpha(const AlphaJob* jobs, OwnerMap map) {
     const AlphaJob& j = jobs[owner_of_tile(map, blockIdx.x)];
     const uint32_t base = (blockIdx.x - j.tile_first) * kAlphaTilePx, npx = j.width * j.rows, C = j.channels;
+    const bool words = C == 4 && ((reinterpret_cast<uintptr_t>(j.src) | reinterpret_cast<uintptr_t>(j.dst) | j.src_pitch | j.dst_pitch) & 3u) == 0;
+#pragma unroll 4
     for (uint32_t k = threadIdx.x; k < kAlphaTilePx; k += 256) {
         const uint32_t i = base + k;
         if (i >= npx) break;
         const uint32_t y = i / j.width, x = i - y * j.width;
         const uint8_t* s = j.src + (size_t)y * j.src_pitch + (size_t)x * C;
         uint8_t* d = j.dst + (size_t)y * j.dst_pitch + (size_t)x * C;
+        if (words) {  // RGBA pixels on word boundaries: one load, one store
+            const uint32_t px = *reinterpret_cast<const uint32_t*>(s), a = px >> 24, recip = a ? ((255u << 17) / a + 1u) >> 1 : 0u;
+            uint32_t r = px & 0xFF000000u;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const uint32_t v = (px >> (8 * c)) & 255u, t = v * a + 128u;
+                r |= (j.divide ? min(255u, (v * recip + (1u << 15)) >> 16) : ((t >> 8) + t) >> 8) << (8 * c);
+            }
+            *reinterpret_cast<uint32_t*>(d) = r;
+            continue;
+        }
         const uint32_t a = s[C - 1];
         const uint32_t recip = a ? ((255u << 17) / a + 1u) >> 1 : 0u;
         for (uint32_t c = 0; c + 1 < C; ++c) {
