@@ -278,18 +278,46 @@ __device__ __forceinline__ void ycc_to_rgb8(uint32_t y0, uint32_t y1, const int3
     }
 }
 
-__device__ __forceinline__ void store_rgb8(uint8_t* o, const uint32_t (&px)[6], int npx) {
-    if (npx == 8 && (reinterpret_cast<uintptr_t>(o) & 7u) == 0) {
-        uint2* o2 = reinterpret_cast<uint2*>(o);
-        __stcs(o2, make_uint2(px[0], px[1])); __stcs(o2 + 1, make_uint2(px[2], px[3])); __stcs(o2 + 2, make_uint2(px[4], px[5]));
-    } else {  // ragged right edge or an odd row start: byte by byte, the word index resolved at compile time
-        const int nb = npx * 3;
+// The lanes of `lanes` (lane 0 and its neighbours up, called by all of them together) store the 24 bytes of eight pixels each,
+// at consecutive places of a row.  Rows of odd-sized images start at any byte: a lane then stores the words that begin in
+// its piece, the first of them with the last bytes of its left neighbour's; the ends of the run go byte by byte (a byte at
+// a time for all of it, as before: 503 us for 96 images of 0.6 Mpixel, 141 by words).  npx < 8: the ragged piece at the right edge.
+__device__ __forceinline__ void store_rgb8(uint8_t* o, const uint32_t (&px)[6], int npx, uint32_t lanes) {
+    const uint32_t m = (uint32_t)(reinterpret_cast<uintptr_t>(o) & 7u);  // the same for all lanes
+    if (m == 0) {
+        if (npx == 8) {
+            uint2* o2 = reinterpret_cast<uint2*>(o);
+            __stcs(o2, make_uint2(px[0], px[1])); __stcs(o2 + 1, make_uint2(px[2], px[3])); __stcs(o2 + 2, make_uint2(px[4], px[5]));
+            return;
+        }
+    } else {
+        const uint32_t lane = threadIdx.x & 31, before = __shfl_up_sync(lanes, px[5], 1), right = __shfl_down_sync(lanes, (uint32_t)npx, 1);
+        if (npx == 8) {
+            const uint32_t k = m & 3u, sh = (32u - 8u * k) & 31u;
+            uint32_t* w = reinterpret_cast<uint32_t*>(o - k);
+            if (k == 0) {
 #pragma unroll
-        for (int wi = 0; wi < 6; ++wi)
+                for (int i = 0; i < 6; ++i) __stcs(w + i, px[i]);
+                return;
+            }
+            if (lane) __stcs(w, __funnelshift_r(before, px[0], sh));
+            else
+                for (uint32_t i = 0; i < 4 - k; ++i) o[i] = (uint8_t)(px[0] >> (8 * i));
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (wi * 4 + k < nb) o[wi * 4 + k] = (uint8_t)(px[wi] >> (8 * k));
+            for (int i = 1; i < 6; ++i) __stcs(w + i, __funnelshift_r(px[i - 1], px[i], sh));
+            const bool last = lane == 31 || !((lanes >> (lane + 1)) & 1u) || right != 8;  // nobody else stores this piece's last bytes
+            if (last)
+                for (uint32_t i = 4 - k; i < 4; ++i) o[20 + i] = (uint8_t)(px[5] >> (8 * i));
+            return;
+        }
     }
+    // ragged right edge: byte by byte, the word index resolved at compile time
+    const int nb = npx * 3;
+#pragma unroll
+    for (int wi = 0; wi < 6; ++wi)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (wi * 4 + k < nb) o[wi * 4 + k] = (uint8_t)(px[wi] >> (8 * k));
 }
 
 struct ChromaPlane {  // per-pixel path
@@ -445,6 +473,7 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
         return;
     }
     const int dw = (W + hs - 1) / hs, dh = (H + vs - 1) / vs;
+    const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, x < W);
     if (hs == 2 && vs == 2 && dw > 2) {
         load_chroma_tile(s_c, w, d, (int)tx, (int)ty, dw, dh);
         if (x >= W) return;
@@ -470,11 +499,11 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
             uint32_t px[6];
             if (yA >= 0) {
                 ycc_to_rgb8(ya.x, ya.y, cbA, crA, px);
-                store_rgb8(out + (size_t)yA * d.out_pitch + x * 3, px, npx);
+                store_rgb8(out + (size_t)yA * d.out_pitch + x * 3, px, npx, lanes);
             }
             if (yB < H) {
                 ycc_to_rgb8(yb.x, yb.y, cbB, crB, px);
-                store_rgb8(out + (size_t)yB * d.out_pitch + x * 3, px, npx);
+                store_rgb8(out + (size_t)yB * d.out_pitch + x * 3, px, npx, lanes);
             }
         }
         return;
@@ -496,7 +525,7 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
             const uint2 yv = __ldg(reinterpret_cast<const uint2*>(yp + (size_t)y * ypitch + x));
             uint32_t px[6];
             ycc_to_rgb8(yv.x, yv.y, cbv, crv, px);
-            store_rgb8(out + (size_t)y * d.out_pitch + x * 3, px, npx);
+            store_rgb8(out + (size_t)y * d.out_pitch + x * 3, px, npx, lanes);
         }
         return;
     }
@@ -535,7 +564,7 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
             const uint2 yv = __ldg(reinterpret_cast<const uint2*>(yp + (size_t)y * ypitch + x));
             uint32_t px[6];
             ycc_to_rgb8(yv.x, yv.y, cbv, crv, px);
-            store_rgb8(out + (size_t)y * d.out_pitch + x * 3, px, npx);
+            store_rgb8(out + (size_t)y * d.out_pitch + x * 3, px, npx, lanes);
         }
         return;
     }
@@ -795,6 +824,7 @@ __global__ void __launch_bounds__(kFusedThreads, DG_FUSED_MIN_CTAS) k_luma_color
     //      chroma tile rows p and p+1).  The tile's first row is the second half of pair 0 and its last row the first
     //      half of the pair after the last whole one: warp 0 converts those two halves in an extra step.
     const int x = (int)t.tx * (int)kColorTileW + (int)lane * 8;
+    const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, x < W);
     if (x >= W) return;
     const int npx = min(8, W - x);
     const int cl = (int)lane * 4 + 4;
@@ -810,7 +840,7 @@ __global__ void __launch_bounds__(kFusedThreads, DG_FUSED_MIN_CTAS) k_luma_color
             uint2* o2 = reinterpret_cast<uint2*>(o);
             __stcs(o2, make_uint2(px[0], px[1])); __stcs(o2 + 1, make_uint2(px[2], px[3])); __stcs(o2 + 2, make_uint2(px[4], px[5]));
         } else {
-            store_rgb8(o, px, npx);
+            store_rgb8(o, px, npx, lanes);
         }
     };
 #pragma unroll 1

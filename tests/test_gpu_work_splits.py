@@ -93,3 +93,14 @@ def test_resize_pass_cuts(h):
         for st, out, _ in ctx(cfg).process([x] * n):
             assert st == 0
             assert_same(out, want, str((h, n)))
+
+
+@pytest.mark.parametrize("sub", ["4:2:0", "4:4:4"])
+def test_colour_rows_at_every_alignment(sub):
+    # rows of odd-sized images start at any byte; tiles of 256 pixels end at, before and behind the right edge
+    rng = np.random.default_rng(340)
+    datas = [synth.encode_jpeg(rng.integers(0, 256, (21, w, 3), dtype=np.uint8), 90, sub, 0)
+             for w in list(range(5, 26)) + list(range(249, 273)) + [511, 513, 519]]
+    for data, (st, out, _) in zip(datas, ctx().process(datas)):
+        assert st == 0
+        assert_same(out, oracle.jpeg_decode(data), str(out.shape))
