@@ -439,7 +439,7 @@ class Batch:
                 it.forced_key = forced_keys[i].encode()
         self._h = C.c_void_p()
         _check(lib().dg_batch_create(ctx._h, self._items, self._n, flags, C.byref(self._h)))
-        self._outs = None
+        self._outs = []  # what copies are queued into: all of it stays alive until they have run (sync or close)
 
     def __len__(self):
         return self._n
@@ -452,8 +452,9 @@ class Batch:
 
     def close(self):
         if self._h:
-            lib().dg_batch_destroy(self._h)
+            lib().dg_batch_destroy(self._h)  # waits for the stream
             self._h = C.c_void_p()
+            self._outs = []
 
     def __del__(self):
         try:
@@ -469,6 +470,7 @@ class Batch:
 
     def sync(self):
         _check(lib().dg_batch_sync(self._h))
+        self._outs = []
 
     def result(self, i):
         r = Result()
@@ -495,7 +497,7 @@ class Batch:
                 return [None if r.status else block[r.packed_offset:r.packed_offset + r.nbytes].reshape(_shape(r)) for r in self.results()]
             outs = self.host_buffers()
         ptrs = (C.c_void_p * max(1, self._n))(*[o.ctypes.data if o is not None else None for o in outs])
-        self._outs = outs
+        self._outs.append(outs)
         _check(lib().dg_batch_download(self._h, ptrs))
         return outs
 
@@ -505,7 +507,7 @@ class Batch:
     def download_packed(self, host_buffer):
         """Queue ONE device->host copy of every payload into `host_buffer` (a writable uint8 numpy array, ideally
         pinned); payload i then sits at result(i).packed_offset.  Valid after sync()."""
-        self._outs = host_buffer
+        self._outs.append(host_buffer)
         _check(lib().dg_batch_download_packed(self._h, host_buffer.ctypes.data, host_buffer.nbytes))
 
     def buckets(self):
