@@ -482,19 +482,19 @@ class DatagoClient:
                     continue
             return False
 
+        units = []  # handed over a few at a time: every hand-over is a switch of threads
         try:
-            units = []  # handed over a few at a time: every hand-over is a switch of threads
             for unit in self._units():
                 units.append(unit)
                 if len(units) == READ_UNITS:
                     if not hand_over(units):
                         return
                     units = []
-            if units:
-                hand_over(units)
         except Exception:  # noqa: BLE001
             log.exception("datago_b200 reader failed")
         finally:
+            if units:  # also those read before a failure
+                hand_over(units)
             while not (self._stop.is_set() or self._reader_stop.is_set()):
                 try:
                     units_q.put(None, timeout=0.1)

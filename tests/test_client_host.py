@@ -5,6 +5,7 @@ import io
 import json
 import os
 import tarfile
+import threading
 
 import numpy as np
 import pytest
@@ -142,3 +143,29 @@ def test_host_decode_of_png_masks_and_other_formats():
     assert p[:4] == b"\x89PNG" and np.array_equal(np.asarray(Image.open(io.BytesIO(p))), mask)
     enc_payload = client.ImagePayload(p, 40, 60, 40, 60, -1, 8, True)
     assert enc_payload().size == (60, 40)
+
+
+def _read(monkeypatch, units, batch_size=32):
+    """What the reader thread of a client over `units` puts on its queue."""
+    import queue
+    c = client.DatagoClient.__new__(client.DatagoClient)
+    c.batch_size, c._stop, c._reader_stop = batch_size, threading.Event(), threading.Event()
+    monkeypatch.setattr(c, "_units", units, raising=False)
+    q = queue.Queue()
+    c._read_ahead(q)
+    got = []
+    while True:
+        x = q.get_nowait()
+        if x is None:
+            assert q.empty()
+            return got
+        got.append(x)
+
+
+@pytest.mark.parametrize("good", [0, 3, 8, 11])
+def test_samples_read_before_the_source_fails_are_handed_over(monkeypatch, good):
+    def units():
+        for i in range(good):
+            yield i
+        raise OSError("damaged shard")
+    assert [u for part in _read(monkeypatch, units) for u in part] == list(range(good))
