@@ -413,7 +413,7 @@ class DatagoClient:
         FIRST_UNITS samples at least, so the GPU starts early and batches grow while it is busy.  Samples leave in source
         order."""
         produced = 0
-        units_q = queue.Queue(maxsize=max(4 * self.batch_size // READ_UNITS, 4))
+        units_q = queue.Queue(maxsize=max(4 * self.batch_size, 16) // min(READ_UNITS, max(self.batch_size, 1)))
         reader = threading.Thread(target=self._read_ahead, args=(units_q,), daemon=True)
         reader.start()
         in_flight, flight_units = None, 0
@@ -482,11 +482,13 @@ class DatagoClient:
                     continue
             return False
 
-        units = []  # handed over a few at a time: every hand-over is a switch of threads
+        # Handed over a few at a time, because every hand-over is a switch of threads, but nothing that completes a batch or
+        # reaches the limit is held back: the source may take long to give the next sample.
+        units = []
         try:
-            for unit in self._units():
+            for n, unit in enumerate(self._units(), 1):
                 units.append(unit)
-                if len(units) == READ_UNITS:
+                if len(units) == READ_UNITS or n % max(self.batch_size, 1) == 0 or n >= self.limit:
                     if not hand_over(units):
                         return
                     units = []

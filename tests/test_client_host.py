@@ -145,11 +145,11 @@ def test_host_decode_of_png_masks_and_other_formats():
     assert enc_payload().size == (60, 40)
 
 
-def _read(monkeypatch, units, batch_size=32):
+def _read(monkeypatch, units, batch_size=32, limit=1000):
     """What the reader thread of a client over `units` puts on its queue."""
     import queue
     c = client.DatagoClient.__new__(client.DatagoClient)
-    c.batch_size, c._stop, c._reader_stop = batch_size, threading.Event(), threading.Event()
+    c.batch_size, c.limit, c._stop, c._reader_stop = batch_size, limit, threading.Event(), threading.Event()
     monkeypatch.setattr(c, "_units", units, raising=False)
     q = queue.Queue()
     c._read_ahead(q)
@@ -169,3 +169,12 @@ def test_samples_read_before_the_source_fails_are_handed_over(monkeypatch, good)
             yield i
         raise OSError("damaged shard")
     assert [u for part in _read(monkeypatch, units) for u in part] == list(range(good))
+
+
+@pytest.mark.parametrize("batch_size,limit", [(1, 100), (3, 100), (8, 100), (12, 100), (32, 100), (32, 5), (12, 14)])
+def test_the_reader_holds_back_nothing_a_batch_waits_for(monkeypatch, batch_size, limit):
+    parts = _read(monkeypatch, lambda: iter(range(40)), batch_size, limit)
+    assert [u for part in parts for u in part] == list(range(40))
+    assert max(len(p) for p in parts) <= client.READ_UNITS
+    handed = set(np.cumsum([len(p) for p in parts]).tolist())  # units the engine has whenever a part has been handed over
+    assert {n for n in range(1, 41) if n % batch_size == 0 or n >= limit} <= handed
