@@ -38,6 +38,7 @@ FILE_EXTENSIONS = ("jpg", "jpeg", "png", "bmp", "gif", "webp")  # src/generator_
 TIMEOUT_S = 300                             # src/client.rs:12
 READ_UNITS = 8                              # samples the reader thread hands over at a time
 FIRST_UNITS = 16                            # samples that are worth a batch
+_PAYLOAD_LOCK = threading.Lock()            # the switch of a payload from the view it arrived as to bytes
 
 
 class ImagePayload:
@@ -55,13 +56,18 @@ class ImagePayload:
 
     @property
     def data(self):
-        if self._view is not None:
-            self._data, self._view = self._view.tobytes(), None
+        view = self._view  # read once: another thread may be at the same place
+        if view is not None:
+            data = view.tobytes()
+            with _PAYLOAD_LOCK:
+                if self._view is view:
+                    self._data, self._view = data, None
         return self._data
 
     @data.setter
     def data(self, value):
-        self._data, self._view = value, None
+        with _PAYLOAD_LOCK:
+            self._data, self._view = value, None
 
     def _shape(self):
         return (self.height, self.width, self.channels) if self.channels > 1 else (self.height, self.width)
@@ -72,8 +78,9 @@ class ImagePayload:
             import io
             from PIL import Image
             return np.asarray(Image.open(io.BytesIO(self.data)).convert("RGB"))
-        if self._view is not None:
-            return self._view.reshape(self._shape())
+        view = self._view
+        if view is not None:
+            return view.reshape(self._shape())
         if self._device_ptr and not len(self.data):
             return self._keepalive.ctx.copy_to_host(self._device_ptr, self.height * self.width * self.channels).reshape(self._shape())
         return np.frombuffer(self.data, np.uint8).reshape(self._shape())

@@ -178,3 +178,27 @@ def test_the_reader_holds_back_nothing_a_batch_waits_for(monkeypatch, batch_size
     assert max(len(p) for p in parts) <= client.READ_UNITS
     handed = set(np.cumsum([len(p) for p in parts]).tolist())  # units the engine has whenever a part has been handed over
     assert {n for n in range(1, 41) if n % batch_size == 0 or n >= limit} <= handed
+
+
+@pytest.mark.parametrize("read", [lambda p: p.data, lambda p: p.to_numpy_array().tobytes()])
+def test_a_payload_is_read_by_two_threads_at_once(read):
+    class Payload(client.ImagePayload):  # whenever one thread looks at the view, another one turns it into bytes
+        busy = True
+
+        def __getattribute__(self, name):
+            value = super().__getattribute__(name)
+            if name == "_view" and not self.busy:
+                self.busy = True
+                t = threading.Thread(target=lambda: seen.append(self.data))
+                t.start()
+                t.join()
+                self.busy = False
+            return value
+
+    seen = []
+    a = np.arange(48, dtype=np.uint8)
+    p = Payload(height=4, width=4, channels=3, view=a)
+    p.busy = False
+    assert read(p) == a.tobytes() and seen[0] == a.tobytes()
+    p.data = b"other"
+    assert p.data == b"other"
