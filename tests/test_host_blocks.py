@@ -1,0 +1,122 @@
+"""The pool of page-locked blocks (csrc/host_blocks.cpp), built against a stand-in for the CUDA runtime: sizes, references,
+bounds, and what a forked child sees."""
+import ctypes as C
+import os
+import subprocess
+import sys
+import threading
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "datago_b200", "csrc")
+MB = 1 << 20
+E_TOO_LARGE = 11
+
+
+@pytest.fixture(scope="session")
+def library(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("fake") / "libhost_blocks.so")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-pthread", "-Wl,-Bsymbolic", "-I", os.path.join(cuda, "include"),
+                    os.path.join(ROOT, "tests", "fake_cuda.cpp"), os.path.join(CSRC, "host_blocks.cpp"), "-o", out], check=True)
+    return out
+
+
+@pytest.fixture
+def pool(library, tmp_path, monkeypatch):
+    monkeypatch.setenv("DATAGO_B200_HOST_BLOCKS_MB", "8")
+    private = str(tmp_path / "lib.so")  # a copy of its own: the pool starts empty
+    with open(library, "rb") as f, open(private, "wb") as g:
+        g.write(f.read())
+    L = C.CDLL(private)
+    L.hb_acquire.argtypes = [C.c_size_t, C.c_int, C.POINTER(C.c_void_p)]
+    L.dg_host_alloc.argtypes = [C.c_uint64, C.POINTER(C.c_void_p)]
+    L.dg_host_release.argtypes = L.hb_retain.argtypes = L.fake_locked_on.argtypes = [C.c_void_p]
+    L.fake_locked_bytes.restype = C.c_size_t
+    return L
+
+
+def take(L, n, optional=1):
+    p = C.c_void_p()
+    assert L.hb_acquire(n, optional, C.byref(p)) == 0
+    return p.value
+
+
+def test_blocks_are_reused_counted_and_given_back(pool):
+    pool.hb_context(0, 1)
+    a = take(pool, 3 * MB - 5)
+    C.memset(a, 1, 3 * MB - 5)
+    b = take(pool, 100)
+    pool.hb_retain(a)
+    pool.dg_host_release(a)
+    assert take(pool, 3 * MB) != a                # one reference is left
+    pool.dg_host_release(a)
+    assert take(pool, 3 * MB - 5) == a            # idle now
+    pool.dg_host_release(b)
+    assert take(pool, 2 * MB) != b                # far too small
+    pool.dg_host_release(a)
+    pool.dg_host_release(a)                       # once too often: nothing happens
+    before = pool.fake_locked_bytes()
+    pool.hb_context(0, -1)                        # the last context: idle blocks go, referenced ones stay
+    assert 0 < pool.fake_locked_bytes() < before
+
+
+def test_limits_hold_for_what_is_referenced_and_for_what_is_idle(pool):
+    pool.hb_context(0, 1)
+    held = [take(pool, MB) for _ in range(8)]
+    p = C.c_void_p()
+    assert not pool.hb_scarce()
+    assert pool.dg_host_alloc(1, C.byref(p)) == E_TOO_LARGE and not p.value
+    more = [take(pool, 2 * MB, 0) for _ in range(3)]  # a caller without an alternative gets its block
+    assert pool.hb_scarce()
+    for x in more + held:
+        pool.dg_host_release(x)
+    assert not pool.hb_scarce() and pool.fake_locked_bytes() <= 8 * MB
+    assert pool.dg_host_alloc(8 * MB, C.byref(p)) == 0
+
+
+def test_threads_at_once(pool):
+    pool.hb_context(0, 1)
+
+    def work(seed):
+        for i in range(300):
+            p = C.c_void_p()
+            if pool.hb_acquire(1 + (i * seed) % (2 * MB), 1, C.byref(p)) == 0:
+                C.memset(p.value, seed, 16)
+                pool.hb_retain(p)
+                pool.dg_host_release(p)
+                assert C.string_at(p.value, 16) == bytes([seed]) * 16
+                pool.dg_host_release(p)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in (3, 7, 11, 201)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    pool.hb_context(0, -1)
+    assert pool.fake_locked_bytes() == 0
+
+
+@pytest.mark.parametrize("nbytes", [1000, 3 * MB])
+def test_a_forked_child_keeps_its_own_copy(pool, nbytes):
+    script = """
+import ctypes as C, os, sys
+L = C.CDLL(sys.argv[1]); n = int(sys.argv[2])
+L.hb_acquire.argtypes = [C.c_size_t, C.c_int, C.POINTER(C.c_void_p)]
+p = C.c_void_p()
+assert L.hb_acquire(n, 1, C.byref(p)) == 0
+C.memset(p.value, 7, n)
+r, w = os.pipe()
+pid = os.fork()
+if pid == 0:
+    os.read(r, 1)
+    ok = C.string_at(p.value, n) == bytes([7]) * n
+    C.memset(p.value, 9, n)
+    os._exit(0 if ok else 1)
+C.memset(p.value, 8, n)  # the pool has handed the block on
+os.write(w, b"x")
+_, status = os.waitpid(pid, 0)
+sys.exit(0 if status == 0 and C.string_at(p.value, n) == bytes([8]) * n else 1)
+"""
+    subprocess.run([sys.executable, "-c", script, pool._name, str(nbytes)], check=True)
