@@ -256,7 +256,7 @@ static int ctx_create(int device, const dg_image_config* cfg, void* stream, bool
     if (!encode_tiled_fn()) c->hmma = false;  // a driver without tensor maps: every horizontal pass takes the dp2a kernel
     if (const char* mb = getenv("DATAGO_B200_MAX_IMAGE_MB")) { long v = atol(mb); if (v >= 1) c->max_image_bytes = (uint64_t)v << 20; }
     if (const char* mb = getenv("DATAGO_B200_WAVE_MB")) { long v = atol(mb); if (v >= 16) c->wave_bytes = (size_t)v << 20; }
-    host_blocks_context(+1);
+    host_blocks_context(device, +1);
     *out = c;
     return DG_OK;
 }
@@ -282,8 +282,8 @@ extern "C" void dg_ctx_destroy(dg_ctx* c) {
     }
     cudaStreamDestroy(c->stream2);
     if (c->own_stream) cudaStreamDestroy(c->stream);
+    host_blocks_context(c->device, -1);
     delete c;
-    host_blocks_context(-1);
 }
 
 extern "C" void* dg_ctx_stream(dg_ctx* c) { return c ? (void*)c->stream : nullptr; }

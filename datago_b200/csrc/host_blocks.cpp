@@ -8,6 +8,8 @@
 #include <map>
 #include <mutex>
 #include <new>
+#include <system_error>
+#include <thread>
 #include <unordered_map>
 #include <utility>
 #include <vector>
@@ -25,7 +27,8 @@ struct Pool {
     std::unordered_map<void*, Entry> blocks;
     std::multimap<size_t, void*> free;  // those with refs == 0, by size
     size_t busy = 0, idle = 0, limit;
-    int contexts = 0;
+    std::map<int, int> contexts;  // live ones per device
+    int last_device = -1;
     Pool() {
         const char* mb = getenv("DATAGO_B200_HOST_BLOCKS_MB");
         const long v = mb ? atol(mb) : 1024;
@@ -41,6 +44,7 @@ struct Pool {
             free.erase(it);
         }
     }
+    int device() const { return contexts.empty() ? last_device : contexts.count(last_device) ? last_device : contexts.begin()->first; }
 };
 
 Pool& pool() {
@@ -56,6 +60,20 @@ size_t rounded(size_t n) {  // eight sizes per power of two, so that blocks of s
     return (n + step - 1) / step * step;
 }
 
+// Runs f with `device` current and leaves the calling thread as it is: making another device current, or going back to one
+// that was never used, creates a context there, so a thread of its own does it.  False: no thread to be had, f has not run.
+template <class F>
+bool on_device(int device, F&& f) {
+    int now = -1;
+    if (device < 0 || (cudaGetDevice(&now) == cudaSuccess && now == device)) { f(); return true; }
+    try {
+        std::thread([&] { cudaSetDevice(device); f(); }).join();
+    } catch (const std::system_error&) {
+        return false;
+    }
+    return true;
+}
+
 void* map_block(size_t size) {
     const size_t extra = size >= kHuge ? kHuge : 0;  // large blocks start at a huge page: locking them is four times as quick
     void* at = mmap(nullptr, size + extra, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
@@ -69,17 +87,20 @@ void* map_block(size_t size) {
     return p;
 }
 
-void free_all(const std::vector<std::pair<void*, size_t>>& gone) {
-    for (const auto& b : gone) {
-        cudaHostUnregister(b.first);
-        munmap(b.first, b.second);
-    }
-    if (!gone.empty()) cudaGetLastError();
+void free_all(const std::vector<std::pair<void*, size_t>>& gone, int device) {
+    if (gone.empty()) return;
+    const auto unlock = [&] {
+        for (const auto& b : gone) cudaHostUnregister(b.first);
+        cudaGetLastError();
+    };
+    if (!on_device(device, unlock)) unlock();
+    for (const auto& b : gone) munmap(b.first, b.second);
 }
 
 int acquire(size_t nbytes, bool optional, void** out) {
     Pool& p = pool();
     const size_t need = rounded(nbytes ? nbytes : 1);
+    int device;
     {
         std::lock_guard<std::mutex> lock(p.mu);
         if (optional && p.busy + need > p.limit) return dg_set_error(DG_E_TOO_LARGE, "host blocks: too much is in use");
@@ -93,10 +114,11 @@ int acquire(size_t nbytes, bool optional, void** out) {
             return DG_OK;
         }
         p.busy += need;
+        device = p.device();
     }
     void* const ptr = map_block(need);
     cudaError_t err = cudaErrorMemoryAllocation;
-    if (ptr && (err = cudaHostRegister(ptr, need, cudaHostRegisterPortable)) != cudaSuccess) cudaGetLastError();
+    if (ptr) on_device(device, [&] { if ((err = cudaHostRegister(ptr, need, cudaHostRegisterPortable)) != cudaSuccess) cudaGetLastError(); });
     std::lock_guard<std::mutex> lock(p.mu);
     if (err != cudaSuccess) {
         if (ptr) munmap(ptr, need);
@@ -130,6 +152,7 @@ void host_block_release(void* base) {
     if (!base) return;
     Pool& p = pool();
     std::vector<std::pair<void*, size_t>> gone;
+    int device;
     {
         std::lock_guard<std::mutex> lock(p.mu);
         auto it = p.blocks.find(base);
@@ -138,9 +161,10 @@ void host_block_release(void* base) {
         p.busy -= it->second.size;
         p.idle += it->second.size;
         p.free.emplace(it->second.size, base);
-        p.trim(p.contexts <= 0 ? 0 : p.limit, &gone);
+        p.trim(p.contexts.empty() ? 0 : p.limit, &gone);
+        device = p.device();
     }
-    free_all(gone);
+    free_all(gone, device);
 }
 
 bool host_blocks_scarce() {
@@ -149,15 +173,16 @@ bool host_blocks_scarce() {
     return p.busy > p.limit;
 }
 
-void host_blocks_context(int change) {
+void host_blocks_context(int device, int change) {
     Pool& p = pool();
     std::vector<std::pair<void*, size_t>> gone;
     {
         std::lock_guard<std::mutex> lock(p.mu);
-        p.contexts += change;
-        if (p.contexts <= 0) p.trim(0, &gone);
+        if ((p.contexts[device] += change) <= 0) p.contexts.erase(device);
+        p.last_device = device;
+        if (p.contexts.empty()) p.trim(0, &gone);
     }
-    free_all(gone);
+    free_all(gone, device);
 }
 
 }  // namespace dg

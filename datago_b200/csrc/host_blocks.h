@@ -22,6 +22,8 @@ int host_block_acquire(size_t nbytes, bool optional, void** out);  // dg_status;
 void host_block_retain(void* base);
 void host_block_release(void* base);
 bool host_blocks_scarce();  // whether more than the limit is referenced
-void host_blocks_context(int change);  // +1 / -1 device context
+// +1 / -1 context on `device`.  Blocks are page-locked on a device that has one: the calling thread's current device may be
+// another rank's, and locking there would create a context on it.
+void host_blocks_context(int device, int change);
 
 }  // namespace dg

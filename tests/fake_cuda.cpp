@@ -83,7 +83,7 @@ void fake_device_limit(size_t n) { std::lock_guard<std::mutex> l(mu); device_lim
 int hb_acquire(size_t n, int optional, void** out) { return dg::host_block_acquire(n, optional != 0, out); }
 void hb_retain(void* p) { dg::host_block_retain(p); }
 int hb_scarce() { return dg::host_blocks_scarce(); }
-void hb_context(int, int change) { dg::host_blocks_context(change); }
+void hb_context(int device, int change) { dg::host_blocks_context(device, change); }
 }
 
 int dg::dg_set_error(int code, const char*) { return code; }

@@ -1,5 +1,5 @@
 """The pool of page-locked blocks (csrc/host_blocks.cpp), built against a stand-in for the CUDA runtime: sizes, references,
-bounds, and what a forked child sees."""
+bounds, the device the locking happens on, and what a forked child sees."""
 import ctypes as C
 import os
 import subprocess
@@ -74,6 +74,16 @@ def test_limits_hold_for_what_is_referenced_and_for_what_is_idle(pool):
         pool.dg_host_release(x)
     assert not pool.hb_scarce() and pool.fake_locked_bytes() <= 8 * MB
     assert pool.dg_host_alloc(8 * MB, C.byref(p)) == 0
+
+
+def test_locking_happens_on_a_device_that_has_a_context(pool):
+    pool.hb_context(3, 1)  # (this thread has never made a CUDA call: its current device is 0)
+    a, b = take(pool, 100), take(pool, 5 * MB)
+    assert pool.fake_locked_on(a) == pool.fake_locked_on(b) == 3
+    pool.dg_host_release(a)
+    pool.hb_context(3, -1)
+    pool.dg_host_release(b)
+    assert pool.fake_locked_bytes() == 0 and not pool.fake_contexts(0)
 
 
 def test_threads_at_once(pool):
