@@ -183,6 +183,7 @@ extern "C" {
     pub fn dg_batch_run(b: *mut dg_batch) -> c_int;
     pub fn dg_batch_download(b: *mut dg_batch, host_out: *const *mut u8) -> c_int;
     pub fn dg_batch_download_packed(b: *mut dg_batch, host_base: *mut u8, capacity: u64) -> c_int;
+    pub fn dg_batch_download_views(b: *mut dg_batch, host_out: *mut *const u8, blocks: *mut *mut c_void) -> c_int;
     pub fn dg_batch_packed_bytes(b: *const dg_batch) -> u64;
     pub fn dg_batch_sync(b: *mut dg_batch) -> c_int;
     pub fn dg_batch_result(b: *const dg_batch, i: c_int, out: *mut dg_result) -> c_int;

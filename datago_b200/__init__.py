@@ -179,6 +179,7 @@ def lib():
         "dg_batch_download": (C.c_int, [vp, C.POINTER(vp)]),
         "dg_batch_download_packed": (C.c_int, [vp, vp, C.c_uint64]),
         "dg_batch_packed_bytes": (C.c_uint64, [vp]),
+        "dg_batch_download_views": (C.c_int, [vp, C.POINTER(vp), C.POINTER(vp)]),
         "dg_batch_sync": (C.c_int, [vp]),
         "dg_batch_result": (C.c_int, [vp, C.c_int, C.POINTER(Result)]),
         "dg_batch_results": (C.c_int, [vp, C.POINTER(Result)]),
@@ -216,7 +217,7 @@ def lib():
 EXPORTS = ("dg_set_log_callback dg_ctx_get_counters dg_last_error dg_version dg_ctx_create dg_ctx_create_on_stream dg_ctx_destroy dg_ctx_stream dg_size_list "
            "dg_bucket_table dg_closest_aspect_ratio dg_aspect_ratio_to_str dg_plan_geometry dg_jpeg_probe dg_rank_slice "
            "dg_key_hash dg_key_rank dg_batch_create dg_batch_upload dg_batch_run dg_batch_download dg_batch_sync "
-           "dg_batch_download_packed dg_batch_packed_bytes dg_batch_bucket_count dg_batch_bucket "
+           "dg_batch_download_packed dg_batch_download_views dg_batch_packed_bytes dg_batch_bucket_count dg_batch_bucket "
            "dg_batch_result dg_batch_results dg_batch_stage_ms dg_batch_counters dg_batch_huffman_stats dg_batch_debug dg_batch_destroy dg_process "
            "dg_copy_to_host dg_resize_device_static dg_feeder_create dg_feeder_ctx dg_submit dg_wait dg_fetch dg_peek dg_fetch_view dg_release dg_host_alloc dg_host_release "
            "dg_feeder_get_stats dg_feeder_destroy").split()
@@ -489,17 +490,28 @@ class Batch:
 
     def download(self, outs=None):
         """Queue device->host copies into `outs` (from host_buffers()); valid after sync().  Without `outs` the payloads arrive in
-        one copy in page-locked memory, and the arrays returned are views of it (which lives as long as any of them)."""
+        page-locked memory, and the arrays returned are views of it (see download_views)."""
         if outs is None:
-            block = host_block(self.packed_bytes())
-            if block is not None:
-                self.download_packed(block)
-                return [None if r.status else block[r.packed_offset:r.packed_offset + r.nbytes].reshape(_shape(r)) for r in self.results()]
+            outs = self.download_views()
+            if outs is not None:
+                return outs
             outs = self.host_buffers()
         ptrs = (C.c_void_p * max(1, self._n))(*[o.ctypes.data if o is not None else None for o in outs])
         self._outs.append(outs)
         _check(lib().dg_batch_download(self._h, ptrs))
         return outs
+
+    def download_views(self):
+        """Queue copies of the payloads into page-locked blocks of the library, a few payloads to a block of about 4 MB (which
+        lives as long as any of their arrays): one writable array per ok payload, None for the others; valid after sync().
+        None while so much of this memory is in use that ordinary memory has to do."""
+        ptrs, blocks = (C.c_void_p * max(1, self._n))(), (C.c_void_p * max(1, self._n))()
+        rc = lib().dg_batch_download_views(self._h, ptrs, blocks)
+        if rc == E_TOO_LARGE:
+            return None
+        _check(rc)
+        return [np.asarray(_HostBlock(ptrs[i], r.nbytes, C.c_void_p(blocks[i]))).reshape(_shape(r)) if blocks[i] else None
+                for i, r in enumerate(self.results())]
 
     def packed_bytes(self):
         return int(lib().dg_batch_packed_bytes(self._h))

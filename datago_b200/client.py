@@ -28,7 +28,7 @@ import threading
 
 import numpy as np
 
-from . import BATCH_DECODE_ONLY, Context, DatagoB200Error, aspect_ratio_to_str, host_block, jpeg_probe, key_rank, rank_slice
+from . import BATCH_DECODE_ONLY, Context, DatagoB200Error, aspect_ratio_to_str, jpeg_probe, key_rank, rank_slice
 
 log = logging.getLogger("datago_b200")
 
@@ -571,21 +571,18 @@ class DatagoClient:
         batch = self.ctx.batch(inputs, keys, 0 if has_tfm else BATCH_DECODE_ONLY, to_rgb8=to_rgb8)
         batch.upload()
         batch.run()
-        buf, views = None, False
+        buf, views = None, None
         if not self.device_payloads and len(batch):
-            buf = None if self.pre_encode else host_block(batch.packed_bytes())  # samples keep views of it
-            views = buf is not None
-            if not views:
+            views = None if self.pre_encode else batch.download_views()  # samples keep them
+            if views is None:
                 buf = self._host_buffer(lane, batch.packed_bytes())
-            batch.download_packed(buf)  # one copy; payload i lands at result(i).packed_offset
+                batch.download_packed(buf)  # one copy; payload i lands at result(i).packed_offset
         return batch, units, slots, buf, views
 
     def _finish(self, launched):
         """Waits for a launched batch and puts its samples on the queue; returns how many it made."""
         batch, units, slots, buf, views = launched
         batch.sync()
-        if views:
-            buf.flags.writeable = False  # payloads are read-only, as bytes are
         results = batch.results()
         made = 0
         payloads = {}
@@ -600,8 +597,13 @@ class DatagoClient:
                                   original_height=r.original_height, original_width=r.original_width, height=r.height,
                                   width=r.width, channels=-1, bit_depth=8, is_encoded=True)
             else:
-                px = None if self.device_payloads else buf[r.packed_offset:r.packed_offset + r.nbytes]
-                pl = ImagePayload(data=b"" if px is None or views else px.tobytes(), view=px if views else None, original_height=r.original_height,
+                data, view = b"", None
+                if views is not None:
+                    view = views[i].reshape(-1)
+                    view.flags.writeable = False  # payloads are read-only, as bytes are
+                elif not self.device_payloads:
+                    data = buf[r.packed_offset:r.packed_offset + r.nbytes].tobytes()
+                pl = ImagePayload(data=data, view=view, original_height=r.original_height,
                                   original_width=r.original_width, height=r.height, width=r.width, channels=r.channels,
                                   bit_depth=8, is_encoded=False, device_ptr=r.device_data if self.device_payloads else 0,
                                   keepalive=batch if self.device_payloads else None)

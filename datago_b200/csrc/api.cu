@@ -488,6 +488,7 @@ struct dg_batch {
     size_t blob_bytes = 0, rawin_bytes = 0, out_bytes = 0;
     size_t arena_bytes = 0;  // out_bytes plus the pre-conversion images of DG_ITEM_TO_RGB8 items (never downloaded)
     size_t m_huff = 0, m_qt = 0, m_tables = 0, meta_total = 0;  // meta_total: meta.bytes plus the filter tables behind it
+    std::vector<void*> landing;  // page-locked blocks that copies are queued into: a reference each until they have run
     std::vector<const uint8_t*> raw_src;  // caller memory of raw items (used inside dg_batch_create only)
     uint64_t h2d = 0, d2h = 0;
     uint32_t launches = 0;
@@ -1677,6 +1678,56 @@ extern "C" int dg_batch_download(dg_batch* b, uint8_t* const* host_out) {
     return DG_OK;
 }
 
+// One copy per kLandingBytes of payloads: a caller that keeps a payload keeps what came with it, so a block must not hold a whole
+// batch; copies of 4 MB run at 54 GB/s, of 1 MB at 48 (one copy for everything: 57).
+constexpr size_t kLandingBytes = (size_t)4 << 20;
+
+int dg::batch_download_blocks(dg_batch* b, uint8_t** host, void** blocks) {
+    dg_ctx* ctx = b->ctx;
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    CU(cudaSetDevice(ctx->device));
+    std::vector<int> order;  // as the payloads lie in the arena
+    for (int i = 0; i < b->n; ++i) {
+        host[i] = nullptr; blocks[i] = nullptr;
+        if (!b->items[i].status) order.push_back(i);
+    }
+    const auto off = [&](size_t k) { return b->items[order[k]].out_off; };
+    const auto end = [&](size_t k) { return off(k) + b->items[order[k]].out_bytes; };
+    std::sort(order.begin(), order.end(), [&](int x, int y) { return b->items[x].out_off < b->items[y].out_off; });
+    b->d2h = 0;
+    int rc = DG_OK;
+    for (size_t k = 0, next; k < order.size() && !rc; k = next) {
+        for (next = k + 1; next < order.size() && end(next) - off(k) <= kLandingBytes;) ++next;
+        void* block = nullptr;
+        const size_t len = end(next - 1) - off(k);
+        rc = host_block_acquire(len, false, &block);
+        if (rc) break;
+        b->landing.push_back(block);
+        const cudaError_t e = cudaMemcpyAsync(block, b->d_persist + b->off_out + off(k), len, cudaMemcpyDeviceToHost, ctx->stream);
+        if (e != cudaSuccess) { rc = fail(DG_E_CUDA, "download: %s", cudaGetErrorString(e)); break; }
+        for (size_t j = k; j < next; ++j) {
+            host_block_retain(block);
+            host[order[j]] = (uint8_t*)block + (off(j) - off(k));
+            blocks[order[j]] = block;
+            b->d2h += b->items[order[j]].out_bytes;
+        }
+    }
+    if (rc)
+        for (int i = 0; i < b->n; ++i) { host_block_release(blocks[i]); host[i] = nullptr; blocks[i] = nullptr; }
+    return rc;
+}
+
+extern "C" int dg_batch_download_views(dg_batch* b, const uint8_t** host_out, void** blocks) {
+    if (!b || !host_out || !blocks) return fail(DG_E_INVALID, "NULL argument");
+    if (!host_blocks_room(b->out_bytes)) return fail(DG_E_TOO_LARGE, "too much page-locked memory is in use");
+    return batch_download_blocks(b, const_cast<uint8_t**>(host_out), blocks);
+}
+
+static void landed(dg_batch* b) {  // nothing is queued into them any more
+    for (void* block : b->landing) host_block_release(block);
+    b->landing.clear();
+}
+
 extern "C" uint64_t dg_batch_packed_bytes(const dg_batch* b) { return b ? b->out_bytes : 0; }
 
 extern "C" int dg_batch_download_packed(dg_batch* b, uint8_t* host_base, uint64_t capacity) {
@@ -1708,6 +1759,7 @@ extern "C" int dg_batch_sync(dg_batch* b) {
         b->d2h += (size_t)b->n * 4;
     }
     CU(cudaStreamSynchronize(ctx->stream));
+    landed(b);
     if (b->ran && b->used_hmma) {
         // the tensor-core resize pass bounds its waits for asynchronous copies; a wait that ran out left garbage behind
         const unsigned int t = read_conv_timeouts(ctx->stream);
@@ -1822,6 +1874,7 @@ extern "C" void dg_batch_destroy(dg_batch* b) {
     std::lock_guard<std::mutex> lock(ctx->mu);
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    landed(b);
     for (StageEvent& se : b->events) { cudaEventDestroy(se.a); cudaEventDestroy(se.b); }
     ctx->dev.release(b->blk_persist);
     ctx->dev.release(b->blk_meta);

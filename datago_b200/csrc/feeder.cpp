@@ -31,12 +31,10 @@ using Clock = std::chrono::steady_clock;
 
 struct Lane;
 
-// One finished batch: keeps the device payloads and their page-locked host copy alive until the last ticket lets go (the
-// host copy longer, if somebody took a view of it).
+// One finished batch: keeps the device payloads alive until the last ticket lets go.
 struct Flight {
     Lane* lane = nullptr;
     dg_batch* batch = nullptr;
-    uint8_t* pinned = nullptr;  // a host block
     std::atomic<int> refs{0};
 };
 
@@ -51,6 +49,8 @@ struct Ticket {
     uint64_t host_cap = 0;
     dg_result res{};
     Flight* flight = nullptr;
+    uint8_t* host = nullptr;  // the page-locked host copy of the payload, and the ticket's reference on the block it lies in
+    void* block = nullptr;
     Clock::time_point t_submit;
 };
 
@@ -96,7 +96,6 @@ void bury(Lane& lane) {
     }
     for (Flight* f : dead) {
         if (f->batch) dg_batch_destroy(f->batch);
-        dg::host_block_release(f->pinned);
         delete f;
     }
 }
@@ -118,6 +117,8 @@ void lane_main(dg_feeder* f, Lane* lane) {
     cudaSetDevice(f->device);
     std::vector<Ticket*> group;
     std::vector<dg_item> items;
+    std::vector<uint8_t*> host;
+    std::vector<void*> blocks;
     for (;;) {
         bury(*lane);
         group.clear();
@@ -153,18 +154,18 @@ void lane_main(dg_feeder* f, Lane* lane) {
         if (!rc) rc = dg_batch_upload(batch);
         for (Ticket* t : group) { std::vector<uint8_t>().swap(t->bytes); }  // staged: the copies are no longer needed
         if (!rc) rc = dg_batch_run(batch);
-        void* landing = nullptr;
-        if (!rc) rc = dg::host_block_acquire(dg_batch_packed_bytes(batch), false, &landing);
-        if (!rc) rc = dg_batch_download_packed(batch, (uint8_t*)landing, dg_batch_packed_bytes(batch));
+        host.assign(n, nullptr);
+        blocks.assign(n, nullptr);
+        if (!rc) rc = dg::batch_download_blocks(batch, host.data(), blocks.data());
         if (!rc) rc = dg_batch_sync(batch);
         if (rc) {
             if (batch) dg_batch_destroy(batch);
-            dg::host_block_release(landing);
+            for (void* block : blocks) dg::host_block_release(block);
             fail_all(f, group, rc);
             continue;
         }
         Flight* fl = new Flight();
-        fl->lane = lane; fl->batch = batch; fl->pinned = (uint8_t*)landing;
+        fl->lane = lane; fl->batch = batch;
         fl->refs.store(n + 1);  // one per ticket + this thread's own
         {
             std::lock_guard<std::mutex> lock(f->mu);
@@ -174,6 +175,8 @@ void lane_main(dg_feeder* f, Lane* lane) {
                 t->state = 2;
                 ++f->stats.completed;
                 if (t->res.status) ++f->stats.failed;
+                if (t->orphan || t->res.status) dg::host_block_release(blocks[i]);
+                else { t->host = host[i]; t->block = blocks[i]; }
                 if (t->orphan) { f->tickets.erase(t->id); unref(fl); }
                 else t->flight = fl;
             }
@@ -241,10 +244,10 @@ extern "C" int dg_submit(dg_feeder* f, const dg_item* item, uint8_t* host_out, u
     return DG_OK;
 }
 
-static int copy_out(Ticket* t, Flight* fl, uint8_t* dst, uint64_t cap) {
+static int copy_out(Ticket* t, uint8_t* dst, uint64_t cap) {
     if (t->res.status) return DG_OK;  // nothing to copy; the status travels in the result
     if (cap < t->res.nbytes) return set_error(DG_E_INVALID, "host buffer smaller than the payload");
-    memcpy(dst, fl->pinned + t->res.packed_offset, t->res.nbytes);
+    memcpy(dst, t->host, t->res.nbytes);
     return DG_OK;
 }
 
@@ -269,12 +272,14 @@ extern "C" int dg_wait(dg_feeder* f, dg_ticket id, uint64_t timeout_ns, dg_resul
     // Only this ticket's owner touches it from here on (releasing a ticket another thread is waiting on is a caller bug).
     int rc = DG_OK;
     if (copy) {
-        rc = copy_out(t, fl, t->host_out, t->host_cap);  // on the caller's thread: the copies of a batch run in parallel
+        rc = copy_out(t, t->host_out, t->host_cap);  // on the caller's thread: the copies of a batch run in parallel
         if (!rc) {  // host path: the device copy is not needed any more, let the batch go as soon as its peers agree
             std::lock_guard<std::mutex> lock(f->mu);
             t->flight = nullptr;
             t->res.device_data = nullptr;
             unref(fl);
+            dg::host_block_release(t->block);
+            t->host = nullptr; t->block = nullptr;
         }
     }
     if (out) *out = t->res;
@@ -284,17 +289,15 @@ extern "C" int dg_wait(dg_feeder* f, dg_ticket id, uint64_t timeout_ns, dg_resul
 extern "C" int dg_fetch(dg_feeder* f, dg_ticket id, uint8_t* host_out, uint64_t capacity) {
     if (!f || !host_out) return set_error(DG_E_INVALID, "NULL argument");
     Ticket* t = nullptr;
-    Flight* fl = nullptr;
     {
         std::lock_guard<std::mutex> lock(f->mu);
         auto it = f->tickets.find(id);
         if (it == f->tickets.end() || it->second->orphan) return set_error(DG_E_INVALID, "unknown ticket");
         t = it->second.get();
         if (t->state != 2) return set_error(DG_E_INVALID, "ticket not finished: call dg_wait first");
-        fl = t->flight;
-        if (t->res.status == DG_OK && !fl) return set_error(DG_E_INVALID, "payload already handed over (host buffer given at submit)");
+        if (t->res.status == DG_OK && !t->flight) return set_error(DG_E_INVALID, "payload already handed over (host buffer given at submit)");
     }
-    return copy_out(t, fl, host_out, capacity);
+    return copy_out(t, host_out, capacity);
 }
 
 extern "C" int dg_peek(dg_feeder* f, dg_ticket id, const uint8_t** host_data) {
@@ -307,7 +310,7 @@ extern "C" int dg_peek(dg_feeder* f, dg_ticket id, const uint8_t** host_data) {
     if (t->state != 2) return set_error(DG_E_INVALID, "ticket not finished: call dg_wait first");
     if (t->res.status) return set_error(t->res.status, "the sample failed: there is no payload");
     if (!t->flight) return set_error(DG_E_INVALID, "payload already handed over (host buffer given at submit)");
-    *host_data = t->flight->pinned + t->res.packed_offset;
+    *host_data = t->host;
     return DG_OK;
 }
 
@@ -319,8 +322,8 @@ extern "C" int dg_fetch_view(dg_feeder* f, dg_ticket id, const uint8_t** host_da
     std::lock_guard<std::mutex> lock(f->mu);
     const Ticket* t = f->tickets.find(id)->second.get();  // (a ticket belongs to one thread: it is still there)
     if (dg::host_blocks_scarce()) return set_error(DG_E_TOO_LARGE, "too much page-locked memory is held by views");
-    dg::host_block_retain(t->flight->pinned);
-    *block = t->flight->pinned;
+    dg::host_block_retain(t->block);
+    *block = t->block;
     return DG_OK;
 }
 
@@ -332,6 +335,7 @@ extern "C" int dg_release(dg_feeder* f, dg_ticket id) {
     Ticket* t = it->second.get();
     if (t->state == 2) {
         unref(t->flight);
+        dg::host_block_release(t->block);
         f->tickets.erase(it);
     } else if (t->state == 0) {  // still queued: take it out, nothing ran
         for (auto q = f->queue.begin(); q != f->queue.end(); ++q)
@@ -368,6 +372,7 @@ extern "C" void dg_feeder_destroy(dg_feeder* f) {
     for (auto& kv : f->tickets) {
         Flight* fl = kv.second->flight;
         if (fl && fl->refs.fetch_sub(1) == 1) fl->lane->dead.push_back(fl);
+        dg::host_block_release(kv.second->block);
     }
     f->tickets.clear();
     cudaSetDevice(f->device);

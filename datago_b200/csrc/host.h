@@ -59,6 +59,11 @@ bool huff_lengths_valid(const JpegHeader::RawHuff& raw);  // what build_huff_tab
 // Stores msg as the calling thread's dg_last_error text and returns code.
 int dg_set_error(int code, const char* msg);
 
+// ---- batches --------------------------------------------------------------------------------------------------------
+// Queues copies of all ok payloads into blocks of the page-locked pool: host[i] and blocks[i] (a reference of the caller's,
+// see host_blocks.h) per item, NULL where there is no payload.  On an error the caller gets no references.
+int batch_download_blocks(dg_batch* b, uint8_t** host, void** blocks);
+
 // ---- sharding -------------------------------------------------------------------------------------------------------
 uint64_t siphash13_str(const char* key, uint64_t len);
 

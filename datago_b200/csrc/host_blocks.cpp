@@ -173,6 +173,12 @@ bool host_blocks_scarce() {
     return p.busy > p.limit;
 }
 
+bool host_blocks_room(size_t nbytes) {
+    Pool& p = pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    return p.busy + nbytes <= p.limit;
+}
+
 void host_blocks_context(int device, int change) {
     Pool& p = pool();
     std::vector<std::pair<void*, size_t>> gone;

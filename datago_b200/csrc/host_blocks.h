@@ -1,5 +1,5 @@
 // Page-locked host blocks shared by everything in the process that receives pixels from the GPU: the payloads of one
-// download sit in a few blocks, and a block lives as long as anybody still looks at one of them (reference counted).
+// download sit in blocks of about 4 MB, and a block lives as long as anybody still looks at one of them (reference counted).
 //
 // Why: a fresh pageable buffer per payload costs a page fault per 4 KB (2 GB/s on the virtual machines this runs on) and a
 // staged copy by the driver; handing out views of the block the copy engine wrote costs neither.
@@ -22,6 +22,7 @@ int host_block_acquire(size_t nbytes, bool optional, void** out);  // dg_status;
 void host_block_retain(void* base);
 void host_block_release(void* base);
 bool host_blocks_scarce();  // whether more than the limit is referenced
+bool host_blocks_room(size_t nbytes);  // whether optional requests for that much would be granted
 // +1 / -1 context on `device`.  Blocks are page-locked on a device that has one: the calling thread's current device may be
 // another rank's, and locking there would create a context on it.
 void host_blocks_context(int device, int change);

@@ -210,6 +210,12 @@ DG_API int dg_batch_download(dg_batch* b, uint8_t* const* host_out);
  * asynchronous copies fill the driver's submission queue and stall the calling thread. */
 DG_API int dg_batch_download_packed(dg_batch* b, uint8_t* host_base, uint64_t capacity);
 DG_API uint64_t dg_batch_packed_bytes(const dg_batch* b);
+/* Payloads in page-locked memory of the library, a few of them to a block of about 4 MB (a larger payload has its own): for
+ * every ok item, host_out[i] points at its bytes and blocks[i] is a reference the caller hands to dg_host_release when it is
+ * done with that payload (NULL and NULL for the others).  The copies are queued; valid after dg_batch_sync, and for as long
+ * as the reference is held, also when the batch and the context are gone.  DG_E_TOO_LARGE while too much page-locked memory
+ * is in use (see dg_host_alloc): use dg_batch_download then. */
+DG_API int dg_batch_download_views(dg_batch* b, const uint8_t** host_out, void** blocks);
 DG_API int dg_batch_sync(dg_batch* b);
 DG_API int dg_batch_result(const dg_batch* b, int i, dg_result* out);
 DG_API int dg_batch_results(const dg_batch* b, dg_result* out); /* all of them: out has room for the batch's n items */

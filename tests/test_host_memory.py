@@ -14,7 +14,7 @@ class FakeLibrary:
 
     def __init__(self):
         self.blocks = {}   # address -> [buffer, references]
-        self.queued = []
+        self.queued, self.held, self.scarce = [], [], False
 
     def in_use(self):
         return {a for a, (_, refs) in self.blocks.items() if refs}
@@ -43,12 +43,30 @@ class FakeLibrary:
         self.queued.append(dst)
         return 0
 
+    def dg_batch_download_views(self, b, host, blocks):
+        if self.scarce:
+            return dg.E_TOO_LARGE
+        p = C.c_void_p()
+        self.dg_host_alloc(48, C.byref(p))
+        self.blocks[p.value][1] += 1  # the batch's own reference, until the copy has run
+        self.held.append(p.value)
+        host[0] = blocks[0] = p.value
+        self.queued.append(p.value)
+        return 0
+
+    def dg_batch_download(self, b, ptrs):
+        self.queued.append(ptrs[0])
+        return 0
+
     def dg_batch_sync(self, b):
         self.queued.clear()
+        for p in self.held:
+            self.dg_host_release(p)
+        self.held.clear()
         return 0
 
     def dg_batch_destroy(self, b):
-        self.queued.clear()
+        self.dg_batch_sync(b)
 
 
 @pytest.fixture
@@ -89,4 +107,12 @@ def test_a_landing_buffer_stays_alive_while_a_copy_into_it_is_queued(fake):
     b.sync()
     gc.collect()
     assert not fake.in_use()
+    b.close()
+
+
+def test_payloads_arrive_in_ordinary_memory_while_blocks_are_scarce(fake):
+    fake.scarce = True
+    b = dg.Batch(_Ctx(), [np.zeros((4, 4, 3), np.uint8)])
+    out, = b.download()
+    assert fake.queued == [out.ctypes.data] and out.flags.owndata and out.shape == (4, 4, 3)
     b.close()
