@@ -632,8 +632,9 @@ class Feeder:
         return r
 
     def fetch(self, ticket, result):
-        """The payload of a finished ticket as a numpy array (H x W x 3, or H x W for one channel): a view of the page-locked
-        memory it arrived in (kept alive by the array), or a copy when it is small or too much is held already."""
+        """The payload of a finished ticket as a numpy array of the caller's own (H x W x 3, or H x W for one channel): a view of
+        the page-locked memory it arrived in (kept alive by the array), or a copy when it is small, handed out before or too
+        much is held already."""
         nbytes = int(result.nbytes)
         if nbytes >= 1 << 15:
             ptr, block = C.c_void_p(), C.c_void_p()

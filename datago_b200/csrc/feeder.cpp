@@ -41,7 +41,7 @@ struct Flight {
 struct Ticket {
     uint64_t id = 0;
     int state = 0;  // 0 queued, 1 taken by a lane, 2 done
-    bool orphan = false, fetched = false;
+    bool orphan = false, fetched = false, peeked = false;
     std::vector<uint8_t> bytes;
     uint32_t raw_w = 0, raw_h = 0, raw_c = 0, flags = 0;
     std::string key;
@@ -49,8 +49,8 @@ struct Ticket {
     uint64_t host_cap = 0;
     dg_result res{};
     Flight* flight = nullptr;
-    uint8_t* host = nullptr;  // the page-locked host copy of the payload, and the ticket's reference on the block it lies in
-    void* block = nullptr;
+    uint8_t* host = nullptr;  // the page-locked host copy of the payload, and the ticket's reference on the block it lies in;
+    void* block = nullptr;    // both NULL once dg_fetch_view has handed them on
     Clock::time_point t_submit;
 };
 
@@ -247,8 +247,32 @@ extern "C" int dg_submit(dg_feeder* f, const dg_item* item, uint8_t* host_out, u
 static int copy_out(Ticket* t, uint8_t* dst, uint64_t cap) {
     if (t->res.status) return DG_OK;  // nothing to copy; the status travels in the result
     if (cap < t->res.nbytes) return set_error(DG_E_INVALID, "host buffer smaller than the payload");
-    memcpy(dst, t->host, t->res.nbytes);
+    if (t->host) { memcpy(dst, t->host, t->res.nbytes); return DG_OK; }
+    return dg_copy_to_host(t->flight->lane->ctx, dst, t->res.device_data, t->res.nbytes);  // the host copy belongs to somebody else by now
+}
+
+// The ticket's own host copy, made anew from the device if the first one has been handed on.
+static int own_copy(Ticket* t) {
+    if (t->host) return DG_OK;
+    void* block = nullptr;
+    int rc = dg::host_block_acquire(t->res.nbytes, false, &block);
+    if (!rc) rc = copy_out(t, (uint8_t*)block, t->res.nbytes);
+    if (rc) { dg::host_block_release(block); return rc; }
+    t->host = (uint8_t*)block;
+    t->block = block;
     return DG_OK;
+}
+
+// The ticket `id` if it is finished and its payload is at hand, else NULL and *rc says why.
+static Ticket* finished(dg_feeder* f, dg_ticket id, int* rc) {
+    std::lock_guard<std::mutex> lock(f->mu);
+    const auto it = f->tickets.find(id);
+    if (it == f->tickets.end() || it->second->orphan) *rc = set_error(DG_E_INVALID, "unknown ticket");
+    else if (it->second->state != 2) *rc = set_error(DG_E_INVALID, "ticket not finished: call dg_wait first");
+    else if (it->second->res.status) *rc = set_error(it->second->res.status, "the sample failed: there is no payload");
+    else if (!it->second->flight) *rc = set_error(DG_E_INVALID, "payload already handed over (host buffer given at submit)");
+    else return it->second.get();  // (a ticket belongs to one thread at a time: it stays)
+    return nullptr;
 }
 
 extern "C" int dg_wait(dg_feeder* f, dg_ticket id, uint64_t timeout_ns, dg_result* out) {
@@ -303,27 +327,36 @@ extern "C" int dg_fetch(dg_feeder* f, dg_ticket id, uint8_t* host_out, uint64_t 
 extern "C" int dg_peek(dg_feeder* f, dg_ticket id, const uint8_t** host_data) {
     if (!f || !host_data) return set_error(DG_E_INVALID, "NULL argument");
     *host_data = nullptr;
-    std::lock_guard<std::mutex> lock(f->mu);
-    auto it = f->tickets.find(id);
-    if (it == f->tickets.end() || it->second->orphan) return set_error(DG_E_INVALID, "unknown ticket");
-    const Ticket* t = it->second.get();
-    if (t->state != 2) return set_error(DG_E_INVALID, "ticket not finished: call dg_wait first");
-    if (t->res.status) return set_error(t->res.status, "the sample failed: there is no payload");
-    if (!t->flight) return set_error(DG_E_INVALID, "payload already handed over (host buffer given at submit)");
+    int rc = DG_OK;
+    Ticket* const t = finished(f, id, &rc);
+    if (!t || (rc = own_copy(t))) return rc;
+    t->peeked = true;
     *host_data = t->host;
     return DG_OK;
 }
 
 extern "C" int dg_fetch_view(dg_feeder* f, dg_ticket id, const uint8_t** host_data, void** block) {
-    if (!block) return set_error(DG_E_INVALID, "NULL argument");
+    if (!f || !host_data || !block) return set_error(DG_E_INVALID, "NULL argument");
+    *host_data = nullptr;
     *block = nullptr;
-    const int rc = dg_peek(f, id, host_data);
-    if (rc) return rc;
-    std::lock_guard<std::mutex> lock(f->mu);
-    const Ticket* t = f->tickets.find(id)->second.get();  // (a ticket belongs to one thread: it is still there)
+    int rc = DG_OK;
+    Ticket* const t = finished(f, id, &rc);
+    if (!t) return rc;
     if (dg::host_blocks_scarce()) return set_error(DG_E_TOO_LARGE, "too much page-locked memory is held by views");
-    dg::host_block_retain(t->block);
+    if (t->peeked) {  // somebody reads the ticket's copy: the caller gets one of its own
+        void* own = nullptr;
+        rc = dg::host_block_acquire(t->res.nbytes, false, &own);
+        if (rc) return rc;
+        memcpy(own, t->host, t->res.nbytes);
+        *host_data = (const uint8_t*)own;
+        *block = own;
+        return DG_OK;
+    }
+    if ((rc = own_copy(t))) return rc;
+    *host_data = t->host;
     *block = t->block;
+    t->host = nullptr;
+    t->block = nullptr;
     return DG_OK;
 }
 

@@ -287,9 +287,10 @@ DG_API int dg_fetch(dg_feeder* f, dg_ticket ticket, uint8_t* host_out, uint64_t 
 /* The payload where the feeder's own device -> host copy left it (page-locked host memory of the library), valid until
  * dg_release: lets a caller consume the pixels without a second host copy. */
 DG_API int dg_peek(dg_feeder* f, dg_ticket ticket, const uint8_t** host_data);
-/* Like dg_peek, for a caller that keeps the pixels: *host_data stays valid after dg_release and after the feeder is gone, until
- * the caller hands *block to dg_host_release.  DG_E_TOO_LARGE while too much page-locked memory is held this way (see
- * dg_host_alloc): copy with dg_fetch instead. */
+/* For a caller that keeps the pixels: *host_data is the caller's alone (what other calls on the ticket return is another copy,
+ * taken from the device if need be) and stays valid after dg_release and after the feeder is gone, until the caller hands
+ * *block to dg_host_release.  DG_E_TOO_LARGE while too much page-locked memory is held this way (see dg_host_alloc): copy
+ * with dg_fetch instead. */
 DG_API int dg_fetch_view(dg_feeder* f, dg_ticket ticket, const uint8_t** host_data, void** block);
 DG_API int dg_release(dg_feeder* f, dg_ticket ticket);
 DG_API int dg_feeder_get_stats(dg_feeder* f, dg_feeder_stats* out);

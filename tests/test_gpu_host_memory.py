@@ -50,6 +50,38 @@ def test_a_block_is_not_lent_on_while_a_copy_into_it_may_be_queued(end):
     b.close()
 
 
+@pytest.mark.parametrize("shape", [(40, 50, 3), (400, 500, 3)])  # copied, handed on as a view
+def test_what_a_ticket_returns_is_the_callers_own(shape):
+    rng = np.random.default_rng(403)
+    x = rng.integers(0, 256, shape, dtype=np.uint8)
+    with dg.Feeder(0, None, max_batch=4, max_wait_us=500) as f:
+        for order in ("ffpp", "pfpf", "fpf"):
+            t, other = f.submit(x), f.submit(x)
+            r = f.wait(t)
+            got = [f.fetch(t, r) if c == "f" else f.peek(t, r) for c in order]
+            for c, a in zip(order, got):
+                assert np.array_equal(a, x), order
+                if c == "f":
+                    a[:] = 0  # nobody else's pixels change
+            for c, a in zip(order, got):
+                assert np.array_equal(a, x) == (c == "p"), order
+            kept = f.fetch(t, r)
+            f.release(t)
+            assert np.array_equal(f.fetch(other, f.wait(other)), x)
+            f.release(other)
+        landing = np.zeros(shape, np.uint8)  # a buffer given at submit is filled by wait, after a fetch as well
+        t = f.submit(x, host_out=landing)
+        while f.stats()["completed"] < f.stats()["submitted"]:
+            pass
+        r = dg.Result()
+        r.nbytes, r.height, r.width, r.channels = x.nbytes, *shape
+        f.fetch(t, r)[:] = 0
+        f.wait(t)
+        assert np.array_equal(landing, x)
+        f.release(t)
+    assert np.array_equal(kept, x)
+
+
 @pytest.mark.parametrize("collate", [0, dg.BATCH_COLLATE])
 def test_payloads_are_whole_and_share_small_blocks_only(collate):
     rng = np.random.default_rng(402)
