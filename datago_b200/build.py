@@ -7,7 +7,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libdatago_b200.so")
 SOURCES = ["api.cu", "kernels_huff.cu", "kernels_jpeg.cu", "kernels_resize.cu", "host_logic.cpp", "jpeg_header.cpp", "host_blocks.cpp", "feeder.cpp"]
-HEADERS = ["desc.h", "host.h", "host_blocks.h", "host_pool.h", "kernels.h", os.path.join("..", "..", "include", "datago_b200.h")]
+HEADERS = ["block_cache.h", "desc.h", "host.h", "host_blocks.h", "host_pool.h", "kernels.h", os.path.join("..", "..", "include", "datago_b200.h")]
 
 
 def _stale():

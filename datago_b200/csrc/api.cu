@@ -23,6 +23,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "block_cache.h"
 #include "host.h"
 #include "host_blocks.h"
 #include "host_pool.h"
@@ -93,72 +94,6 @@ extern "C" const char* dg_version(void) { return "datago_b200 0.1 (sm_100a)"; }
 // ---------------------------------------------------------------------------------------------------------------
 namespace {
 
-struct Block {
-    void* ptr = nullptr;
-    size_t size = 0;
-    bool busy = false;
-};
-
-// Cache of blocks: a batch borrows them and hands them back; nothing is freed in the steady state, so it makes no allocation
-// calls.  A request takes the smallest idle block that fits and is not far too large for it (a large block lent to a small
-// request is missing when the next large one comes, and then the cache allocates on every batch).
-struct BlockCache {
-    bool pinned;
-    std::vector<Block> blocks;
-    explicit BlockCache(bool p) : pinned(p) {}
-    void give_back(Block& b) {
-        if (b.ptr) { if (pinned) cudaFreeHost(b.ptr); else cudaFree(b.ptr); }
-        b = Block();
-    }
-    int smallest_fit(size_t size, size_t most) const {
-        int best = -1;
-        for (size_t i = 0; i < blocks.size(); ++i)
-            if (!blocks[i].busy && blocks[i].size >= size && blocks[i].size <= most && (best < 0 || blocks[i].size < blocks[best].size)) best = (int)i;
-        return best;
-    }
-    int acquire(size_t size, int* index) {
-        if (size == 0) size = 256;
-        int best = smallest_fit(size, 2 * size + ((size_t)4 << 20));
-        if (best < 0) {
-            // the largest idle block that is too small makes room, so that the cache does not pile up stale sizes
-            int victim = -1;
-            for (size_t i = 0; i < blocks.size(); ++i)
-                if (!blocks[i].busy && blocks[i].size < size && (victim < 0 || blocks[i].size > blocks[victim].size)) victim = (int)i;
-            // ... once the idle ones add up to something, and not a much smaller one, which serves other requests
-            size_t idle = 0;
-            for (const Block& b : blocks) idle += b.busy ? 0 : b.size;
-            if (victim >= 0 && (blocks[victim].size < size / 2 || idle < ((size_t)1 << 30))) victim = -1;
-            if (victim < 0) { blocks.emplace_back(); victim = (int)blocks.size() - 1; }
-            give_back(blocks[victim]);
-            Block nb;
-            nb.size = size + size / 8 + 4096;
-            auto allocate = [&] { return pinned ? cudaHostAlloc(&nb.ptr, nb.size, cudaHostAllocDefault) : cudaMalloc(&nb.ptr, nb.size); };
-            cudaError_t e = allocate();
-            if (e != cudaSuccess) {  // out of memory: whatever fits, else without the idle blocks
-                cudaGetLastError();  // a failed allocation must not surface again as the next healthy batch's error
-                best = smallest_fit(size, ~(size_t)0);
-                if (best < 0) {
-                    for (Block& b : blocks) if (!b.busy) give_back(b);
-                    e = allocate();
-                    if (e != cudaSuccess) {
-                        cudaGetLastError();
-                        return fail(DG_E_CUDA, "%s of %zu bytes: %s", pinned ? "cudaHostAlloc" : "cudaMalloc", nb.size, cudaGetErrorString(e));
-                    }
-                }
-            }
-            if (best < 0) { blocks[victim] = nb; best = victim; }
-        }
-        blocks[best].busy = true;
-        *index = best;
-        return DG_OK;
-    }
-    void release(int index) { if (index >= 0) blocks[index].busy = false; }
-    void clear() {
-        for (auto& b : blocks) if (b.ptr) { if (pinned) cudaFreeHost(b.ptr); else cudaFree(b.ptr); }
-        blocks.clear();
-    }
-};
-
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 }  // namespace
@@ -175,7 +110,8 @@ struct dg_ctx {
     dg_image_config cfg{};
     Transform tfm;
     std::mutex mu;
-    BlockCache dev{false}, pin{true};
+    BlockCache dev{false}, pin{true};            // intermediates, inputs and payloads; staged inputs
+    BlockCache dev_meta{false}, pin_meta{true};  // metadata and status words: small requests must not take the large blocks
     // Lanczos tables built so far, by (input size, box, output size): data sets repeat image sizes, and every epoch
     // repeats all of them, while a table costs two sin() per weight.  Dropped wholesale when it outgrows its cap.
     std::map<std::array<uint64_t, 4>, std::shared_ptr<const FilterTable>> table_cache;
@@ -270,8 +206,7 @@ extern "C" void dg_ctx_destroy(dg_ctx* c) {
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     cudaStreamSynchronize(c->stream2);
-    c->dev.clear();
-    c->pin.clear();
+    for (BlockCache* cache : {&c->dev, &c->pin, &c->dev_meta, &c->pin_meta}) cache->clear();
     cudaEventDestroy(c->ev_fork);
     cudaEventDestroy(c->ev_join);
     for (int i = 0; i < 2; ++i) {
@@ -893,12 +828,12 @@ template <typename F> static void parallel_items(int n, F&& fn) {
 static int abandon(dg_batch* b, int rc) {
     dg_ctx* ctx = b->ctx;
     ctx->dev.release(b->blk_persist);
-    ctx->dev.release(b->blk_meta);
+    ctx->dev_meta.release(b->blk_meta);
     ctx->dev.release(b->blk_scratch);
     ctx->dev.release(b->blk_scratch2);
     ctx->pin.release(b->blk_pin);
-    ctx->pin.release(b->blk_pin_meta);
-    ctx->pin.release(b->blk_pin_status);
+    ctx->pin_meta.release(b->blk_pin_meta);
+    ctx->pin_meta.release(b->blk_pin_status);
     delete b;
     return rc;
 }
@@ -1376,15 +1311,15 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
     // ---- page-locked staging -------------------------------------------------------------------------------------------
     // Raw inputs are staged too: a copy from pageable caller memory is serialised by the driver at a fraction of the
     // link rate, while host threads fill page-locked memory in parallel and the upload becomes one large transfer.
-    rc = ctx->dev.acquire(b->meta_total, &b->blk_meta);
+    rc = ctx->dev_meta.acquire(b->meta_total, &b->blk_meta);
     if (!rc) rc = ctx->pin.acquire(b->off_rawin + align_up(rawin, 256), &b->blk_pin);
-    if (!rc) rc = ctx->pin.acquire(b->meta_total, &b->blk_pin_meta);
-    if (!rc) rc = ctx->pin.acquire(std::max<size_t>((size_t)n * 4, 256), &b->blk_pin_status);
+    if (!rc) rc = ctx->pin_meta.acquire(b->meta_total, &b->blk_pin_meta);
+    if (!rc) rc = ctx->pin_meta.acquire(std::max<size_t>((size_t)n * 4, 256), &b->blk_pin_status);
     if (rc) return abandon(b, rc);
-    b->d_meta = (uint8_t*)ctx->dev.blocks[b->blk_meta].ptr;
+    b->d_meta = (uint8_t*)ctx->dev_meta.blocks[b->blk_meta].ptr;
     b->h_pin = (uint8_t*)ctx->pin.blocks[b->blk_pin].ptr;
-    b->h_meta = (uint8_t*)ctx->pin.blocks[b->blk_pin_meta].ptr;
-    b->h_status = (uint32_t*)ctx->pin.blocks[b->blk_pin_status].ptr;
+    b->h_meta = (uint8_t*)ctx->pin_meta.blocks[b->blk_pin_meta].ptr;
+    b->h_status = (uint32_t*)ctx->pin_meta.blocks[b->blk_pin_status].ptr;
     memset(b->h_pin, 0, b->off_blob);
     {
         // One list of copies for everything: pieces of about 128 KB, or one filter table each, so that a few large inputs
@@ -1877,12 +1812,12 @@ extern "C" void dg_batch_destroy(dg_batch* b) {
     landed(b);
     for (StageEvent& se : b->events) { cudaEventDestroy(se.a); cudaEventDestroy(se.b); }
     ctx->dev.release(b->blk_persist);
-    ctx->dev.release(b->blk_meta);
+    ctx->dev_meta.release(b->blk_meta);
     ctx->dev.release(b->blk_scratch);
     ctx->dev.release(b->blk_scratch2);
     ctx->pin.release(b->blk_pin);
-    ctx->pin.release(b->blk_pin_meta);
-    ctx->pin.release(b->blk_pin_status);
+    ctx->pin_meta.release(b->blk_pin_meta);
+    ctx->pin_meta.release(b->blk_pin_status);
     delete b;
 }
 

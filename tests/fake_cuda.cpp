@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 #include <sys/mman.h>
 
+#include "../datago_b200/csrc/block_cache.h"
 #include "../datago_b200/csrc/host.h"
 #include "../datago_b200/csrc/host_blocks.h"
 
@@ -84,6 +85,11 @@ int hb_acquire(size_t n, int optional, void** out) { return dg::host_block_acqui
 void hb_retain(void* p) { dg::host_block_retain(p); }
 int hb_scarce() { return dg::host_blocks_scarce(); }
 void hb_context(int device, int change) { dg::host_blocks_context(device, change); }
+
+void* bc_new() { return new dg::BlockCache(false); }
+int bc_acquire(void* c, size_t n) { int i = -1; return ((dg::BlockCache*)c)->acquire(n, &i) ? -1 : i; }
+void bc_release(void* c, int i) { ((dg::BlockCache*)c)->release(i); }
+void bc_delete(void* c) { ((dg::BlockCache*)c)->clear(); delete (dg::BlockCache*)c; }
 }
 
 int dg::dg_set_error(int code, const char*) { return code; }

@@ -1,7 +1,9 @@
-"""The pool of page-locked blocks (csrc/host_blocks.cpp), built against a stand-in for the CUDA runtime: sizes, references,
-bounds, the device the locking happens on, and what a forked child sees."""
+"""The pool of page-locked blocks (csrc/host_blocks.cpp) and the blocks a context lends to its batches (csrc/block_cache.h),
+built against a stand-in for the CUDA runtime: sizes, references, bounds, the device the locking happens on, and what a forked
+child sees."""
 import ctypes as C
 import os
+import random
 import subprocess
 import sys
 import threading
@@ -33,7 +35,10 @@ def pool(library, tmp_path, monkeypatch):
     L.hb_acquire.argtypes = [C.c_size_t, C.c_int, C.POINTER(C.c_void_p)]
     L.dg_host_alloc.argtypes = [C.c_uint64, C.POINTER(C.c_void_p)]
     L.dg_host_release.argtypes = L.hb_retain.argtypes = L.fake_locked_on.argtypes = [C.c_void_p]
-    L.fake_locked_bytes.restype = C.c_size_t
+    L.fake_locked_bytes.restype = L.fake_device_bytes.restype = C.c_size_t
+    L.bc_new.restype = C.c_void_p
+    L.bc_acquire.argtypes, L.bc_release.argtypes, L.bc_delete.argtypes = [C.c_void_p, C.c_size_t], [C.c_void_p, C.c_int], [C.c_void_p]
+    L.fake_device_limit.argtypes = [C.c_size_t]
     return L
 
 
@@ -130,3 +135,57 @@ _, status = os.waitpid(pid, 0)
 sys.exit(0 if status == 0 and C.string_at(p.value, n) == bytes([8]) * n else 1)
 """
     subprocess.run([sys.executable, "-c", script, pool._name, str(nbytes)], check=True)
+
+
+class Cache:
+    """Batches that borrow some blocks at once, and hand them back."""
+
+    def __init__(self, L):
+        self.L, self.c = L, L.bc_new()
+
+    def batch(self, *sizes):
+        got = [self.L.bc_acquire(self.c, n) for n in sizes]
+        assert len(set(got)) == len(got)
+        return got
+
+    def done(self, got):
+        for i in got:
+            self.L.bc_release(self.c, i)
+
+
+def test_a_smaller_batch_borrows_what_is_there(pool):
+    cache = Cache(pool)
+    cache.done(cache.batch(4000 * MB, 700 * MB))
+    n = pool.fake_allocations()
+    for scale in (1, 3, 40, 5000):
+        cache.done(cache.batch(4000 * MB // scale, 700 * MB // scale))
+    assert pool.fake_allocations() == n
+    pool.bc_delete(cache.c)
+    assert pool.fake_device_bytes() == 0
+
+
+@pytest.mark.parametrize("in_flight", [1, 2])
+def test_batches_of_many_sizes_neither_pile_up_blocks_nor_allocate_for_ever(pool, in_flight):
+    rng = random.Random(5)
+    sizes = [tuple(int(2 ** rng.uniform(20, 32)) for _ in range(3)) for _ in range(40)]
+    most = max(max(s) for s in sizes)
+    cache, flying = Cache(pool), []
+    for i in range(3000):
+        if i == 2000:
+            n = pool.fake_allocations()
+        flying.append(cache.batch(*rng.choice(sizes)))
+        if len(flying) > in_flight - 1:
+            cache.done(flying.pop(0))
+        assert pool.fake_device_bytes() <= 3 * in_flight * (most + most // 8 + 4096)
+    assert pool.fake_allocations() == n
+
+
+def test_idle_blocks_go_before_an_allocation_fails(pool):
+    pool.fake_device_limit(1000 * MB)
+    cache = Cache(pool)
+    cache.done(cache.batch(300 * MB, 300 * MB, 200 * MB))
+    big, = cache.batch(800 * MB)
+    assert big >= 0
+    assert cache.batch(300 * MB) == [-1]
+    cache.done([big])
+    assert cache.batch(300 * MB, 50 * MB)[0] >= 0
