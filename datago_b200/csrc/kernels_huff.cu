@@ -727,6 +727,7 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
 // ---- blocks with their values --------------------------------------------------------------------------------------
 namespace {
 
+constexpr uint32_t kBlankBlock = (uint32_t)kClsDc << 16;  // in info[]: a block the stream does not hold
 constexpr uint32_t kNotDc = 1u << 28, kNot2x2 = 1u << 29, kNot4x4 = 1u << 30;
 
 // Zig-zag position -> byte offset of the coefficient in a lane's block buffer (row r of the lane's block sits at
@@ -909,7 +910,13 @@ __global__ void __launch_bounds__(kRestartThreads) k_huff_restart(JpegWave w) {
     if (k0 == 0 && tid == 0 && found != d.nseg) atomicOr(w.status + d.item, kStBadMarker);
     const uint32_t* seg = w.seg_start + d.seg_off;
     const uint32_t have = min(found, d.nseg);  // entries of seg[] that exist
-    if (k0 >= have) return;
+    const uint32_t mcus = d.mcux * d.mcuy;
+    const uint32_t m0 = min(k * d.restart, mcus), m1 = min(m0 + d.restart, mcus);
+    const uint32_t blk0 = m0 * d.bpm, blk1 = m1 * d.bpm;
+    uint32_t* info = w.info + d.block_off;
+    // blocks that a damaged file lacks are flat mid-gray, not what an earlier wave left in info[] and coef[]
+    const auto blank = [&](uint32_t from) { for (uint32_t b = from; b < blk1; ++b) info[b] = kBlankBlock; };
+    if (k0 >= have) { blank(blk0); return; }
     // the CTA's piece of the stream: from the 16-byte piece its first segment starts in to its end plus what a block that
     // is not whole may run over
     const uint32_t lo = seg[k0] & ~15u, hi = (k0 + kSegsPerCta < have ? seg[k0 + kSegsPerCta] : us_len) + 272u;
@@ -925,21 +932,19 @@ __global__ void __launch_bounds__(kRestartThreads) k_huff_restart(JpegWave w) {
     __syncthreads();
     const bool mine = k < have;
     const uint32_t b0 = mine ? seg[k] : lo, b1 = k + 1 < have ? seg[k + 1] : us_len;
-    const uint32_t mcus = d.mcux * d.mcuy;
-    const uint32_t m0 = mine ? k * d.restart : 0u, m1 = mine ? min(m0 + d.restart, mcus) : 0u;
-    const uint32_t blk0 = m0 * d.bpm, blk1 = m1 * d.bpm;
+    const uint32_t end = mine ? blk1 : blk0;
     int16_t* coef = w.coef + d.block_off * 64;
-    uint32_t* info = w.info + d.block_off;
     uint32_t err = 0, n;
     if (staged) {
         const uint32_t sbase = smem_addr(stage) - lo;
-        n = decode_blocks<kRestartThreads, true>(shared_source([&](uint32_t p) { return sbase + ((p >> 3) & ~3u); }), b0 * 8u, blk0, blk1, b1 * 8u, b1 * 8u, 0u,
+        n = decode_blocks<kRestartThreads, true>(shared_source([&](uint32_t p) { return sbase + ((p >> 3) & ~3u); }), b0 * 8u, blk0, end, b1 * 8u, b1 * 8u, 0u,
                                                  d.hs * d.vs, sh, w.huff, coef, info, err);
     } else {
         const GlobalSource source{reinterpret_cast<const uint32_t*>(us), (us_len + 3) / 4 + 2};
-        n = decode_blocks<kRestartThreads, true>(source, b0 * 8u, blk0, blk1, b1 * 8u, b1 * 8u, 0u, d.hs * d.vs, sh, w.huff, coef, info, err);
+        n = decode_blocks<kRestartThreads, true>(source, b0 * 8u, blk0, end, b1 * 8u, b1 * 8u, 0u, d.hs * d.vs, sh, w.huff, coef, info, err);
     }
-    if (n < blk1 - blk0) err |= kStTruncated;
+    if (n < end - blk0) err |= kStTruncated;
+    if (n < blk1 - blk0) blank(blk0 + n);
     if (err) atomicOr(w.status + d.item, err);
 }
 
@@ -956,11 +961,11 @@ constexpr int kDcThreads = 512;
 struct Dc3 { int32_t a, b, c; };
 __device__ __forceinline__ Dc3 operator+(Dc3 x, Dc3 y) { return {x.a + y.a, x.b + y.b, x.c + y.c}; }
 
-// four MCUs per thread: BPM 16-byte pieces
+// four MCUs per thread: BPM 16-byte pieces.  have: blocks that the stream holds.
 template <int BPM>
-__device__ __forceinline__ Dc3 load_mcus(const uint32_t* diff, uint32_t m4, uint32_t nblocks, uint32_t (&v)[4 * BPM]) {
+__device__ __forceinline__ Dc3 load_mcus(const uint32_t* diff, uint32_t m4, uint32_t have, uint32_t (&v)[4 * BPM]) {
     const uint32_t b0 = m4 * 4 * BPM;
-    if (b0 + 4 * BPM <= nblocks) {
+    if (b0 + 4 * BPM <= have) {
 #pragma unroll
         for (int i = 0; i < BPM; ++i) {
             const uint4 q = reinterpret_cast<const uint4*>(diff + b0)[i];
@@ -968,7 +973,7 @@ __device__ __forceinline__ Dc3 load_mcus(const uint32_t* diff, uint32_t m4, uint
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < 4 * BPM; ++i) v[i] = b0 + i < nblocks ? diff[b0 + i] : 0u;
+        for (int i = 0; i < 4 * BPM; ++i) v[i] = b0 + i < have ? diff[b0 + i] : 0u;
     }
     Dc3 s{0, 0, 0};
 #pragma unroll
@@ -983,14 +988,14 @@ __device__ __forceinline__ Dc3 load_mcus(const uint32_t* diff, uint32_t m4, uint
 }
 
 template <int BPM>
-__device__ void dc_range(const uint32_t* diff, uint32_t* info, uint32_t range, uint32_t nblocks, Dc3* s_warp) {
+__device__ void dc_range(const uint32_t* diff, uint32_t* info, uint32_t range, uint32_t nblocks, uint32_t have, Dc3* s_warp) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr uint32_t kStep = kDcThreads;  // groups of four MCUs per turn
     const uint32_t groups = (nblocks + 4 * BPM - 1) / (4 * BPM);
     const uint32_t g0 = range * (kDcMcus / 4), g1 = min(g0 + kDcMcus / 4, groups);
     uint32_t v[4 * BPM];
     Dc3 before{0, 0, 0};
-    for (uint32_t g = tid; g < g0; g += kStep) before = before + load_mcus<BPM>(diff, g, nblocks, v);
+    for (uint32_t g = tid; g < g0; g += kStep) before = before + load_mcus<BPM>(diff, g, have, v);
     auto total = [&](Dc3 x) -> Dc3 {  // sum over the CTA, in every thread
 #pragma unroll
         for (int o = 16; o; o >>= 1) { x.a += __shfl_xor_sync(0xFFFFFFFFu, x.a, o); x.b += __shfl_xor_sync(0xFFFFFFFFu, x.b, o); x.c += __shfl_xor_sync(0xFFFFFFFFu, x.c, o); }
@@ -1008,7 +1013,7 @@ __device__ void dc_range(const uint32_t* diff, uint32_t* info, uint32_t range, u
     for (uint32_t g = g0; g < g1; g += kStep) {
         const uint32_t m4 = g + tid;
         Dc3 mine{0, 0, 0};
-        if (m4 < g1) mine = load_mcus<BPM>(diff, m4, nblocks, v);
+        if (m4 < g1) mine = load_mcus<BPM>(diff, m4, have, v);
         Dc3 inc = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1034,12 +1039,12 @@ __device__ void dc_range(const uint32_t* diff, uint32_t* info, uint32_t range, u
             pred += x;
             v[i] = (v[i] & 0xFFFF0000u) | ((uint32_t)pred & 0xFFFFu);
         }
-        if (b0 + 4 * BPM <= nblocks) {
+        if (b0 + 4 * BPM <= have) {
 #pragma unroll
             for (int i = 0; i < BPM; ++i) reinterpret_cast<uint4*>(info + b0)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
         } else {
 #pragma unroll
-            for (int i = 0; i < 4 * BPM; ++i) if (b0 + i < nblocks) info[b0 + i] = v[i];
+            for (int i = 0; i < 4 * BPM; ++i) if (b0 + i < nblocks) info[b0 + i] = b0 + i < have ? v[i] : kBlankBlock;
         }
     }
 }
@@ -1053,11 +1058,12 @@ __global__ void __launch_bounds__(kDcThreads) k_dc(JpegWave w) {
     const uint32_t range = blockIdx.x - __ldg(w.dc_ctas.first + o);
     const uint32_t* diff = w.diff + d.block_off;
     uint32_t* info = w.info + d.block_off;
+    const uint32_t ncell = (w.us_len[w.spec_list[o]] * 8u + w.cell_bits - 1) / w.cell_bits, have = min(w.cells[d.cell_off + ncell].y, d.nblocks);
     switch (d.bpm) {
-        case 1: dc_range<1>(diff, info, range, d.nblocks, s_warp); break;
-        case 3: dc_range<3>(diff, info, range, d.nblocks, s_warp); break;
-        case 4: dc_range<4>(diff, info, range, d.nblocks, s_warp); break;
-        default: dc_range<6>(diff, info, range, d.nblocks, s_warp); break;
+        case 1: dc_range<1>(diff, info, range, d.nblocks, have, s_warp); break;
+        case 3: dc_range<3>(diff, info, range, d.nblocks, have, s_warp); break;
+        case 4: dc_range<4>(diff, info, range, d.nblocks, have, s_warp); break;
+        default: dc_range<6>(diff, info, range, d.nblocks, have, s_warp); break;
     }
 }
 
@@ -1138,10 +1144,12 @@ void launch_huff_chain(const JpegWave& w, cudaStream_t s) {
 }
 
 void launch_huff_write(const JpegWave& w, cudaStream_t s) {
-    if (!w.write_ctas.total) return;
+    if (!w.n_spec) return;
     configure_once();
-    if (w.cell_bits == (uint32_t)kCellBits) launch_write<kCellBits>(w, s);
-    else launch_write<kShortCellBits>(w, s);
+    if (w.write_ctas.total) {  // (streams may be empty)
+        if (w.cell_bits == (uint32_t)kCellBits) launch_write<kCellBits>(w, s);
+        else launch_write<kShortCellBits>(w, s);
+    }
     k_dc<<<w.dc_ctas.total, kDcThreads, 0, s>>>(w);
 }
 
