@@ -1079,7 +1079,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
                 d.cell_off = cells;
                 cells += stream_cells(d.raw_len, wv.cell_bits) + 1;
             }
-            wv.tile_first.push_back(wv.tile_first.back() + std::max(1u, (d.raw_len + kUnstuffTile - 1) / kUnstuffTile));
+            wv.tile_first.push_back(wv.tile_first.back() + std::max(1u, (uint32_t)(((uint64_t)d.raw_len + kUnstuffTile - 1) / kUnstuffTile)));
             {
                 const uint32_t distinct = 1 + (d.pair[1] != d.pair[0]) + (d.pair[2] != d.pair[0] && d.pair[2] != d.pair[1]);
                 wv.max_pairs = std::max(wv.max_pairs, distinct);

@@ -33,6 +33,9 @@ inline uint32_t guess_spans(uint32_t bpm, uint32_t span) {
 }
 constexpr uint32_t kDcMcus = 8192;       // MCUs per CTA of the DC prediction
 constexpr uint32_t kCodeTablesBytes = 20544;  // look-up tables of one (DC, AC) pair of Huffman tables
+// Bit positions are 32-bit numbers.  A stream counts up to this length, which leaves room for what the decoders add to a
+// position at its end (the cells of a CTA, a block); what lies behind is as good as cut off.
+constexpr uint32_t kMaxStream = (1u << 29) - (1u << 16);
 constexpr uint32_t kStreamPad = 512;     // bytes behind an image's unstuffed stream that the bit readers may touch
 
 // How much of a block is non-zero decides how much of the inverse DCT is needed: everything, the top-left 4x4 or 2x2

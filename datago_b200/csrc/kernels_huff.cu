@@ -201,7 +201,7 @@ __device__ __forceinline__ Unit classify(const uint8_t* in, uint32_t i0, uint32_
     if (i0 < len) v = __ldg(reinterpret_cast<const uint4*>(in + i0));  // blob slices are padded to 16 bytes with zeros
     u.w[0] = v.x; u.w[1] = v.y; u.w[2] = v.z; u.w[3] = v.w;
     const uint32_t prev = (i0 > 0 && i0 <= len) ? __ldg(in + i0 - 1) : 0u;
-    const uint32_t next = (i0 + 16 < len) ? __ldg(in + i0 + 16) : 0u;
+    const uint32_t next = (i0 < len && len - i0 > 16) ? __ldg(in + i0 + 16) : 0u;
     uint32_t F = 0, Z = 0, R = 0;  // FF bytes, zero bytes, bytes D0..D7
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kUnstuffThreads) k_unstuff_write(JpegWave w) {
     if (tile + 1 == ntile) {
         const uint32_t total = base + n;
         if (tid < 32) out[(total + tid) ^ 3u] = 0;  // the bit readers may look a few bytes past the end
-        if (tid == 0) { w.us_len[o] = total; w.seg_found[o] = rbase + (tot >> 16) + 1; }
+        if (tid == 0) { w.us_len[o] = min(total, kMaxStream); w.seg_found[o] = rbase + (tot >> 16) + 1; }
     }
 }
 
@@ -496,6 +496,7 @@ struct Staged {
     static __device__ __forceinline__ uint32_t at(uint32_t base, uint32_t p) { return base + ((p >> 3) & ~3u) + (p / CELL) * 16; }
 };
 static_assert(kStreamPad >= (2048 + 1024) / 8 + 16, "rows behind the end of a stream are copied");
+static_assert((1ull << 32) - kMaxStream * 8ull > 2ull * kCellsPerCta * kCellBits + 4096, "positions behind the end of a stream do not wrap");
 
 // A state at or behind the first bit of a cell, relative to it: bits 0-11 distance of the block start (less than 2048: a
 // block has 64 symbols of 31 bits at most), 12-14 its block c.
@@ -919,7 +920,8 @@ __global__ void __launch_bounds__(kRestartThreads) k_huff_restart(JpegWave w) {
     if (k0 >= have) { blank(blk0); return; }
     // the CTA's piece of the stream: from the 16-byte piece its first segment starts in to its end plus what a block that
     // is not whole may run over
-    const uint32_t lo = seg[k0] & ~15u, hi = (k0 + kSegsPerCta < have ? seg[k0 + kSegsPerCta] : us_len) + 272u;
+    const auto begin = [&](uint32_t i) { return i < have ? min(seg[i], us_len) : us_len; };  // of a segment (us_len: see kMaxStream)
+    const uint32_t lo = begin(k0) & ~15u, hi = begin(k0 + kSegsPerCta) + 272u;
     const bool staged = hi - lo <= kRestartStage;
     const uint8_t* us = w.us + d.us_off;
     if (staged) {
@@ -931,7 +933,7 @@ __global__ void __launch_bounds__(kRestartThreads) k_huff_restart(JpegWave w) {
     copy_wait<0>();
     __syncthreads();
     const bool mine = k < have;
-    const uint32_t b0 = mine ? seg[k] : lo, b1 = k + 1 < have ? seg[k + 1] : us_len;
+    const uint32_t b0 = mine ? begin(k) : lo, b1 = begin(k + 1);
     const uint32_t end = mine ? blk1 : blk0;
     int16_t* coef = w.coef + d.block_off * 64;
     uint32_t err = 0, n;
