@@ -546,6 +546,7 @@ class Batch:
         return dict(h2d_bytes=int(h2d.value), d2h_bytes=int(d2h.value), kernel_launches=int(k.value))
 
     def huffman_stats(self):
+        """Of the last run, over its restart-free JPEGs: cells of the streams (chunks), rounds of linking them, decodes of a cell."""
         out = (C.c_uint64 * 3)()
         _check(lib().dg_batch_huffman_stats(self._h, out))
         return dict(chunks=int(out[0]), rounds=int(out[1]), subsequence_decodes=int(out[2]))

@@ -65,7 +65,7 @@ struct JpegWave {
     uint8_t* planes;         // component planes after the IDCT
     uint8_t* out;            // decoded images
     uint32_t* status;        // [items of the batch]
-    unsigned long long* spec_stats;  // [0] stretches of 256 cells, [1] synchronisation rounds, [2] decodes of a thread's run
+    unsigned long long* spec_stats;  // [0] cells, [1] rounds of the linking kernel, [2] decodes of a cell (candidates, open states, values)
     const HuffTable* huff;   // table pool
     const uint2* table_pairs; uint32_t n_pairs;  // the (DC, AC) pairs of tables the images of the wave use
     uint8_t* codes;          // [n_pairs] look-up tables made from them, kCodeTablesBytes each

@@ -545,6 +545,7 @@ __global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
     SyncLane L{};
     L.start(source, mcu0, k ? k * CELL - kLeadBits : 0u, k ? 1u : 0u, live && k ? myh : 0u);
     L.run_to(live && k, k * CELL, source, w.huff);
+    uint32_t decodes = 0;
     s_state[tid] = (uint16_t)(live ? pack_state(L.p, k * CELL, L.mb.w, total) : kStNone);
     for (uint32_t step = 0; step < span; ++step) {
         __syncthreads();
@@ -559,6 +560,7 @@ __global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
         uint32_t before = 0, all = 0;
 #pragma unroll
         for (int i = 0; i < kGuessThreads / 32; ++i) { const uint32_t n = s_warp[i]; if (i < warp) before += n; all += n; }
+        decodes += all;
         if (keep) s_list[before + __popc(kept & ((1u << lane) - 1u))] = (uint16_t)tid;
         __syncthreads();
         // ---- through their cell
@@ -578,6 +580,7 @@ __global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
             }
         }
     }
+    if (tid == 0) atomicAdd(w.spec_stats + 2, (unsigned long long)decodes);
 }
 
 namespace {
@@ -665,7 +668,7 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
     }
     follow(active, kbeg, entry, false);
     sh.exit[tid] = exit;
-    uint32_t walks = active ? 1u : 0u, rounds = 1, round = 0;
+    uint32_t decodes = active ? kend - kbeg : 0u, rounds = 1, round = 0;  // decodes: once each for the values, and those below
     __syncthreads();
     // Look-ups until nothing changes any more; then what is open is decoded, one cell per thread; and again.  Opened cells have
     // their turn in every eighth round in any case: of eight rounds, one settles the first thread that is not final yet or
@@ -679,7 +682,6 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
         if (!any_need || (round & 7u) == 7u) any_decode = __syncthreads_or(decode);
         if (!any_need && !any_decode) break;
         if (!any_decode) {
-            walks += need;
             if (need) entry = prev;
             follow(need, kbeg, entry, true);
         } else {
@@ -690,6 +692,7 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
                 L.run_to(decode, min(bound, total + 1), source, w.huff);
                 __syncwarp();
                 if (decode) {
+                    ++decodes;
                     const uint32_t n = L.nb - (L.p > total ? 1u : 0u), next = pack_state(L.p, bound, L.mb.w, total);
                     found += n - (recs[k].y & 0xFFFu);
                     recs[k] = make_uint2(p, open_state << 12 | n);
@@ -707,8 +710,8 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, o); if (lane >= o) inc += t; }
     if (lane == 31) sh.warp[warp] = inc;
-    walks = __reduce_add_sync(0xFFFFFFFFu, walks);
-    if (lane == 0) atomicAdd(w.spec_stats + 2, (unsigned long long)walks);
+    decodes = __reduce_add_sync(0xFFFFFFFFu, decodes);
+    if (lane == 0) atomicAdd(w.spec_stats + 2, (unsigned long long)decodes);
     __syncthreads();
     uint32_t base = inc - found;
 #pragma unroll
@@ -720,7 +723,7 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
         if (base < d.nblocks) err |= kStTruncated;
         if (round > limit) err |= kStSyncLimit;
         if (err) atomicOr(w.status + d.item, err);
-        atomicAdd(w.spec_stats, (unsigned long long)max(1u, (ncell + 255u) / 256u));
+        atomicAdd(w.spec_stats, (unsigned long long)ncell);
         atomicAdd(w.spec_stats + 1, (unsigned long long)rounds);
     }
 }

@@ -231,8 +231,9 @@ DG_API int dg_batch_bucket(const dg_batch* b, int k, dg_bucket* out);
 DG_API int dg_batch_stage_ms(const dg_batch* b, float ms[DG_STAGE_COUNT]);
 /* Bytes copied host->device by upload, and kernels launched by one run. */
 DG_API int dg_batch_counters(const dg_batch* b, uint64_t* h2d_bytes, uint64_t* d2h_bytes, uint32_t* kernel_launches);
-/* Counters of the speculative entropy decoder over the last run: chunks of subsequences processed, synchronisation
- * rounds, subsequence decodes (guess + re-decodes + write pass).  Synchronises the stream. */
+/* Counters of the speculative entropy decoder over the last run: cells (of 512 or 1024 bits) that the restart-free streams
+ * are cut into, rounds of linking them (added up over the images), decodes of a cell (by every candidate state, again where
+ * no candidate was the right one, once for the values).  Synchronises the stream. */
 DG_API int dg_batch_huffman_stats(dg_batch* b, uint64_t out[3]);
 /* Intermediate device buffers, for stage-by-stage parity tests: coefficient words (int16, scan order) and, for
  * decode+resize batches, the full-size decoded image of item i (its rows padded to a multiple of 16 bytes unless the

@@ -82,6 +82,22 @@ def test_entropy_cells_and_spans(copies):
             assert_same(out, want[i % len(distinct)], str(i))
 
 
+def test_decoder_counters():
+    # cells of 512 bits with this little work: each is decoded by one candidate at least, by one per block of the MCU at most,
+    # and once for the values; where no candidate was right once more or oftener
+    rng = np.random.default_rng(321)
+    data = _noisy(rng, 600, 400, "4:2:0", 90)
+    stream = data[data.index(b"\xff\xda") + 14:-2].replace(b"\xff\x00", b"\xff")
+    cells = (len(stream) * 8 + 511) // 512
+    for copies in (1, 3):
+        with ctx().batch([data] * copies) as b:
+            b.upload(); b.run(); b.sync()
+            st = b.huffman_stats()
+        assert st["chunks"] == copies * cells
+        assert copies <= st["rounds"] <= copies * 200
+        assert 2 * copies * (cells - 2) <= st["subsequence_decodes"] <= 8 * copies * cells
+
+
 @pytest.mark.parametrize("h", [1, 40, 700, 2300])
 def test_resize_pass_cuts(h):
     # one image (CTAs of two chunks) and forty (longer ones), as tall and as flat as a pass gets
