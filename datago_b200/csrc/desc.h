@@ -25,7 +25,6 @@ struct alignas(16) HuffTable {
     // length of the code at the head of window v is 10 + the number of i < 6 with v >= limit[i], and v >= limit[6]
     // means that no code matches.  limit[7] is unused.  (16-byte aligned: read as two vectors.)
     uint32_t limit[8];
-    int32_t maxcode[18];          // [l], l = 1..16: largest code of length l, -1 if none; [17] = INT_MAX
     int32_t valoff[17];           // [l]: index of the first symbol of length l minus its first code
     uint8_t vals[256];
 };

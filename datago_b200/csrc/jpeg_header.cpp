@@ -2,7 +2,6 @@
 // Stands in for what `image::ImageReader::decode()` / zune-jpeg reads before the entropy-coded data
 // (datago call sites: src/worker_files.rs:14-16, src/worker_wds.rs:45, src/worker_http.rs:64).
 // Only what the baseline path needs: SOF0/SOF1, 8-bit, 1 or 3 components, one interleaved scan.
-#include <climits>
 #include <cstring>
 
 #include "host.h"
@@ -173,13 +172,9 @@ bool build_huff_table(const JpegHeader::RawHuff& raw, HuffTable& out) {
                     for (int f = 0; f < span; ++f) out.lut[(code << (kLutBits - l)) | f] = huff_pack((uint32_t)l, raw.vals[k]);
                 }
             }
-            out.maxcode[l] = code - 1;
-        } else {
-            out.maxcode[l] = -1;
         }
         code <<= 1;
     }
-    out.maxcode[17] = INT_MAX;
     // left-aligned end of the code space used by lengths <= l (the first code of the next length, shifted to 16 bits)
     uint32_t used = 0;  // in units of 2^-16 of the code space
     for (int l = 1; l <= 16; ++l) {

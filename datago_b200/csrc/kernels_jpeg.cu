@@ -241,7 +241,7 @@ void launch_idct(const JpegWave& w, uint32_t first, uint32_t count, cudaStream_t
 
 // ---------------------------------------------------------------------------------------------------------------
 // K3  chroma upsampling + YCbCr -> RGB (16-bit fixed point constants 1.402, 0.34414, 0.71414, 1.772), interleaved
-//     RGB8 out.  A CTA owns 256 pixels of two MCU rows, a thread 8 pixels of every eighth row of the tile.
+//     RGB8 out.  A CTA owns 256 pixels of four MCU rows, a thread 8 pixels of every eighth row of the tile.
 //       4:2:0  triangle filter: every output sample is (9a + 3b + 3c + d + bias) >> 4 over its 2x2 chroma
 //              neighbourhood -- one dp4a on bytes gathered from a shared-memory tile (1-sample halo, clamped to the
 //              real plane extent, which is what the edge rules of the filter amount to);
@@ -323,27 +323,12 @@ __device__ __forceinline__ void store_rgb8(uint8_t* o, const uint32_t (&px)[6], 
 struct ChromaPlane {  // per-pixel path
     const uint8_t* p;
     uint32_t pitch;
-    int dw, dh, hs, vs;
+    int dh, hs, vs;
     __device__ __forceinline__ int px(int x, int y) const { return __ldg(p + (size_t)y * pitch + x); }
-    __device__ __forceinline__ int colsum(int cx, int y) const {
-        const int cy = y >> 1;
-        int far = (y & 1) ? cy + 1 : cy - 1;
-        far = min(max(far, 0), dh - 1);
-        return 3 * px(cx, cy) + px(cx, far);
-    }
     __device__ __forceinline__ int at(int x, int y) const {
-        if (hs == 1 && vs == 1) return px(x, y);
-        if (hs == 2 && dw <= 2) return px(x >> 1, vs == 2 ? y >> 1 : y);
-        if (hs == 1) return (colsum(x, y) + ((y & 1) ? 2 : 1)) >> 2;
-        const int cx = x >> 1;
-        if (vs == 1) {
-            const int t = px(cx, y);
-            if (x & 1) return cx == dw - 1 ? t : (3 * t + px(cx + 1, y) + 2) >> 2;
-            return cx == 0 ? t : (3 * t + px(cx - 1, y) + 1) >> 2;
-        }
-        const int t = colsum(cx, y);
-        if (x & 1) return cx == dw - 1 ? (t * 4 + 7) >> 4 : (t * 3 + colsum(cx + 1, y) + 7) >> 4;
-        return cx == 0 ? (t * 4 + 8) >> 4 : (t * 3 + colsum(cx - 1, y) + 8) >> 4;
+        if (hs == 2) return px(x >> 1, vs == 2 ? y >> 1 : y);  // planes at most two samples wide: replicated
+        const int cy = y >> 1, far = min(max((y & 1) ? cy + 1 : cy - 1, 0), dh - 1);  // 4:4:0: triangle filter down the column
+        return (3 * px(x, cy) + px(x, far) + ((y & 1) ? 2 : 1)) >> 2;
     }
 };
 
@@ -569,8 +554,8 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
         return;
     }
     // remaining samplings (4:4:0, chroma planes at most two samples wide): one pixel at a time
-    const ChromaPlane cbp{w.planes + d.plane_off[1], d.plane_pitch[1], dw, dh, hs, vs};
-    const ChromaPlane crp{w.planes + d.plane_off[2], d.plane_pitch[2], dw, dh, hs, vs};
+    const ChromaPlane cbp{w.planes + d.plane_off[1], d.plane_pitch[1], dh, hs, vs};
+    const ChromaPlane crp{w.planes + d.plane_off[2], d.plane_pitch[2], dh, hs, vs};
 #pragma unroll 1
     for (int k = 0; k < nsteps; ++k) {
         const int y = y_base + rowi + 8 * k;

@@ -125,12 +125,12 @@ typedef struct dg_batch dg_batch;
 enum {
     DG_BATCH_DECODE_ONLY = 1u,  /* ignore the ctx transform: payload = decoded image (image_to_payload with img_tfm None) */
     DG_BATCH_TIMING = 2u,       /* record CUDA events around each stage of dg_batch_run */
-    DG_BATCH_KEEP_COEFFICIENTS = 4u, /* leave the decoded coefficients in place for dg_batch_debug (they are normally
-                                        zeroed again as they are consumed) */
+    DG_BATCH_KEEP_COEFFICIENTS = 4u, /* store whole coefficient blocks for dg_batch_debug (normally only the rows that
+                                        hold something are written, and DC terms elsewhere) */
     DG_BATCH_COLLATE = 8u       /* lay the payloads out bucket by bucket, see dg_batch_bucket */
 };
 
-/* Stages reported by dg_batch_stage_ms. */
+/* Stages reported by dg_batch_stage_ms.  DG_STAGE_COEF_CLEAR is always 0: nothing is cleared any more. */
 enum { DG_STAGE_UNSTUFF = 0, DG_STAGE_COEF_CLEAR, DG_STAGE_HUFF_RESTART, DG_STAGE_HUFF_SPEC, DG_STAGE_IDCT, DG_STAGE_COLOR,
        DG_STAGE_RESIZE_H, DG_STAGE_RESIZE_V, DG_STAGE_RESIZE_SHIFT, DG_STAGE_TO_RGB8, DG_STAGE_COUNT };
 
