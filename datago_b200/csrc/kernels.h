@@ -14,6 +14,8 @@ struct OwnerMap {
     uint32_t n, shift, total;
 };
 
+constexpr uint32_t kSms = 148;  // of a B200
+
 // ---- entropy decoding: work splits (see kernels_huff.cu) ------------------------------------------------------------------
 constexpr uint32_t kUnstuffTile = 4096;  // bytes of an entropy-coded segment per CTA of the unstuffing kernels
 // bits of an unstuffed stream per thread of the value decoder; the short form while all threads are resident at once
@@ -22,7 +24,7 @@ constexpr uint32_t kCellsPerCta = 128, kSegsPerCta = 128;
 // synchronising decoder: threads per CTA, the entries of the candidate array per cell, and the cells of a span once a thread
 // per cell and block of the MCU would be more than the chip holds at once
 constexpr uint32_t kGuessLanes = 384, kCandidates = 6, kGuessSpan = 4;
-constexpr uint64_t kGuessSpanThreads = 148 * 2048;
+constexpr uint64_t kGuessSpanThreads = kSms * 2048ull;
 // spans of cells a CTA takes, each with a thread per block of the MCU: what the threads allow, 256 staged cells at most
 #ifdef __CUDACC__
 __host__ __device__
@@ -147,6 +149,10 @@ inline uint32_t conv_tiles(const ConvPass& p, bool vertical) {
 // chunks: two CTAs per resident place of the chip keep its SMs evenly busy to the end, one per place is better where that
 // leaves a CTA only a few chunks, and two chunks are the least a CTA gets.  (One image of 1.5 Mpixel: horizontal pass 20.6 us
 // at four CTAs per place, 15.7 at two, 10.9 at one; 48 images of 5 Mpixel: 275, 253, 252 us, and 268 with CTAs of 2048 rows.)
+#ifndef DG_HMMA_CTAS
+#define DG_HMMA_CTAS 3
+#endif
+constexpr uint32_t kHMmaCtasPerSm = DG_HMMA_CTAS, kVMmaCtasPerSm = 2;
 constexpr uint32_t kMmaMinChunks = 2, kMmaFewChunks = 4, kMmaMaxChunks = 64;
 inline void cut_pass_tiles(ConvPass* passes, size_t n, bool vertical) {
     uint64_t work = 0;  // chunks of all CTAs together
@@ -154,7 +160,7 @@ inline void cut_pass_tiles(ConvPass* passes, size_t n, bool vertical) {
     auto chunks_of = [&](const ConvPass& p) -> uint64_t { return vertical ? (p.out_w * p.channels + kVMmaChunk - 1) / kVMmaChunk : (p.out_h + kHMmaChunk - 1) / kHMmaChunk; };
     for (size_t i = 0; i < n; ++i)
         if (passes[i].fast == 2) work += rows_of_ctas(passes[i]) * chunks_of(passes[i]);
-    const uint64_t places = 148 * (vertical ? 2 : 3), one = (work + places - 1) / places;
+    const uint64_t places = kSms * (vertical ? kVMmaCtasPerSm : kHMmaCtasPerSm), one = (work + places - 1) / places;
     uint64_t chunks = (one + 1) / 2;
     if (chunks < kMmaFewChunks) chunks = one < kMmaFewChunks ? one : kMmaFewChunks;
     chunks = chunks < kMmaMinChunks ? kMmaMinChunks : chunks > kMmaMaxChunks ? kMmaMaxChunks : chunks;

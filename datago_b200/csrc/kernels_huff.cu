@@ -3,7 +3,8 @@
 //
 // Output of this file, per 8x8 block in scan (MCU-interleaved) order:
 //   info[block]  low half: the DC coefficient (int16, prediction resolved); bits 16-17: the block's class
-//   coef[block]  64 int16 in natural order, DC slot zero -- only the rows the class covers are written (and read)
+//   coef[block]  64 int16 in natural order -- only the rows the class covers are written (and read), and the DC slot holds
+//                nothing to rely on: the term is in info[]
 // The class says where the AC coefficients end (kClsFull / kCls4x4 / kCls2x2 / kClsDc).  On photographs at ordinary
 // qualities half of the blocks or more carry a handful of low-frequency coefficients or none, so keeping the DC terms
 // dense and skipping the rows that hold nothing is worth several times the memory traffic of whole blocks, and nothing has
@@ -957,8 +958,8 @@ __global__ void __launch_bounds__(kRestartThreads) k_huff_restart(JpegWave w) {
 // K1b  DC prediction of restart-free images: diff[] holds what info[] will hold, with DC differences, in scan order; the
 //      predictor runs over the blocks of a component.  Kept out of the bit-serial kernels on purpose: there it would cost every symbol of the
 //      synchronising pass a value extraction, here it is a prefix sum over four bytes per block.
-//      One CTA per kDcMcus MCUs of an image; it adds up what lies before its range itself (L2 reads, 32 ranges at most for a
-//      50-megapixel image), so that no CTA waits on another.
+//      One CTA per kDcMcus MCUs of an image; it adds up what lies before its range itself (L2 reads; a 50-megapixel
+//      image has 24 ranges in 4:2:0, 96 in 4:4:4 or gray), so that no CTA waits on another.
 // ---------------------------------------------------------------------------------------------------------------
 namespace {
 
@@ -1116,13 +1117,13 @@ void launch_guess(const JpegWave& w, cudaStream_t s) {
     k_huff_guess<CELL><<<w.guess_ctas.total, kGuessThreads, rows * Staged<CELL>::kPitch + w.max_pairs * 2 * sizeof(SyncTab), s>>>(w);
 }
 
-// With an image per SM or more, 256 threads each leave the most room for other kernels beside them (1024 files of 0.4 Mbit:
-// 3.37 ms a pass against 3.48 with 1024 threads; 256 files of 5 Mbit: 4.29 against 4.30); with fewer, an image gets 1024, so
-// that its threads' runs are short.
+// With an image for most SMs or more, 256 threads each leave the most room for other kernels beside them (1024 files of 0.4
+// Mbit: 3.37 ms a pass against 3.48 with 1024 threads; 256 files of 5 Mbit: 4.29 against 4.30); with fewer, an image gets
+// 1024, so that its threads' runs are short.
 template <int CELL>
 void launch_chain(const JpegWave& w, cudaStream_t s) {
     const size_t tables = w.max_pairs * 2 * sizeof(SyncTab);
-    if (w.n_spec >= 120) k_huff_chain<256, CELL><<<w.n_spec, 256, sizeof(ChainMisc<256>) + tables, s>>>(w);
+    if (w.n_spec >= kSms * 4 / 5) k_huff_chain<256, CELL><<<w.n_spec, 256, sizeof(ChainMisc<256>) + tables, s>>>(w);
     else k_huff_chain<1024, CELL><<<w.n_spec, 1024, sizeof(ChainMisc<1024>) + tables, s>>>(w);
 }
 

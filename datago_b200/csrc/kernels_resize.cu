@@ -160,10 +160,6 @@ __device__ __forceinline__ void conv_h_rows(const ConvPass& p, const Table& tb, 
 constexpr int kHMmaConsumers = 256;   // eight warps multiply
 constexpr int kHMmaProducers = 32;    // one more warp, of which one thread issues the copies into the ring
 constexpr int kHMmaThreads = kHMmaConsumers + kHMmaProducers;
-#ifndef DG_HMMA_CTAS
-#define DG_HMMA_CTAS 3
-#endif
-constexpr int kHMmaCtasPerSm = DG_HMMA_CTAS;
 constexpr int kHMmaRing = kHMmaCtasPerSm == 3 ? 69632 : 98304;  // bytes of the A ring: the CTAs of an SM keep ~200 KB of source rows in flight
 constexpr int kHMmaMaxStages = 8;
 constexpr int kHMmaOutPitch = kHMmaStrip + 8;         // 18 words: the tiles' two-byte writes fall into different banks
@@ -618,7 +614,7 @@ struct VMmaSmem {
     uint8_t out[kVMmaConsumers / 32][8][kVMmaChunk + 16];  // per warp: a chunk's 8 x 64 output bytes (rows padded against bank conflicts)
 };
 
-__global__ void __launch_bounds__(kVMmaThreads, 2) k_conv_v_mma(const ConvPass* passes, OwnerMap map, const uint32_t* tables,
+__global__ void __launch_bounds__(kVMmaThreads, kVMmaCtasPerSm) k_conv_v_mma(const ConvPass* passes, OwnerMap map, const uint32_t* tables,
                                                                 unsigned int* timeouts) {
     extern __shared__ __align__(1024) unsigned char conv_v_smem[];
     VMmaSmem& sm = *reinterpret_cast<VMmaSmem*>(conv_v_smem);
