@@ -1119,11 +1119,13 @@ void launch_guess(const JpegWave& w, cudaStream_t s) {
 
 // With an image for most SMs or more, 256 threads each leave the most room for other kernels beside them (1024 files of 0.4
 // Mbit: 3.37 ms a pass against 3.48 with 1024 threads; 256 files of 5 Mbit: 4.29 against 4.30); with fewer, an image gets
-// 1024, so that its threads' runs are short.
+// 1024, so that its threads' runs are short (waves of 118 and 138 files of 5 Mbit: 270 us for the two launches as the line
+// lies, 319 with 256 threads in both).
+constexpr uint32_t kChainManyImages = 120;
 template <int CELL>
 void launch_chain(const JpegWave& w, cudaStream_t s) {
     const size_t tables = w.max_pairs * 2 * sizeof(SyncTab);
-    if (w.n_spec >= kSms * 4 / 5) k_huff_chain<256, CELL><<<w.n_spec, 256, sizeof(ChainMisc<256>) + tables, s>>>(w);
+    if (w.n_spec >= kChainManyImages) k_huff_chain<256, CELL><<<w.n_spec, 256, sizeof(ChainMisc<256>) + tables, s>>>(w);
     else k_huff_chain<1024, CELL><<<w.n_spec, 1024, sizeof(ChainMisc<1024>) + tables, s>>>(w);
 }
 
