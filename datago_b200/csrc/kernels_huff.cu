@@ -1119,8 +1119,8 @@ void launch_guess(const JpegWave& w, cudaStream_t s) {
 
 // With an image for most SMs or more, 256 threads each leave the most room for other kernels beside them (1024 files of 0.4
 // Mbit: 3.37 ms a pass against 3.48 with 1024 threads; 256 files of 5 Mbit: 4.29 against 4.30); with fewer, an image gets
-// 1024, so that its threads' runs are short (waves of 118 and 138 files of 5 Mbit: 270 us for the two launches as the line
-// lies, 319 with 256 threads in both).
+// 1024, so that its threads' runs are short.  (The launches alone are shorter with 1024 threads even then, 270 against 319 us
+// for the two of the 256 files; a pass, in which other kernels run beside them, is not.)
 constexpr uint32_t kChainManyImages = 120;
 template <int CELL>
 void launch_chain(const JpegWave& w, cudaStream_t s) {
