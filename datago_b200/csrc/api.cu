@@ -1635,7 +1635,8 @@ int dg::batch_download_blocks(dg_batch* b, uint8_t** host, void** blocks) {
         for (next = k + 1; next < order.size() && end(next) - off(k) <= kLandingBytes;) ++next;
         void* block = nullptr;
         const size_t len = end(next - 1) - off(k);
-        rc = host_block_acquire(len, false, &block);
+        // (blocks inside a batch are all of one size, so that those of the next batch are the same ones)
+        rc = host_block_acquire(next < order.size() ? std::max(len, kLandingBytes) : len, false, &block);
         if (rc) break;
         b->landing.push_back(block);
         const cudaError_t e = cudaMemcpyAsync(block, b->d_persist + b->off_out + off(k), len, cudaMemcpyDeviceToHost, ctx->stream);

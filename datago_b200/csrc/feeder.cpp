@@ -214,6 +214,7 @@ extern "C" int dg_feeder_create(int device, const dg_image_config* image_config,
         }
         f->lanes.push_back(std::move(lane));
     }
+    dg::host_blocks_feeder(+1);
     for (auto& l : f->lanes) l->thread = std::thread(lane_main, f.get(), l.get());
     *out = f.release();
     return DG_OK;
@@ -409,6 +410,7 @@ extern "C" void dg_feeder_destroy(dg_feeder* f) {
     }
     f->tickets.clear();
     cudaSetDevice(f->device);
+    dg::host_blocks_feeder(-1);
     for (auto& l : f->lanes) {
         bury(*l);
         dg_ctx_destroy(l->ctx);

@@ -26,9 +26,17 @@ struct Pool {
     struct Entry { size_t size; int refs; };
     std::unordered_map<void*, Entry> blocks;
     std::multimap<size_t, void*> free;  // those with refs == 0, by size
-    size_t busy = 0, idle = 0, limit;
     std::map<int, int> contexts;  // live ones per device
     int last_device = -1;
+    size_t busy = 0, idle = 0, limit;
+    size_t peak = 0;  // most that was referenced at one time while there were feeders
+    int feeders = 0;
+    void add_busy(size_t n) {
+        busy += n;
+        if (feeders > 0 && busy > peak) peak = busy;
+    }
+    // idle bytes to keep
+    size_t keep() const { return contexts.empty() ? 0 : peak > busy + limit ? peak - busy : limit; }
     Pool() {
         const char* mb = getenv("DATAGO_B200_HOST_BLOCKS_MB");
         const long v = mb ? atol(mb) : 1024;
@@ -108,12 +116,12 @@ int acquire(size_t nbytes, bool optional, void** out) {
         if (it != p.free.end() && it->first <= 2 * need) {
             *out = it->second;
             p.idle -= it->first;
-            p.busy += it->first;
+            p.add_busy(it->first);
             p.blocks[it->second].refs = 1;
             p.free.erase(it);
             return DG_OK;
         }
-        p.busy += need;
+        p.add_busy(need);
         device = p.device();
     }
     void* const ptr = map_block(need);
@@ -161,7 +169,7 @@ void host_block_release(void* base) {
         p.busy -= it->second.size;
         p.idle += it->second.size;
         p.free.emplace(it->second.size, base);
-        p.trim(p.contexts.empty() ? 0 : p.limit, &gone);
+        p.trim(p.keep(), &gone);
         device = p.device();
     }
     free_all(gone, device);
@@ -186,7 +194,21 @@ void host_blocks_context(int device, int change) {
         std::lock_guard<std::mutex> lock(p.mu);
         if ((p.contexts[device] += change) <= 0) p.contexts.erase(device);
         p.last_device = device;
-        if (p.contexts.empty()) p.trim(0, &gone);
+        p.trim(p.keep(), &gone);
+    }
+    free_all(gone, device);
+}
+
+void host_blocks_feeder(int change) {
+    Pool& p = pool();
+    std::vector<std::pair<void*, size_t>> gone;
+    int device;
+    {
+        std::lock_guard<std::mutex> lock(p.mu);
+        p.feeders += change;
+        if (p.feeders <= 0) p.peak = 0;
+        p.trim(p.keep(), &gone);
+        device = p.device();
     }
     free_all(gone, device);
 }

@@ -12,7 +12,9 @@
 // Bounds: blocks nobody references are kept for reuse up to a limit (DATAGO_B200_HOST_BLOCKS_MB, default 1024) and freed
 // beyond it, all of them when the last device context of the process goes away.  Requests that have an alternative (`optional`)
 // are refused when they would bring what is referenced above the same amount, so a caller that hoards payloads does not lock
-// all of its memory.
+// all of its memory.  While there are feeders, whose batches have no alternative, blocks are kept for reuse up to the most that
+// was referenced at one time: a batch of 512 photos is 1.6 GB, and locking that anew each time took longer than the decoding
+// (8192 photos through a feeder: 589 images/s, 13 800 with blocks that stay).
 #pragma once
 #include <cstddef>
 
@@ -23,6 +25,7 @@ void host_block_retain(void* base);
 void host_block_release(void* base);
 bool host_blocks_scarce();  // whether more than the limit is referenced
 bool host_blocks_room(size_t nbytes);  // whether optional requests for that much would be granted
+void host_blocks_feeder(int change);  // +1 / -1 feeder
 // +1 / -1 context on `device`.  Blocks are page-locked on a device that has one: the calling thread's current device may be
 // another rank's, and locking there would create a context on it.
 void host_blocks_context(int device, int change);

@@ -17,7 +17,7 @@ std::mutex mu;
 std::set<int> contexts;
 std::map<const void*, std::pair<size_t, int>> locked, allocated;  // page-locked memory with its device; device memory
 size_t device_limit = ~(size_t)0;
-int allocations = 0;
+int allocations = 0, locks = 0;
 thread_local int current = 0;
 size_t total(const std::map<const void*, std::pair<size_t, int>>& m) {
     size_t n = 0;
@@ -34,6 +34,7 @@ cudaError_t cudaHostRegister(void* p, size_t n, unsigned int) {
     std::lock_guard<std::mutex> l(mu);
     contexts.insert(current);
     locked[p] = {n, current};
+    ++locks;
     return cudaSuccess;
 }
 cudaError_t cudaHostUnregister(void* p) {
@@ -78,12 +79,14 @@ int fake_contexts(int device) { std::lock_guard<std::mutex> l(mu); return (int)c
 int fake_locked_on(const void* p) { std::lock_guard<std::mutex> l(mu); auto it = locked.find(p); return it == locked.end() ? -1 : it->second.second; }
 size_t fake_locked_bytes() { std::lock_guard<std::mutex> l(mu); return total(locked); }
 size_t fake_device_bytes() { std::lock_guard<std::mutex> l(mu); return total(allocated); }
+int fake_locks() { std::lock_guard<std::mutex> l(mu); return locks; }
 int fake_allocations() { std::lock_guard<std::mutex> l(mu); return allocations; }
 void fake_device_limit(size_t n) { std::lock_guard<std::mutex> l(mu); device_limit = n; }
 
 int hb_acquire(size_t n, int optional, void** out) { return dg::host_block_acquire(n, optional != 0, out); }
 void hb_retain(void* p) { dg::host_block_retain(p); }
 int hb_scarce() { return dg::host_blocks_scarce(); }
+void hb_feeder(int change) { dg::host_blocks_feeder(change); }
 void hb_context(int device, int change) { dg::host_blocks_context(device, change); }
 
 void* bc_new() { return new dg::BlockCache(false); }

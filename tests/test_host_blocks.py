@@ -81,6 +81,28 @@ def test_limits_hold_for_what_is_referenced_and_for_what_is_idle(pool):
     assert pool.dg_host_alloc(8 * MB, C.byref(p)) == 0
 
 
+def test_a_feeder_keeps_the_blocks_its_batches_need(pool):
+    pool.hb_context(0, 1)
+    pool.hb_feeder(1)
+    for i in range(10):  # 24 MB a batch, two at a time, over a limit of 8
+        batch = [take(pool, 4 * MB, 0) for _ in range(6)]
+        if i:
+            for x in last:
+                pool.dg_host_release(x)
+        last = batch
+        if i == 1:
+            locks = pool.fake_locks()
+    assert pool.fake_locks() == locks and pool.fake_locked_bytes() == 48 * MB
+    p = C.c_void_p()
+    assert pool.dg_host_alloc(MB, C.byref(p)) == E_TOO_LARGE  # others are bounded as before
+    for x in last:
+        pool.dg_host_release(x)
+    assert pool.dg_host_alloc(MB, C.byref(p)) == 0
+    pool.dg_host_release(p)
+    pool.hb_feeder(-1)
+    assert pool.fake_locked_bytes() <= 8 * MB
+
+
 def test_locking_happens_on_a_device_that_has_a_context(pool):
     pool.hb_context(3, 1)  # (this thread has never made a CUDA call: its current device is 0)
     a, b = take(pool, 100), take(pool, 5 * MB)
