@@ -384,10 +384,13 @@ def measure(wl, local_rank, world, barrier, all_max, steps, warmup, e2e_steps, c
     if pms > 0:
         out["post_entropy"] = {"ms": round(pms, 3), "bytes": pbytes, "gbs": round(pbytes / pms / 1e6, 1),
                                "frac": round(pbytes / pms / 1e6 / peak, 4)}
+        # Algorithmic bytes count whole coefficient blocks; the kernels leave out the rows that a block's class does not
+        # cover.  Where the traffic is known and less, it is what was moved.
         per_px = (traffic.get(wl.name) or {}).get("dram_bytes_per_pixel")
-        roofline = {"kernel": kern, "bound": "hbm", "achieved": out["post_entropy"]["gbs"], "peak": peak, "unit": "GB/s",
-                    "frac": out["post_entropy"]["frac"], "traffic": int(per_px * stats["pixels"]) if per_px else None,
-                    "algorithmic_bytes": pbytes,
+        dram = int(per_px * stats["pixels"]) if per_px else None
+        moved = min(pbytes, dram) if dram else pbytes
+        roofline = {"kernel": kern, "bound": "hbm", "achieved": round(moved / pms / 1e6, 1), "peak": peak, "unit": "GB/s",
+                    "frac": round(moved / pms / 1e6 / peak, 4), "traffic": dram, "algorithmic_bytes": pbytes,
                     "longest_stage": max(stages, key=lambda k: stages[k]["ms"]) if stages else None}
     out["roofline"] = roofline
     huff_ms = stage_ms.get("huff_restart", 0.0) + stage_ms.get("huff_spec", 0.0)
