@@ -1,6 +1,7 @@
 #include "host_blocks.h"
 
 #include <cuda_runtime.h>
+#include <pthread.h>
 #include <sys/mman.h>
 
 #include <cstdint>
@@ -56,7 +57,12 @@ struct Pool {
 };
 
 Pool& pool() {
-    static Pool* p = new Pool();  // deliberately leaked: arrays may outlive static destructors
+    static Pool* p = [] {
+        static Pool* made = new Pool();  // deliberately leaked: arrays may outlive static destructors
+        // no other thread is in the middle of it when a process forks: the child hands its inherited arrays back as well
+        pthread_atfork([] { made->mu.lock(); }, [] { made->mu.unlock(); }, [] { made->mu.unlock(); });
+        return made;
+    }();
     return *p;
 }
 
@@ -115,6 +121,7 @@ int acquire(size_t nbytes, bool optional, void** out) {
         const auto it = p.free.lower_bound(need);
         if (it != p.free.end() && it->first <= 2 * need) {
             *out = it->second;
+            madvise(it->second, it->first, MADV_DOFORK);
             p.idle -= it->first;
             p.add_busy(it->first);
             p.blocks[it->second].refs = 1;
@@ -168,6 +175,7 @@ void host_block_release(void* base) {
         if (--it->second.refs) return;
         p.busy -= it->second.size;
         p.idle += it->second.size;
+        madvise(base, it->second.size, MADV_DONTFORK);
         p.free.emplace(it->second.size, base);
         p.trim(p.keep(), &gone);
         device = p.device();
