@@ -321,7 +321,8 @@ DG_API int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, uint3
 
 /* Page-locked host memory for dg_batch_download_packed (or any other use), from a pool the process shares: blocks that have
  * been released are reused, because page-locking is slow and a fresh pageable buffer costs a page fault per 4 KB.  Idle
- * blocks beyond DATAGO_B200_HOST_BLOCKS_MB (default 1024) are freed, and so are all of them with the last context.
+ * blocks beyond DATAGO_B200_HOST_BLOCKS_MB (default 1024; while there are feeders, beyond what their batches need) are
+ * freed, and so are all of them with the last context.
  * DG_E_TOO_LARGE while more than the same amount is in use: fall back to ordinary memory.  Thread-safe. */
 DG_API int dg_host_alloc(uint64_t nbytes, void** out);
 DG_API void dg_host_release(void* block);

@@ -1,7 +1,7 @@
-"""Parity of the code paths that only large batches reach: the narrow-CTA instantiation of the speculative entropy
-decoder (picked when a launch holds at least 1024 restart-free images), batches of several waves (two stream lanes,
-auxiliary streams, scratch blocks reused with a carried zero prefix, the IDCT's zero write-back) and the L2-sized
-IDCT / colour launch groups.  Every payload is compared with the oracle, bit for bit."""
+"""Parity of the code paths that only large batches reach: the narrow-CTA instantiation of the entropy decoder's linking
+kernel (picked when a launch holds at least 120 restart-free images), batches of several waves (two stream lanes,
+auxiliary streams, scratch blocks reused with whatever the last wave left in them) and the L2-sized IDCT / colour launch
+groups.  Every payload is compared with the oracle, bit for bit."""
 import os
 from concurrent.futures import ThreadPoolExecutor
 
@@ -22,8 +22,8 @@ def _oracle_all(datas):
 
 
 def test_many_restart_free_images_in_one_launch():
-    # >= 1024 restart-free images in one wave select the 256-thread decoder CTA; a few long streams need more
-    # than 256 subsequences, i.e. several chunks with the decoder state carried between them
+    # >= 120 restart-free images in one wave select 256 linking threads per image; in a few long streams each of them
+    # owns several cells, in the short ones most own none
     rng = np.random.default_rng(101)
     datas = []
     for i in range(1100):
@@ -43,7 +43,7 @@ def test_many_restart_free_images_in_one_launch():
             coefs, _, _ = oracle.jpeg_decode_stages(datas[i])
             assert np.array_equal(b.debug_coefficients(i), scan_order(coefs, oracle.jpeg_info(datas[i]))), i
         st = b.huffman_stats()
-        assert st["chunks"] >= 1100 + 3 * 2  # every image at least one chunk, the long ones several
+        assert st["chunks"] >= 1100 + 3 * 600  # every image at least one cell, the long ones hundreds
 
 
 def _with_env(name, value):
@@ -75,14 +75,14 @@ def _multi_wave_case(extra_env=None):
     try:
         with c.batch(datas) as b:
             b.upload()
-            for rerun in range(2):  # the second pass reuses both scratch blocks: they must have been left zeroed
+            for rerun in range(2):  # the second pass reuses both scratch blocks, which still hold the first one's coefficients
                 b.run()
                 outs = b.download(); b.sync()
                 for i in range(len(datas)):
                     assert b.result(i).status == 0, (rerun, i)
                     assert_same(outs[i], want[i], f"pass {rerun} image {i}")
             assert b.counters()["kernel_launches"] >= 3 * 4  # at least three waves
-        # a second, different batch on the same context inherits the scratch blocks and their zero prefix
+        # a second, different batch on the same context inherits the scratch blocks with all that is in them
         other = [datas[i] for i in (5, 2, 40, 9, 12, 1)]
         with c.batch(other) as b:
             b.upload(); b.run()
@@ -142,8 +142,8 @@ def test_general_kernels_still_decode_420_images():
 
 
 def test_longest_images_take_the_widest_decoder_beside_the_others():
-    # images with more than 1024 subsequences are decoded by 1024-thread CTAs on the lane's auxiliary stream while the
-    # rest of the wave goes through the ordinary variant; alone in a batch they run on the main stream
+    # images of some hundred thousand bytes, whose linking threads (1024 of them here) own several cells each, beside small
+    # ones and one for the restart decoder on the lane's auxiliary stream; then alone in a batch
     rng = np.random.default_rng(303)
     big = [synth.encode_jpeg(rng.integers(0, 256, (1024, 1024, 3), dtype=np.uint8), 97, "4:4:4", 0),
            synth.encode_jpeg(rng.integers(0, 256, (1400, 900, 3), dtype=np.uint8), 95, "4:2:0", 0)]
