@@ -502,7 +502,7 @@ class Batch:
         return outs
 
     def download_views(self):
-        """Queue copies of the payloads into page-locked blocks of the library, a few payloads to a block of about 4 MB (which
+        """Queue copies of the payloads into page-locked blocks of the library, a few payloads to a block of about 8 MB (which
         lives as long as any of their arrays): one writable array per ok payload, None for the others; valid after sync().
         None while so much of this memory is in use that ordinary memory has to do."""
         ptrs, blocks = (C.c_void_p * max(1, self._n))(), (C.c_void_p * max(1, self._n))()
@@ -510,8 +510,21 @@ class Batch:
         if rc == E_TOO_LARGE:
             return None
         _check(rc)
-        return [np.asarray(_HostBlock(ptrs[i], r.nbytes, C.c_void_p(blocks[i]))).reshape(_shape(r)) if blocks[i] else None
-                for i, r in enumerate(self.results())]
+        blocks, results, ends, memory, outs = list(blocks), self.results(), {}, {}, []
+        for r, p, block in zip(results, ptrs, blocks):
+            if block:
+                ends[block] = max(ends.get(block, 0), p - block + r.nbytes)
+        for r, p, block in zip(results, ptrs, blocks):
+            if not block:
+                outs.append(None)
+                continue
+            whole = memory.get(block)
+            if whole is None:
+                whole = memory[block] = np.asarray(_HostBlock(block, ends[block], C.c_void_p(block)))
+            else:
+                lib().dg_host_release(block)  # one reference for all arrays over the block
+            outs.append(whole[p - block:p - block + r.nbytes].reshape(_shape(r)))
+        return outs
 
     def packed_bytes(self):
         return int(lib().dg_batch_packed_bytes(self._h))

@@ -210,7 +210,7 @@ DG_API int dg_batch_download(dg_batch* b, uint8_t* const* host_out);
  * asynchronous copies fill the driver's submission queue and stall the calling thread. */
 DG_API int dg_batch_download_packed(dg_batch* b, uint8_t* host_base, uint64_t capacity);
 DG_API uint64_t dg_batch_packed_bytes(const dg_batch* b);
-/* Payloads in page-locked memory of the library, a few of them to a block of about 4 MB (a larger payload has its own): for
+/* Payloads in page-locked memory of the library, a few of them to a block of about 8 MB (a larger payload has its own): for
  * every ok item, host_out[i] points at its bytes and blocks[i] is a reference the caller hands to dg_host_release when it is
  * done with that payload (NULL and NULL for the others).  The copies are queued; valid after dg_batch_sync, and for as long
  * as the reference is held, also when the batch and the context are gone.  DG_E_TOO_LARGE while too much page-locked memory
