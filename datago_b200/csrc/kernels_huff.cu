@@ -30,11 +30,6 @@ __device__ __forceinline__ uint32_t owner_of(const OwnerMap& m, uint32_t idx) {
     return o;
 }
 
-__device__ __forceinline__ uint32_t shr_clamp(uint32_t x, uint32_t n) {  // shift counts >= 32 give 0
-    uint32_t r;
-    asm("shr.b32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(n));
-    return r;
-}
 // shared-memory reads by 32-bit address (volatile: the memory behind them changes under asynchronous copies)
 __device__ __forceinline__ uint32_t lds32(uint32_t a) {
     uint32_t v;
@@ -71,40 +66,53 @@ __device__ __forceinline__ uint32_t code_at(const HuffTable* t, uint32_t v) {
     if (!e) return long_code(t, v);
     return ((e >> 6) & 31u) | ((e >> 11) & 255u) << 8;
 }
-__device__ __forceinline__ uint32_t advance_of(uint32_t symbol, bool is_ac) {  // slots a symbol advances
+// slots a symbol advances, or kBlockEnd
+constexpr uint32_t kBlockEnd = 128;
+__device__ __forceinline__ uint32_t advance_of(uint32_t symbol, bool is_ac) {
     const uint32_t s = symbol & 15u, r = symbol >> 4;
-    return !is_ac ? 1u : (s || r == 15u) ? r + 1u : 64u;  // coefficient after a run, ZRL, or end of block
+    return !is_ac ? 1u : (s || r == 15u) ? r + 1u : kBlockEnd;  // coefficient after a run, ZRL, or end of block
 }
 
 // Look-up tables of the two decoders for one (DC, AC) pair of Huffman tables, made on the device (k_unstuff_count), because
-// they are several times the size of what the host sends.  Codes longer than the index: entry 0, and far[] takes over --
-// canonical codes grow with their length, so all of them lie above far_base, and the 16-bit windows from there on are few
-// (190 to 640 for the tables most files carry).  One comparison with far_base picks the array, so that a long code costs no
-// second look-up and no branch: some lane of a warp has one in nearly every step (see entry_at).  Windows behind the end
-// of far[], whose last entry is 0, go to the host's table.
+// they are several times the size of what the host sends.  Both decoders are chains of dependent instructions with few
+// warps to hide them, so the tables are laid out for as few instructions per symbol as possible:
+//   * A lane keeps its place in one register: bits 0-15 the bit position inside the block (relative to a word boundary),
+//     16-21 the slot inside the block, 22-23 "the block has ended" (slot 64 reached, or end of block: kBlockEnd).  A symbol
+//     adds to both fields at once.
+//   * The codes of at most kBits bits fill entries [0, N) by the next kBits bits; the 16-bit windows of longer codes all lie
+//     above those (canonical codes grow with their length) and follow from entry N on, window by window.  The index is then
+//     the larger of (top >> 32 - kBits) and (top >> 16) + off: both are N at the first long window, and the first grows
+//     slower.  No branch and no second look-up for long codes -- some lane of a warp has one in nearly every step.  Windows
+//     behind the last entry, which is 0, and (value decoder) codes that do not exist take the host's table: rare_entry.
 constexpr int kSyncBits = 10, kValueBits = 9;
-// Synchronising decoder: as many whole symbols as the index shows.  bits 0-4 / 5-11: bits consumed and slots advanced by the
-// first symbol alone, 12-16 / 17-23: by all of them, 24-29: slots before the last one (the last counts only if that many do
-// not end the block).  64 slots or more end the block.  A DC symbol is followed by AC symbols of the same component.
+// Synchronising decoder: as many whole symbols as the index shows.  byte 0 / 1: bits consumed and slots advanced (kBlockEnd on
+// top if the last one ends the block) by all of them, byte 2 / 3: by the first alone.  Where all would reach slot 64, the
+// first is taken alone.  A DC symbol is followed by AC symbols of the same component.
 struct SyncTab {
-    uint32_t lut[1 << kSyncBits];
-    uint32_t far[384];
-    uint32_t far_base, huff, is_ac, pad;
+    static constexpr int kBits = kSyncBits, kEntries = (1 << kSyncBits) + 384;
+    uint32_t entry[kEntries];
+    int32_t off;
+    uint32_t huff, is_ac, pad;
 };
-// Value decoder: bits 0-4 code and extra bits together, 5-9 code length, 10-13 extra bits s, 24 no such code, 25-31 slots
-// advanced (the coefficient sits in the last of them; 64: end of block).
+// Value decoder, to be added to a lane's place as it is: bits 0-4 code and extra bits together, 16-23 slots advanced (the
+// coefficient sits in the last of them) or kBlockEnd, 27-31 (32 - s) % 32 for s extra bits: negative if there are any.
 struct ValueTab {
-    uint32_t lut[1 << kValueBits];
-    uint32_t far[640];
-    uint32_t far_base, huff, is_ac, pad;
+    static constexpr int kBits = kValueBits, kEntries = (1 << kValueBits) + 640;
+    uint32_t entry[kEntries];
+    int32_t off;
+    uint32_t huff, is_ac, pad;
 };
 struct CodeTables { SyncTab sync[2]; ValueTab value[2]; };  // [0] DC, [1] AC
 static_assert(sizeof(SyncTab) % 16 == 0 && sizeof(ValueTab) % 16 == 0 && sizeof(CodeTables) == kCodeTablesBytes, "tables are copied in 16-byte pieces");
+constexpr uint32_t kPosMask = 0xFFFFu, kEndMask = 0xC0u << 16;  // of a lane's place
 
-__device__ __forceinline__ uint32_t sync_entry(uint32_t u, uint32_t a) { return u | a << 5 | u << 12 | a << 17; }
+// code: see long_code
+__device__ __forceinline__ uint32_t sync_entry(uint32_t code, bool is_ac) {  // of one symbol
+    return ((code & 31u) + ((code >> 8) & 15u) | advance_of((code >> 8) & 255u, is_ac) << 8) * 0x10001u;
+}
 __device__ __forceinline__ uint32_t value_entry(uint32_t code, bool is_ac) {
     const uint32_t len = code & 31u, s = (code >> 8) & 15u;
-    return (len + s) | len << 5 | s << 10 | (code >> 31) << 24 | advance_of((code >> 8) & 255u, is_ac) << 25;
+    return (len + s) | advance_of((code >> 8) & 255u, is_ac) << 16 | (32u - s) << 27;
 }
 
 __device__ void build_tables(CodeTables& out, const HuffTable* pool, uint32_t dc_id, uint32_t ac_id, int tid, int nthreads) {
@@ -113,64 +121,52 @@ __device__ void build_tables(CodeTables& out, const HuffTable* pool, uint32_t dc
         const HuffTable* const t = pool + (side ? ac_id : dc_id);
         SyncTab& st = out.sync[side];
         ValueTab& vt = out.value[side];
-        for (uint32_t i = tid; i < (1u << kSyncBits); i += nthreads) {
-            const uint32_t window = i << (16 - kSyncBits);
-            uint32_t c = code_at(t, window), e = 0;
-            if ((c & 31u) <= (uint32_t)kSyncBits) {
-                uint32_t u = (c & 31u) + ((c >> 8) & 15u), a = advance_of((c >> 8) & 255u, side != 0), pre = 0;
-                const uint32_t first = u | a << 5;
-                while (u < (uint32_t)kSyncBits && a < 64u) {
-                    c = code_at(ac, (window << u) & 0xFFFFu);
-                    const uint32_t len = c & 31u;
-                    if (u + len > (uint32_t)kSyncBits) break;
-                    pre = a;
-                    u += len + ((c >> 8) & 15u);
-                    a += advance_of((c >> 8) & 255u, true);
-                }
-                e = first | u << 12 | a << 17 | pre << 24;
-            }
-            st.lut[i] = e;
-        }
-        // the windows from the first one that no code of at most kLutBits / kSyncBits bits covers
+        // the first windows that no code of at most kLutBits / kSyncBits bits covers
         uint32_t covered = 0;
         for (int k = 0; k < (1 << kLutBits); k += 32) covered += __popc(__ballot_sync(0xFFFFFFFFu, __ldg(t->lut + k + (tid & 31)) != 0u));
-        const uint32_t vbase = covered << (16 - kLutBits), sbase = __ldg(t->limit + 0);
+        const uint32_t vfar = covered << (16 - kLutBits), sfar = __ldg(t->limit + 0);
+        const uint32_t vnear = vfar >> (16 - kValueBits), snear = sfar >> (16 - kSyncBits);
         static_assert(kValueBits == kLutBits && kSyncBits == 10, "limit[0] covers ten bits");
-        for (uint32_t i = tid; i < sizeof(st.far) / 4; i += nthreads) {
-            const uint32_t c = code_at(t, min(sbase + i, 0xFFFFu));
-            st.far[i] = i + 1 < sizeof(st.far) / 4 ? sync_entry((c & 31u) + ((c >> 8) & 15u), advance_of((c >> 8) & 255u, side != 0)) : 0u;
+        for (uint32_t i = tid; i < (uint32_t)SyncTab::kEntries; i += nthreads) {
+            const uint32_t window = i < snear ? i << (16 - kSyncBits) : min(sfar + (i - snear), 0xFFFFu);
+            uint32_t c = code_at(t, window), e = sync_entry(c, side != 0);
+            if (i < snear) {
+                uint32_t u = e & 31u, a = (e >> 8) & 255u;
+                while (u < (uint32_t)kSyncBits && a < 64u) {
+                    c = code_at(ac, (window << u) & 0xFFFFu);
+                    const uint32_t len = c & 31u, more = advance_of((c >> 8) & 255u, true);
+                    if (u + len > (uint32_t)kSyncBits || (more < kBlockEnd && a + more > 63u)) break;
+                    u += len + ((c >> 8) & 15u);
+                    a += more;
+                }
+                e = (e & 0xFFFF0000u) | u | a << 8;
+            }
+            st.entry[i] = i + 1 < (uint32_t)SyncTab::kEntries ? e : 0u;
         }
-        for (uint32_t i = tid; i < (1u << kValueBits); i += nthreads) {
-            const uint32_t c = code_at(t, i << (16 - kValueBits));
-            vt.lut[i] = (c & 31u) <= (uint32_t)kValueBits ? value_entry(c, side != 0) : 0u;
+        for (uint32_t i = tid; i < (uint32_t)ValueTab::kEntries; i += nthreads) {
+            const uint32_t c = code_at(t, i < vnear ? i << (16 - kValueBits) : min(vfar + (i - vnear), 0xFFFFu));
+            vt.entry[i] = i + 1 < (uint32_t)ValueTab::kEntries && !(c >> 31) ? value_entry(c, side != 0) : 0u;
         }
-        for (uint32_t i = tid; i < sizeof(vt.far) / 4; i += nthreads) vt.far[i] = i + 1 < sizeof(vt.far) / 4 ? value_entry(code_at(t, min(vbase + i, 0xFFFFu)), side != 0) : 0u;
         if (tid == 0) {
-            st.far_base = sbase; vt.far_base = vbase;
+            st.off = (int32_t)snear - (int32_t)sfar; vt.off = (int32_t)vnear - (int32_t)vfar;
             st.huff = vt.huff = side ? ac_id : dc_id;
             st.is_ac = vt.is_ac = side;
         }
     }
 }
 
-// The entry of the code at the head of `top`, 0: see rare_entry.  tab: shared-memory address of the table, off: far_offset()
-// of it.
-template <class Tab> __device__ __forceinline__ uint32_t far_offset(uint32_t far_base) { return (uint32_t)(sizeof(Tab::lut) / 4) - far_base; }
+// The entry of the code at the head of `top`, 0: see rare_entry.  tab: shared-memory address of the table, off: its `off`.
 template <class Tab>
-__device__ __forceinline__ uint32_t entry_at(uint32_t tab, uint32_t off, uint32_t top) {
-    constexpr int kNear = (int)(sizeof(Tab::lut) / 4), kBits = kNear == 1 << kSyncBits ? kSyncBits : kValueBits, kAll = kNear + (int)(sizeof(Tab::far) / 4);
-    static_assert(kNear == 1 << kBits && offsetof(Tab, far) == sizeof(Tab::lut), "far[] follows lut[]");
-    const int32_t behind = (int32_t)((top >> 16) + off);
-    const uint32_t i = behind >= kNear ? (uint32_t)min(behind, kAll - 1) : top >> (32 - kBits);
-    return lds32(tab + i * 4);
+__device__ __forceinline__ uint32_t entry_at(uint32_t tab, int32_t off, uint32_t top) {
+    const int32_t i = min(__viaddmax_s32((int32_t)(top >> 16), off, (int32_t)(top >> (32 - Tab::kBits))), Tab::kEntries - 1);
+    return lds32(tab + (uint32_t)i * 4u);
 }
-// ... of a code whose window lies behind the end of far[]
+// ... of a code whose window lies behind the last entry (x), and the code (y; bit 31: there is no such code).
 template <class Tab>
-__device__ __noinline__ uint32_t rare_entry(uint32_t tab, uint32_t top, const HuffTable* pool) {
+__device__ __noinline__ uint2 rare_entry(uint32_t tab, uint32_t top, const HuffTable* pool) {
     const uint32_t c = long_code(pool + lds32(tab + (uint32_t)offsetof(Tab, huff)), top >> 16);
     const bool is_ac = lds32(tab + (uint32_t)offsetof(Tab, is_ac)) != 0;
-    if (sizeof(Tab) == sizeof(SyncTab)) return sync_entry((c & 31u) + ((c >> 8) & 15u), advance_of((c >> 8) & 255u, is_ac));
-    return value_entry(c, is_ac);
+    return make_uint2(sizeof(Tab) == sizeof(SyncTab) ? sync_entry(c, is_ac) : value_entry(c, is_ac), c);
 }
 
 }  // namespace
@@ -369,18 +365,18 @@ void launch_unstuff(const JpegWave& w, cudaStream_t s) {
 // ---------------------------------------------------------------------------------------------------------------
 namespace {
 
-// Where a decoder stands inside the MCU: the tables of the current block as shared-memory addresses, and the entry of the
-// block after it.  Two reads per block instead of arithmetic on indices.
-struct alignas(16) McuBlock { uint32_t dc, ac, next, index; uint32_t dc_off, ac_off, pad[2]; };
-__device__ __forceinline__ uint2 lds64(uint32_t a) {
-    uint2 v;
-    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+// Where a decoder stands inside the MCU: the DC table of the current block as a shared-memory address (the AC table follows
+// it), the tables' `off`, and the entry of the block after it.  One read per block instead of arithmetic on indices.
+struct alignas(16) McuBlock { uint32_t dc; int32_t dc_off, ac_off; uint32_t next; };
+__device__ __forceinline__ McuBlock lds_mcu(uint32_t a) {
+    McuBlock v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.dc), "=r"(v.dc_off), "=r"(v.ac_off), "=r"(v.next) : "r"(a));
     return v;
 }
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-    return v;
+// index inside the MCU of the block whose entry names `next`
+__device__ __forceinline__ uint32_t mcu_index(uint32_t mcu0, uint32_t next, uint32_t bpm) {
+    const uint32_t n = (next - mcu0) / (uint32_t)sizeof(McuBlock);
+    return (n ? n : bpm) - 1u;
 }
 // The image's tables into shared memory, each distinct pair once.  Tab: SyncTab or ValueTab; which: offset of its [2] array
 // inside CodeTables.
@@ -400,78 +396,82 @@ __device__ __forceinline__ void load_tables(const JpegWave& w, const JpegDesc& d
         const uint32_t luma = d.hs * d.vs, slot = (uint32_t)tid < luma ? 0u : (uint32_t)tid == luma ? slot1 : slot2;
         const uint32_t at = smem_addr(tab0) + slot * 2 * (uint32_t)sizeof(Tab);
         const Tab* const tabs = reinterpret_cast<const Tab*>(w.codes + (size_t)(slot == 0 ? p0 : slot == slot1 ? p1 : p2) * kCodeTablesBytes + which);
-        mcu[tid] = McuBlock{at, at + (uint32_t)sizeof(Tab), smem_addr(&mcu[(uint32_t)tid + 1 == d.bpm ? 0 : tid + 1]), (uint32_t)tid,
-                            far_offset<Tab>(__ldg(&tabs[0].far_base)), far_offset<Tab>(__ldg(&tabs[1].far_base)), {0, 0}};
+        mcu[tid] = McuBlock{at, __ldg(&tabs[0].off), __ldg(&tabs[1].off), smem_addr(&mcu[(uint32_t)tid + 1 == d.bpm ? 0 : tid + 1])};
     }
 }
 
-// Window of two stream words (w0 holds the current bit): when bit position `was` -> `now` crosses a word boundary (one at
-// most: symbols have 31 bits at most), w0 takes w1 and w1 the word behind the one at address `word`.  Predicated by hand:
-// some lane of a warp crosses in nearly every step.
-__device__ __forceinline__ void advance_window(uint32_t& w0, uint32_t& w1, uint32_t was, uint32_t now, uint32_t word) {
-    asm volatile("{\n .reg .pred q;\n setp.ge.u32 q, %2, 32;\n @q mov.u32 %0, %1;\n @q ld.shared.u32 %1, [%3+4];\n}" : "+r"(w0), "+r"(w1) : "r"(was ^ now), "r"(word));
-}
-// Streams in shared memory: at(p) is the address of the word that holds bit p; the word behind it follows.
-template <class Address>
+// Streams in shared memory: a lane's window is two words (w0 holds its current bit), `cur` the address of the first.  base: the
+// address bit 0 of the stream would have.  step: w0 takes w1 and w1 the word behind it where `crossed` is not zero; predicated
+// by hand, because some lane of a warp crosses in nearly every step.
 struct SharedSource {
-    Address at;
-    __device__ __forceinline__ void start(uint32_t& w0, uint32_t& w1, uint32_t p) const { w0 = lds32(at(p)); w1 = lds32(at(p) + 4); }
-    __device__ __forceinline__ void advance(uint32_t& w0, uint32_t& w1, uint32_t was, uint32_t now) const { advance_window(w0, w1, was, now, at(now)); }
+    uint32_t base;
+    __device__ __forceinline__ uint32_t start(uint32_t& w0, uint32_t& w1, uint32_t p) const {
+        const uint32_t cur = base + ((p >> 3) & ~3u);
+        w0 = lds32(cur); w1 = lds32(cur + 4);
+        return cur;
+    }
+    __device__ __forceinline__ void step(uint32_t& w0, uint32_t& w1, uint32_t& cur, uint32_t crossed) const {
+        asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %3, 0;\n @q mov.u32 %0, %1;\n @q ld.shared.u32 %1, [%2+8];\n @q add.u32 %2, %2, 4;\n}"
+                     : "+r"(w0), "+r"(w1), "+r"(cur) : "r"(crossed));
+    }
 };
-template <class Address> __device__ __forceinline__ SharedSource<Address> shared_source(Address at) { return SharedSource<Address>{at}; }
-// ... and in global memory
+// ... and in global memory; `cur` is the index of the first word
 struct GlobalSource {
     const uint32_t* words;
     uint32_t n;
     __device__ __forceinline__ uint32_t word(uint32_t i) const { return i < n ? __ldg(words + i) : 0u; }
-    __device__ __forceinline__ void start(uint32_t& w0, uint32_t& w1, uint32_t p) const { w0 = word(p >> 5); w1 = word((p >> 5) + 1); }
-    __device__ __forceinline__ void advance(uint32_t& w0, uint32_t& w1, uint32_t was, uint32_t now) const {
-        if ((was ^ now) >= 32u) { w0 = w1; w1 = word((now >> 5) + 1); }
+    __device__ __forceinline__ uint32_t start(uint32_t& w0, uint32_t& w1, uint32_t p) const {
+        w0 = word(p >> 5); w1 = word((p >> 5) + 1);
+        return p >> 5;
+    }
+    __device__ __forceinline__ void step(uint32_t& w0, uint32_t& w1, uint32_t& cur, uint32_t crossed) const {
+        if (crossed) { w0 = w1; w1 = word(++cur + 1); }
     }
 };
 
 // A lane of a synchronising decoder.
 struct SyncLane {
-    uint32_t p, z, nb;   // bit position, slot inside the block, blocks ended since nb was last set to zero
-    uint32_t w0, w1, tab, off;
-    uint4 mb;            // McuBlock of the current block
-    uint2 mo;
+    uint32_t base, at;   // a word boundary of the stream; the lane's place (see SyncTab), its bit position counted from there
+    uint32_t nb;         // blocks ended since nb was last set to zero
+    uint32_t w0, w1, cur, tab;
+    int32_t off;
+    McuBlock mb;         // of the current block
+    // at a block start, or (`inside`) as if the DC term of the block had been passed
     template <class Source>
-    __device__ __forceinline__ void start(const Source& src, uint32_t mcu0, uint32_t bit, uint32_t slot, uint32_t c) {
-        p = bit; z = slot; nb = 0;
-        src.start(w0, w1, p);
-        mb = lds128(mcu0 + c * (uint32_t)sizeof(McuBlock));
-        mo = lds64(mcu0 + c * (uint32_t)sizeof(McuBlock) + 16);
-        tab = z ? mb.y : mb.x;
-        off = z ? mo.y : mo.x;
+    __device__ __forceinline__ void start(const Source& src, uint32_t mcu0, uint32_t bit, bool inside, uint32_t c) {
+        base = bit & ~31u; at = (bit & 31u) | (inside ? 1u << 16 : 0u); nb = 0;
+        cur = src.start(w0, w1, bit);
+        mb = lds_mcu(mcu0 + c * (uint32_t)sizeof(McuBlock));
+        tab = inside ? mb.dc + (uint32_t)sizeof(SyncTab) : mb.dc;
+        off = inside ? mb.ac_off : mb.dc_off;
     }
-    // Lanes with `live` decode to the first block start at p >= stop.  Called by whole warps: the loop has one exit, taken by
-    // all lanes together, and no other jump out of it -- with returns from inside, the lanes of a warp never met again
-    // after their first different turn and went on alone.
+    __device__ __forceinline__ uint32_t pos() const { return base + (at & kPosMask); }
+    // Lanes with `live` decode to the first block start at a position of at least `stop`.  Called by whole warps: the loop has
+    // one exit, taken by all lanes together, and no other jump out of it -- with returns from inside, the lanes of a warp
+    // never met again after their first different turn and went on alone.
     template <class Source>
     __device__ __forceinline__ void run_to(bool live, uint32_t stop, const Source& src, const HuffTable* pool) {
+        const uint32_t stop_at = stop > base ? stop - base : 0u;
         while (__any_sync(0xFFFFFFFFu, live)) {
 #pragma unroll
             for (int step = 0; step < 4; ++step) {
                 if (live) {
-                    const uint32_t top = __funnelshift_l(w1, w0, p);
+                    const uint32_t top = __funnelshift_l(w1, w0, at);
                     uint32_t e = entry_at<SyncTab>(tab, off, top);
-                    if (e == 0) e = rare_entry<SyncTab>(tab, top, pool);
-                    const uint32_t h = z + (e >> 24) >= 64u ? e : e >> 12;
-                    const uint32_t was = p;
-                    p += h & 31u;
-                    z += (h >> 5) & 127u;
-                    tab = mb.y;
-                    off = mo.y;
-                    src.advance(w0, w1, was, p);
-                    if (z >= 64u) {
-                        z = 0;
+                    if (e == 0) e = rare_entry<SyncTab>(tab, top, pool).x;
+                    const uint32_t was = at;
+                    at = was + __byte_perm(e, 0u, 0x4140);                                 // all symbols
+                    if (at & (64u << 16)) at = was + __byte_perm(e, 0u, 0x4342);           // slot 64: the first alone
+                    src.step(w0, w1, cur, (was ^ at) & 32u);
+                    tab = mb.dc + (uint32_t)sizeof(SyncTab);
+                    off = mb.ac_off;
+                    if (at & kEndMask) {
+                        at &= kPosMask;
                         ++nb;
-                        mo = lds64(mb.z + 16);
-                        mb = lds128(mb.z);
-                        tab = mb.x;
-                        off = mo.x;
-                        live = p < stop;
+                        mb = lds_mcu(mb.next);
+                        tab = mb.dc;
+                        off = mb.dc_off;
+                        live = at < stop_at;
                     }
                 }
             }
@@ -479,22 +479,19 @@ struct SyncLane {
     }
 };
 
-// Streams staged in shared memory, a cell per row and the first 16 bytes of the next cell behind it (which spreads the rows
-// over the banks and makes the word behind any word its neighbour).  A block may run 1984 bits (64 symbols of 31 bits) into
-// what follows the last cell, and the padding of a stream covers that: kRowsBehind, kRowsPadded.
+// Streams staged in shared memory: consecutive cells.  A block may run 1984 bits (64 symbols of 31 bits) into what follows the
+// last cell, and the padding of a stream covers that: kRowsBehind, kRowsPadded.  (Cells of 1024 bits start in the same bank;
+// padding them apart costs more instructions per symbol than the conflicts of the few lanes that load in one step.)
 template <int CELL>
 struct Staged {
-    static constexpr int kPitch = CELL / 8 + 16, kRowsBehind = 1984 / CELL + 2, kRowsPadded = 2048 / CELL;
+    static constexpr int kPitch = CELL / 8, kRowsBehind = 1984 / CELL + 2, kRowsPadded = 2048 / CELL;
     // cells [row0, row0 + rows) of the stream `us`
     static __device__ __forceinline__ void copy(unsigned char* stage, const uint8_t* us, uint32_t row0, int rows, int tid, int nthreads) {
-        constexpr int kPieces = CELL / 128 + 1;  // 16-byte pieces per row
-        const uint8_t* src = us + (size_t)row0 * (CELL / 8);
+        const uint8_t* src = us + (size_t)row0 * kPitch;
         const uint32_t dst = smem_addr(stage);
-        for (int i = tid; i < rows * kPieces; i += nthreads) copy16(dst + i * 16, src + (i / kPieces) * (CELL / 8) + (i % kPieces) * 16);
+        for (int i = tid; i < rows * (kPitch / 16); i += nthreads) copy16(dst + i * 16, src + i * 16);
         copy_commit();
     }
-    // shared-memory address of the word with bit p; base: address row 0 of the stream would have
-    static __device__ __forceinline__ uint32_t at(uint32_t base, uint32_t p) { return base + ((p >> 3) & ~3u) + (p / CELL) * 16; }
 };
 static_assert(kStreamPad >= (2048 + 1024) / 8 + 16, "rows behind the end of a stream are copied");
 static_assert((1ull << 32) - kMaxStream * 8ull > 2ull * kCellsPerCta * kCellBits + 4096, "positions behind the end of a stream do not wrap");
@@ -536,18 +533,18 @@ __global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
         reinterpret_cast<uint4*>(cand)[i] = make_uint4(kStDropped, 0, kStDropped, 0);
     copy_wait<0>();
     __syncthreads();
-    const uint32_t sbase = smem_addr(stage) - row0 * Staged<CELL>::kPitch, mcu0 = smem_addr(&mcu[0]);
-    const auto source = shared_source([&](uint32_t p) { return Staged<CELL>::at(sbase, p); });
+    const uint32_t mcu0 = smem_addr(&mcu[0]);
+    const SharedSource source{smem_addr(stage) - row0 * (uint32_t)Staged<CELL>::kPitch};
 
     // ---- the lead: from its first bit on, as if inside each of the MCU's blocks
     const uint32_t mine = cell0 + (uint32_t)tid / bpm * span, myh = (uint32_t)tid % bpm;  // first cell of this thread's span
     const bool live = (uint32_t)tid < nspans * bpm && mine < ncell;
     uint32_t k = live ? mine : cell0;
     SyncLane L{};
-    L.start(source, mcu0, k ? k * CELL - kLeadBits : 0u, k ? 1u : 0u, live && k ? myh : 0u);
+    L.start(source, mcu0, k ? k * CELL - kLeadBits : 0u, k != 0u, live && k ? myh : 0u);
     L.run_to(live && k, k * CELL, source, w.huff);
     uint32_t decodes = 0;
-    s_state[tid] = (uint16_t)(live ? pack_state(L.p, k * CELL, L.mb.w, total) : kStNone);
+    s_state[tid] = (uint16_t)(live ? pack_state(L.pos(), k * CELL, mcu_index(mcu0, L.mb.next, bpm), total) : kStNone);
     for (uint32_t step = 0; step < span; ++step) {
         __syncthreads();
         // ---- the distinct states, in as few warps as they fill
@@ -570,12 +567,12 @@ __global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
             const uint32_t t = s_list[on ? tid : warp * 32], entry = s_state[t];
             k = cell0 + t / bpm * span + step;
             const uint32_t bound = (k + 1) * CELL, p = k * CELL + (entry & 0xFFFu);
-            L.start(source, mcu0, p, 0, entry >> 12);
+            L.start(source, mcu0, p, false, entry >> 12);
             L.run_to(on && p < bound, min(bound, total + 1), source, w.huff);
             __syncwarp();
             if (on) {
-                const uint32_t exit = pack_state(L.p, bound, L.mb.w, total);
-                if (L.p > total) --L.nb;  // the block that ended here is not whole
+                const uint32_t exit = pack_state(L.pos(), bound, mcu_index(mcu0, L.mb.next, bpm), total);
+                if (L.pos() > total) --L.nb;  // the block that ended here is not whole
                 cand[(size_t)k * kCandidates + t % bpm] = make_uint2(entry | exit << 16, L.nb);
                 s_state[t] = (uint16_t)exit;
             }
@@ -689,12 +686,12 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
             if (__any_sync(0xFFFFFFFFu, decode)) {
                 const uint32_t k = decode ? open_at : 0, bound = (k + 1) * CELL, p = k * CELL + (decode ? open_state & 0xFFFu : 0u);
                 SyncLane L;
-                L.start(source, mcu0, p, 0, decode ? open_state >> 12 : 0u);
+                L.start(source, mcu0, p, false, decode ? open_state >> 12 : 0u);
                 L.run_to(decode, min(bound, total + 1), source, w.huff);
                 __syncwarp();
                 if (decode) {
                     ++decodes;
-                    const uint32_t n = L.nb - (L.p > total ? 1u : 0u), next = pack_state(L.p, bound, L.mb.w, total);
+                    const uint32_t n = L.nb - (L.pos() > total ? 1u : 0u), next = pack_state(L.pos(), bound, mcu_index(mcu0, L.mb.next, d.bpm), total);
                     found += n - (recs[k].y & 0xFFFu);
                     recs[k] = make_uint2(p, open_state << 12 | n);
                     if (k + 1 == kend) { exit = next; open_at = ~0u; last_open = 0; }
@@ -733,14 +730,15 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
 namespace {
 
 constexpr uint32_t kBlankBlock = (uint32_t)kClsDc << 16;  // in info[]: a block the stream does not hold
-constexpr uint32_t kNotDc = 1u << 28, kNot2x2 = 1u << 29, kNot4x4 = 1u << 30;
+constexpr uint32_t kNotDc = 1u, kNot2x2 = 2u, kNot4x4 = 4u;
 
 // Zig-zag position -> byte offset of the coefficient in a lane's block buffer (row r of the lane's block sits at
-// r * T * 16: rows of neighbouring lanes are neighbours, so whole-row accesses are conflict free) | class flags.
+// r * T * 16: rows of neighbouring lanes are neighbours, so whole-row accesses are conflict free) << 16 | class flags.
 template <int T>
 __device__ __forceinline__ uint32_t place_of(uint32_t zz) {
+    static_assert(8 * T * 16 <= 65536, "offsets are 16-bit numbers");
     const uint32_t nat = kNatural[zz], r = nat >> 3, c = nat & 7u;
-    return r * (T * 16) + c * 2 | (zz ? kNotDc : 0u) | (r > 1 || c > 1 ? kNot2x2 : 0u) | (r > 3 || c > 3 ? kNot4x4 : 0u);
+    return (r * (T * 16) + c * 2) << 16 | (zz ? kNotDc : 0u) | (r > 1 || c > 1 ? kNot2x2 : 0u) | (r > 3 || c > 3 ? kNot4x4 : 0u);
 }
 
 template <int T>
@@ -748,7 +746,6 @@ struct ValueMisc {
     uint4 block[8 * T];    // the lanes' current blocks
     uint32_t place[64];
     McuBlock mcu[6];
-    uint32_t pad[8];
 };
 
 // Shared memory of the value decoder: [ValueMisc | ... | tables].  The caller waits for the copies and the barrier.
@@ -770,59 +767,68 @@ __device__ __forceinline__ void value_setup(const JpegWave& w, const JpegDesc& d
 // One code path for DC and AC symbols, the DC difference going to slot 0 of the block buffer like any coefficient: the lanes
 // of a warp are at unrelated places.  For the same reason a lane whose block is complete waits until kFlushLanes lanes
 // have one (or no lane has anything else to do): writing a block out takes more instructions than decoding a symbol,
-// and they cost the same whether two lanes execute them or ten.
+// and they cost the same whether two lanes execute them or ten.  The warp looks for such lanes after every other symbol.
 constexpr int kFlushLanes = 8;
 
 template <int T, bool ABSOLUTE, class Source>
-__device__ __forceinline__ uint32_t decode_blocks(const Source& src, uint32_t p, uint32_t blk, const uint32_t end, const uint32_t limit, const uint32_t stop,
-                                                  uint32_t c, const uint32_t luma, ValueMisc<T>& sh, const HuffTable* pool, int16_t* __restrict__ coef,
+__device__ __forceinline__ uint32_t decode_blocks(const Source& src, const uint32_t p, uint32_t blk, const uint32_t end, const uint32_t limit, const uint32_t stop,
+                                                  uint32_t c, const JpegDesc& d, ValueMisc<T>& sh, const HuffTable* pool, int16_t* __restrict__ coef,
                                                   uint32_t* __restrict__ info, uint32_t& err) {
-    const uint32_t first = blk;
+    const uint32_t first = blk, mcu0 = smem_addr(&sh.mcu[0]);
     bool live = blk < end;
-    uint32_t w0, w1;
-    src.start(w0, w1, p);
+    uint32_t w0, w1, cur = src.start(w0, w1, p);
+    uint32_t base = p & ~31u, at = p & 31u;  // of the current block: a word boundary, the lane's place (see ValueTab)
     const uint32_t place = smem_addr(sh.place) - 4, buf = smem_addr(&sh.block[threadIdx.x]);
-    uint4 mb = lds128(smem_addr(&sh.mcu[0]) + c * sizeof(McuBlock));
-    uint2 mo = lds64(smem_addr(&sh.mcu[0]) + c * sizeof(McuBlock) + 16);
-    uint32_t tab = mb.x, off = mo.x, z = 0, seen = 0;
+    McuBlock mb = lds_mcu(mcu0 + c * (uint32_t)sizeof(McuBlock));
+    uint32_t tab = mb.dc, seen = 0, e = 0;
+    int32_t off = mb.dc_off;
     int32_t pred0 = 0, pred1 = 0, pred2 = 0;
     for (;;) {
         const uint32_t alive = __ballot_sync(0xFFFFFFFFu, live);
         if (!alive) break;  // one exit for the whole warp, see SyncLane::run_to
-        if (live && z < 64u) {
-            const uint32_t top = __funnelshift_l(w1, w0, p);
-            uint32_t e = entry_at<ValueTab>(tab, off, top);
-            if (e == 0) e = rare_entry<ValueTab>(tab, top, pool);
-            if (((e >> 24) & 1u) && p < limit) err |= kStBadCode;
-            const uint32_t was = p, s = (e >> 10) & 15u;
-            // the s extra bits (T.81 EXTEND): a leading 1 means the value itself, a leading 0 the complement of its magnitude
-            const uint32_t bits = top << ((e >> 5) & 31u);
-            const int32_t neg = ~((int32_t)bits >> 31);
-            const int32_t v = (int32_t)(shr_clamp(bits ^ (uint32_t)neg, 32u - s) ^ (uint32_t)neg) - neg;
-            p += e & 31u;
-            z += e >> 25;
-            src.advance(w0, w1, was, p);
-            if (s && z <= 64u) {
-                const uint32_t pl = lds32(place + z * 4);
-                asm volatile("st.shared.u16 [%0], %1;" ::"r"(buf + (pl & 0xFFFFu)), "h"((uint16_t)v) : "memory");
-                seen |= pl;
+#pragma unroll
+        for (int step = 0; step < 2; ++step) {
+            if (live && !(at & kEndMask)) {
+                const uint32_t top = __funnelshift_l(w1, w0, at);
+                e = entry_at<ValueTab>(tab, off, top);
+                if (e == 0) {
+                    const uint2 rare = rare_entry<ValueTab>(tab, top, pool);
+                    e = rare.x;
+                    if (rare.y >> 31 && base + (at & kPosMask) < limit) err |= kStBadCode;
+                }
+                const uint32_t was = at;
+                at += e;
+                src.step(w0, w1, cur, (was ^ at) & 32u);
+                // the s extra bits (T.81 EXTEND), first moved to the top: a leading 1 means the value itself, a leading 0 the
+                // complement of its magnitude
+                const uint32_t n = e >> 27, bits = __funnelshift_l(0u, __funnelshift_l(top, 0u, e), n);
+                const uint32_t neg = ~(uint32_t)((int32_t)bits >> 31);
+                const uint32_t v = __funnelshift_r(bits, neg, n) - neg;
+                const uint32_t slot = at >> 14 & 0x3FCu;  // (times four)
+                if ((int32_t)e < 0 && slot <= 256u) {
+                    const uint32_t pl = lds32(place + slot);
+                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(buf + (pl >> 16)), "h"((uint16_t)v) : "memory");
+                    seen |= pl;
+                }
+                tab = mb.dc + (uint32_t)sizeof(ValueTab);
+                off = mb.ac_off;
             }
-            if (s && z > 64u && p <= limit) err |= kStCoefRange;
-            tab = mb.y;
-            off = mo.y;
         }
-        const uint32_t done = __ballot_sync(0xFFFFFFFFu, live && z >= 64u);
+        const uint32_t done = __ballot_sync(0xFFFFFFFFu, live && (at & kEndMask));
         if (__popc(done) >= kFlushLanes || done == alive) {
-            if (live && z >= 64u) {
-                if (p > limit) live = false;  // (what the buffer holds is of no use, and neither is the rest of the span)
+            if (live && (at & kEndMask)) {
+                const uint32_t now = base + (at & kPosMask);
+                if (now > limit) live = false;  // (what the buffer holds is of no use, and neither is the rest of the span)
                 else {
+                    if ((int32_t)e < 0 && (at >> 14 & 0x3FCu) > 256u) err |= kStCoefRange;
                     uint4* const b = sh.block + threadIdx.x;
                     uint4* const rows = reinterpret_cast<uint4*>(coef) + (size_t)blk * 8;
                     const uint4 zero = make_uint4(0, 0, 0, 0), q0 = b[0];
                     int32_t dc = (int16_t)(q0.x & 0xFFFFu);
                     if (ABSOLUTE) {
-                        if (mb.w < luma) dc = pred0 += dc;
-                        else if (mb.w == luma) dc = pred1 += dc;
+                        const uint32_t luma = d.hs * d.vs, k = mcu_index(mcu0, mb.next, d.bpm);
+                        if (k < luma) dc = pred0 += dc;
+                        else if (k == luma) dc = pred1 += dc;
                         else dc = pred2 += dc;
                     }
                     const uint32_t cls = seen & kNot4x4 ? (uint32_t)kClsFull : seen & kNot2x2 ? (uint32_t)kCls4x4 : seen & kNotDc ? (uint32_t)kCls2x2 : (uint32_t)kClsDc;
@@ -841,12 +847,12 @@ __device__ __forceinline__ uint32_t decode_blocks(const Source& src, uint32_t p,
                         for (int q = 4; q < 8; ++q) { rows[q] = b[q * T]; b[q * T] = zero; }
                     }
                     ++blk;
-                    live = blk < end && p < stop;
-                    z = 0; seen = 0;
-                    mo = lds64(mb.z + 16);
-                    mb = lds128(mb.z);
-                    tab = mb.x;
-                    off = mo.x;
+                    live = blk < end && now < stop;
+                    base = now & ~31u; at = now & 31u;
+                    seen = 0;
+                    mb = lds_mcu(mb.next);
+                    tab = mb.dc;
+                    off = mb.dc_off;
                 }
             }
         }
@@ -887,10 +893,9 @@ __global__ void __launch_bounds__(kWriteThreads) k_huff_write(JpegWave w) {
     copy_wait<0>();
     __syncthreads();
     uint32_t err = 0;
-    const uint32_t sbase = smem_addr(stage) - cell0 * Staged<CELL>::kPitch;
-    const auto source = shared_source([&](uint32_t p) { return Staged<CELL>::at(sbase, p); });
+    const SharedSource source{smem_addr(stage) - cell0 * (uint32_t)Staged<CELL>::kPitch};
     const uint32_t p0 = a.y < b1 ? a.x : cell0 * CELL;
-    decode_blocks<kWriteThreads, false>(source, p0, a.y, b1, total, (cell0 + kCellsPerCta) * CELL, a.y % d.bpm, d.hs * d.vs, sh, w.huff,
+    decode_blocks<kWriteThreads, false>(source, p0, a.y, b1, total, (cell0 + kCellsPerCta) * CELL, a.y % d.bpm, d, sh, w.huff,
                                         w.coef + d.block_off * 64, w.diff + d.block_off, err);
     if (err) atomicOr(w.status + d.item, err);
 }
@@ -942,12 +947,10 @@ __global__ void __launch_bounds__(kRestartThreads) k_huff_restart(JpegWave w) {
     int16_t* coef = w.coef + d.block_off * 64;
     uint32_t err = 0, n;
     if (staged) {
-        const uint32_t sbase = smem_addr(stage) - lo;
-        n = decode_blocks<kRestartThreads, true>(shared_source([&](uint32_t p) { return sbase + ((p >> 3) & ~3u); }), b0 * 8u, blk0, end, b1 * 8u, b1 * 8u, 0u,
-                                                 d.hs * d.vs, sh, w.huff, coef, info, err);
+        n = decode_blocks<kRestartThreads, true>(SharedSource{smem_addr(stage) - lo}, b0 * 8u, blk0, end, b1 * 8u, b1 * 8u, 0u, d, sh, w.huff, coef, info, err);
     } else {
         const GlobalSource source{reinterpret_cast<const uint32_t*>(us), (us_len + 3) / 4 + 2};
-        n = decode_blocks<kRestartThreads, true>(source, b0 * 8u, blk0, end, b1 * 8u, b1 * 8u, 0u, d.hs * d.vs, sh, w.huff, coef, info, err);
+        n = decode_blocks<kRestartThreads, true>(source, b0 * 8u, blk0, end, b1 * 8u, b1 * 8u, 0u, d, sh, w.huff, coef, info, err);
     }
     if (n < end - blk0) err |= kStTruncated;
     if (n < blk1 - blk0) blank(blk0 + n);
