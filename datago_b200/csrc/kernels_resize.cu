@@ -177,14 +177,31 @@ __device__ __forceinline__ void load_a(uint32_t (&a)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr) : "memory");
 }
-__device__ __forceinline__ void mma_u8s8(int32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+// (first: the accumulators start at zero, which the instruction takes as its third operand)
+__device__ __forceinline__ void mma_u8s8(int32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, bool first) {
+    if (first)
+        asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+            : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
+    else
+        asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mma_u8u8(int32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+__device__ __forceinline__ void mma_u8u8(int32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, bool first) {
+    if (first)
+        asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+            : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
+    else
+        asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// A chunk's place in the ring: the slot, and the parity of the slot's fillings before it.  (Chunk number % and / ring length,
+// per warp and chunk, were a fifth of the horizontal kernel's instructions.)
+struct RingPlace {
+    uint32_t slot = 0, phase = 0;
+    __device__ __forceinline__ void next(uint32_t nstage) {
+        if (++slot == nstage) { slot = 0; phase ^= 1u; }
+    }
+};
 
 // mbarrier helpers: two barriers per ring slot, "filled" (the copies into it have landed) and "drained"
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -279,9 +296,10 @@ __global__ void __launch_bounds__(kHMmaThreads, kHMmaCtasPerSm) k_conv_h_mma(con
         // the descriptor sits in global memory that earlier batches may have used for other descriptors
         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
         const int32_t x_word = strip_lo >> 2;
-        for (uint32_t c = 0; c < nchunks && !gave_up; ++c) {
-            const uint32_t slot = c % nstage, use = c / nstage;
-            if (use > 0) wait_for(bar0 + 8 * (kHMmaMaxStages + slot), (use - 1) & 1u);
+        RingPlace at;
+        for (uint32_t c = 0; c < nchunks && !gave_up; ++c, at.next(nstage)) {
+            const uint32_t slot = at.slot;
+            if (c >= nstage) wait_for(bar0 + 8 * (kHMmaMaxStages + slot), at.phase ^ 1u);
             if (gave_up) break;
             mbar_expect_tx(bar0 + 8 * slot, stage_bytes);
             tensor_copy_2d(a_base + slot * stage_bytes, map, x_word, (int32_t)(y_first + c * kHMmaChunk), bar0 + 8 * slot);
@@ -332,14 +350,11 @@ __global__ void __launch_bounds__(kHMmaThreads, kHMmaCtasPerSm) k_conv_h_mma(con
     // of loads and tensor-core instructions.
     auto consume = [&](auto ks_tag) {
     constexpr int KS = decltype(ks_tag)::value;
-    for (uint32_t c = 0; c < nchunks; ++c) {
-        const uint32_t slot = c % nstage;
-        wait_for(bar0 + 8 * slot, (c / nstage) & 1u);  // chunk c is the (c / nstage)-th filling of its slot
+    RingPlace at;
+    for (uint32_t c = 0; c < nchunks; ++c, at.next(nstage)) {
+        const uint32_t slot = at.slot;
+        wait_for(bar0 + 8 * slot, at.phase);
         int32_t acc_hi[2][4], acc_lo[2][4];
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { acc_hi[mt][i] = 0; acc_lo[mt][i] = half; }
         if (warp_active) {
             const uint32_t a_addr = a_base + slot * stage_bytes + a_lane;
             uint32_t a[2][2][4];  // [k step parity][row tile]
@@ -354,8 +369,8 @@ __global__ void __launch_bounds__(kHMmaThreads, kHMmaCtasPerSm) k_conv_h_mma(con
                 }
 #pragma unroll
                 for (int mt = 0; mt < 2; ++mt) {
-                    mma_u8s8(acc_hi[mt], a[ks & 1][mt], bfr[ks][0], bfr[ks][1]);
-                    mma_u8u8(acc_lo[mt], a[ks & 1][mt], bfr[ks][2], bfr[ks][3]);
+                    mma_u8s8(acc_hi[mt], a[ks & 1][mt], bfr[ks][0], bfr[ks][1], ks == 0);
+                    mma_u8u8(acc_lo[mt], a[ks & 1][mt], bfr[ks][2], bfr[ks][3], ks == 0);
                 }
             }
         }
@@ -370,8 +385,8 @@ __global__ void __launch_bounds__(kHMmaThreads, kHMmaCtasPerSm) k_conv_h_mma(con
             for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const int32_t v0 = (acc_hi[mt][2 * h] * 256 + acc_lo[mt][2 * h]) >> precision;
-                    const int32_t v1 = (acc_hi[mt][2 * h + 1] * 256 + acc_lo[mt][2 * h + 1]) >> precision;
+                    const int32_t v0 = (acc_hi[mt][2 * h] * 256 + (acc_lo[mt][2 * h] + half)) >> precision;
+                    const int32_t v1 = (acc_hi[mt][2 * h + 1] * 256 + (acc_lo[mt][2 * h + 1] + half)) >> precision;
                     uint32_t pk;
                     asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(pk) : "r"(v1), "r"(v0), "r"(0));
                     *reinterpret_cast<uint16_t*>(&ob[mt * 16 + g + 8 * h][warp * 8 + 2 * t4]) = (uint16_t)pk;
@@ -665,9 +680,10 @@ __global__ void __launch_bounds__(kVMmaThreads, kVMmaCtasPerSm) k_conv_v_mma(con
         if (lane != 0) return;
         const void* tmap = pg.tmap;
         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmap) : "memory");
-        for (uint32_t c = 0; c < nchunks && !gave_up; ++c) {
-            const uint32_t slot = c % nstage, use = c / nstage;
-            if (use > 0) wait_for(bar0 + 8 * (kVMmaMaxStages + slot), (use - 1) & 1u);
+        RingPlace at;
+        for (uint32_t c = 0; c < nchunks && !gave_up; ++c, at.next(nstage)) {
+            const uint32_t slot = at.slot;
+            if (c >= nstage) wait_for(bar0 + 8 * (kVMmaMaxStages + slot), at.phase ^ 1u);
             if (gave_up) break;
             mbar_expect_tx(bar0 + 8 * slot, stage_bytes);
             for (uint32_t bx = 0; bx < boxes; ++bx)
@@ -713,14 +729,15 @@ __global__ void __launch_bounds__(kVMmaThreads, kVMmaCtasPerSm) k_conv_v_mma(con
     constexpr uint32_t kOutPitch = kVMmaChunk + 16;
     auto consume = [&](auto ks_tag) {
     constexpr int KS = decltype(ks_tag)::value;
-    for (uint32_t c = 0; c < nchunks; ++c) {
-        const uint32_t slot = c % nstage;
-        wait_for(bar0 + 8 * slot, (c / nstage) & 1u);
+    RingPlace at;
+    for (uint32_t c = 0; c < nchunks; ++c, at.next(nstage)) {
+        const uint32_t slot = at.slot;
+        wait_for(bar0 + 8 * slot, at.phase);
         if (warp_active) {
             const uint32_t stage = a_base + slot * stage_bytes;
 #pragma unroll
             for (int mt = 0; mt < 4; ++mt) {
-                int32_t acc_hi[4] = {0, 0, 0, 0}, acc_lo[4] = {half, half, half, half};
+                int32_t acc_hi[4], acc_lo[4];
 #pragma unroll
                 for (int ks = 0; ks < KS; ++ks) {
                     // lane i names staged row band_lo + 32 ks + i; its 16-byte piece mt sits at piece mt ^ (row / 2 % 4)
@@ -734,13 +751,13 @@ __global__ void __launch_bounds__(kVMmaThreads, kVMmaCtasPerSm) k_conv_v_mma(con
                     a[1] = __byte_perm(r[0], r[1], 0x7531);  // column 2g + 1
                     a[2] = __byte_perm(r[2], r[3], 0x6420);
                     a[3] = __byte_perm(r[2], r[3], 0x7531);
-                    mma_u8s8(acc_hi, a, bfr[ks][0], bfr[ks][1]);
-                    mma_u8u8(acc_lo, a, bfr[ks][2], bfr[ks][3]);
+                    mma_u8s8(acc_hi, a, bfr[ks][0], bfr[ks][1], ks == 0);
+                    mma_u8u8(acc_lo, a, bfr[ks][2], bfr[ks][3], ks == 0);
                 }
                 // accumulators: (column 2g, row 2t), (column 2g, row 2t+1), (column 2g+1, row 2t), (column 2g+1, row 2t+1)
                 int32_t v[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) v[i] = (acc_hi[i] * 256 + acc_lo[i]) >> precision;
+                for (int i = 0; i < 4; ++i) v[i] = (acc_hi[i] * 256 + (acc_lo[i] + half)) >> precision;
                 uint32_t pk;
                 asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(pk) : "r"(v[2]), "r"(v[0]), "r"(0));
                 asm volatile("st.shared.u16 [%0], %1;" ::"r"(out_base + (2 * t4) * kOutPitch + 16 * mt + 2 * g), "h"((uint16_t)pk) : "memory");
