@@ -357,6 +357,7 @@ struct WavePlan {
     std::map<std::array<uint32_t, 2>, uint32_t> pair_ids;
     uint32_t cell_bits = kCellBits;              // of the wave's streams: bits per thread of the value decoder
     uint32_t guess_span = 1;                     // cells a thread of the synchronising decoder goes through
+    uint32_t write_cells = kDecodeThreads, restart_segs = kDecodeThreads;  // threads per CTA of the value decoders
     uint32_t max_pairs = 1;                      // most distinct ones in one image
     uint32_t pair_id(uint32_t dc, uint32_t ac) {
         const std::array<uint32_t, 2> key{dc, ac};
@@ -1048,7 +1049,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             if (!d.restart) guess_bits += (uint64_t)d.raw_len * 8 * d.bpm;
         wv.cell_bits = guess_bits / kShortCellBits > kGuessSpanThreads ? kCellBits : kShortCellBits;
         wv.guess_span = guess_bits / kCellBits > kGuessSpanThreads ? kGuessSpan : 1;
-        uint32_t color_total = 0, restart_total = 0, fchroma_total = 0, ftile_total = 0;
+        uint32_t color_total = 0, fchroma_total = 0, ftile_total = 0;
         size_t group_bytes = 0, fgroup_bytes = 0;
         wv.block_first.push_back(0);
         wv.color_first.push_back(0);
@@ -1056,7 +1057,6 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         wv.fchroma_first.push_back(0);
         wv.ftile_first.push_back(0);
         wv.fgroups.push_back({0, 0, 0, 0});
-        wv.restart_first.push_back(0);
         wv.tile_first.push_back(0);
         wv.fused_first = (uint32_t)built.size();
         for (size_t k : order) {
@@ -1072,8 +1072,6 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             it.wave_local = (int)wv.descs.size();
             if (d.restart) {
                 wv.restart_list.push_back((uint32_t)wv.descs.size());
-                restart_total += (d.nseg + kSegsPerCta - 1) / kSegsPerCta;
-                wv.restart_first.push_back(restart_total);
             } else {
                 wv.spec_list.push_back((uint32_t)wv.descs.size());
                 d.cell_off = cells;
@@ -1119,6 +1117,16 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         // longest streams first: one CTA links the cells of an image, and the launch ends with its slowest CTA
         std::stable_sort(wv.spec_list.begin(), wv.spec_list.end(),
                          [&](uint32_t a, uint32_t c) { return wv.descs[a].raw_len > wv.descs[c].raw_len; });
+        {
+            uint64_t all_cells = 0, all_segs = 0;
+            for (const JpegDesc& d : wv.descs)
+                if (d.restart) all_segs += d.nseg;
+                else all_cells += stream_cells(d.raw_len, wv.cell_bits);
+            wv.write_cells = decode_threads(all_cells);
+            wv.restart_segs = decode_threads(all_segs);
+        }
+        wv.restart_first.assign(1, 0);
+        for (uint32_t k : wv.restart_list) wv.restart_first.push_back(wv.restart_first.back() + (wv.descs[k].nseg + wv.restart_segs - 1) / wv.restart_segs);
         wv.guess_first.assign(1, 0);
         wv.write_first.assign(1, 0);
         wv.dc_first.assign(1, 0);
@@ -1126,7 +1134,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             const JpegDesc& d = wv.descs[k];
             const uint32_t guess_step = guess_spans(d.bpm, wv.guess_span) * wv.guess_span;
             wv.guess_first.push_back(wv.guess_first.back() + (stream_cells(d.raw_len, wv.cell_bits) + guess_step - 1) / guess_step);
-            wv.write_first.push_back(wv.write_first.back() + (stream_cells(d.raw_len, wv.cell_bits) + kCellsPerCta - 1) / kCellsPerCta);
+            wv.write_first.push_back(wv.write_first.back() + (stream_cells(d.raw_len, wv.cell_bits) + wv.write_cells - 1) / wv.write_cells);
             wv.dc_first.push_back(wv.dc_first.back() + (d.mcux * d.mcuy + kDcMcus - 1) / kDcMcus);
         }
         wv.us_bytes = us; wv.coef_blocks = blocks; wv.plane_bytes = planes; wv.decoded_bytes = decoded; wv.mid_bytes = mids; wv.nseg = segs; wv.cells = cells;
@@ -1483,6 +1491,8 @@ static int batch_run_locked(dg_batch* b) {
             w.restart_ctas = resolve(b, wv.m_restart);
             w.cell_bits = wv.cell_bits;
             w.guess_span = wv.guess_span;
+            w.write_cells = wv.write_cells;
+            w.restart_segs = wv.restart_segs;
             w.guess_ctas = resolve(b, wv.m_guess);
             w.write_ctas = resolve(b, wv.m_write);
             w.dc_ctas = resolve(b, wv.m_dc);

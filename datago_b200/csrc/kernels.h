@@ -20,7 +20,11 @@ constexpr uint32_t kSms = 148;  // of a B200
 constexpr uint32_t kUnstuffTile = 4096;  // bytes of an entropy-coded segment per CTA of the unstuffing kernels
 // bits of an unstuffed stream per thread of the value decoder; the short form while all threads are resident at once
 constexpr int kCellBits = 1024, kShortCellBits = 512;
-constexpr uint32_t kCellsPerCta = 128, kSegsPerCta = 128;
+// threads per CTA of the value decoders, one per cell or restart segment: the second form once there is more than the chip holds
+// of the first at a time.  Shared memory bounds the warps of an SM (128 bytes of block buffer and up to 128 of stream per
+// thread, 18 KB of tables per CTA): four CTAs of 128 threads, or three of 224.
+constexpr uint32_t kDecodeThreads = 128, kDecodeThreadsMany = 224;
+inline uint32_t decode_threads(uint64_t threads) { return threads > kSms * 4ull * kDecodeThreads ? kDecodeThreadsMany : kDecodeThreads; }
 // synchronising decoder: threads per CTA, the entries of the candidate array per cell, and the cells of a span once a thread
 // per cell and block of the MCU would be more than the chip holds at once
 constexpr uint32_t kGuessLanes = 384, kCandidates = 6, kGuessSpan = 4;
@@ -78,8 +82,9 @@ struct JpegWave {
     const uint32_t* spec_list; uint32_t n_spec;
     OwnerMap guess_ctas, write_ctas, dc_ctas;
     uint32_t cell_bits;      // kCellBits or kShortCellBits
+    uint32_t write_cells, restart_segs;  // cells / segments per CTA of the value decoders: kDecodeThreads or kDecodeThreadsMany
     uint32_t guess_span;     // cells a thread of the synchronising decoder goes through
-    // restart-interval images: kSegsPerCta segments per CTA, owner = index into restart_list
+    // restart-interval images: restart_segs segments per CTA, owner = index into restart_list
     OwnerMap restart_ctas;
     const uint32_t* restart_list;
     OwnerMap blocks;         // owner = image

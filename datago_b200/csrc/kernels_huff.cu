@@ -494,7 +494,7 @@ struct Staged {
     }
 };
 static_assert(kStreamPad >= (2048 + 1024) / 8 + 16, "rows behind the end of a stream are copied");
-static_assert((1ull << 32) - kMaxStream * 8ull > 2ull * kCellsPerCta * kCellBits + 4096, "positions behind the end of a stream do not wrap");
+static_assert((1ull << 32) - kMaxStream * 8ull > 2ull * kDecodeThreadsMany * kCellBits + 4096, "positions behind the end of a stream do not wrap");
 
 // A state at or behind the first bit of a cell, relative to it: bits 0-11 distance of the block start (less than 2048: a
 // block has 64 symbols of 31 bits at most), 12-14 its block c.
@@ -863,25 +863,24 @@ __device__ __forceinline__ uint32_t decode_blocks(const Source& src, const uint3
 }  // namespace
 
 // ---- restart-free images: one thread per cell -----------------------------------------------------------------------
-constexpr int kWriteThreads = (int)kCellsPerCta;
-// The CTA's cells are consecutive: their stream is staged in shared memory.
-template <int CELL>
-__global__ void __launch_bounds__(kWriteThreads) k_huff_write(JpegWave w) {
+// The CTA's T cells are consecutive: their stream is staged in shared memory.
+template <int T, int CELL>
+__global__ void __launch_bounds__(T) k_huff_write(JpegWave w) {
     extern __shared__ __align__(16) unsigned char write_smem[];
-    ValueMisc<kWriteThreads>& sh = *reinterpret_cast<ValueMisc<kWriteThreads>*>(write_smem);
-    unsigned char* const stage = write_smem + sizeof(ValueMisc<kWriteThreads>);
-    unsigned char* const tab0 = stage + (kWriteThreads + Staged<CELL>::kRowsBehind) * Staged<CELL>::kPitch;
+    ValueMisc<T>& sh = *reinterpret_cast<ValueMisc<T>*>(write_smem);
+    unsigned char* const stage = write_smem + sizeof(ValueMisc<T>);
+    unsigned char* const tab0 = stage + (T + Staged<CELL>::kRowsBehind) * Staged<CELL>::kPitch;
     const uint32_t o = owner_of(w.write_ctas, blockIdx.x);
     const uint32_t img = w.spec_list[o];
     const JpegDesc& d = w.descs[img];
-    const uint32_t cell0 = (blockIdx.x - __ldg(w.write_ctas.first + o)) * kCellsPerCta;
+    const uint32_t cell0 = (blockIdx.x - __ldg(w.write_ctas.first + o)) * T;
     const uint32_t total = w.us_len[img] * 8u;
     const uint32_t ncell = (total + CELL - 1) / CELL;
     if (cell0 >= ncell) return;
     const int tid = threadIdx.x;
     // (no further than the stream and its padding reach)
-    Staged<CELL>::copy(stage, w.us + d.us_off, cell0, (int)min((uint32_t)(kWriteThreads + Staged<CELL>::kRowsBehind), ncell - cell0 + Staged<CELL>::kRowsPadded), tid, kWriteThreads);
-    value_setup<kWriteThreads>(w, d, sh, tab0);
+    Staged<CELL>::copy(stage, w.us + d.us_off, cell0, (int)min((uint32_t)(T + Staged<CELL>::kRowsBehind), ncell - cell0 + Staged<CELL>::kRowsPadded), tid, T);
+    value_setup<T>(w, d, sh, tab0);
     const uint32_t k = cell0 + tid;
     const uint2* recs = w.cells + d.cell_off;
     uint2 a = make_uint2(0, 0);
@@ -895,7 +894,7 @@ __global__ void __launch_bounds__(kWriteThreads) k_huff_write(JpegWave w) {
     uint32_t err = 0;
     const SharedSource source{smem_addr(stage) - cell0 * (uint32_t)Staged<CELL>::kPitch};
     const uint32_t p0 = a.y < b1 ? a.x : cell0 * CELL;
-    decode_blocks<kWriteThreads, false>(source, p0, a.y, b1, total, (cell0 + kCellsPerCta) * CELL, a.y % d.bpm, d, sh, w.huff,
+    decode_blocks<T, false>(source, p0, a.y, b1, total, (cell0 + T) * CELL, a.y % d.bpm, d, sh, w.huff,
                                         w.coef + d.block_off * 64, w.diff + d.block_off, err);
     if (err) atomicOr(w.status + d.item, err);
 }
@@ -903,18 +902,18 @@ __global__ void __launch_bounds__(kWriteThreads) k_huff_write(JpegWave w) {
 // ---- restart-interval images: one thread per segment -----------------------------------------------------------------
 // A segment's first MCU and the zero DC predictors are known, so one pass does it.  The segments of a CTA are consecutive
 // in one image; the stream under them is staged when it fits (it does for intervals of a few MCUs), else read in place.
-constexpr int kRestartThreads = (int)kSegsPerCta;
-constexpr uint32_t kRestartStage = 16384;
+template <int T> constexpr uint32_t kRestartStage = T * 128;
 
-__global__ void __launch_bounds__(kRestartThreads) k_huff_restart(JpegWave w) {
+template <int T>
+__global__ void __launch_bounds__(T) k_huff_restart(JpegWave w) {
     extern __shared__ __align__(16) unsigned char restart_smem[];
-    ValueMisc<kRestartThreads>& sh = *reinterpret_cast<ValueMisc<kRestartThreads>*>(restart_smem);
-    unsigned char* const stage = restart_smem + sizeof(ValueMisc<kRestartThreads>);
-    unsigned char* const tab0 = stage + kRestartStage;
+    ValueMisc<T>& sh = *reinterpret_cast<ValueMisc<T>*>(restart_smem);
+    unsigned char* const stage = restart_smem + sizeof(ValueMisc<T>);
+    unsigned char* const tab0 = stage + kRestartStage<T>;
     const uint32_t o = owner_of(w.restart_ctas, blockIdx.x);
     const uint32_t img = w.restart_list[o];
     const JpegDesc& d = w.descs[img];
-    const uint32_t k0 = (blockIdx.x - __ldg(w.restart_ctas.first + o)) * kSegsPerCta;
+    const uint32_t k0 = (blockIdx.x - __ldg(w.restart_ctas.first + o)) * T;
     const int tid = threadIdx.x;
     const uint32_t found = w.seg_found[img], us_len = w.us_len[img], k = k0 + tid;
     if (k0 == 0 && tid == 0 && found != d.nseg) atomicOr(w.status + d.item, kStBadMarker);
@@ -930,15 +929,15 @@ __global__ void __launch_bounds__(kRestartThreads) k_huff_restart(JpegWave w) {
     // the CTA's piece of the stream: from the 16-byte piece its first segment starts in to its end plus what a block that
     // is not whole may run over
     const auto begin = [&](uint32_t i) { return i < have ? min(seg[i], us_len) : us_len; };  // of a segment (us_len: see kMaxStream)
-    const uint32_t lo = begin(k0) & ~15u, hi = begin(k0 + kSegsPerCta) + 272u;
-    const bool staged = hi - lo <= kRestartStage;
+    const uint32_t lo = begin(k0) & ~15u, hi = begin(k0 + T) + 272u;
+    const bool staged = hi - lo <= kRestartStage<T>;
     const uint8_t* us = w.us + d.us_off;
     if (staged) {
         const uint32_t dst = smem_addr(stage);
-        for (uint32_t i = tid; i * 16 < hi - lo; i += kRestartThreads) copy16(dst + i * 16, us + lo + (size_t)i * 16);
+        for (uint32_t i = tid; i * 16 < hi - lo; i += T) copy16(dst + i * 16, us + lo + (size_t)i * 16);
         copy_commit();
     }
-    value_setup<kRestartThreads>(w, d, sh, tab0);
+    value_setup<T>(w, d, sh, tab0);
     copy_wait<0>();
     __syncthreads();
     const bool mine = k < have;
@@ -947,10 +946,10 @@ __global__ void __launch_bounds__(kRestartThreads) k_huff_restart(JpegWave w) {
     int16_t* coef = w.coef + d.block_off * 64;
     uint32_t err = 0, n;
     if (staged) {
-        n = decode_blocks<kRestartThreads, true>(SharedSource{smem_addr(stage) - lo}, b0 * 8u, blk0, end, b1 * 8u, b1 * 8u, 0u, d, sh, w.huff, coef, info, err);
+        n = decode_blocks<T, true>(SharedSource{smem_addr(stage) - lo}, b0 * 8u, blk0, end, b1 * 8u, b1 * 8u, 0u, d, sh, w.huff, coef, info, err);
     } else {
         const GlobalSource source{reinterpret_cast<const uint32_t*>(us), (us_len + 3) / 4 + 2};
-        n = decode_blocks<kRestartThreads, true>(source, b0 * 8u, blk0, end, b1 * 8u, b1 * 8u, 0u, d, sh, w.huff, coef, info, err);
+        n = decode_blocks<T, true>(source, b0 * 8u, blk0, end, b1 * 8u, b1 * 8u, 0u, d, sh, w.huff, coef, info, err);
     }
     if (n < end - blk0) err |= kStTruncated;
     if (n < blk1 - blk0) blank(blk0 + n);
@@ -1092,6 +1091,14 @@ namespace {
 
 template <class K>
 void allow_smem(K kernel, size_t bytes) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); }
+template <int CELL>
+void allow_cells(size_t most) {
+    allow_smem(k_huff_guess<CELL>, most - 4096);  // (it has static arrays as well)
+    allow_smem(k_huff_chain<256, CELL>, most);
+    allow_smem(k_huff_chain<1024, CELL>, most);
+    allow_smem(k_huff_write<kDecodeThreads, CELL>, most);
+    allow_smem(k_huff_write<kDecodeThreadsMany, CELL>, most);
+}
 
 // Dynamic shared memory beyond the default limit has to be allowed once per device and kernel.
 void configure_once() {
@@ -1101,15 +1108,10 @@ void configure_once() {
     if (dev < 0 || dev >= 64) dev = 0;
     std::call_once(done[dev], [] {
         const size_t most = 227 * 1024 - 1024;
-        allow_smem(k_huff_guess<kCellBits>, most - 4096);  // (it has static arrays as well)
-        allow_smem(k_huff_guess<kShortCellBits>, most - 4096);
-        allow_smem(k_huff_chain<256, kCellBits>, most);
-        allow_smem(k_huff_chain<1024, kCellBits>, most);
-        allow_smem(k_huff_chain<256, kShortCellBits>, most);
-        allow_smem(k_huff_chain<1024, kShortCellBits>, most);
-        allow_smem(k_huff_write<kCellBits>, most);
-        allow_smem(k_huff_write<kShortCellBits>, most);
-        allow_smem(k_huff_restart, most);
+        allow_cells<kCellBits>(most);
+        allow_cells<kShortCellBits>(most);
+        allow_smem(k_huff_restart<kDecodeThreads>, most);
+        allow_smem(k_huff_restart<kDecodeThreadsMany>, most);
     });
 }
 
@@ -1132,10 +1134,20 @@ void launch_chain(const JpegWave& w, cudaStream_t s) {
     else k_huff_chain<1024, CELL><<<w.n_spec, 1024, sizeof(ChainMisc<1024>) + tables, s>>>(w);
 }
 
+template <int T, int CELL>
+void launch_write(const JpegWave& w, cudaStream_t s) {
+    const size_t smem = sizeof(ValueMisc<T>) + (size_t)(T + Staged<CELL>::kRowsBehind) * Staged<CELL>::kPitch + w.max_pairs * 2 * sizeof(ValueTab);
+    k_huff_write<T, CELL><<<w.write_ctas.total, T, smem, s>>>(w);
+}
 template <int CELL>
 void launch_write(const JpegWave& w, cudaStream_t s) {
-    const size_t smem = sizeof(ValueMisc<kWriteThreads>) + (size_t)(kWriteThreads + Staged<CELL>::kRowsBehind) * Staged<CELL>::kPitch + w.max_pairs * 2 * sizeof(ValueTab);
-    k_huff_write<CELL><<<w.write_ctas.total, kWriteThreads, smem, s>>>(w);
+    if (w.write_cells == kDecodeThreads) launch_write<kDecodeThreads, CELL>(w, s);
+    else launch_write<kDecodeThreadsMany, CELL>(w, s);
+}
+
+template <int T>
+void launch_restart(const JpegWave& w, cudaStream_t s) {
+    k_huff_restart<T><<<w.restart_ctas.total, T, sizeof(ValueMisc<T>) + kRestartStage<T> + w.max_pairs * 2 * sizeof(ValueTab), s>>>(w);
 }
 
 }  // namespace
@@ -1167,8 +1179,8 @@ void launch_huff_write(const JpegWave& w, cudaStream_t s) {
 void launch_huff_restart(const JpegWave& w, cudaStream_t s) {
     if (!w.restart_ctas.total) return;
     configure_once();
-    const size_t smem = sizeof(ValueMisc<kRestartThreads>) + kRestartStage + w.max_pairs * 2 * sizeof(ValueTab);
-    k_huff_restart<<<w.restart_ctas.total, kRestartThreads, smem, s>>>(w);
+    if (w.restart_segs == kDecodeThreads) launch_restart<kDecodeThreads>(w, s);
+    else launch_restart<kDecodeThreadsMany>(w, s);
 }
 
 void launch_whole_blocks(const JpegWave& w, uint32_t nblocks, cudaStream_t s) {

@@ -82,6 +82,20 @@ def test_entropy_cells_and_spans(copies):
             assert_same(out, want[i % len(distinct)], str(i))
 
 
+@pytest.mark.parametrize("copies", [1, 30])
+def test_restart_segments_per_cta(copies):
+    # 3 106 segments of one MCU, or 93 180: CTAs of 128 threads, or of 224
+    rng = np.random.default_rng(322)
+    distinct = [jpeg(rng, w, h, q=92, rst=1) for w, h in [(640, 480), (1201, 400), (17, 33)]]
+    want = [oracle.jpeg_decode(d) for d in distinct]
+    with ctx().batch(distinct * copies) as b:
+        b.upload(); b.run()
+        outs = b.download(); b.sync()
+        for i, out in enumerate(outs):
+            assert b.result(i).status == 0, i
+            assert_same(out, want[i % len(distinct)], str(i))
+
+
 def test_decoder_counters():
     # cells of 512 bits with this little work: each is decoded by one candidate at least, by one per block of the MCU at most,
     # and once for the values; where no candidate was right once more or oftener
