@@ -352,7 +352,7 @@ struct ItemPlan {
 struct WavePlan {
     int first_item = 0, last_item = 0;  // [first, last)
     std::vector<JpegDesc> descs;
-    std::vector<uint32_t> tile_first, spec_list, guess_first, write_first, dc_first, restart_list, restart_first, block_first, color_first;
+    std::vector<uint32_t> tile_first, spec_list, guess_first, write_first, restart_list, restart_first, block_first, color_first;
     std::vector<std::array<uint32_t, 2>> pairs;  // (DC, AC) pairs of Huffman tables in use
     std::map<std::array<uint32_t, 2>, uint32_t> pair_ids;
     uint32_t cell_bits = kCellBits;              // of the wave's streams: bits per thread of the value decoder
@@ -387,7 +387,7 @@ struct WavePlan {
     size_t off_us = 0, off_uslen = 0, off_segstart = 0, off_segfound = 0, off_tiles = 0, off_codes = 0, off_cells = 0, off_cand = 0, off_diff = 0, off_info = 0, off_coef = 0, off_planes = 0, off_decoded = 0, off_mid = 0, total = 0;
     // meta offsets
     size_t m_descs = 0, m_pairs = 0, m_spec = 0, m_restart_list = 0, m_passes[4] = {0, 0, 0, 0}, m_copies = 0, m_torgbs = 0, m_alphas[4] = {0, 0, 0, 0};
-    OwnerMapOff m_tiles, m_guess, m_write, m_dc, m_restart, m_blocks, m_color, m_fchroma, m_ftile, m_pass[4], m_copy, m_torgb, m_alpha[4];
+    OwnerMapOff m_tiles, m_guess, m_write, m_restart, m_blocks, m_color, m_fchroma, m_ftile, m_pass[4], m_copy, m_torgb, m_alpha[4];
 };
 
 struct StageEvent { int stage; cudaEvent_t a, b; };
@@ -1129,13 +1129,11 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         for (uint32_t k : wv.restart_list) wv.restart_first.push_back(wv.restart_first.back() + (wv.descs[k].nseg + wv.restart_segs - 1) / wv.restart_segs);
         wv.guess_first.assign(1, 0);
         wv.write_first.assign(1, 0);
-        wv.dc_first.assign(1, 0);
         for (uint32_t k : wv.spec_list) {
             const JpegDesc& d = wv.descs[k];
             const uint32_t guess_step = guess_spans(d.bpm, wv.guess_span) * wv.guess_span;
             wv.guess_first.push_back(wv.guess_first.back() + (stream_cells(d.raw_len, wv.cell_bits) + guess_step - 1) / guess_step);
             wv.write_first.push_back(wv.write_first.back() + (stream_cells(d.raw_len, wv.cell_bits) + wv.write_cells - 1) / wv.write_cells);
-            wv.dc_first.push_back(wv.dc_first.back() + (d.mcux * d.mcuy + kDcMcus - 1) / kDcMcus);
         }
         wv.us_bytes = us; wv.coef_blocks = blocks; wv.plane_bytes = planes; wv.decoded_bytes = decoded; wv.mid_bytes = mids; wv.nseg = segs; wv.cells = cells;
         size_t o = 0;
@@ -1287,7 +1285,6 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             wv.m_tiles = put_owner_map(m, wv.tile_first);
             wv.m_guess = put_owner_map(m, wv.guess_first);
             wv.m_write = put_owner_map(m, wv.write_first);
-            wv.m_dc = put_owner_map(m, wv.dc_first);
             wv.m_restart = put_owner_map(m, wv.restart_first);
             wv.m_blocks = put_owner_map(m, wv.block_first);
             wv.m_color = put_owner_map(m, wv.color_first);
@@ -1495,7 +1492,6 @@ static int batch_run_locked(dg_batch* b) {
             w.restart_segs = wv.restart_segs;
             w.guess_ctas = resolve(b, wv.m_guess);
             w.write_ctas = resolve(b, wv.m_write);
-            w.dc_ctas = resolve(b, wv.m_dc);
             w.blocks = resolve(b, wv.m_blocks);
             w.color_tiles = resolve(b, wv.m_color);
             w.fused_first = wv.fused_first;

@@ -37,7 +37,6 @@ inline uint32_t guess_spans(uint32_t bpm, uint32_t span) {
     const uint32_t lanes = kGuessLanes / bpm, stage = span == 1 ? 128u : 256u / span;
     return lanes < stage ? lanes : stage;
 }
-constexpr uint32_t kDcMcus = 8192;       // MCUs per CTA of the DC prediction
 constexpr uint32_t kCodeTablesBytes = 20544;  // look-up tables of one (DC, AC) pair of Huffman tables
 // Bit positions are 32-bit numbers.  A stream counts up to this length, which leaves room for what the decoders add to a
 // position at its end (the cells of a CTA, a block); what lies behind is as good as cut off.
@@ -77,10 +76,10 @@ struct JpegWave {
     uint8_t* codes;          // [n_pairs] look-up tables made from them, kCodeTablesBytes each
     uint32_t max_pairs;      // most distinct pairs one image of the wave uses
     const uint32_t* qt32;    // quantisation pool, 32 words per table: word i holds q[2i] in byte 0 and q[2i+1] in byte 3
-    // restart-free images of this wave, longest first; CTAs of the synchronising decoder, the value decoder and the DC
-    // prediction: owner = index into spec_list
+    // restart-free images of this wave, longest first; CTAs of the synchronising decoder and the value decoder: owner =
+    // index into spec_list
     const uint32_t* spec_list; uint32_t n_spec;
-    OwnerMap guess_ctas, write_ctas, dc_ctas;
+    OwnerMap guess_ctas, write_ctas;
     uint32_t cell_bits;      // kCellBits or kShortCellBits
     uint32_t write_cells, restart_segs;  // cells / segments per CTA of the value decoders: kDecodeThreads or kDecodeThreadsMany
     uint32_t guess_span;     // cells a thread of the synchronising decoder goes through

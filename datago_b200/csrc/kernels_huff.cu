@@ -13,6 +13,8 @@
 #include <cstdint>
 #include <mutex>
 
+#include <cooperative_groups.h>
+
 #include "kernels.h"
 
 namespace dg {
@@ -960,8 +962,11 @@ __global__ void __launch_bounds__(T) k_huff_restart(JpegWave w) {
 // K1b  DC prediction of restart-free images: diff[] holds what info[] will hold, with DC differences, in scan order; the
 //      predictor runs over the blocks of a component.  Kept out of the bit-serial kernels on purpose: there it would cost every symbol of the
 //      synchronising pass a value extraction, here it is a prefix sum over four bytes per block.
-//      One CTA per kDcMcus MCUs of an image; it adds up what lies before its range itself (L2 reads; a 50-megapixel
-//      image has 24 ranges in 4:2:0, 96 in 4:4:4 or gray), so that no CTA waits on another.
+//      A cluster of CTAs per image, each with an equal run of its MCUs: a CTA adds up its run, the cluster exchanges the
+//      sums, and the CTA writes its run -- from registers where a thread has no more than four MCUs.  What bounds it is the
+//      latency of its few dependent loads, so the blocks are fetched before it is known how many the stream holds.  (One CTA
+//      per 8192 MCUs, which read again what lay before its range: 16 us for one photo, 43 for 8 images of 4:4:4 up to 4096
+//      pixels.)
 // ---------------------------------------------------------------------------------------------------------------
 namespace {
 
@@ -969,11 +974,11 @@ constexpr int kDcThreads = 512;
 struct Dc3 { int32_t a, b, c; };
 __device__ __forceinline__ Dc3 operator+(Dc3 x, Dc3 y) { return {x.a + y.a, x.b + y.b, x.c + y.c}; }
 
-// four MCUs per thread: BPM 16-byte pieces.  have: blocks that the stream holds.
+// four MCUs per thread: BPM 16-byte pieces
 template <int BPM>
-__device__ __forceinline__ Dc3 load_mcus(const uint32_t* diff, uint32_t m4, uint32_t have, uint32_t (&v)[4 * BPM]) {
+__device__ __forceinline__ void load_mcus(const uint32_t* diff, uint32_t m4, uint32_t nblocks, uint32_t (&v)[4 * BPM]) {
     const uint32_t b0 = m4 * 4 * BPM;
-    if (b0 + 4 * BPM <= have) {
+    if (b0 + 4 * BPM <= nblocks) {
 #pragma unroll
         for (int i = 0; i < BPM; ++i) {
             const uint4 q = reinterpret_cast<const uint4*>(diff + b0)[i];
@@ -981,7 +986,16 @@ __device__ __forceinline__ Dc3 load_mcus(const uint32_t* diff, uint32_t m4, uint
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < 4 * BPM; ++i) v[i] = b0 + i < have ? diff[b0 + i] : 0u;
+        for (int i = 0; i < 4 * BPM; ++i) v[i] = b0 + i < nblocks ? diff[b0 + i] : 0u;
+    }
+}
+// their differences; blocks from `have` on, which the stream does not hold, count as nothing
+template <int BPM>
+__device__ __forceinline__ Dc3 sum_mcus(uint32_t m4, uint32_t have, uint32_t (&v)[4 * BPM]) {
+    const uint32_t b0 = m4 * 4 * BPM;
+    if (b0 + 4 * BPM > have) {
+#pragma unroll
+        for (int i = 0; i < 4 * BPM; ++i) if (b0 + i >= have) v[i] = 0;
     }
     Dc3 s{0, 0, 0};
 #pragma unroll
@@ -995,33 +1009,54 @@ __device__ __forceinline__ Dc3 load_mcus(const uint32_t* diff, uint32_t m4, uint
     return s;
 }
 
-template <int BPM>
-__device__ void dc_range(const uint32_t* diff, uint32_t* info, uint32_t range, uint32_t nblocks, uint32_t have, Dc3* s_warp) {
+struct DcSmem { Dc3 warp[kDcThreads / 32], total, carry; };
+
+// blocks: how many of the image's blocks the stream holds (called once the first loads are under way)
+template <int BPM, class Blocks>
+__device__ void dc_image(const uint32_t* diff, uint32_t* info, uint32_t nblocks, Blocks&& blocks, DcSmem& sh) {
+    const auto cluster = cooperative_groups::this_cluster();
+    const uint32_t rank = cluster.block_rank(), size = cluster.num_blocks();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr uint32_t kStep = kDcThreads;  // groups of four MCUs per turn
-    const uint32_t groups = (nblocks + 4 * BPM - 1) / (4 * BPM);
-    const uint32_t g0 = range * (kDcMcus / 4), g1 = min(g0 + kDcMcus / 4, groups);
+    const uint32_t groups = (nblocks + 4 * BPM - 1) / (4 * BPM), run = (groups + size - 1) / size;  // of four MCUs
+    const uint32_t g0 = min(rank * run, groups), g1 = min(g0 + run, groups);
+    const bool once = run <= (uint32_t)kDcThreads;  // the run stays in registers
     uint32_t v[4 * BPM];
-    Dc3 before{0, 0, 0};
-    for (uint32_t g = tid; g < g0; g += kStep) before = before + load_mcus<BPM>(diff, g, have, v);
-    auto total = [&](Dc3 x) -> Dc3 {  // sum over the CTA, in every thread
+    if (g0 + tid < g1) load_mcus<BPM>(diff, g0 + tid, nblocks, v);
+    const uint32_t have = blocks();
+    Dc3 x{0, 0, 0};
+    if (g0 + tid < g1) x = sum_mcus<BPM>(g0 + tid, have, v);
+    const Dc3 first = x;
+    for (uint32_t g = g0 + tid + kDcThreads; g < g1; g += kDcThreads) {
+        load_mcus<BPM>(diff, g, nblocks, v);
+        x = x + sum_mcus<BPM>(g, have, v);
+    }
 #pragma unroll
-        for (int o = 16; o; o >>= 1) { x.a += __shfl_xor_sync(0xFFFFFFFFu, x.a, o); x.b += __shfl_xor_sync(0xFFFFFFFFu, x.b, o); x.c += __shfl_xor_sync(0xFFFFFFFFu, x.c, o); }
-        __syncthreads();
-        if (lane == 0) s_warp[warp] = x;
-        __syncthreads();
+    for (int o = 16; o; o >>= 1) { x.a += __shfl_xor_sync(0xFFFFFFFFu, x.a, o); x.b += __shfl_xor_sync(0xFFFFFFFFu, x.b, o); x.c += __shfl_xor_sync(0xFFFFFFFFu, x.c, o); }
+    if (lane == 0) sh.warp[warp] = x;
+    __syncthreads();
+    if (tid == 0) {
         Dc3 t{0, 0, 0};
 #pragma unroll
-        for (int i = 0; i < kDcThreads / 32; ++i) t = t + s_warp[i];
-        return t;
-    };
-    Dc3 carry{0, 0, 0};
-    if (g0) carry = total(before);
+        for (int i = 0; i < kDcThreads / 32; ++i) t = t + sh.warp[i];
+        sh.total = t;
+    }
+    cluster.sync();
+    if (warp == 0) {  // what the CTAs before this one add up to
+        Dc3 t{0, 0, 0};
+        if ((uint32_t)lane < rank) t = *cluster.map_shared_rank(&sh.total, lane);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) { t.a += __shfl_xor_sync(0xFFFFFFFFu, t.a, o); t.b += __shfl_xor_sync(0xFFFFFFFFu, t.b, o); t.c += __shfl_xor_sync(0xFFFFFFFFu, t.c, o); }
+        if (lane == 0) sh.carry = t;
+    }
+    cluster.barrier_arrive();  // this CTA has read the others' sums
+    __syncthreads();
+    Dc3 carry = sh.carry;
     // (info keeps 16 bits, so nothing is lost when a damaged stream makes the sums wrap)
-    for (uint32_t g = g0; g < g1; g += kStep) {
+    for (uint32_t g = g0; g < g1; g += kDcThreads) {
         const uint32_t m4 = g + tid;
         Dc3 mine{0, 0, 0};
-        if (m4 < g1) mine = load_mcus<BPM>(diff, m4, have, v);
+        if (once) mine = first;
+        else if (m4 < g1) { load_mcus<BPM>(diff, m4, nblocks, v); mine = sum_mcus<BPM>(m4, have, v); }
         Dc3 inc = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1029,11 +1064,11 @@ __device__ void dc_range(const uint32_t* diff, uint32_t* info, uint32_t range, u
             if (lane >= o) { inc.a += ta; inc.b += tb; inc.c += tc; }
         }
         __syncthreads();
-        if (lane == 31) s_warp[warp] = inc;
+        if (lane == 31) sh.warp[warp] = inc;
         __syncthreads();
         Dc3 pre{0, 0, 0}, all{0, 0, 0};
 #pragma unroll
-        for (int i = 0; i < kDcThreads / 32; ++i) { const Dc3 t = s_warp[i]; if (i < warp) pre = pre + t; all = all + t; }
+        for (int i = 0; i < kDcThreads / 32; ++i) { const Dc3 t = sh.warp[i]; if (i < warp) pre = pre + t; all = all + t; }
         int32_t a = carry.a + pre.a + inc.a - mine.a, b = carry.b + pre.b + inc.b - mine.b, c = carry.c + pre.c + inc.c - mine.c;
         carry = carry + all;
         if (m4 >= g1) continue;
@@ -1055,23 +1090,24 @@ __device__ void dc_range(const uint32_t* diff, uint32_t* info, uint32_t range, u
             for (int i = 0; i < 4 * BPM; ++i) if (b0 + i < nblocks) info[b0 + i] = b0 + i < have ? v[i] : kBlankBlock;
         }
     }
+    cluster.barrier_wait();  // the sums stay until every CTA has read them
 }
 
 }  // namespace
 
 __global__ void __launch_bounds__(kDcThreads) k_dc(JpegWave w) {
-    __shared__ Dc3 s_warp[kDcThreads / 32];
-    const uint32_t o = owner_of(w.dc_ctas, blockIdx.x);
-    const JpegDesc& d = w.descs[w.spec_list[o]];
-    const uint32_t range = blockIdx.x - __ldg(w.dc_ctas.first + o);
+    __shared__ DcSmem sh;
+    const uint32_t img = w.spec_list[blockIdx.x / cooperative_groups::this_cluster().num_blocks()];
+    const JpegDesc& d = w.descs[img];
+    const uint32_t us_len = w.us_len[img], nblocks = d.nblocks;
     const uint32_t* diff = w.diff + d.block_off;
     uint32_t* info = w.info + d.block_off;
-    const uint32_t ncell = (w.us_len[w.spec_list[o]] * 8u + w.cell_bits - 1) / w.cell_bits, have = min(w.cells[d.cell_off + ncell].y, d.nblocks);
+    const auto blocks = [&] { return min(w.cells[d.cell_off + (us_len * 8u + w.cell_bits - 1) / w.cell_bits].y, nblocks); };
     switch (d.bpm) {
-        case 1: dc_range<1>(diff, info, range, d.nblocks, have, s_warp); break;
-        case 3: dc_range<3>(diff, info, range, d.nblocks, have, s_warp); break;
-        case 4: dc_range<4>(diff, info, range, d.nblocks, have, s_warp); break;
-        default: dc_range<6>(diff, info, range, d.nblocks, have, s_warp); break;
+        case 1: dc_image<1>(diff, info, nblocks, blocks, sh); break;
+        case 3: dc_image<3>(diff, info, nblocks, blocks, sh); break;
+        case 4: dc_image<4>(diff, info, nblocks, blocks, sh); break;
+        default: dc_image<6>(diff, info, nblocks, blocks, sh); break;
     }
 }
 
@@ -1150,6 +1186,19 @@ void launch_restart(const JpegWave& w, cudaStream_t s) {
     k_huff_restart<T><<<w.restart_ctas.total, T, sizeof(ValueMisc<T>) + kRestartStage<T> + w.max_pairs * 2 * sizeof(ValueTab), s>>>(w);
 }
 
+// CTAs per image: eight while they all run at once; with many images that only adds CTAs (1024 files: passes of 3170 us with two to four,
+// see the commit for one).
+void launch_dc(const JpegWave& w, cudaStream_t s) {
+    const uint32_t size = w.n_spec <= kSms / 4 ? 8 : w.n_spec <= kSms ? 2 : 1;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = size; cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cudaLaunchConfig_t at{};
+    at.gridDim = dim3(w.n_spec * size); at.blockDim = dim3(kDcThreads); at.stream = s;
+    at.attrs = &cluster; at.numAttrs = 1;
+    cudaLaunchKernelEx(&at, k_dc, w);
+}
+
 }  // namespace
 
 void launch_huff_guess(const JpegWave& w, cudaStream_t s) {
@@ -1173,7 +1222,7 @@ void launch_huff_write(const JpegWave& w, cudaStream_t s) {
         if (w.cell_bits == (uint32_t)kCellBits) launch_write<kCellBits>(w, s);
         else launch_write<kShortCellBits>(w, s);
     }
-    k_dc<<<w.dc_ctas.total, kDcThreads, 0, s>>>(w);
+    launch_dc(w, s);
 }
 
 void launch_huff_restart(const JpegWave& w, cudaStream_t s) {
