@@ -402,81 +402,93 @@ __device__ __forceinline__ void load_tables(const JpegWave& w, const JpegDesc& d
     }
 }
 
-// Streams in shared memory: a lane's window is two words (w0 holds its current bit), `cur` the address of the first.  base: the
-// address bit 0 of the stream would have.  step: w0 takes w1 and w1 the word behind it where `crossed` is not zero; predicated
-// by hand, because some lane of a warp crosses in nearly every step.
+// Streams in shared memory: a lane's window is two words (w0 holds its current bit) and the one behind them, which is on its way
+// while they are used; `at` is the address of the first.  base: the address bit 0 of the stream would have.  step: the window
+// moves on by a word where `crossed` is not zero; predicated by hand, because some lane of a warp crosses in nearly every step.
 struct SharedSource {
+    struct Cursor { uint32_t at, w2; };
     uint32_t base;
-    __device__ __forceinline__ uint32_t start(uint32_t& w0, uint32_t& w1, uint32_t p) const {
-        const uint32_t cur = base + ((p >> 3) & ~3u);
-        w0 = lds32(cur); w1 = lds32(cur + 4);
-        return cur;
+    __device__ __forceinline__ Cursor start(uint32_t& w0, uint32_t& w1, uint32_t p) const {
+        const uint32_t at = base + ((p >> 3) & ~3u);
+        w0 = lds32(at); w1 = lds32(at + 4);
+        return Cursor{at, lds32(at + 8)};
     }
-    __device__ __forceinline__ void step(uint32_t& w0, uint32_t& w1, uint32_t& cur, uint32_t crossed) const {
-        asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %3, 0;\n @q mov.u32 %0, %1;\n @q ld.shared.u32 %1, [%2+8];\n @q add.u32 %2, %2, 4;\n}"
-                     : "+r"(w0), "+r"(w1), "+r"(cur) : "r"(crossed));
+    __device__ __forceinline__ void step(uint32_t& w0, uint32_t& w1, Cursor& cur, uint32_t crossed) const {
+        asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %4, 0;\n @q mov.u32 %0, %1;\n @q mov.u32 %1, %2;\n @q ld.shared.u32 %2, [%3+12];\n @q add.u32 %3, %3, 4;\n}"
+                     : "+r"(w0), "+r"(w1), "+r"(cur.w2), "+r"(cur.at) : "r"(crossed));
     }
 };
-// ... and in global memory; `cur` is the index of the first word
+// ... and in global memory; `at` is the index of the first word
 struct GlobalSource {
+    struct Cursor { uint32_t at, w2; };
     const uint32_t* words;
     uint32_t n;
     __device__ __forceinline__ uint32_t word(uint32_t i) const { return i < n ? __ldg(words + i) : 0u; }
-    __device__ __forceinline__ uint32_t start(uint32_t& w0, uint32_t& w1, uint32_t p) const {
+    __device__ __forceinline__ Cursor start(uint32_t& w0, uint32_t& w1, uint32_t p) const {
         w0 = word(p >> 5); w1 = word((p >> 5) + 1);
-        return p >> 5;
+        return Cursor{p >> 5, word((p >> 5) + 2)};
     }
-    __device__ __forceinline__ void step(uint32_t& w0, uint32_t& w1, uint32_t& cur, uint32_t crossed) const {
-        if (crossed) { w0 = w1; w1 = word(++cur + 1); }
+    __device__ __forceinline__ void step(uint32_t& w0, uint32_t& w1, Cursor& cur, uint32_t crossed) const {
+        if (crossed) { w0 = w1; w1 = cur.w2; cur.w2 = word(++cur.at + 2); }
     }
 };
 
 // A lane of a synchronising decoder.
+template <class Source>
 struct SyncLane {
     uint32_t base, at;   // a word boundary of the stream; the lane's place (see SyncTab), its bit position counted from there
     uint32_t nb;         // blocks ended since nb was last set to zero
-    uint32_t w0, w1, cur, tab;
+    uint32_t w0, w1, tab;
+    typename Source::Cursor cur;
     int32_t off;
-    McuBlock mb;         // of the current block
+    uint32_t ac;         // AC table of the current block
+    int32_t ac_off;
+    McuBlock nx;         // of the block after it
     // at a block start, or (`inside`) as if the DC term of the block had been passed
-    template <class Source>
     __device__ __forceinline__ void start(const Source& src, uint32_t mcu0, uint32_t bit, bool inside, uint32_t c) {
         base = bit & ~31u; at = (bit & 31u) | (inside ? 1u << 16 : 0u); nb = 0;
         cur = src.start(w0, w1, bit);
-        mb = lds_mcu(mcu0 + c * (uint32_t)sizeof(McuBlock));
-        tab = inside ? mb.dc + (uint32_t)sizeof(SyncTab) : mb.dc;
-        off = inside ? mb.ac_off : mb.dc_off;
+        const McuBlock mb = lds_mcu(mcu0 + c * (uint32_t)sizeof(McuBlock));
+        ac = mb.dc + (uint32_t)sizeof(SyncTab);
+        ac_off = mb.ac_off;
+        tab = inside ? ac : mb.dc;
+        off = inside ? ac_off : mb.dc_off;
+        nx = lds_mcu(mb.next);
     }
     __device__ __forceinline__ uint32_t pos() const { return base + (at & kPosMask); }
+    __device__ __forceinline__ uint32_t index(uint32_t mcu0, uint32_t bpm) const {  // of the current block, inside the MCU
+        const uint32_t k = mcu_index(mcu0, nx.next, bpm);
+        return (k ? k : bpm) - 1u;
+    }
+    // One look-up: an entry of 0 (a lane that is not `live`, a rare code) changes nothing.
+    __device__ __forceinline__ void apply(uint32_t e, bool& live, uint32_t stop_at, const Source& src) {
+        const uint32_t was = at;
+        at = was + __byte_perm(e, 0u, 0x4140);                        // all symbols
+        if (at & (64u << 16)) at = was + __byte_perm(e, 0u, 0x4342);  // slot 64: the first alone
+        src.step(w0, w1, cur, (was ^ at) & 32u);
+        if (e) { tab = ac; off = ac_off; }
+        const uint32_t end = at & kEndMask;
+        // the next block, whose tables are here already
+        asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %9, 0;\n @q mov.u32 %0, %5;\n @q mov.u32 %1, %6;\n @q add.u32 %2, %5, %10;\n @q mov.u32 %3, %7;\n"
+                     " @q add.u32 %4, %4, 1;\n @q ld.shared.v4.u32 {%5,%6,%7,%8}, [%8];\n}"
+                     : "+r"(tab), "+r"(off), "+r"(ac), "+r"(ac_off), "+r"(nb), "+r"(nx.dc), "+r"(nx.dc_off), "+r"(nx.ac_off), "+r"(nx.next)
+                     : "r"(end), "n"((int)sizeof(SyncTab)));
+        if (end) { at &= kPosMask; live = at < stop_at; }
+    }
     // Lanes with `live` decode to the first block start at a position of at least `stop`.  Called by whole warps: the loop has
     // one exit, taken by all lanes together, and no other jump out of it -- with returns from inside, the lanes of a warp
-    // never met again after their first different turn and went on alone.
-    template <class Source>
+    // never met again after their first different turn and went on alone.  The steps themselves are free of branches: a lane
+    // waits for every instruction of its chain, and jumps were a third of the chain.
     __device__ __forceinline__ void run_to(bool live, uint32_t stop, const Source& src, const HuffTable* pool) {
         const uint32_t stop_at = stop > base ? stop - base : 0u;
         while (__any_sync(0xFFFFFFFFu, live)) {
+            uint32_t e = 0;
 #pragma unroll
             for (int step = 0; step < 4; ++step) {
-                if (live) {
-                    const uint32_t top = __funnelshift_l(w1, w0, at);
-                    uint32_t e = entry_at<SyncTab>(tab, off, top);
-                    if (e == 0) e = rare_entry<SyncTab>(tab, top, pool).x;
-                    const uint32_t was = at;
-                    at = was + __byte_perm(e, 0u, 0x4140);                                 // all symbols
-                    if (at & (64u << 16)) at = was + __byte_perm(e, 0u, 0x4342);           // slot 64: the first alone
-                    src.step(w0, w1, cur, (was ^ at) & 32u);
-                    tab = mb.dc + (uint32_t)sizeof(SyncTab);
-                    off = mb.ac_off;
-                    if (at & kEndMask) {
-                        at &= kPosMask;
-                        ++nb;
-                        mb = lds_mcu(mb.next);
-                        tab = mb.dc;
-                        off = mb.dc_off;
-                        live = at < stop_at;
-                    }
-                }
+                e = entry_at<SyncTab>(tab, off, __funnelshift_l(w1, w0, at));
+                apply(live ? e : 0u, live, stop_at, src);
             }
+            if (live && e == 0) apply(rare_entry<SyncTab>(tab, __funnelshift_l(w1, w0, at), pool).x, live, stop_at, src);
         }
     }
 };
@@ -542,11 +554,11 @@ __global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
     const uint32_t mine = cell0 + (uint32_t)tid / bpm * span, myh = (uint32_t)tid % bpm;  // first cell of this thread's span
     const bool live = (uint32_t)tid < nspans * bpm && mine < ncell;
     uint32_t k = live ? mine : cell0;
-    SyncLane L{};
+    SyncLane<SharedSource> L{};
     L.start(source, mcu0, k ? k * CELL - kLeadBits : 0u, k != 0u, live && k ? myh : 0u);
     L.run_to(live && k, k * CELL, source, w.huff);
     uint32_t decodes = 0;
-    s_state[tid] = (uint16_t)(live ? pack_state(L.pos(), k * CELL, mcu_index(mcu0, L.mb.next, bpm), total) : kStNone);
+    s_state[tid] = (uint16_t)(live ? pack_state(L.pos(), k * CELL, L.index(mcu0, bpm), total) : kStNone);
     for (uint32_t step = 0; step < span; ++step) {
         __syncthreads();
         // ---- the distinct states, in as few warps as they fill
@@ -573,7 +585,7 @@ __global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
             L.run_to(on && p < bound, min(bound, total + 1), source, w.huff);
             __syncwarp();
             if (on) {
-                const uint32_t exit = pack_state(L.pos(), bound, mcu_index(mcu0, L.mb.next, bpm), total);
+                const uint32_t exit = pack_state(L.pos(), bound, L.index(mcu0, bpm), total);
                 if (L.pos() > total) --L.nb;  // the block that ended here is not whole
                 cand[(size_t)k * kCandidates + t % bpm] = make_uint2(entry | exit << 16, L.nb);
                 s_state[t] = (uint16_t)exit;
@@ -687,13 +699,13 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
         } else {
             if (__any_sync(0xFFFFFFFFu, decode)) {
                 const uint32_t k = decode ? open_at : 0, bound = (k + 1) * CELL, p = k * CELL + (decode ? open_state & 0xFFFu : 0u);
-                SyncLane L;
+                SyncLane<GlobalSource> L;
                 L.start(source, mcu0, p, false, decode ? open_state >> 12 : 0u);
                 L.run_to(decode, min(bound, total + 1), source, w.huff);
                 __syncwarp();
                 if (decode) {
                     ++decodes;
-                    const uint32_t n = L.nb - (L.pos() > total ? 1u : 0u), next = pack_state(L.pos(), bound, mcu_index(mcu0, L.mb.next, d.bpm), total);
+                    const uint32_t n = L.nb - (L.pos() > total ? 1u : 0u), next = pack_state(L.pos(), bound, L.index(mcu0, d.bpm), total);
                     found += n - (recs[k].y & 0xFFFu);
                     recs[k] = make_uint2(p, open_state << 12 | n);
                     if (k + 1 == kend) { exit = next; open_at = ~0u; last_open = 0; }
@@ -778,43 +790,46 @@ __device__ __forceinline__ uint32_t decode_blocks(const Source& src, const uint3
                                                   uint32_t* __restrict__ info, uint32_t& err) {
     const uint32_t first = blk, mcu0 = smem_addr(&sh.mcu[0]);
     bool live = blk < end;
-    uint32_t w0, w1, cur = src.start(w0, w1, p);
+    uint32_t w0, w1;
+    typename Source::Cursor cur = src.start(w0, w1, p);
     uint32_t base = p & ~31u, at = p & 31u;  // of the current block: a word boundary, the lane's place (see ValueTab)
     const uint32_t place = smem_addr(sh.place) - 4, buf = smem_addr(&sh.block[threadIdx.x]);
     McuBlock mb = lds_mcu(mcu0 + c * (uint32_t)sizeof(McuBlock));
-    uint32_t tab = mb.dc, seen = 0, e = 0;
+    uint32_t tab = mb.dc, seen = 0, last = 0;  // last: the entry of the last symbol
     int32_t off = mb.dc_off;
     int32_t pred0 = 0, pred1 = 0, pred2 = 0;
+    // one symbol; an entry of 0 (a lane that waits, a rare code) changes nothing
+    const auto apply = [&](uint32_t e, uint32_t top) {
+        const uint32_t was = at;
+        at += e;
+        src.step(w0, w1, cur, (was ^ at) & 32u);
+        // the s extra bits (T.81 EXTEND), first moved to the top: a leading 1 means the value itself, a leading 0 the complement
+        // of its magnitude
+        const uint32_t n = e >> 27, bits = __funnelshift_l(0u, __funnelshift_l(top, 0u, e), n);
+        const uint32_t neg = ~(uint32_t)((int32_t)bits >> 31);
+        const uint32_t v = __funnelshift_r(bits, neg, n) - neg;
+        const uint32_t slot = at >> 14 & 0x3FCu;  // (times four)
+        const bool store = (int32_t)e < 0 && slot <= 256u;
+        asm volatile("{\n .reg .pred q;\n .reg .u32 a, o;\n .reg .u16 h;\n setp.ne.u32 q, %1, 0;\n @q ld.shared.u32 a, [%2];\n cvt.u16.u32 h, %3;\n"
+                     " shr.u32 o, a, 16;\n add.u32 o, o, %4;\n @q st.shared.u16 [o], h;\n @q or.b32 %0, %0, a;\n}"
+                     : "+r"(seen) : "r"((uint32_t)store), "r"(place + slot), "r"(v), "r"(buf) : "memory");
+        if (e) { tab = mb.dc + (uint32_t)sizeof(ValueTab); off = mb.ac_off; last = e; }
+    };
     for (;;) {
         const uint32_t alive = __ballot_sync(0xFFFFFFFFu, live);
         if (!alive) break;  // one exit for the whole warp, see SyncLane::run_to
+        uint32_t e = 0;
 #pragma unroll
         for (int step = 0; step < 2; ++step) {
-            if (live && !(at & kEndMask)) {
-                const uint32_t top = __funnelshift_l(w1, w0, at);
-                e = entry_at<ValueTab>(tab, off, top);
-                if (e == 0) {
-                    const uint2 rare = rare_entry<ValueTab>(tab, top, pool);
-                    e = rare.x;
-                    if (rare.y >> 31 && base + (at & kPosMask) < limit) err |= kStBadCode;
-                }
-                const uint32_t was = at;
-                at += e;
-                src.step(w0, w1, cur, (was ^ at) & 32u);
-                // the s extra bits (T.81 EXTEND), first moved to the top: a leading 1 means the value itself, a leading 0 the
-                // complement of its magnitude
-                const uint32_t n = e >> 27, bits = __funnelshift_l(0u, __funnelshift_l(top, 0u, e), n);
-                const uint32_t neg = ~(uint32_t)((int32_t)bits >> 31);
-                const uint32_t v = __funnelshift_r(bits, neg, n) - neg;
-                const uint32_t slot = at >> 14 & 0x3FCu;  // (times four)
-                if ((int32_t)e < 0 && slot <= 256u) {
-                    const uint32_t pl = lds32(place + slot);
-                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(buf + (pl >> 16)), "h"((uint16_t)v) : "memory");
-                    seen |= pl;
-                }
-                tab = mb.dc + (uint32_t)sizeof(ValueTab);
-                off = mb.ac_off;
-            }
+            const uint32_t top = __funnelshift_l(w1, w0, at);
+            e = entry_at<ValueTab>(tab, off, top);
+            apply(live && !(at & kEndMask) ? e : 0u, top);
+        }
+        if (e == 0 && live && !(at & kEndMask)) {
+            const uint32_t top = __funnelshift_l(w1, w0, at);
+            const uint2 rare = rare_entry<ValueTab>(tab, top, pool);
+            if (rare.y >> 31 && base + (at & kPosMask) < limit) err |= kStBadCode;
+            apply(rare.x, top);
         }
         const uint32_t done = __ballot_sync(0xFFFFFFFFu, live && (at & kEndMask));
         if (__popc(done) >= kFlushLanes || done == alive) {
@@ -822,7 +837,7 @@ __device__ __forceinline__ uint32_t decode_blocks(const Source& src, const uint3
                 const uint32_t now = base + (at & kPosMask);
                 if (now > limit) live = false;  // (what the buffer holds is of no use, and neither is the rest of the span)
                 else {
-                    if ((int32_t)e < 0 && (at >> 14 & 0x3FCu) > 256u) err |= kStCoefRange;
+                    if ((int32_t)last < 0 && (at >> 14 & 0x3FCu) > 256u) err |= kStCoefRange;
                     uint4* const b = sh.block + threadIdx.x;
                     uint4* const rows = reinterpret_cast<uint4*>(coef) + (size_t)blk * 8;
                     const uint4 zero = make_uint4(0, 0, 0, 0), q0 = b[0];
