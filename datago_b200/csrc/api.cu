@@ -357,6 +357,8 @@ struct WavePlan {
     std::map<std::array<uint32_t, 2>, uint32_t> pair_ids;
     uint32_t cell_bits = kCellBits;              // of the wave's streams: bits per thread of the value decoder
     uint32_t guess_span = 1;                     // cells a thread of the synchronising decoder goes through
+    uint32_t chain_threads = 1024;               // of the linking kernel per image
+    bool mixed = false;                          // see JpegWave
     uint32_t write_cells = kDecodeThreads, restart_segs = kDecodeThreads;  // threads per CTA of the value decoders
     uint32_t max_pairs = 1;                      // most distinct ones in one image
     uint32_t pair_id(uint32_t dc, uint32_t ac) {
@@ -1049,6 +1051,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             if (!d.restart) guess_bits += (uint64_t)d.raw_len * 8 * d.bpm;
         wv.cell_bits = guess_bits / kShortCellBits > kGuessSpanThreads ? kCellBits : kShortCellBits;
         wv.guess_span = guess_bits / kCellBits > kGuessSpanThreads ? kGuessSpan : 1;
+        wv.chain_threads = chain_threads(std::count_if(built.begin(), built.end(), [](const JpegDesc& d) { return !d.restart; }));
         uint32_t color_total = 0, fchroma_total = 0, ftile_total = 0;
         size_t group_bytes = 0, fgroup_bytes = 0;
         wv.block_first.push_back(0);
@@ -1075,7 +1078,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             } else {
                 wv.spec_list.push_back((uint32_t)wv.descs.size());
                 d.cell_off = cells;
-                cells += stream_cells(d.raw_len, wv.cell_bits) + 1;
+                cells += align_up(stream_cells(d.raw_len, wv.cell_bits), wv.chain_threads) + 1;
             }
             wv.tile_first.push_back(wv.tile_first.back() + std::max(1u, (uint32_t)(((uint64_t)d.raw_len + kUnstuffTile - 1) / kUnstuffTile)));
             {
@@ -1127,6 +1130,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         }
         wv.restart_first.assign(1, 0);
         for (uint32_t k : wv.restart_list) wv.restart_first.push_back(wv.restart_first.back() + (wv.descs[k].nseg + wv.restart_segs - 1) / wv.restart_segs);
+        wv.mixed = !wv.spec_list.empty() && wv.chain_threads == 1024 && stream_cells(wv.descs[wv.spec_list[0]].raw_len, wv.cell_bits) > kMixedRun * 1024;
         wv.guess_first.assign(1, 0);
         wv.write_first.assign(1, 0);
         for (uint32_t k : wv.spec_list) {
@@ -1468,7 +1472,7 @@ static int batch_run_locked(dg_batch* b) {
             w.seg_start = (uint32_t*)(sc + wv.off_segstart);
             w.seg_found = (uint32_t*)(sc + wv.off_segfound);
             w.cells = (uint2*)(sc + wv.off_cells);
-            w.cand = (uint2*)(sc + wv.off_cand);
+            w.cand = (uint4*)(sc + wv.off_cand);
             w.coef = (int16_t*)(sc + wv.off_coef);
             w.diff = (uint32_t*)(sc + wv.off_diff);
             w.info = (uint32_t*)(sc + wv.off_info);
@@ -1488,6 +1492,8 @@ static int batch_run_locked(dg_batch* b) {
             w.restart_ctas = resolve(b, wv.m_restart);
             w.cell_bits = wv.cell_bits;
             w.guess_span = wv.guess_span;
+            w.chain_threads = wv.chain_threads;
+            w.mixed = wv.mixed;
             w.write_cells = wv.write_cells;
             w.restart_segs = wv.restart_segs;
             w.guess_ctas = resolve(b, wv.m_guess);

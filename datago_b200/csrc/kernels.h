@@ -29,6 +29,11 @@ inline uint32_t decode_threads(uint64_t threads) { return threads > kSms * 4ull 
 // per cell and block of the MCU would be more than the chip holds at once
 constexpr uint32_t kGuessLanes = 384, kCandidates = 6, kGuessSpan = 4;
 constexpr uint64_t kGuessSpanThreads = kSms * 2048ull;
+// Threads of the linking kernel per image.  With an image for most SMs or more, 256 leave the most room for other kernels beside
+// them (1024 files of 0.4 Mbit: 3.37 ms a pass against 3.48 with 1024 threads; 256 files of 5 Mbit: 4.29 against 4.30); with fewer,
+// an image gets 1024, so that its threads' runs are short.
+constexpr uint32_t kMixedRun = 4;
+inline uint32_t chain_threads(size_t images) { return images >= 120 ? 256 : 1024; }
 // spans of cells a CTA takes, each with a thread per block of the MCU: what the threads allow, 256 staged cells at most
 #ifdef __CUDACC__
 __host__ __device__
@@ -61,9 +66,10 @@ struct JpegWave {
     uint32_t* us_len;        // [n] bytes of each unstuffed stream
     uint32_t* seg_start;     // restart-segment starts (bytes into the image's unstuffed stream)
     uint32_t* seg_found;     // [n] segments actually present
-    uint2* cells;            // per cell of a restart-free stream: bit position of its first block, index of that block
-    uint2* cand;             // [cells][kCandidates] entry state | exit state << 16, blocks that start in the cell (see k_huff_guess);
-                             // lies over what is written after the entropy stage
+    uint2* cells;            // of a restart-free stream: -, its blocks; then per cell (see CellOrder): bit position of its first
+                             // block, index of that block
+    uint4* cand;             // [cells][kCandidates / 2], see CellOrder: two candidates: entry state | exit state << 16, blocks that
+                             // start in the cell (see k_huff_guess); lies over what is written after the entropy stage
     int16_t* coef;           // [blocks][64], scan order, natural order inside a block; AC terms, rows the class covers
     uint32_t* diff;          // [blocks] restart-free images: DC difference | class << 16
     uint32_t* info;          // [blocks] DC coefficient (low half) | class << 16
@@ -83,6 +89,8 @@ struct JpegWave {
     uint32_t cell_bits;      // kCellBits or kShortCellBits
     uint32_t write_cells, restart_segs;  // cells / segments per CTA of the value decoders: kDecodeThreads or kDecodeThreadsMany
     uint32_t guess_span;     // cells a thread of the synchronising decoder goes through
+    uint32_t chain_threads;  // of the linking kernel per image, see chain_threads()
+    uint32_t mixed;          // see CellOrder: 1024 linking threads, and more than kMixedRun cells for one of them
     // restart-interval images: restart_segs segments per CTA, owner = index into restart_list
     OwnerMap restart_ctas;
     const uint32_t* restart_list;

@@ -515,7 +515,29 @@ static_assert((1ull << 32) - kMaxStream * 8ull > 2ull * kDecodeThreadsMany * kCe
 constexpr uint32_t kStNone = 0xFFFFu, kStDropped = 0xFFFEu;  // the stream ends before; no candidate
 __device__ __forceinline__ uint32_t pack_state(uint32_t p, uint32_t cell_bit, uint32_t c, uint32_t total) { return p > total ? kStNone : (p - cell_bit) | c << 12; }
 
-constexpr uint32_t kLeadBits = 256;
+// Where cell k of an image stands in w.cells and w.cand.  A thread of the linking kernel walks `run` consecutive cells.  Where
+// runs are long (`mixed`, see JpegWave), the cells that all threads read in the same step are neighbours instead: in order, a load
+// of a warp touched 32 lines, and the loads of a step queued for 2 900 cycles (8 images of 4:4:4, up to 17 cells a thread: 66 us
+// for the kernel, 50 like this).
+struct CellOrder {
+    uint32_t run, threads;
+    bool mixed;
+    __device__ __forceinline__ CellOrder(uint32_t ncell, uint32_t threads, bool mixed) : run((ncell + threads - 1) >> (threads == 256 ? 8 : 10)), threads(threads), mixed(mixed) {}
+    __device__ __forceinline__ uint32_t at(uint32_t k) const {
+        if (!mixed) return k;
+        const uint32_t t = k / run;
+        return (k - t * run) * threads + t;
+    }
+    // pieces of two candidates: in order all of a cell's together, else one of each cell together
+    static constexpr uint32_t kPieces = kCandidates / 2;
+    __device__ __forceinline__ uint32_t piece_step() const { return mixed ? run * threads : 1u; }  // from a cell's piece to its next one
+    __device__ __forceinline__ uint32_t piece(uint32_t k, uint32_t h) const { return mixed ? h * piece_step() + at(k) : k * kPieces + h; }
+};
+
+// Bits before a cell from which its candidates are decoded.  512 leave a third of the open states that 256 leave; that costs the
+// candidates 3 us and saves a long stream's linking more (one photo of 5 234 cells: 16.3 + 41.3 us with 256, 19.1 + 33.9 with 512;
+// 8 images of 4:4:4: 51 + 50 and 60 + 39; a thumbnail of 312 cells has few open states anyway).
+constexpr uint32_t kLead = 256, kLeadMixed = 512;
 constexpr int kGuessThreads = (int)kGuessLanes;
 
 }  // namespace
@@ -523,7 +545,7 @@ constexpr int kGuessThreads = (int)kGuessLanes;
 // A CTA takes guess_spans() spans of w.guess_span cells, a thread per span and block of the MCU.  Decoders that meet are one
 // from then on, so in a span of several cells the lead is run once and fewer decoders are left from cell to cell; with few
 // images a span is one cell, because then the length of a thread's way is what counts.
-template <int CELL>
+template <int CELL, bool MIXED>
 __global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
     extern __shared__ __align__(16) unsigned char guess_smem[];
     __shared__ McuBlock mcu[6];
@@ -538,13 +560,16 @@ __global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
     unsigned char* const tab0 = guess_smem;
     unsigned char* const stage = tab0 + w.max_pairs * 2 * sizeof(SyncTab);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr uint32_t lead = MIXED ? kLeadMixed : kLead;
+    static_assert(lead <= (uint32_t)CELL, "the lead lies in the cell before");
     const uint32_t row0 = cell0 ? cell0 - 1 : 0, cell1 = min(cell0 + nspans * span, ncell);
     Staged<CELL>::copy(stage, w.us + d.us_off, row0, (int)(min(cell0 + nspans * span + Staged<CELL>::kRowsBehind, ncell + Staged<CELL>::kRowsPadded) - row0), tid, kGuessThreads);
     load_tables<SyncTab>(w, d, mcu, tab0, (uint32_t)offsetof(CodeTables, sync), tid, kGuessThreads);
     copy_commit();
-    uint2* const cand = w.cand + (size_t)d.cell_off * kCandidates;
+    const CellOrder order(ncell, 1024, MIXED);
+    uint2* const cand = reinterpret_cast<uint2*>(w.cand + (size_t)d.cell_off * CellOrder::kPieces);
     for (uint32_t i = cell0 * (kCandidates / 2) + tid; i < cell1 * (kCandidates / 2); i += kGuessThreads)
-        reinterpret_cast<uint4*>(cand)[i] = make_uint4(kStDropped, 0, kStDropped, 0);
+        reinterpret_cast<uint4*>(cand)[order.mixed ? order.piece(i / CellOrder::kPieces, i % CellOrder::kPieces) : i] = make_uint4(kStDropped, 0, kStDropped, 0);
     copy_wait<0>();
     __syncthreads();
     const uint32_t mcu0 = smem_addr(&mcu[0]);
@@ -555,7 +580,7 @@ __global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
     const bool live = (uint32_t)tid < nspans * bpm && mine < ncell;
     uint32_t k = live ? mine : cell0;
     SyncLane<SharedSource> L{};
-    L.start(source, mcu0, k ? k * CELL - kLeadBits : 0u, k != 0u, live && k ? myh : 0u);
+    L.start(source, mcu0, k ? k * CELL - lead : 0u, k != 0u, live && k ? myh : 0u);
     L.run_to(live && k, k * CELL, source, w.huff);
     uint32_t decodes = 0;
     s_state[tid] = (uint16_t)(live ? pack_state(L.pos(), k * CELL, L.index(mcu0, bpm), total) : kStNone);
@@ -587,7 +612,8 @@ __global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
             if (on) {
                 const uint32_t exit = pack_state(L.pos(), bound, L.index(mcu0, bpm), total);
                 if (L.pos() > total) --L.nb;  // the block that ended here is not whole
-                cand[(size_t)k * kCandidates + t % bpm] = make_uint2(entry | exit << 16, L.nb);
+                const uint32_t h = t % bpm;
+                cand[order.mixed ? (size_t)order.piece(k, h / 2) * 2 + (h & 1u) : (size_t)k * kCandidates + h] = make_uint2(entry | exit << 16, L.nb);
                 s_state[t] = (uint16_t)exit;
             }
         }
@@ -607,7 +633,7 @@ static_assert(sizeof(ChainMisc<256>) % 16 == 0, "tables follow in shared memory"
 
 }  // namespace
 
-template <int T, int CELL>
+template <int T, int CELL, bool MIXED>
 __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
     extern __shared__ __align__(16) unsigned char chain_smem[];
     ChainMisc<T>& sh = *reinterpret_cast<ChainMisc<T>*>(chain_smem);
@@ -620,10 +646,12 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
     const uint32_t us_len = w.us_len[img], total = us_len * 8u;
     const uint32_t ncell = (total + CELL - 1) / CELL;
     const GlobalSource source{reinterpret_cast<const uint32_t*>(w.us + d.us_off), (us_len + 3) / 4 + 2};
-    uint2* const recs = w.cells + d.cell_off;  // while linking: block start, state << 12 | blocks that start in the cell
-    const uint4* const cand = reinterpret_cast<const uint4*>(w.cand + (size_t)d.cell_off * kCandidates);
-    const uint32_t run = (ncell + T - 1) / T;
-    const uint32_t kbeg = min(tid * run, ncell), kend = min(kbeg + run, ncell);
+    const CellOrder order(ncell, T, MIXED);
+    const uint32_t run = order.run, kbeg = min(tid * run, ncell), kend = min(kbeg + run, ncell);
+    // of this thread's cell k: [(k - kbeg) * step]
+    const uint32_t step = order.mixed ? T : 1, cand_step = order.mixed ? T : CellOrder::kPieces, piece = order.piece_step();
+    uint2* const recs = w.cells + d.cell_off + 1 + tid * (order.mixed ? 1 : run);  // while linking: block start, state << 12 | blocks that start in the cell
+    const uint4* const cand = w.cand + (size_t)d.cell_off * CellOrder::kPieces + tid * (order.mixed ? 1 : run * CellOrder::kPieces);
     const bool active = kbeg < kend;
     const uint32_t mcu0 = smem_addr(&sh.mcu[0]);
     uint32_t found = 0;  // blocks that start in this thread's cells
@@ -644,14 +672,14 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
             uint32_t next = kStNone, n = 0;
             uint2 had = make_uint2(0, 0);
             if (redo) {
-                had = recs[k];
+                had = recs[(k - kbeg) * step];
                 if (k != first && k >= last_open && (had.y >> 12) == state) break;  // met
             }
             if (state != kStNone) {
                 if ((state & 0xFFFu) >= (uint32_t)CELL) next = state - CELL;  // no block starts in this cell
                 else {
-                    const uint4* const c = cand + (size_t)k * (kCandidates / 2);
-                    const uint4 a = __ldg(c), b = __ldg(c + 1), e = __ldg(c + 2);
+                    const uint4* const c = cand + (k - kbeg) * cand_step;
+                    const uint4 a = __ldg(c), b = __ldg(c + piece), e = __ldg(c + 2 * piece);
                     bool known = false;
                     auto look = [&](uint32_t x, uint32_t y) { if ((x & 0xFFFFu) == state) { next = x >> 16; n = y; known = true; } };
                     look(a.x, a.y); look(a.z, a.w); look(b.x, b.y); look(b.z, b.w); look(e.x, e.y); look(e.z, e.w);
@@ -665,7 +693,7 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
                     }
                 }
             }
-            recs[k] = make_uint2(state == kStNone ? kNoState : cell_bit + (state & 0xFFFu), state << 12 | n);
+            recs[(k - kbeg) * step] = make_uint2(state == kStNone ? kNoState : cell_bit + (state & 0xFFFu), state << 12 | n);
             found += n - (had.y & 0xFFFu);
             state = next;
             if (k + 1 == kend) { exit = state; break; }
@@ -675,7 +703,7 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
 
     uint32_t entry = 0;  // thread 0: bit 0, block 0
     if (active && tid) {
-        entry = __ldg(&cand[(size_t)kbeg * (kCandidates / 2)].x) & 0xFFFFu;
+        entry = __ldg(&cand->x) & 0xFFFFu;
         if (entry == kStDropped) entry = kStNone;
     }
     follow(active, kbeg, entry, false);
@@ -706,8 +734,8 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
                 if (decode) {
                     ++decodes;
                     const uint32_t n = L.nb - (L.pos() > total ? 1u : 0u), next = pack_state(L.pos(), bound, L.index(mcu0, d.bpm), total);
-                    found += n - (recs[k].y & 0xFFFu);
-                    recs[k] = make_uint2(p, open_state << 12 | n);
+                    found += n - (recs[(k - kbeg) * step].y & 0xFFFu);
+                    recs[(k - kbeg) * step] = make_uint2(p, open_state << 12 | n);
                     if (k + 1 == kend) { exit = next; open_at = ~0u; last_open = 0; }
                     else follow(true, k + 1, next, true);
                 }
@@ -728,9 +756,10 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
     uint32_t base = inc - found;
 #pragma unroll
     for (int i = 0; i < T / 32; ++i) if (i < warp) base += sh.warp[i];
-    for (uint32_t k = kbeg; k < kend; ++k) { const uint32_t n = recs[k].y & 0xFFFu; recs[k].y = base; base += n; }
+#pragma unroll 4
+    for (uint32_t i = 0; i < kend - kbeg; ++i) { const uint32_t n = recs[i * step].y & 0xFFFu; recs[i * step].y = base; base += n; }
     if (tid == T - 1) {
-        recs[ncell] = make_uint2(kNoState, base);
+        w.cells[d.cell_off] = make_uint2(kNoState, base);
         uint32_t err = 0;
         if (base < d.nblocks) err |= kStTruncated;
         if (round > limit) err |= kStSyncLimit;
@@ -899,12 +928,13 @@ __global__ void __launch_bounds__(T) k_huff_write(JpegWave w) {
     Staged<CELL>::copy(stage, w.us + d.us_off, cell0, (int)min((uint32_t)(T + Staged<CELL>::kRowsBehind), ncell - cell0 + Staged<CELL>::kRowsPadded), tid, T);
     value_setup<T>(w, d, sh, tab0);
     const uint32_t k = cell0 + tid;
+    const CellOrder order(ncell, w.chain_threads, w.mixed);
     const uint2* recs = w.cells + d.cell_off;
     uint2 a = make_uint2(0, 0);
     uint32_t b1 = 0;
     if (k < ncell) {
-        a = recs[k];
-        b1 = min(recs[k + 1].y, d.nblocks);
+        a = recs[1 + order.at(k)];
+        b1 = min(recs[k + 1 < ncell ? 1 + order.at(k + 1) : 0].y, d.nblocks);
     }
     copy_wait<0>();
     __syncthreads();
@@ -1114,10 +1144,10 @@ __global__ void __launch_bounds__(kDcThreads) k_dc(JpegWave w) {
     __shared__ DcSmem sh;
     const uint32_t img = w.spec_list[blockIdx.x / cooperative_groups::this_cluster().num_blocks()];
     const JpegDesc& d = w.descs[img];
-    const uint32_t us_len = w.us_len[img], nblocks = d.nblocks;
+    const uint32_t nblocks = d.nblocks;
     const uint32_t* diff = w.diff + d.block_off;
     uint32_t* info = w.info + d.block_off;
-    const auto blocks = [&] { return min(w.cells[d.cell_off + (us_len * 8u + w.cell_bits - 1) / w.cell_bits].y, nblocks); };
+    const auto blocks = [&] { return min(w.cells[d.cell_off].y, nblocks); };
     switch (d.bpm) {
         case 1: dc_image<1>(diff, info, nblocks, blocks, sh); break;
         case 3: dc_image<3>(diff, info, nblocks, blocks, sh); break;
@@ -1144,9 +1174,11 @@ template <class K>
 void allow_smem(K kernel, size_t bytes) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); }
 template <int CELL>
 void allow_cells(size_t most) {
-    allow_smem(k_huff_guess<CELL>, most - 4096);  // (it has static arrays as well)
-    allow_smem(k_huff_chain<256, CELL>, most);
-    allow_smem(k_huff_chain<1024, CELL>, most);
+    allow_smem(k_huff_guess<CELL, false>, most - 4096);  // (it has static arrays as well)
+    allow_smem(k_huff_guess<CELL, true>, most - 4096);
+    allow_smem(k_huff_chain<256, CELL, false>, most);
+    allow_smem(k_huff_chain<1024, CELL, false>, most);
+    allow_smem(k_huff_chain<1024, CELL, true>, most);
     allow_smem(k_huff_write<kDecodeThreads, CELL>, most);
     allow_smem(k_huff_write<kDecodeThreadsMany, CELL>, most);
 }
@@ -1170,19 +1202,17 @@ template <int CELL>
 void launch_guess(const JpegWave& w, cudaStream_t s) {
     // the cell before the first, the cells, and what a block may run over
     const size_t rows = 1 + (size_t)guess_spans(1, w.guess_span) * w.guess_span + Staged<CELL>::kRowsBehind;
-    k_huff_guess<CELL><<<w.guess_ctas.total, kGuessThreads, rows * Staged<CELL>::kPitch + w.max_pairs * 2 * sizeof(SyncTab), s>>>(w);
+    const size_t smem = rows * Staged<CELL>::kPitch + w.max_pairs * 2 * sizeof(SyncTab);
+    if (w.mixed) k_huff_guess<CELL, true><<<w.guess_ctas.total, kGuessThreads, smem, s>>>(w);
+    else k_huff_guess<CELL, false><<<w.guess_ctas.total, kGuessThreads, smem, s>>>(w);
 }
 
-// With an image for most SMs or more, 256 threads each leave the most room for other kernels beside them (1024 files of 0.4
-// Mbit: 3.37 ms a pass against 3.48 with 1024 threads; 256 files of 5 Mbit: 4.29 against 4.30); with fewer, an image gets
-// 1024, so that its threads' runs are short.  (The launches alone are shorter with 1024 threads even then, 270 against 319 us
-// for the two of the 256 files; a pass, in which other kernels run beside them, is not.)
-constexpr uint32_t kChainManyImages = 120;
 template <int CELL>
 void launch_chain(const JpegWave& w, cudaStream_t s) {
     const size_t tables = w.max_pairs * 2 * sizeof(SyncTab);
-    if (w.n_spec >= kChainManyImages) k_huff_chain<256, CELL><<<w.n_spec, 256, sizeof(ChainMisc<256>) + tables, s>>>(w);
-    else k_huff_chain<1024, CELL><<<w.n_spec, 1024, sizeof(ChainMisc<1024>) + tables, s>>>(w);
+    if (w.chain_threads == 256) k_huff_chain<256, CELL, false><<<w.n_spec, 256, sizeof(ChainMisc<256>) + tables, s>>>(w);
+    else if (w.mixed) k_huff_chain<1024, CELL, true><<<w.n_spec, 1024, sizeof(ChainMisc<1024>) + tables, s>>>(w);
+    else k_huff_chain<1024, CELL, false><<<w.n_spec, 1024, sizeof(ChainMisc<1024>) + tables, s>>>(w);
 }
 
 template <int T, int CELL>
