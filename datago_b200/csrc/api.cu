@@ -127,7 +127,6 @@ struct dg_ctx {
     // Horizontal resize passes run on the tensor cores where their geometry fits; DATAGO_B200_HMMA=0 keeps them on the
     // dp2a kernel (measurements, and the test-suite's coverage of that kernel).
     bool hmma = true;
-    unsigned int conv_timeouts_seen = 0;
     dg_ctx_counters counters{};  // guarded by mu
     // Largest decoded image accepted (width * height * channels bytes); the `image` crate's default allocation limit is 512 MiB.
     uint64_t max_image_bytes = (uint64_t)512 << 20;
@@ -296,6 +295,12 @@ extern "C" uint64_t dg_key_rank(const char* key, uint64_t len, uint64_t world) {
 // ---------------------------------------------------------------------------------------------------------------
 namespace {
 
+// What the kernels report, one copy at dg_batch_sync: n status words, three 64-bit counters of the synchronising Huffman decoder,
+// the CTAs of resize passes that gave up waiting.
+inline size_t stats_at(int n) { return align_up((size_t)n * 4, 8); }
+inline size_t timeouts_at(int n) { return stats_at(n) + 24; }
+inline size_t status_bytes(int n) { return stats_at(n) + 32; }
+
 // Appends arrays to one host image of the batch's device metadata; offsets become device pointers after upload.
 struct Meta {
     std::vector<uint8_t> bytes;
@@ -432,7 +437,6 @@ struct dg_batch {
     uint32_t launches = 0;
     bool uploaded = false, ran = false;
     bool counted = false;    // its items have been added to the context's counters
-    bool used_hmma = false;  // a pass of this batch ran on the tensor-core resize kernel, whose waits are bounded
     std::vector<StageEvent> events;
     float stage_ms[DG_STAGE_COUNT] = {0};
 };
@@ -1170,8 +1174,8 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         if (rc) return abandon(b, rc);
         b->d_scratch2 = (uint8_t*)ctx->dev.blocks[b->blk_scratch2].ptr;
     }
-    b->off_status = 0;  // n status words, then 4 counters of the speculative Huffman kernel
-    b->off_blob = align_up((size_t)n * 4 + 32, 256);
+    b->off_status = 0;  // see status_bytes
+    b->off_blob = align_up(status_bytes(n), 256);
     b->off_rawin = b->off_blob + align_up(blob, 256);
     b->off_out = b->off_rawin + align_up(rawin, 256);
     rc = ctx->dev.acquire(b->off_out + align_up(b->arena_bytes, 256), &b->blk_persist);
@@ -1323,7 +1327,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
     rc = ctx->dev_meta.acquire(b->meta_total, &b->blk_meta);
     if (!rc) rc = ctx->pin.acquire(b->off_rawin + align_up(rawin, 256), &b->blk_pin);
     if (!rc) rc = ctx->pin_meta.acquire(b->meta_total, &b->blk_pin_meta);
-    if (!rc) rc = ctx->pin_meta.acquire(std::max<size_t>((size_t)n * 4, 256), &b->blk_pin_status);
+    if (!rc) rc = ctx->pin_meta.acquire(std::max<size_t>(status_bytes(n), 256), &b->blk_pin_status);
     if (rc) return abandon(b, rc);
     b->d_meta = (uint8_t*)ctx->dev_meta.blocks[b->blk_meta].ptr;
     b->h_pin = (uint8_t*)ctx->pin.blocks[b->blk_pin].ptr;
@@ -1448,7 +1452,7 @@ static int batch_run_locked(dg_batch* b) {
         return cudaEventRecord(b->events[ev++].b, s);
     };
     b->launches = 0;
-    if (b->ran) CU(cudaMemsetAsync(b->d_persist + b->off_status, 0, align_up((size_t)b->n * 4, 8) + 32, s));  // status words of the previous run
+    if (b->ran) CU(cudaMemsetAsync(b->d_persist + b->off_status, 0, status_bytes(b->n), s));  // of the previous run
     if (two_lanes) {
         CU(cudaEventRecord(ctx->ev_fork, ctx->stream));
         CU(cudaStreamWaitEvent(ctx->stream2, ctx->ev_fork, 0));
@@ -1479,7 +1483,7 @@ static int batch_run_locked(dg_batch* b) {
             w.planes = sc + wv.off_planes;
             w.out = transform ? sc + wv.off_decoded : b->d_persist + b->off_out;
             w.status = (uint32_t*)(b->d_persist + b->off_status);
-            w.spec_stats = (unsigned long long*)(b->d_persist + b->off_status + align_up((size_t)b->n * 4, 8));
+            w.spec_stats = (unsigned long long*)(b->d_persist + b->off_status + stats_at(b->n));
             w.huff = (const HuffTable*)(meta + b->m_huff);
             w.table_pairs = (const uint2*)(meta + wv.m_pairs);
             w.n_pairs = (uint32_t)wv.pairs.size();
@@ -1579,9 +1583,9 @@ static int batch_run_locked(dg_batch* b) {
                 if (!wv.passes[st].empty()) {
                     CU(mark(kStageOf[st], true));
                     const ConvPass* passes = (const ConvPass*)(meta + wv.m_passes[st]);
-                    if (st & 1) launch_conv_v(passes, resolve(b, wv.m_pass[st]), tables, wv.mma_tiles[st], s);
-                    else launch_conv_h(passes, resolve(b, wv.m_pass[st]), tables, wv.mma_tiles[st], s);
-                    b->used_hmma = b->used_hmma || wv.mma_tiles[st] != 0;
+                    unsigned int* const timeouts = (unsigned int*)(b->d_persist + b->off_status + timeouts_at(b->n));
+                    if (st & 1) launch_conv_v(passes, resolve(b, wv.m_pass[st]), tables, wv.mma_tiles[st], timeouts, s);
+                    else launch_conv_h(passes, resolve(b, wv.m_pass[st]), tables, wv.mma_tiles[st], timeouts, s);
                     ++b->launches;
                     CU(mark(kStageOf[st], false));
                 }
@@ -1703,20 +1707,15 @@ extern "C" int dg_batch_sync(dg_batch* b) {
     std::lock_guard<std::mutex> lock(ctx->mu);
     CU(cudaSetDevice(ctx->device));
     if (b->ran) {
-        CU(cudaMemcpyAsync(b->h_status, b->d_persist + b->off_status, (size_t)b->n * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        CU(cudaMemcpyAsync(b->h_status, b->d_persist + b->off_status, status_bytes(b->n), cudaMemcpyDeviceToHost, ctx->stream));
         b->d2h += (size_t)b->n * 4;
     }
     CU(cudaStreamSynchronize(ctx->stream));
     landed(b);
-    if (b->ran && b->used_hmma) {
-        // the tensor-core resize pass bounds its waits for asynchronous copies; a wait that ran out left garbage behind
-        const unsigned int t = read_conv_timeouts(ctx->stream);
-        if (t != ctx->conv_timeouts_seen) {
-            ctx->conv_timeouts_seen = t;
-            return fail(DG_E_CUDA, "resize: a copy into shared memory did not complete in time (%u CTAs gave up); the batch's pixels are not valid", t);
-        }
-    }
     if (b->ran) {
+        // the tensor-core resize passes bound their waits for asynchronous copies; a wait that ran out left garbage behind
+        const unsigned int t = *(const unsigned int*)((const uint8_t*)b->h_status + timeouts_at(b->n));
+        if (t) return fail(DG_E_CUDA, "resize: a copy into shared memory did not complete in time (%u CTAs gave up); the batch's pixels are not valid", t);
         for (int i = 0; i < b->n; ++i)
             if (b->items[i].status == DG_OK && b->h_status[i]) b->items[i].status = device_status_to_code(b->h_status[i]);
         if (!b->counted) {  // once per batch, however often it is run and synchronised
@@ -1798,7 +1797,7 @@ extern "C" int dg_batch_huffman_stats(dg_batch* b, uint64_t out[3]) {
     dg_ctx* ctx = b->ctx;
     std::lock_guard<std::mutex> lock(ctx->mu);
     CU(cudaSetDevice(ctx->device));
-    CU(cudaMemcpyAsync(out, b->d_persist + b->off_status + align_up((size_t)b->n * 4, 8), 24, cudaMemcpyDeviceToHost, ctx->stream));
+    CU(cudaMemcpyAsync(out, b->d_persist + b->off_status + stats_at(b->n), 24, cudaMemcpyDeviceToHost, ctx->stream));
     CU(cudaStreamSynchronize(ctx->stream));
     return DG_OK;
 }
@@ -1954,6 +1953,8 @@ extern "C" int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, u
     }
     const size_t m_copies = m.put(wv.copies, 16);
     m_copy = put_owner_map(m, wv.copy_first);
+    const uint32_t no_timeouts = 0;
+    const size_t m_timeouts = m.put(&no_timeouts, sizeof no_timeouts);
     if (m.bytes.size() > meta_cap)
         return fail(DG_E_TOO_LARGE, "filter tables (%zu bytes) and intermediates (%zu bytes) exceed the %zu-byte static scratch",
                     m.bytes.size(), mid_bound, kStaticScratchBytes);
@@ -1973,8 +1974,9 @@ extern "C" int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, u
     for (int st = 0; st < 4; ++st) {
         if (wv.passes[st].empty()) continue;
         const ConvPass* passes = (const ConvPass*)(scratch + m_passes[st]);
-        if (st & 1) launch_conv_v(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], s);
-        else launch_conv_h(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], s);
+        unsigned int* const timeouts = (unsigned int*)(scratch + m_timeouts);
+        if (st & 1) launch_conv_v(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], timeouts, s);
+        else launch_conv_h(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], timeouts, s);
     }
     if (!wv.copies.empty()) launch_copy((const CopyJob*)(scratch + m_copies), map_at(m_copy), s);
     CU(cudaGetLastError());

@@ -190,11 +190,11 @@ inline uint32_t copy_tiles(const CopyJob& j) {  // tiles start at multiples of 1
     return (uint32_t)(((uint64_t)j.row_bytes * j.rows + 15 + kCopyTileBytes - 1) / kCopyTileBytes);
 }
 
-// the passes that take the tensor-core kernel (fast == 2) come first in `passes` and own tiles [0, mma_tiles)
-void launch_conv_h(const ConvPass* passes, OwnerMap map, const uint32_t* tables, uint32_t mma_tiles, cudaStream_t s);
-// CTAs of the tensor-core horizontal pass that ran out of patience waiting for a copy since the library was loaded
-unsigned int read_conv_timeouts(cudaStream_t s);
-void launch_conv_v(const ConvPass* passes, OwnerMap map, const uint32_t* tables, uint32_t mma_tiles, cudaStream_t s);
+// the passes that take the tensor-core kernel (fast == 2) come first in `passes` and own tiles [0, mma_tiles).  timeouts: counts
+// the CTAs of those kernels that ran out of patience waiting for a copy (never expected; it exists so that a wait can be
+// bounded without the failure going unnoticed).
+void launch_conv_h(const ConvPass* passes, OwnerMap map, const uint32_t* tables, uint32_t mma_tiles, unsigned int* timeouts, cudaStream_t s);
+void launch_conv_v(const ConvPass* passes, OwnerMap map, const uint32_t* tables, uint32_t mma_tiles, unsigned int* timeouts, cudaStream_t s);
 void launch_copy(const CopyJob* jobs, OwnerMap map, cudaStream_t s);
 constexpr uint32_t kAlphaTilePx = 2048;  // pixels per CTA of the alpha multiply / divide kernel
 void launch_alpha(const AlphaJob* jobs, OwnerMap map, cudaStream_t s);

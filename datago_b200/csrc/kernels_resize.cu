@@ -460,27 +460,9 @@ __global__ void __launch_bounds__(kConvHThreads) k_conv_h(const ConvPass* passes
     else conv_h_rows<1, false>(p, tb, x, y0);
 }
 
-// Counts CTAs of the tensor-core pass that gave up waiting for a copy (never expected; the counter exists so that a wait
-// can be bounded without the failure going unnoticed).  One counter per device.
-static __device__ unsigned int g_conv_timeouts;
-static unsigned int* conv_timeouts() {
-    static unsigned int* ptr[64] = {nullptr};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) dev = 0;
-    if (!ptr[dev]) cudaGetSymbolAddress(reinterpret_cast<void**>(&ptr[dev]), g_conv_timeouts);
-    return ptr[dev];
-}
-unsigned int read_conv_timeouts(cudaStream_t s) {
-    unsigned int v = 0;
-    cudaMemcpyFromSymbolAsync(&v, g_conv_timeouts, sizeof v, 0, cudaMemcpyDeviceToHost, s);
-    cudaStreamSynchronize(s);
-    return v;
-}
-
 // Horizontal passes of one stage: the tensor-core passes come first in `passes` and own tiles [0, mma_tiles) of the map,
 // the others the rest.
-void launch_conv_h(const ConvPass* passes, OwnerMap map, const uint32_t* tables, uint32_t mma_tiles, cudaStream_t s) {
+void launch_conv_h(const ConvPass* passes, OwnerMap map, const uint32_t* tables, uint32_t mma_tiles, unsigned int* timeouts, cudaStream_t s) {
     if (!map.total) return;
     if (mma_tiles) {
         static bool configured[64] = {false};
@@ -491,7 +473,7 @@ void launch_conv_h(const ConvPass* passes, OwnerMap map, const uint32_t* tables,
             cudaFuncSetAttribute(k_conv_h_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HMmaSmem));
             configured[dev] = true;
         }
-        k_conv_h_mma<<<mma_tiles, kHMmaThreads, sizeof(HMmaSmem), s>>>(passes, map, tables, conv_timeouts());
+        k_conv_h_mma<<<mma_tiles, kHMmaThreads, sizeof(HMmaSmem), s>>>(passes, map, tables, timeouts);
     }
     if (map.total > mma_tiles) k_conv_h<<<map.total - mma_tiles, kConvHThreads, 0, s>>>(passes, map, tables, mma_tiles);
 }
@@ -804,7 +786,7 @@ __global__ void __launch_bounds__(kConvVThreads) k_conv_v(const ConvPass* passes
 }
 
 // Vertical passes of one stage: the tensor-core passes come first in `passes` and own tiles [0, mma_tiles) of the map.
-void launch_conv_v(const ConvPass* passes, OwnerMap map, const uint32_t* tables, uint32_t mma_tiles, cudaStream_t s) {
+void launch_conv_v(const ConvPass* passes, OwnerMap map, const uint32_t* tables, uint32_t mma_tiles, unsigned int* timeouts, cudaStream_t s) {
     if (!map.total) return;
     if (mma_tiles) {
         static bool configured[64] = {false};
@@ -815,7 +797,7 @@ void launch_conv_v(const ConvPass* passes, OwnerMap map, const uint32_t* tables,
             cudaFuncSetAttribute(k_conv_v_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(VMmaSmem));
             configured[dev] = true;
         }
-        k_conv_v_mma<<<mma_tiles, kVMmaThreads, sizeof(VMmaSmem), s>>>(passes, map, tables, conv_timeouts());
+        k_conv_v_mma<<<mma_tiles, kVMmaThreads, sizeof(VMmaSmem), s>>>(passes, map, tables, timeouts);
     }
     if (map.total > mma_tiles) k_conv_v<<<map.total - mma_tiles, kConvVThreads, 0, s>>>(passes, map, tables, mma_tiles);
 }
