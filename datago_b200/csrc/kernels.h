@@ -16,6 +16,39 @@ struct OwnerMap {
 
 constexpr uint32_t kSms = 148;  // of a B200
 
+#ifdef __CUDACC__
+// ---- launches that overlap the end of the kernel before them --------------------------------------------------------------
+// A batch is a chain of ten or more kernels, many of them shorter than 20 us when the batch is small.  All of them are launched with
+// programmatic stream serialisation: a kernel may start while the one before it ends.  Rules:
+//   * every thread calls wait_for_previous() before it reads what an earlier kernel wrote, before it writes anything, and before
+//     it returns (so the end of a kernel implies the end of all kernels before it);
+//   * before that it may read what the host uploaded: descriptors, owner maps, code, quantisation and filter tables;
+//   * pointers to what earlier kernels wrote pass through from_previous() after the wait where they are read with __ldg(), which
+//     the compiler may otherwise move ahead of the wait.
+//   * the reconstruction and resize kernels call let_next_start() first when they have few CTAs: the next kernel then fetches its
+//     descriptors and weights meanwhile.  Large grids do not: it would only hand over places that other streams can use.  Nor do
+//     the entropy kernels, whose successors want much shared memory and sit in it until the slowest stream is through (256 files:
+//     3 810 us a pass against 3 571; one photo 314 against 280).
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() {
+    if (gridDim.x <= 2 * kSms) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class T> __device__ __forceinline__ T* from_previous(T* p) {
+    asm volatile("" : "+l"(p));
+    return p;
+}
+template <class... P, class... A>
+void launch_after(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute overlap;
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t at{};
+    at.gridDim = dim3(grid); at.blockDim = dim3(block); at.dynamicSmemBytes = smem; at.stream = s;
+    at.attrs = &overlap; at.numAttrs = 1;
+    cudaLaunchKernelEx(&at, kernel, P(args)...);
+}
+#endif
+
 // ---- entropy decoding: work splits (see kernels_huff.cu) ------------------------------------------------------------------
 constexpr uint32_t kUnstuffTile = 4096;  // bytes of an entropy-coded segment per CTA of the unstuffing kernels
 // bits of an unstuffed stream per thread of the value decoder; the short form while all threads are resident at once

@@ -223,6 +223,7 @@ __device__ __forceinline__ Unit classify(const uint8_t* in, uint32_t i0, uint32_
 // (The CTAs behind the last tile make the code tables of the wave: work of the same length, for which a launch of its own
 // would be too much.)
 __global__ void __launch_bounds__(kUnstuffThreads) k_unstuff_count(JpegWave w) {
+    wait_for_previous();
     if (blockIdx.x >= w.us_tiles.total) {
         const uint32_t k = blockIdx.x - w.us_tiles.total;
         const uint2 ids = w.table_pairs[k];
@@ -262,6 +263,7 @@ __global__ void __launch_bounds__(kUnstuffThreads) k_unstuff_write(JpegWave w) {
     __syncthreads();
     const uint32_t i0 = tile * kUnstuffTile + tid * 16;
     Unit u = classify(w.raw + d.raw_off, i0, d.raw_len);
+    wait_for_previous();
     // what the tiles before this one kept
     uint32_t kept = 0, rst = 0;
     bool ended = false;
@@ -337,8 +339,8 @@ __global__ void __launch_bounds__(kUnstuffThreads) k_unstuff_write(JpegWave w) {
 
 void launch_unstuff(const JpegWave& w, cudaStream_t s) {
     if (!w.n) return;
-    k_unstuff_count<<<w.us_tiles.total + w.n_pairs, kUnstuffThreads, 0, s>>>(w);
-    k_unstuff_write<<<w.us_tiles.total, kUnstuffThreads, 0, s>>>(w);
+    launch_after(k_unstuff_count, w.us_tiles.total + w.n_pairs, kUnstuffThreads, 0, s, w);
+    launch_after(k_unstuff_write, w.us_tiles.total, kUnstuffThreads, 0, s, w);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -398,7 +400,7 @@ __device__ __forceinline__ void load_tables(const JpegWave& w, const JpegDesc& d
         const uint32_t luma = d.hs * d.vs, slot = (uint32_t)tid < luma ? 0u : (uint32_t)tid == luma ? slot1 : slot2;
         const uint32_t at = smem_addr(tab0) + slot * 2 * (uint32_t)sizeof(Tab);
         const Tab* const tabs = reinterpret_cast<const Tab*>(w.codes + (size_t)(slot == 0 ? p0 : slot == slot1 ? p1 : p2) * kCodeTablesBytes + which);
-        mcu[tid] = McuBlock{at, __ldg(&tabs[0].off), __ldg(&tabs[1].off), smem_addr(&mcu[(uint32_t)tid + 1 == d.bpm ? 0 : tid + 1])};
+        mcu[tid] = McuBlock{at, tabs[0].off, tabs[1].off, smem_addr(&mcu[(uint32_t)tid + 1 == d.bpm ? 0 : tid + 1])};
     }
 }
 
@@ -554,7 +556,9 @@ __global__ void __launch_bounds__(kGuessThreads) k_huff_guess(JpegWave w) {
     const uint32_t o = owner_of(w.guess_ctas, blockIdx.x);
     const uint32_t img = w.spec_list[o];
     const JpegDesc& d = w.descs[img];
-    const uint32_t span = w.guess_span, bpm = d.bpm, nspans = guess_spans(bpm, span), cell0 = (blockIdx.x - __ldg(w.guess_ctas.first + o)) * nspans * span;
+    const uint32_t bpm = d.bpm;
+    wait_for_previous();
+    const uint32_t span = w.guess_span, nspans = guess_spans(bpm, span), cell0 = (blockIdx.x - __ldg(w.guess_ctas.first + o)) * nspans * span;
     const uint32_t total = w.us_len[img] * 8u, ncell = (total + CELL - 1) / CELL;
     if (cell0 >= ncell) return;
     unsigned char* const tab0 = guess_smem;
@@ -641,17 +645,18 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t img = w.spec_list[blockIdx.x];
     const JpegDesc& d = w.descs[img];
+    wait_for_previous();
     load_tables<SyncTab>(w, d, sh.mcu, tab0, (uint32_t)offsetof(CodeTables, sync), tid, T);
     copy_commit();
     const uint32_t us_len = w.us_len[img], total = us_len * 8u;
     const uint32_t ncell = (total + CELL - 1) / CELL;
-    const GlobalSource source{reinterpret_cast<const uint32_t*>(w.us + d.us_off), (us_len + 3) / 4 + 2};
+    const GlobalSource source{from_previous(reinterpret_cast<const uint32_t*>(w.us + d.us_off)), (us_len + 3) / 4 + 2};
     const CellOrder order(ncell, T, MIXED);
     const uint32_t run = order.run, kbeg = min(tid * run, ncell), kend = min(kbeg + run, ncell);
     // of this thread's cell k: [(k - kbeg) * step]
     const uint32_t step = order.mixed ? T : 1, cand_step = order.mixed ? T : CellOrder::kPieces, piece = order.piece_step();
     uint2* const recs = w.cells + d.cell_off + 1 + tid * (order.mixed ? 1 : run);  // while linking: block start, state << 12 | blocks that start in the cell
-    const uint4* const cand = w.cand + (size_t)d.cell_off * CellOrder::kPieces + tid * (order.mixed ? 1 : run * CellOrder::kPieces);
+    const uint4* const cand = from_previous(w.cand) + (size_t)d.cell_off * CellOrder::kPieces + tid * (order.mixed ? 1 : run * CellOrder::kPieces);
     const bool active = kbeg < kend;
     const uint32_t mcu0 = smem_addr(&sh.mcu[0]);
     uint32_t found = 0;  // blocks that start in this thread's cells
@@ -791,15 +796,19 @@ struct ValueMisc {
     McuBlock mcu[6];
 };
 
-// Shared memory of the value decoder: [ValueMisc | ... | tables].  The caller waits for the copies and the barrier.
+// Shared memory of the value decoder: [ValueMisc | ... | tables].
 template <int T>
-__device__ __forceinline__ void value_setup(const JpegWave& w, const JpegDesc& d, ValueMisc<T>& sh, unsigned char* tab0) {
+__device__ __forceinline__ void value_setup(ValueMisc<T>& sh) {
     const int tid = threadIdx.x;
-    load_tables<ValueTab>(w, d, sh.mcu, tab0, (uint32_t)offsetof(CodeTables, value), tid, T);
-    copy_commit();
     if (tid < 64) sh.place[tid] = place_of<T>(tid);
 #pragma unroll
     for (int r = 0; r < 8; ++r) sh.block[r * T + tid] = make_uint4(0, 0, 0, 0);
+}
+// ... and its tables; the caller waits for the copies and the barrier.
+template <int T>
+__device__ __forceinline__ void value_tables(const JpegWave& w, const JpegDesc& d, ValueMisc<T>& sh, unsigned char* tab0) {
+    load_tables<ValueTab>(w, d, sh.mcu, tab0, (uint32_t)offsetof(CodeTables, value), threadIdx.x, T);
+    copy_commit();
 }
 
 // Decodes blocks [blk, end) of an image from bit p on.  src: the image's stream, see SharedSource.
@@ -920,13 +929,15 @@ __global__ void __launch_bounds__(T) k_huff_write(JpegWave w) {
     const uint32_t img = w.spec_list[o];
     const JpegDesc& d = w.descs[img];
     const uint32_t cell0 = (blockIdx.x - __ldg(w.write_ctas.first + o)) * T;
+    const int tid = threadIdx.x;
+    value_setup<T>(sh);
+    wait_for_previous();
     const uint32_t total = w.us_len[img] * 8u;
     const uint32_t ncell = (total + CELL - 1) / CELL;
     if (cell0 >= ncell) return;
-    const int tid = threadIdx.x;
     // (no further than the stream and its padding reach)
     Staged<CELL>::copy(stage, w.us + d.us_off, cell0, (int)min((uint32_t)(T + Staged<CELL>::kRowsBehind), ncell - cell0 + Staged<CELL>::kRowsPadded), tid, T);
-    value_setup<T>(w, d, sh, tab0);
+    value_tables<T>(w, d, sh, tab0);
     const uint32_t k = cell0 + tid;
     const CellOrder order(ncell, w.chain_threads, w.mixed);
     const uint2* recs = w.cells + d.cell_off;
@@ -962,6 +973,8 @@ __global__ void __launch_bounds__(T) k_huff_restart(JpegWave w) {
     const JpegDesc& d = w.descs[img];
     const uint32_t k0 = (blockIdx.x - __ldg(w.restart_ctas.first + o)) * T;
     const int tid = threadIdx.x;
+    value_setup<T>(sh);
+    wait_for_previous();
     const uint32_t found = w.seg_found[img], us_len = w.us_len[img], k = k0 + tid;
     if (k0 == 0 && tid == 0 && found != d.nseg) atomicOr(w.status + d.item, kStBadMarker);
     const uint32_t* seg = w.seg_start + d.seg_off;
@@ -984,7 +997,7 @@ __global__ void __launch_bounds__(T) k_huff_restart(JpegWave w) {
         for (uint32_t i = tid; i * 16 < hi - lo; i += T) copy16(dst + i * 16, us + lo + (size_t)i * 16);
         copy_commit();
     }
-    value_setup<T>(w, d, sh, tab0);
+    value_tables<T>(w, d, sh, tab0);
     copy_wait<0>();
     __syncthreads();
     const bool mine = k < have;
@@ -995,7 +1008,7 @@ __global__ void __launch_bounds__(T) k_huff_restart(JpegWave w) {
     if (staged) {
         n = decode_blocks<T, true>(SharedSource{smem_addr(stage) - lo}, b0 * 8u, blk0, end, b1 * 8u, b1 * 8u, 0u, d, sh, w.huff, coef, info, err);
     } else {
-        const GlobalSource source{reinterpret_cast<const uint32_t*>(us), (us_len + 3) / 4 + 2};
+        const GlobalSource source{from_previous(reinterpret_cast<const uint32_t*>(us)), (us_len + 3) / 4 + 2};
         n = decode_blocks<T, true>(source, b0 * 8u, blk0, end, b1 * 8u, b1 * 8u, 0u, d, sh, w.huff, coef, info, err);
     }
     if (n < end - blk0) err |= kStTruncated;
@@ -1147,8 +1160,10 @@ __global__ void __launch_bounds__(kDcThreads) k_dc(JpegWave w) {
     const uint32_t nblocks = d.nblocks;
     const uint32_t* diff = w.diff + d.block_off;
     uint32_t* info = w.info + d.block_off;
+    const uint32_t bpm = d.bpm;
+    wait_for_previous();
     const auto blocks = [&] { return min(w.cells[d.cell_off].y, nblocks); };
-    switch (d.bpm) {
+    switch (bpm) {
         case 1: dc_image<1>(diff, info, nblocks, blocks, sh); break;
         case 3: dc_image<3>(diff, info, nblocks, blocks, sh); break;
         case 4: dc_image<4>(diff, info, nblocks, blocks, sh); break;
@@ -1159,6 +1174,7 @@ __global__ void __launch_bounds__(kDcThreads) k_dc(JpegWave w) {
 // Stage-by-stage parity tests look at whole coefficient blocks: fills in the rows the class left out and the DC term.
 __global__ void __launch_bounds__(256) k_whole_blocks(JpegWave w, uint32_t nblocks) {
     const uint32_t i = blockIdx.x * 256 + threadIdx.x, blk = i >> 3, row = i & 7u;
+    wait_for_previous();
     if (blk >= nblocks) return;
     const uint32_t v = w.info[blk];
     uint4* const at = reinterpret_cast<uint4*>(w.coef) + (size_t)blk * 8 + row;
@@ -1203,22 +1219,22 @@ void launch_guess(const JpegWave& w, cudaStream_t s) {
     // the cell before the first, the cells, and what a block may run over
     const size_t rows = 1 + (size_t)guess_spans(1, w.guess_span) * w.guess_span + Staged<CELL>::kRowsBehind;
     const size_t smem = rows * Staged<CELL>::kPitch + w.max_pairs * 2 * sizeof(SyncTab);
-    if (w.mixed) k_huff_guess<CELL, true><<<w.guess_ctas.total, kGuessThreads, smem, s>>>(w);
-    else k_huff_guess<CELL, false><<<w.guess_ctas.total, kGuessThreads, smem, s>>>(w);
+    if (w.mixed) launch_after(k_huff_guess<CELL, true>, w.guess_ctas.total, kGuessThreads, smem, s, w);
+    else launch_after(k_huff_guess<CELL, false>, w.guess_ctas.total, kGuessThreads, smem, s, w);
 }
 
 template <int CELL>
 void launch_chain(const JpegWave& w, cudaStream_t s) {
     const size_t tables = w.max_pairs * 2 * sizeof(SyncTab);
-    if (w.chain_threads == 256) k_huff_chain<256, CELL, false><<<w.n_spec, 256, sizeof(ChainMisc<256>) + tables, s>>>(w);
-    else if (w.mixed) k_huff_chain<1024, CELL, true><<<w.n_spec, 1024, sizeof(ChainMisc<1024>) + tables, s>>>(w);
-    else k_huff_chain<1024, CELL, false><<<w.n_spec, 1024, sizeof(ChainMisc<1024>) + tables, s>>>(w);
+    if (w.chain_threads == 256) launch_after(k_huff_chain<256, CELL, false>, w.n_spec, 256, sizeof(ChainMisc<256>) + tables, s, w);
+    else if (w.mixed) launch_after(k_huff_chain<1024, CELL, true>, w.n_spec, 1024, sizeof(ChainMisc<1024>) + tables, s, w);
+    else launch_after(k_huff_chain<1024, CELL, false>, w.n_spec, 1024, sizeof(ChainMisc<1024>) + tables, s, w);
 }
 
 template <int T, int CELL>
 void launch_write(const JpegWave& w, cudaStream_t s) {
     const size_t smem = sizeof(ValueMisc<T>) + (size_t)(T + Staged<CELL>::kRowsBehind) * Staged<CELL>::kPitch + w.max_pairs * 2 * sizeof(ValueTab);
-    k_huff_write<T, CELL><<<w.write_ctas.total, T, smem, s>>>(w);
+    launch_after(k_huff_write<T, CELL>, w.write_ctas.total, T, smem, s, w);
 }
 template <int CELL>
 void launch_write(const JpegWave& w, cudaStream_t s) {
@@ -1228,19 +1244,21 @@ void launch_write(const JpegWave& w, cudaStream_t s) {
 
 template <int T>
 void launch_restart(const JpegWave& w, cudaStream_t s) {
-    k_huff_restart<T><<<w.restart_ctas.total, T, sizeof(ValueMisc<T>) + kRestartStage<T> + w.max_pairs * 2 * sizeof(ValueTab), s>>>(w);
+    launch_after(k_huff_restart<T>, w.restart_ctas.total, T, sizeof(ValueMisc<T>) + kRestartStage<T> + w.max_pairs * 2 * sizeof(ValueTab), s, w);
 }
 
 // CTAs per image: eight while they all run at once; with many images that only adds CTAs (1024 files: passes of 3170 us with two to four,
 // see the commit for one).
 void launch_dc(const JpegWave& w, cudaStream_t s) {
     const uint32_t size = w.n_spec <= kSms / 4 ? 8 : w.n_spec <= kSms ? 2 : 1;
-    cudaLaunchAttribute cluster;
-    cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim.x = size; cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeClusterDimension;
+    attrs[0].val.clusterDim.x = size; attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
+    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t at{};
     at.gridDim = dim3(w.n_spec * size); at.blockDim = dim3(kDcThreads); at.stream = s;
-    at.attrs = &cluster; at.numAttrs = 1;
+    at.attrs = attrs; at.numAttrs = 2;
     cudaLaunchKernelEx(&at, k_dc, w);
 }
 
@@ -1278,7 +1296,7 @@ void launch_huff_restart(const JpegWave& w, cudaStream_t s) {
 }
 
 void launch_whole_blocks(const JpegWave& w, uint32_t nblocks, cudaStream_t s) {
-    if (nblocks) k_whole_blocks<<<(nblocks + 31) / 32, 256, 0, s>>>(w, nblocks);
+    if (nblocks) launch_after(k_whole_blocks, (nblocks + 31) / 32, 256, 0, s, w, nblocks);
 }
 
 }  // namespace dg

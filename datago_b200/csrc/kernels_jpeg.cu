@@ -196,7 +196,11 @@ __global__ void __launch_bounds__(kIdctThreads, DG_IDCT_MIN_CTAS) k_idct(JpegWav
     // (One 16-byte load per lane and row straight from global memory makes every instruction touch 32 lines.)
     __shared__ __align__(16) uint4 s_coef[kIdctThreads / 32][256];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t v = __ldg(w.info + g);
+    const uint32_t img = owner_of(w.blocks, g);
+    const JpegDesc& d = w.descs[img];
+    let_next_start();
+    wait_for_previous();
+    const uint32_t v = w.info[g];
     const int cls = (int)((v >> 16) & 3u);
     const uint32_t nrows = class_rows(cls);
     {
@@ -213,8 +217,6 @@ __global__ void __launch_bounds__(kIdctThreads, DG_IDCT_MIN_CTAS) k_idct(JpegWav
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    const uint32_t img = owner_of(w.blocks, g);
-    const JpegDesc& d = w.descs[img];
     const uint32_t blk = g - (uint32_t)d.block_off;
     const bool valid = local < count && blk < d.nblocks;  // (images start at multiples of eight blocks)
     const uint32_t mcu = blk / d.bpm, k = blk - mcu * d.bpm;
@@ -236,7 +238,7 @@ __global__ void __launch_bounds__(kIdctThreads, DG_IDCT_MIN_CTAS) k_idct(JpegWav
 }
 
 void launch_idct(const JpegWave& w, uint32_t first, uint32_t count, cudaStream_t s) {
-    if (count) k_idct<<<(count + kIdctThreads - 1) / kIdctThreads, kIdctThreads, 0, s>>>(w, first, count);
+    if (count) launch_after(k_idct, (count + kIdctThreads - 1) / kIdctThreads, kIdctThreads, 0, s, w, first, count);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -340,7 +342,7 @@ constexpr int kCTileRows = 8 * (int)kColorMcuRows + 2;  // chroma rows of a 4:2:
 // Warp q loads tile rows q, q + 8, ... of both components; a lane loads word `lane` and, for two lanes, word 32 + lane.
 // Two steps, both by every thread of the CTA (256), with a __syncthreads() after each: chroma_tile_fetch, chroma_tile_edges.
 template <int ROWS>
-__device__ __forceinline__ void chroma_tile_fetch(uint8_t (&s_c)[2][ROWS][kCTileCols], const JpegWave& w, const JpegDesc& d,
+__device__ __forceinline__ void chroma_tile_fetch(uint8_t (&s_c)[2][ROWS][kCTileCols], const uint8_t* planes, const JpegDesc& d,
                                                   int tx, int ty, int dh) {
     constexpr int kCTileRows = ROWS;
     const int lane = threadIdx.x & 31, rowi = threadIdx.x >> 5;
@@ -348,8 +350,8 @@ __device__ __forceinline__ void chroma_tile_fetch(uint8_t (&s_c)[2][ROWS][kCTile
     constexpr int kWords = kCTileCols / 4;  // 34
     const uint32_t cpitch = d.plane_pitch[1];
     const int wmax = (int)(cpitch / 4) - 1, w0 = cx0 / 4 - 1;
-    const uint8_t* cb_base = w.planes + d.plane_off[1];
-    const uint8_t* cr_base = w.planes + d.plane_off[2];
+    const uint8_t* cb_base = planes + d.plane_off[1];
+    const uint8_t* cr_base = planes + d.plane_off[2];
 #pragma unroll
     for (int rr = 0; rr < (kCTileRows + 7) / 8; ++rr) {
         const int r = rowi + 8 * rr;
@@ -383,9 +385,9 @@ __device__ __forceinline__ void chroma_tile_edges(uint8_t (&s_c)[2][ROWS][kCTile
     }
 }
 
-__device__ __forceinline__ void load_chroma_tile(uint8_t (&s_c)[2][kCTileRows][kCTileCols], const JpegWave& w, const JpegDesc& d,
+__device__ __forceinline__ void load_chroma_tile(uint8_t (&s_c)[2][kCTileRows][kCTileCols], const uint8_t* planes, const JpegDesc& d,
                                                  int tx, int ty, int dw, int dh) {
-    chroma_tile_fetch(s_c, w, d, tx, ty, dh);
+    chroma_tile_fetch(s_c, planes, d, tx, ty, dh);
     __syncthreads();
     chroma_tile_edges(s_c, tx, dw);
     __syncthreads();
@@ -429,7 +431,10 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
     __shared__ __align__(16) uint8_t s_c[2][kCTileRows][kCTileCols];
     __shared__ uint32_t s_img;
     if (threadIdx.x == 0) s_img = owner_of(w.color_tiles, first_tile + blockIdx.x);
+    let_next_start();
+    wait_for_previous();
     __syncthreads();
+    const uint8_t* const planes = from_previous(w.planes);
     const uint32_t img = s_img;
     const JpegDesc& d = w.descs[img];
     const uint32_t tile = first_tile + blockIdx.x - w.color_tiles.first[img];
@@ -441,7 +446,7 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
     const int y_base = (int)ty * 8 * vs * (int)kColorMcuRows;
     const int nsteps = vs * (int)kColorMcuRows;  // a thread converts rows rowi, rowi + 8, ... of the tile
     uint8_t* out = w.out + d.out_off;
-    const uint8_t* yp = w.planes + d.plane_off[0];
+    const uint8_t* yp = planes + d.plane_off[0];
     const uint32_t ypitch = d.plane_pitch[0];
 
     if (d.ncomp == 1) {  // grayscale: copy the real extent of the luma plane
@@ -460,7 +465,7 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
     const int dw = (W + hs - 1) / hs, dh = (H + vs - 1) / vs;
     const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, x < W);
     if (hs == 2 && vs == 2 && dw > 2) {
-        load_chroma_tile(s_c, w, d, (int)tx, (int)ty, dw, dh);
+        load_chroma_tile(s_c, planes, d, (int)tx, (int)ty, dw, dh);
         if (x >= W) return;
         const int cl = lane * 4 + 4;  // s_c column of this thread's first chroma sample (a word boundary)
         const int npx = min(8, W - x);
@@ -499,8 +504,8 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
         for (int k = 0; k < nsteps; ++k) {
             const int y = y_base + rowi + 8 * k;
             if (y >= H) break;
-            const uint2 b = __ldg(reinterpret_cast<const uint2*>(w.planes + d.plane_off[1] + (size_t)y * d.plane_pitch[1] + x));
-            const uint2 r = __ldg(reinterpret_cast<const uint2*>(w.planes + d.plane_off[2] + (size_t)y * d.plane_pitch[2] + x));
+            const uint2 b = __ldg(reinterpret_cast<const uint2*>(planes + d.plane_off[1] + (size_t)y * d.plane_pitch[1] + x));
+            const uint2 r = __ldg(reinterpret_cast<const uint2*>(planes + d.plane_off[2] + (size_t)y * d.plane_pitch[2] + x));
             int32_t cbv[8], crv[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -527,7 +532,7 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
             int32_t cbv[8], crv[8];
 #pragma unroll
             for (int comp = 1; comp <= 2; ++comp) {
-                const uint8_t* row = w.planes + d.plane_off[comp] + (size_t)y * d.plane_pitch[comp];
+                const uint8_t* row = planes + d.plane_off[comp] + (size_t)y * d.plane_pitch[comp];
                 const uint32_t q = __ldg(reinterpret_cast<const uint32_t*>(row + c0));
                 int32_t t[6];
                 t[0] = __ldg(row + max(c0 - 1, 0));
@@ -554,8 +559,8 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
         return;
     }
     // remaining samplings (4:4:0, chroma planes at most two samples wide): one pixel at a time
-    const ChromaPlane cbp{w.planes + d.plane_off[1], d.plane_pitch[1], dh, hs, vs};
-    const ChromaPlane crp{w.planes + d.plane_off[2], d.plane_pitch[2], dh, hs, vs};
+    const ChromaPlane cbp{planes + d.plane_off[1], d.plane_pitch[1], dh, hs, vs};
+    const ChromaPlane crp{planes + d.plane_off[2], d.plane_pitch[2], dh, hs, vs};
 #pragma unroll 1
     for (int k = 0; k < nsteps; ++k) {
         const int y = y_base + rowi + 8 * k;
@@ -573,7 +578,7 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
 }
 
 void launch_color(const JpegWave& w, uint32_t first_tile, uint32_t count, cudaStream_t s) {
-    if (count) k_color<<<count, kColorThreads, 0, s>>>(w, first_tile);
+    if (count) launch_after(k_color, count, kColorThreads, 0, s, w, first_tile);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -597,7 +602,9 @@ __global__ void __launch_bounds__(kIdctThreads, DG_IDCT_MIN_CTAS) k_idct_chroma(
     const uint32_t ql = q - __ldg(w.fused_chroma.first + o);
     const uint32_t mcu = ql >> 1, which = ql & 1u;
     const uint32_t blk = (uint32_t)d.block_off + mcu * 6u + 4u + which;  // this lane's block in the coefficient array
-    const uint32_t v = __ldg(w.info + blk);
+    let_next_start();
+    wait_for_previous();
+    const uint32_t v = w.info[blk];
     const int cls = (int)((v >> 16) & 3u);
     const uint32_t nrows = class_rows(cls);
     // Lanes 2j and 2j + 1 hold the Cb and Cr block of one MCU: 256 consecutive bytes.  Step i copies the rows of blocks
@@ -628,7 +635,7 @@ __global__ void __launch_bounds__(kIdctThreads, DG_IDCT_MIN_CTAS) k_idct_chroma(
 }
 
 void launch_idct_chroma(const JpegWave& w, uint32_t first, uint32_t count, cudaStream_t s) {
-    if (count) k_idct_chroma<<<(count + kIdctThreads - 1) / kIdctThreads, kIdctThreads, 0, s>>>(w, first, count);
+    if (count) launch_after(k_idct_chroma, (count + kIdctThreads - 1) / kIdctThreads, kIdctThreads, 0, s, w, first, count);
 }
 
 constexpr int kFusedThreads = 64 * (int)kFusedMcuRows;
@@ -722,6 +729,8 @@ __global__ void __launch_bounds__(kFusedThreads, DG_FUSED_MIN_CTAS) k_luma_color
     const TileInfo& t = sm.info;  // read where needed: a copy in registers would not fit beside the butterfly
 
     if (threadIdx.x == 0) fill_tile_info(sm.info, w, first_tile + blockIdx.x);
+    let_next_start();
+    wait_for_previous();
     __syncthreads();
     // ---- inputs.  Luma coefficients: warp q owns MCU row q / 2 of the tile and MCUs 8 (q % 2) .. + 7 of it, lane l block
     //      l % 4 of MCU l / 4.  MCUs outside the image are replaced by the nearest one inside: their results land in tile
@@ -732,7 +741,7 @@ __global__ void __launch_bounds__(kFusedThreads, DG_FUSED_MIN_CTAS) k_luma_color
         const uint32_t mrow = warp >> 1, half = warp & 1u;
         const uint32_t myc = min(t.ty * kFusedMcuRows + mrow, t.mcuy - 1), mx0 = t.tx * 16 + half * 8;
         const uint32_t mcu_row = myc * t.mcux;
-        v = __ldg(t.info + (size_t)(mcu_row + min(mx0 + (lane >> 2), t.mcux - 1)) * 6 + (lane & 3u)) & 0x3FFFFu;
+        v = *(t.info + (size_t)(mcu_row + min(mx0 + (lane >> 2), t.mcux - 1)) * 6 + (lane & 3u)) & 0x3FFFFu;
         queue_chroma_tile(sm, t);
         const uint32_t nrows = class_rows((int)(v >> 16));
         const int16_t* row_base = t.coef + (size_t)mcu_row * 384;
@@ -860,7 +869,7 @@ void launch_luma_color(const JpegWave& w, uint32_t first_tile, uint32_t count, c
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     std::call_once(done[dev], [] { cudaFuncSetAttribute(k_luma_color, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FusedSmem)); });
-    k_luma_color<<<count, kFusedThreads, sizeof(FusedSmem), s>>>(w, first_tile);
+    launch_after(k_luma_color, count, kFusedThreads, sizeof(FusedSmem), s, w, first_tile);
 }
 
 }  // namespace dg

@@ -291,11 +291,13 @@ __global__ void __launch_bounds__(kHMmaThreads, kHMmaCtasPerSm) k_conv_h_mma(con
     };
     if (warp >= kHMmaConsumers / 32) {
         // ---- the copying thread
-        if (lane != 0) return;
+        if (lane != 0) { let_next_start(); wait_for_previous(); return; }
         const void* map = pg.tmap;
         // the descriptor sits in global memory that earlier batches may have used for other descriptors
         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
         const int32_t x_word = strip_lo >> 2;
+        let_next_start();
+        wait_for_previous();
         RingPlace at;
         for (uint32_t c = 0; c < nchunks && !gave_up; ++c, at.next(nstage)) {
             const uint32_t slot = at.slot;
@@ -346,6 +348,8 @@ __global__ void __launch_bounds__(kHMmaThreads, kHMmaCtasPerSm) k_conv_h_mma(con
             bfr[ks][0] = hi[0]; bfr[ks][1] = hi[1]; bfr[ks][2] = lo[0]; bfr[ks][3] = lo[1];
         }
     }
+    let_next_start();
+    wait_for_previous();
     // The chunk loop is compiled once per number of k steps, so that the multiplies of a chunk form one straight run
     // of loads and tensor-core instructions.
     auto consume = [&](auto ks_tag) {
@@ -444,6 +448,9 @@ __device__ void conv_h_rows_any(const ConvPass& p, const Table& tb, uint32_t x, 
 }
 
 __global__ void __launch_bounds__(kConvHThreads) k_conv_h(const ConvPass* passes, OwnerMap map, const uint32_t* tables, uint32_t first_tile) {
+    let_next_start();
+    wait_for_previous();
+    passes = from_previous(passes);  // (their sources are earlier kernels' results)
     const uint32_t tile_index = first_tile + blockIdx.x;
     const ConvPass& p = passes[owner_of_tile(map, tile_index)];
     const uint32_t tile = tile_index - p.tile_first;
@@ -473,9 +480,9 @@ void launch_conv_h(const ConvPass* passes, OwnerMap map, const uint32_t* tables,
             cudaFuncSetAttribute(k_conv_h_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HMmaSmem));
             configured[dev] = true;
         }
-        k_conv_h_mma<<<mma_tiles, kHMmaThreads, sizeof(HMmaSmem), s>>>(passes, map, tables, timeouts);
+        launch_after(k_conv_h_mma, mma_tiles, kHMmaThreads, sizeof(HMmaSmem), s, passes, map, tables, timeouts);
     }
-    if (map.total > mma_tiles) k_conv_h<<<map.total - mma_tiles, kConvHThreads, 0, s>>>(passes, map, tables, mma_tiles);
+    if (map.total > mma_tiles) launch_after(k_conv_h, map.total - mma_tiles, kConvHThreads, 0, s, passes, map, tables, mma_tiles);
 }
 
 // ---- vertical pass -----------------------------------------------------------------------------------------------------
@@ -659,9 +666,11 @@ __global__ void __launch_bounds__(kVMmaThreads, kVMmaCtasPerSm) k_conv_v_mma(con
     };
     if (warp >= kVMmaConsumers / 32) {
         // ---- the copying thread: per chunk `boxes` copies of box_rows rows x 64 bytes, one below the other
-        if (lane != 0) return;
+        if (lane != 0) { let_next_start(); wait_for_previous(); return; }
         const void* tmap = pg.tmap;
         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmap) : "memory");
+        let_next_start();
+        wait_for_previous();
         RingPlace at;
         for (uint32_t c = 0; c < nchunks && !gave_up; ++c, at.next(nstage)) {
             const uint32_t slot = at.slot;
@@ -707,6 +716,8 @@ __global__ void __launch_bounds__(kVMmaThreads, kVMmaCtasPerSm) k_conv_v_mma(con
             bfr[ks][0] = hi[0]; bfr[ks][1] = hi[1]; bfr[ks][2] = lo[0]; bfr[ks][3] = lo[1];
         }
     }
+    let_next_start();
+    wait_for_previous();
     const uint32_t out_base = (uint32_t)__cvta_generic_to_shared(&sm.out[warp][0][0]);
     constexpr uint32_t kOutPitch = kVMmaChunk + 16;
     auto consume = [&](auto ks_tag) {
@@ -776,6 +787,9 @@ __global__ void __launch_bounds__(kConvVThreads) k_conv_v(const ConvPass* passes
     __shared__ uint32_t s_pass;
     const uint32_t tile_index = first_tile + blockIdx.x;
     if (threadIdx.x == 0) s_pass = owner_of_tile(map, tile_index);
+    let_next_start();
+    wait_for_previous();
+    passes = from_previous(passes);  // (their sources are earlier kernels' results)
     __syncthreads();
     const ConvPass& p = passes[s_pass];
     const uint32_t tile = tile_index - p.tile_first;
@@ -797,9 +811,9 @@ void launch_conv_v(const ConvPass* passes, OwnerMap map, const uint32_t* tables,
             cudaFuncSetAttribute(k_conv_v_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(VMmaSmem));
             configured[dev] = true;
         }
-        k_conv_v_mma<<<mma_tiles, kVMmaThreads, sizeof(VMmaSmem), s>>>(passes, map, tables, timeouts);
+        launch_after(k_conv_v_mma, mma_tiles, kVMmaThreads, sizeof(VMmaSmem), s, passes, map, tables, timeouts);
     }
-    if (map.total > mma_tiles) k_conv_v<<<map.total - mma_tiles, kConvVThreads, 0, s>>>(passes, map, tables, mma_tiles);
+    if (map.total > mma_tiles) launch_after(k_conv_v, map.total - mma_tiles, kConvVThreads, 0, s, passes, map, tables, mma_tiles);
 }
 
 // ---- plain copies (identity payloads, integral crops without any filtering, raw pixels handed through) ----------------
@@ -807,6 +821,9 @@ void launch_conv_v(const ConvPass* passes, OwnerMap map, const uint32_t* tables,
 // with funnel shifts (payloads of odd sizes start anywhere), one division per 16 bytes.  Pieces that cross a source row go
 // byte by byte, and so do the first and the last ones of a job, whose aligned words may reach outside the source.
 __global__ void __launch_bounds__(256) k_copy(const CopyJob* jobs, OwnerMap map) {
+    let_next_start();
+    wait_for_previous();
+    jobs = from_previous(jobs);  // (their sources are earlier kernels' results)
     const uint32_t ji = owner_of_tile(map, blockIdx.x);
     const CopyJob& j = jobs[ji];
     uint8_t* const dst = j.dst;
@@ -842,13 +859,16 @@ __global__ void __launch_bounds__(256) k_copy(const CopyJob* jobs, OwnerMap map)
 }
 
 void launch_copy(const CopyJob* jobs, OwnerMap map, cudaStream_t s) {
-    if (map.total) k_copy<<<map.total, 256, 0, s>>>(jobs, map);
+    if (map.total) launch_after(k_copy, map.total, 256, 0, s, jobs, map);
 }
 
 // ---- alpha pre-multiplication and division (what fast_image_resize does around a convolution of U8x2 / U8x4 images) ----
 // multiply: colour = ((colour * alpha + 128) + ((colour * alpha + 128) >> 8)) >> 8
 // divide:   colour = min(255, (colour * recip + 2^15) >> 16), recip = ((255 * 2^17) / alpha + 1) >> 1, 0 for alpha 0
 __global__ void __launch_bounds__(256) k_alpha(const AlphaJob* jobs, OwnerMap map) {
+    let_next_start();
+    wait_for_previous();
+    jobs = from_previous(jobs);  // (their sources are earlier kernels' results)
     const AlphaJob& j = jobs[owner_of_tile(map, blockIdx.x)];
     const uint32_t base = (blockIdx.x - j.tile_first) * kAlphaTilePx, npx = j.width * j.rows, C = j.channels;
     const bool words = C == 4 && ((reinterpret_cast<uintptr_t>(j.src) | reinterpret_cast<uintptr_t>(j.dst) | j.src_pitch | j.dst_pitch) & 3u) == 0;
@@ -884,7 +904,7 @@ __global__ void __launch_bounds__(256) k_alpha(const AlphaJob* jobs, OwnerMap ma
 }
 
 void launch_alpha(const AlphaJob* jobs, OwnerMap map, cudaStream_t s) {
-    if (map.total) k_alpha<<<map.total, 256, 0, s>>>(jobs, map);
+    if (map.total) launch_after(k_alpha, map.total, 256, 0, s, jobs, map);
 }
 
 // ---- convert_to_rgb8 (datago src/image_processing.rs:163-186) -------------------------------------------------------
@@ -893,6 +913,9 @@ void launch_alpha(const AlphaJob* jobs, OwnerMap map, cudaStream_t s) {
 // operation rounded once (the _rn intrinsics keep the compiler from fusing a multiply into an add), in the order the
 // `image` crate's Pixel::blend uses, so that the result equals a CPU evaluation of the same expression bit for bit.
 __global__ void __launch_bounds__(256) k_to_rgb8(const ToRgbJob* jobs, OwnerMap map) {
+    let_next_start();
+    wait_for_previous();
+    jobs = from_previous(jobs);  // (their sources are earlier kernels' results)
     const uint32_t ji = owner_of_tile(map, blockIdx.x);
     const ToRgbJob& j = jobs[ji];
     const uint32_t base = (blockIdx.x - j.tile_first) * kToRgbTilePx;
@@ -927,7 +950,7 @@ __global__ void __launch_bounds__(256) k_to_rgb8(const ToRgbJob* jobs, OwnerMap 
 }
 
 void launch_to_rgb8(const ToRgbJob* jobs, OwnerMap map, cudaStream_t s) {
-    if (map.total) k_to_rgb8<<<map.total, 256, 0, s>>>(jobs, map);
+    if (map.total) launch_after(k_to_rgb8, map.total, 256, 0, s, jobs, map);
 }
 
 }  // namespace dg
