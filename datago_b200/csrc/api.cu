@@ -103,6 +103,8 @@ struct dg_ctx {
     cudaStream_t stream = nullptr;   // everything the caller can observe is ordered on this stream
     cudaStream_t stream2 = nullptr;  // odd waves of a batch run here, concurrently with the even ones
     cudaStream_t aux[2] = {nullptr, nullptr};  // per lane: the restart-interval decoder runs beside the speculative one
+    cudaStream_t up = nullptr;                 // inputs of larger batches, copied while the rest is being staged (see dg_batch_create)
+    std::vector<cudaEvent_t> events;           // idle ones, for the waves' inputs
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaEvent_t ev_aux_go[2] = {nullptr, nullptr}, ev_aux_done[2] = {nullptr, nullptr};
     bool own_stream = false;
@@ -173,6 +175,7 @@ static int ctx_create(int device, const dg_image_config* cfg, void* stream, bool
         c->own_stream = true;
     }
     if (cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&c->up, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->aux[0], cudaStreamNonBlocking) != cudaSuccess ||
@@ -205,6 +208,9 @@ extern "C" void dg_ctx_destroy(dg_ctx* c) {
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     cudaStreamSynchronize(c->stream2);
+    cudaStreamSynchronize(c->up);
+    cudaStreamDestroy(c->up);
+    for (cudaEvent_t e : c->events) cudaEventDestroy(e);
     for (BlockCache* cache : {&c->dev, &c->pin, &c->dev_meta, &c->pin_meta}) cache->clear();
     cudaEventDestroy(c->ev_fork);
     cudaEventDestroy(c->ev_join);
@@ -436,6 +442,9 @@ struct dg_batch {
     uint64_t h2d = 0, d2h = 0;
     uint32_t launches = 0;
     bool uploaded = false, ran = false;
+    // Inputs that dg_batch_create has queued on ctx->up already, and arrived[k]: those of wave k are on the device.
+    bool queued = false, in_flight = false;
+    std::vector<cudaEvent_t> arrived;
     bool counted = false;    // its items have been added to the context's counters
     std::vector<StageEvent> events;
     float stage_ms[DG_STAGE_COUNT] = {0};
@@ -810,6 +819,16 @@ static void plan_resize(Planner& pl, WavePlan& wv, const dg_plan& p, uint32_t C,
         add_copy(src + (size_t)ra * src_pitch + (size_t)ca * C, src_pitch, tw * C, th);
 }
 
+// The pool's threads have no device of their own: makes `device` the current one of whoever calls.
+static bool pool_device(int device) {
+    static thread_local int bound = -1;
+    if (bound != device && cudaSetDevice(device) == cudaSuccess) bound = device;
+    return bound == device;
+}
+
+// input bytes from which on a batch is copied to the device while it is staged
+constexpr size_t kQueueBytes = (size_t)2 << 20;
+
 // worst-case scratch of the intermediates of one image's resize
 static size_t resize_mid_bound(const dg_plan& p, uint32_t C) {
     if (p.identity) return 0;
@@ -832,8 +851,16 @@ template <typename F> static void parallel_items(int n, F&& fn) {
     HostPool::get().run((size_t)std::max(n, 0), [&fn](size_t i) { fn((int)i); }, 16);
 }
 
+// Until the copies that dg_batch_create queued have run; a batch whose kernels have run has waited for them.
+static void await_inputs(dg_batch* b) {
+    if (b->in_flight && !b->ran) cudaStreamSynchronize(b->ctx->up);
+    b->in_flight = false;
+}
+
 static int abandon(dg_batch* b, int rc) {
     dg_ctx* ctx = b->ctx;
+    await_inputs(b);
+    for (cudaEvent_t e : b->arrived) ctx->events.push_back(e);
     ctx->dev.release(b->blk_persist);
     ctx->dev_meta.release(b->blk_meta);
     ctx->dev.release(b->blk_scratch);
@@ -1211,8 +1238,7 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
                 if (it.status || it.wave < 0) return;
                 // encoding a tensor map is a driver call and wants a current context, which the pool's threads do not
                 // have by themselves
-                static thread_local int bound_device = -1;
-                if (bound_device != ctx->device) { if (cudaSetDevice(ctx->device) != cudaSuccess) { pl.tmap_failed = true; return; } bound_device = ctx->device; }
+                if (!pool_device(ctx->device)) { pl.tmap_failed = true; return; }
                 WavePlan& part = parts[k];
                 const uint8_t* src = it.is_jpeg ? kBaseS + wv.off_decoded + it.decoded_off : baseP + b->off_rawin + it.raw_in_off;
                 uint8_t* dst = baseP + b->off_out + it.pipe_off;
@@ -1336,52 +1362,111 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
     memset(b->h_pin, 0, b->off_blob);
     {
         // One list of copies for everything: pieces of about 128 KB, or one filter table each, so that a few large inputs
-        // spread over the host threads as well as many small ones.
-        constexpr size_t kPiece = (size_t)128 << 10;
-        struct Piece { uint8_t* dst; const uint8_t* src; size_t len; uint32_t rows, pitch; };  // rows == 0: one flat run of len bytes
+        // spread over the host threads as well as many small ones.  Pieces belong to parts: what goes to the device in one copy,
+        // the metadata, then per wave its files and its raw pixels, kPart bytes or one image at a time.
+        constexpr size_t kPiece = (size_t)128 << 10, kPart = (size_t)4 << 20;
+        struct Piece { uint8_t* dst; const uint8_t* src; size_t len; uint32_t rows, pitch; const FilterTable* table; uint32_t part; };  // rows == 0: one flat run of len bytes
+        struct Part { uint8_t* dst; const uint8_t* src; size_t len; uint32_t wave, pieces; };
         std::vector<Piece> pieces;
-        size_t bytes = b->meta.bytes.size();
-        auto flat = [&](uint8_t* dst, const uint8_t* src, size_t len) {
-            bytes += len;
-            for (size_t o = 0; o < len; o += kPiece) pieces.push_back({dst + o, src + o, std::min(len - o, kPiece), 0, 0});
+        std::vector<Part> parts;
+        size_t bytes = 0;
+        auto add = [&](Piece p) {
+            p.part = (uint32_t)parts.size() - 1;
+            ++parts.back().pieces;
+            bytes += p.table ? p.table->words() * 4 : p.rows ? (size_t)p.rows * p.len : p.len;
+            pieces.push_back(p);
         };
-        size_t off = 0;  // in the blob: same order as the descriptors' raw_off
-        for (WavePlan& wv : b->waves)
-            for (int i = wv.first_item; i < wv.last_item; ++i) {
+        auto flat = [&](uint8_t* dst, const uint8_t* src, size_t len) {
+            for (size_t o = 0; o < len; o += kPiece) add({dst + o, src + o, std::min(len - o, kPiece), 0, 0, nullptr, 0});
+        };
+        parts.push_back({b->d_meta, b->h_meta, b->meta_total, 0, 0});
+        flat(b->h_meta, b->meta.bytes.data(), b->meta.bytes.size());
+        uint32_t* const pool = reinterpret_cast<uint32_t*>(b->h_meta + b->m_tables);
+        for (const auto& e : pl.table_list) add({(uint8_t*)(pool + e.first), nullptr, 0, 0, 0, e.second, 0});
+        // The two regions of the block, [status | files] and raw pixels, are laid out wave by wave: a part is what follows the last.
+        size_t files_sent = 0, raw_sent = b->off_rawin, off = b->off_blob;
+        auto open_part = [&](size_t wave) { parts.push_back({nullptr, nullptr, 0, (uint32_t)wave, 0}); };
+        auto close_part = [&](size_t& from, size_t to) {
+            Part& p = parts.back();
+            p.dst = b->d_persist + from; p.src = b->h_pin + from; p.len = to - from;
+            from = to;
+        };
+        for (size_t wi = 0; wi < b->waves.size(); ++wi) {
+            const WavePlan& wv = b->waves[wi];
+            open_part(wi);
+            for (int i = wv.first_item; i < wv.last_item; ++i) {  // in the order of the descriptors' raw_off
                 const ItemPlan& it = b->items[i];
                 if (it.status || !it.is_jpeg || it.wave_local < 0) continue;
                 const JpegHeader& h = *it.hdr;
-                uint8_t* dst = b->h_pin + b->off_blob + off;
+                uint8_t* dst = b->h_pin + off;
                 const size_t slot = align_up(h.scan_len, 16) + 16;
+                if (off - files_sent >= kPart) { close_part(files_sent, off); open_part(wi); }
                 flat(dst, items[i].data + h.scan_off, h.scan_len);
                 memset(dst + h.scan_len, 0, slot - h.scan_len);
                 off += slot;
             }
-        for (int i = 0; i < n && rawin; ++i) {
-            const ItemPlan& it = b->items[i];
-            if (it.status || it.is_jpeg || !b->raw_src[i]) continue;
-            const size_t row = (size_t)it.w * it.c;
-            uint8_t* dst = b->h_pin + b->off_rawin + it.raw_in_off;
-            if (it.src_pitch == row) flat(dst, b->raw_src[i], row * it.h);
-            else {  // rows are re-pitched on the way: a piece is a run of whole rows
-                const size_t rows_per = std::max<size_t>(1, kPiece / row);
-                bytes += row * it.h;
-                for (size_t y = 0; y < it.h; y += rows_per)
-                    pieces.push_back({dst + y * it.src_pitch, b->raw_src[i] + y * row, row, (uint32_t)std::min<size_t>(rows_per, it.h - y), it.src_pitch});
+            close_part(files_sent, off);
+            open_part(wi);
+            size_t raw_end = raw_sent;
+            for (int i = wv.first_item; i < wv.last_item && rawin; ++i) {
+                const ItemPlan& it = b->items[i];
+                if (it.status || it.is_jpeg || !b->raw_src[i]) continue;
+                const size_t row = (size_t)it.w * it.c, at = b->off_rawin + it.raw_in_off;
+                uint8_t* dst = b->h_pin + at;
+                if (at - raw_sent >= kPart) { close_part(raw_sent, at); open_part(wi); }
+                if (it.src_pitch == row) flat(dst, b->raw_src[i], row * it.h);
+                else {  // rows are re-pitched on the way: a piece is a run of whole rows
+                    const size_t rows_per = std::max<size_t>(1, kPiece / row);
+                    for (size_t y = 0; y < it.h; y += rows_per)
+                        add({dst + y * it.src_pitch, b->raw_src[i] + y * row, row, (uint32_t)std::min<size_t>(rows_per, it.h - y), it.src_pitch, nullptr, 0});
+                }
+                raw_end = at + align_up((size_t)it.src_pitch * it.h, 256);
             }
+            close_part(raw_sent, raw_end);
         }
-        flat(b->h_meta, b->meta.bytes.data(), b->meta.bytes.size());
-        uint32_t* const pool = reinterpret_cast<uint32_t*>(b->h_meta + b->m_tables);
-        const auto& list = pl.table_list;
-        bytes += pl.table_words_total * 4;
-        const size_t np = pieces.size();
-        // below half a megabyte waking the other threads takes longer than the copies
-        HostPool::get().run(np + list.size(), [&](size_t k) {
-            if (k >= np) { list[k - np].second->pack(pool + list[k - np].first); return; }
+        const auto stage = [&](size_t k) {
             const Piece& pc = pieces[k];
+            if (pc.table) { pc.table->pack((uint32_t*)pc.dst); return; }
             if (!pc.rows) { memcpy(pc.dst, pc.src, pc.len); return; }
             for (uint32_t y = 0; y < pc.rows; ++y) memcpy(pc.dst + (size_t)y * pc.pitch, pc.src + (size_t)y * pc.len, pc.len);
-        }, bytes < ((size_t)1 << 19) ? np + list.size() : 1);
+        };
+        // Larger batches: whoever stages the last piece of a part queues its copy, so that the link is busy from the first part on and
+        // a wave's kernels start when its own inputs are there.  Small ones wait for dg_batch_upload, whose two copies on the
+        // batch's own stream are the shorter way.
+        if (bytes < kQueueBytes || b->waves.empty()) {
+            // below half a megabyte waking the other threads takes longer than the copies
+            HostPool::get().run(pieces.size(), stage, bytes < ((size_t)1 << 19) ? pieces.size() : 1);
+        } else {
+            for (size_t wi = 0; wi < b->waves.size(); ++wi) {
+                cudaEvent_t e = nullptr;
+                if (!ctx->events.empty()) { e = ctx->events.back(); ctx->events.pop_back(); }
+                else if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return abandon(b, fail(DG_E_CUDA, "creating an event failed"));
+                b->arrived.push_back(e);
+            }
+            std::mutex mu;  // guards the next three
+            std::vector<uint32_t> left(parts.size()), left_in_wave(b->waves.size(), 0);  // pieces of a part, parts of a wave
+            cudaError_t failed = cudaSuccess;
+            for (size_t k = 0; k < parts.size(); ++k) { left[k] = parts[k].pieces; ++left_in_wave[parts[k].wave]; }
+            b->in_flight = true;
+            const auto queue = [&](size_t k) {
+                const Part& p = parts[k];
+                cudaError_t e = p.len ? cudaMemcpyAsync(p.dst, p.src, p.len, cudaMemcpyHostToDevice, ctx->up) : cudaSuccess;
+                if (e == cudaSuccess && --left_in_wave[p.wave] == 0) e = cudaEventRecord(b->arrived[p.wave], ctx->up);
+                if (e != cudaSuccess) failed = e;
+            };
+            for (size_t k = 0; k < parts.size(); ++k) if (!left[k]) queue(k);
+            std::atomic<size_t> next{0};
+            HostPool::get().run((size_t)HostPool::get().threads(), [&](size_t) {
+                (void)pool_device(ctx->device);  // (copies that fail are noticed below)
+                for (size_t k; (k = next.fetch_add(1)) < pieces.size();) {
+                    stage(k);
+                    std::lock_guard<std::mutex> lock(mu);
+                    if (--left[pieces[k].part] == 0) queue(pieces[k].part);
+                }
+            }, 1);
+            if (failed != cudaSuccess) return abandon(b, fail(DG_E_CUDA, "queueing the inputs failed: %s", cudaGetErrorString(failed)));
+            b->queued = true;
+        }
     }
     b->raw_src.clear();  // caller memory is not needed after this call
     *out = b;
@@ -1393,14 +1478,14 @@ extern "C" int dg_batch_upload(dg_batch* b) {
     dg_ctx* ctx = b->ctx;
     std::lock_guard<std::mutex> lock(ctx->mu);
     CU(cudaSetDevice(ctx->device));
-    b->h2d = 0;
-    // status zeros + compressed blob + raw pixel inputs (contiguous in the staging buffer and on the device)
+    // status zeros + compressed blob + raw pixel inputs (contiguous in the staging buffer and on the device), metadata
     const size_t head = b->off_rawin + align_up(b->rawin_bytes, 256);
-    CU(cudaMemcpyAsync(b->d_persist, b->h_pin, head, cudaMemcpyHostToDevice, ctx->stream));
-    b->h2d += head;
-    // metadata
-    CU(cudaMemcpyAsync(b->d_meta, b->h_meta, b->meta_total, cudaMemcpyHostToDevice, ctx->stream));
-    b->h2d += b->meta_total;
+    b->h2d = head + b->meta_total;
+    if (!b->queued) {
+        CU(cudaMemcpyAsync(b->d_persist, b->h_pin, head, cudaMemcpyHostToDevice, ctx->stream));
+        CU(cudaMemcpyAsync(b->d_meta, b->h_meta, b->meta_total, cudaMemcpyHostToDevice, ctx->stream));
+    }
+    b->queued = false;  // another call copies again
     b->uploaded = true;
     return DG_OK;
 }
@@ -1463,6 +1548,10 @@ static int batch_run_locked(dg_batch* b) {
         // the scratch block belongs to the lane, so in one-stream mode an odd wave must wait for nothing extra:
         // stream order already serialises the waves
         s = (two_lanes && (wi & 1)) ? ctx->stream2 : ctx->stream;
+        if (b->in_flight) {  // (the metadata came with the first wave's inputs)
+            if (wi) CU(cudaStreamWaitEvent(s, b->arrived[0], 0));
+            CU(cudaStreamWaitEvent(s, b->arrived[wi], 0));
+        }
         if (!wv.descs.empty()) {
             JpegWave w;
             memset(&w, 0, sizeof w);
@@ -1711,6 +1800,7 @@ extern "C" int dg_batch_sync(dg_batch* b) {
         b->d2h += (size_t)b->n * 4;
     }
     CU(cudaStreamSynchronize(ctx->stream));
+    await_inputs(b);
     landed(b);
     if (b->ran) {
         // the tensor-core resize passes bound their waits for asynchronous copies; a wait that ran out left garbage behind
@@ -1821,6 +1911,8 @@ extern "C" void dg_batch_destroy(dg_batch* b) {
     std::lock_guard<std::mutex> lock(ctx->mu);
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    await_inputs(b);
+    for (cudaEvent_t e : b->arrived) ctx->events.push_back(e);
     landed(b);
     for (StageEvent& se : b->events) { cudaEventDestroy(se.a); cudaEventDestroy(se.b); }
     ctx->dev.release(b->blk_persist);

@@ -134,3 +134,32 @@ def test_colour_rows_at_every_alignment(sub):
     for data, (st, out, _) in zip(datas, ctx().process(datas)):
         assert st == 0
         assert_same(out, oracle.jpeg_decode(data), str(out.shape))
+
+
+@pytest.mark.parametrize("n", [1, 3, 40])
+def test_inputs_copied_while_they_are_staged(n, monkeypatch):
+    # about 0.4 to 16 MB of files and re-pitched raw pixels in one wave and in many: below 2 MB the upload copies, above it
+    # the pieces are queued as they are staged.  A batch may be dropped before its upload, uploaded again, and run again.
+    cfg = dict(crop_and_resize=True, default_image_size=224, downsampling_ratio=16, min_aspect_ratio=0.5, max_aspect_ratio=2.0)
+    rng = np.random.default_rng(350)
+    files = [jpeg(rng, w, h, q=95, noise=8.0) for w, h in [(640, 480), (333, 222)]]
+    raw = rng.integers(0, 256, (301, 401, 3), dtype=np.uint8)
+    want = [oracle.crop_and_resize(cfg, oracle.jpeg_decode(f))[0] for f in files] + [oracle.crop_and_resize(cfg, raw)[0]]
+    items = (files + [raw]) * n
+    monkeypatch.setenv("DATAGO_B200_WAVE_MB", "16")
+    c = dg.Context(0, cfg)
+    try:
+        c.batch(items).close()
+        with c.batch(items) as b, c.batch(items[::-1]) as other:
+            b.upload(); other.upload(); b.run(); other.run()
+            outs, others = b.download(), other.download()
+            b.sync(); other.sync()
+            for i in range(len(items)):
+                assert_same(outs[i], want[i % 3], str(i))
+                assert_same(others[i], want[2 - i % 3], str(i))
+            b.upload(); b.run(); b.run()
+            outs = b.download(); b.sync()
+            for i in range(len(items)):
+                assert_same(outs[i], want[i % 3], str(i))
+    finally:
+        c.close()
