@@ -999,7 +999,11 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         }
         size_t n_waves = std::max<size_t>(1, std::max((total_coef + ctx->wave_bytes - 1) / ctx->wave_bytes,
                                                       (total_big + 2 * ctx->wave_bytes - 1) / (2 * ctx->wave_bytes)));
-        if (n_waves == 1 && total_coef + total_big > ((size_t)1 << 30)) n_waves = 2;
+        // (one wave / two, us a pass: 48 files of 1 Mpixel, 150 MB of coefficients, decoded 394 / 357; 150 files 835 / 740; 100 files
+        // into buckets 957 / 836; 8 pairs of 4:4:4 and mask, 290 MB, 686 / 641; 48 files into buckets, 133 MB, 502 / 515.  Three
+        // and more: 790 for the pairs, 3 770 instead of 3 570 for 256 files of 5 Mbit.)
+        const bool kept = (flags & DG_BATCH_KEEP_COEFFICIENTS) != 0;  // dg_batch_debug looks into single waves
+        if (n_waves == 1 && (total_coef + total_big > ((size_t)1 << 30) || (total_coef > ((size_t)144 << 20) && !kept))) n_waves = 2;
         const size_t coef_cap = total_coef / n_waves + 1, big_cap = total_big / n_waves + 1;
         WavePlan* wv = nullptr;
         size_t coef_bytes = 0, big_bytes = 0;
@@ -1073,10 +1077,10 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
             for (size_t k = 0; k < built.size(); ++k)
                 if ((int)(ctx->fused_path && fused_decode(built[k].ncomp, built[k].hs, built[k].vs, built[k].width)) == pass) order.push_back(k);
         // While a thread per cell of 512 bits and block of the MCU fits the chip at once, the length of a thread's way is what
-        // counts: short cells (synchronisation + values of one photo 173 us with cells of 1024 bits, 122 with 512; 32 web
-        // images 193 and 118).  Beyond that, less work in all counts more (8 files of 4:4:4, 75 Mbit: a pass 0.84 ms with
-        // 512, 0.80 with 1024), and with several times as many threads, spans of cells as well (256 files, 1.2 Gbit: 1005 us
-        // for single cells, 817 with four in a span; the 4:4:4 files: 52 and 94 us).
+        // counts: short cells (synchronisation + values, when a symbol took half as long again: one photo 173 us with cells of 1024
+        // bits, 122 with 512; 32 web images 193 and 118).  Beyond that, less work in all counts more (8 files of 4:4:4, 75 Mbit: a
+        // pass 0.84 ms with 512, 0.80 with 1024), and with several times as many threads, spans of cells as well (256 files, 1.2
+        // Gbit: 1005 us for single cells, 817 with four in a span; the 4:4:4 files: 52 and 94 us).
         uint64_t guess_bits = 0;
         for (const JpegDesc& d : built)
             if (!d.restart) guess_bits += (uint64_t)d.raw_len * 8 * d.bpm;
