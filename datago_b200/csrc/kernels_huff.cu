@@ -363,9 +363,15 @@ void launch_unstuff(const JpegWave& w, cudaStream_t s) {
 //     candidates through it, then compares what its left neighbour hands over with what it assumed, and so on until
 //     nothing changes; states nobody guessed are then decoded, all at once, and it goes on.  Chains of wrong phases are 5
 //     to 15 cells long: resolving them by decoding, with one guess per cell, took 12 rounds of a cell each for a photo of
-//     2.7 Mbit (276 us in a cluster of eight CTAs; 28 + 54 us for these two kernels).
+//     2.7 Mbit (276 us in a cluster of eight CTAs; 19 + 34 us for these two kernels now).
 //  k_huff_write  one thread per cell decodes the blocks that start in it, values included, collects a block in shared
 //     memory and writes it out whole: DC difference and class to diff[], the rows the class covers to coef[].
+//
+//  What bounds all three is the way of one lane: a chain of dependent instructions per symbol, with three to five warps per
+//  scheduler to hide it, or one where there is little work.  So a step is few instructions (SyncTab, ValueTab), none of them a
+//  jump (SyncLane::run_to, decode_blocks), and what it needs next is on its way before (Cursor, SyncLane::nx).  Before / after
+//  these three, us: values 43 / 21 (one thumbnail), 51 / 28 (one photo), 1 340 / 890 (256 files of 5 Mbit); candidates 19 / 15
+//  (thumbnail), 58 / 50 (8 files of 4:4:4), 789 / 624 (256 files); restart segments 732 / 530 (512 files of 0.4 Mbit).
 // ---------------------------------------------------------------------------------------------------------------
 namespace {
 
