@@ -755,11 +755,11 @@ static void plan_resize(Planner& pl, WavePlan& wv, const dg_plan& p, uint32_t C,
         const bool guarded = caller_owned_src && s >= src && s < src + (size_t)src_pitch * h;
         if (horizontal) {
             cp.fast = 1;
-            if (guarded) { cp.guard_lo = src; cp.guard_hi = src + (size_t)w * h * C; }
-            else if (pl.ctx->hmma && (((uintptr_t)s | spitch) & 15) == 0 && hmma_fits(*T, t0, out_w, C, origin, &cp.box_pieces)) {
+            // (a tensor map covers whole rows of the image and nothing else, so it may read memory that is not the library's)
+            if (pl.ctx->hmma && (((uintptr_t)s | spitch) & 15) == 0 && hmma_fits(*T, t0, out_w, C, origin, &cp.box_pieces)) {
                 cp.fast = 2;
                 if (!encode_source_map(cp)) pl.tmap_failed = true;
-            }
+            } else if (guarded) { cp.guard_lo = src; cp.guard_hi = src + (size_t)w * h * C; }
         } else {
             const uintptr_t bits = (uintptr_t)s | (uintptr_t)d | spitch | dpitch;
             cp.fast = (bits & 15) == 0 && (uint32_t)T->window <= kVFastMaxWindow && (size_t)align_up((size_t)out_w * C, 16) <= spitch &&
@@ -1967,6 +1967,7 @@ extern "C" int dg_copy_to_host(dg_ctx* ctx, void* dst, const void* src, uint64_t
 namespace {
 
 constexpr size_t kStaticScratchBytes = (size_t)32 << 20;
+constexpr size_t kStaticCopyBytes = (size_t)2 << 20, kStaticCopyOut = (size_t)3 << 19;  // see dg_resize_device_static
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
 // In host code `g_static_scratch` is only a handle for the runtime, not an address a kernel can use; the device
@@ -2012,13 +2013,36 @@ extern "C" int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, u
     if (mid_bound + 65536 > kStaticScratchBytes)
         return fail(DG_E_TOO_LARGE, "image needs %zu bytes of intermediates; the static scratch holds %zu in total", mid_bound, kStaticScratchBytes);
     unsigned char* mid_base = scratch + (kStaticScratchBytes - mid_bound);
-    const size_t meta_cap = kStaticScratchBytes - mid_bound;
+    size_t meta_cap = kStaticScratchBytes - mid_bound;
 
     Planner pl{ctx, nullptr};
     WavePlan wv;
     size_t mid_used = 0;
-    plan_resize(pl, wv, plan, channels, device_src, w * channels, device_dst, mid_base, &mid_used, true);
+    // The tensor-core passes want rows that start on 16-byte boundaries.  Where the caller's do not, a copy with padded rows goes
+    // into the array first, if there is room for it and the horizontal pass is long enough to pay for it: long windows on a large
+    // image (1 413 x 1 121 pixels to 512: a call 58 us without the copy, 48 with; 2 813 x 2 241: 89 and 76).  With shorter
+    // windows, or so much output that the plain pass has enough CTAs, it is the better one (to 1024: 58 and 61, 94 and 99).
+    const size_t row = (size_t)w * channels, padded = align_up(row, 16), copy_bytes = align_up(padded * h, 256);
+    // no less than what the descriptors and the filter tables take: 2 * (6 * in / out + 3) + 8 bytes per output of a resize to `out`,
+    // 24 of a half-pixel shift
+    const size_t meta_room = 65536 + 64 * ((size_t)w + h);
+    const bool pays = row * h >= kStaticCopyBytes && row >= 32 && w >= 2 * plan.new_w && (size_t)plan.new_w * h <= kStaticCopyOut;
+    const bool copied = pays && ctx->hmma && !plan.identity && ((uintptr_t)device_src | row) % 16 != 0 && copy_bytes + meta_room <= meta_cap;
+    if (copied) {
+        meta_cap -= copy_bytes;
+        unsigned char* const copy = scratch + meta_cap;
+        plan_resize(pl, wv, plan, channels, copy, (uint32_t)padded, device_dst, mid_base, &mid_used);
+        // the padding of a row is the start of the next one; the last row comes without
+        CopyJob j;
+        j.src = device_src; j.dst = copy; j.src_pitch = (uint32_t)row; j.row_bytes = (uint32_t)padded; j.rows = h - 1; j.tile_first = 0;
+        if (j.rows) wv.copies.push_back(j);  // (a row is longer than its padding)
+        j.src += row * (h - 1); j.dst += padded * (h - 1); j.row_bytes = (uint32_t)row; j.rows = 1;
+        wv.copies.push_back(j);
+    } else {
+        plan_resize(pl, wv, plan, channels, device_src, w * channels, device_dst, mid_base, &mid_used, true);
+    }
     if (mid_used > mid_bound) return fail(DG_E_TOO_LARGE, "internal: intermediates exceed their bound");
+    if (pl.tmap_failed) return fail(DG_E_CUDA, "cuTensorMapEncodeTiled rejected the source of a resize pass");
     Meta m;
     std::vector<uint32_t> packed(pl.table_words_total);
     pl.pack_tables(packed.data());
@@ -2067,6 +2091,7 @@ extern "C" int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, u
         return r;
     };
     const uint32_t* tables = (const uint32_t*)(scratch + m_tables);
+    if (copied) launch_copy((const CopyJob*)(scratch + m_copies), map_at(m_copy), s);
     for (int st = 0; st < 4; ++st) {
         if (wv.passes[st].empty()) continue;
         const ConvPass* passes = (const ConvPass*)(scratch + m_passes[st]);
@@ -2074,7 +2099,7 @@ extern "C" int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, u
         if (st & 1) launch_conv_v(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], timeouts, s);
         else launch_conv_h(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], timeouts, s);
     }
-    if (!wv.copies.empty()) launch_copy((const CopyJob*)(scratch + m_copies), map_at(m_copy), s);
+    if (!copied && !wv.copies.empty()) launch_copy((const CopyJob*)(scratch + m_copies), map_at(m_copy), s);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(s));  // the host-side metadata image dies with this frame
     return DG_OK;

@@ -64,6 +64,26 @@ def test_source_that_ends_where_its_allocation_could_end():
             assert np.array_equal(dst.cpu().numpy(), want), (h, w, c, lead, sentinel)
 
 
+@pytest.mark.parametrize("shape,lead", [((1121, 1413, 3), 0), ((1121, 1413, 3), 5), ((1200, 1408, 3), 0), ((1200, 1408, 3), 16), ((1200, 1408, 3), 8),
+                                        ((2203, 1501, 1), 3), ((2801, 2803, 3), 1), ((3101, 3103, 3), 1)])
+def test_large_images_at_every_alignment(shape, lead):
+    # rows that a tensor map can describe in place, rows that are copied to padded ones first, images too small or too large for
+    # that (the last one leaves no room beside its intermediates)
+    import torch
+    ctx = dg.Context(0, CFG)
+    img = np.random.default_rng(43).integers(0, 256, shape, dtype=np.uint8)
+    (status, want, _), = ctx.process([img[:, :, 0] if shape[2] == 1 else img])
+    assert status == 0
+    n = img.size
+    for sentinel in (0, 255):
+        big = torch.full((lead + n + 64,), sentinel, dtype=torch.uint8, device="cuda")
+        big[lead:lead + n] = torch.from_numpy(img.reshape(-1)).cuda()
+        dst = torch.zeros(want.shape, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        ctx.resize_device_static(big.data_ptr() + lead, shape[1], shape[0], shape[2], dst.data_ptr())
+        assert np.array_equal(dst.cpu().numpy(), want), sentinel
+
+
 def test_identity_and_copy_only_plans():
     ctx = dg.Context(0, CFG)
     rng = np.random.default_rng(42)
