@@ -117,22 +117,21 @@ __device__ __forceinline__ uint32_t value_entry(uint32_t code, bool is_ac) {
     return (len + s) | advance_of((code >> 8) & 255u, is_ac) << 16 | (32u - s) << 27;
 }
 
-__device__ void build_tables(CodeTables& out, const HuffTable* pool, uint32_t dc_id, uint32_t ac_id, int tid, int nthreads) {
-    const HuffTable* const ac = pool + ac_id;
-    for (int side = 0; side < 2; ++side) {
-        const HuffTable* const t = pool + (side ? ac_id : dc_id);
+// One CTA per table: part 0 / 1 sync[0] / sync[1], 2 / 3 value[0] / value[1].  (One CTA for all four took 8 us, twice what the tiles
+// beside it take for an ordinary file.)
+constexpr uint32_t kTableParts = 4;
+__device__ void build_table(CodeTables& out, const HuffTable* pool, uint32_t dc_id, uint32_t ac_id, uint32_t part, int tid, int nthreads) {
+    const uint32_t side = part & 1u;
+    const HuffTable* const t = pool + (side ? ac_id : dc_id);
+    static_assert(kValueBits == kLutBits && kSyncBits == 10, "limit[0] covers ten bits");
+    if (part < 2) {
         SyncTab& st = out.sync[side];
-        ValueTab& vt = out.value[side];
-        // the first windows that no code of at most kLutBits / kSyncBits bits covers
-        uint32_t covered = 0;
-        for (int k = 0; k < (1 << kLutBits); k += 32) covered += __popc(__ballot_sync(0xFFFFFFFFu, __ldg(t->lut + k + (tid & 31)) != 0u));
-        const uint32_t vfar = covered << (16 - kLutBits), sfar = __ldg(t->limit + 0);
-        const uint32_t vnear = vfar >> (16 - kValueBits), snear = sfar >> (16 - kSyncBits);
-        static_assert(kValueBits == kLutBits && kSyncBits == 10, "limit[0] covers ten bits");
+        const HuffTable* const ac = pool + ac_id;
+        const uint32_t far = __ldg(t->limit + 0), near = far >> (16 - kSyncBits);  // the first window that no code of at most kSyncBits bits covers
         for (uint32_t i = tid; i < (uint32_t)SyncTab::kEntries; i += nthreads) {
-            const uint32_t window = i < snear ? i << (16 - kSyncBits) : min(sfar + (i - snear), 0xFFFFu);
+            const uint32_t window = i < near ? i << (16 - kSyncBits) : min(far + (i - near), 0xFFFFu);
             uint32_t c = code_at(t, window), e = sync_entry(c, side != 0);
-            if (i < snear) {
+            if (i < near) {
                 uint32_t u = e & 31u, a = (e >> 8) & 255u;
                 while (u < (uint32_t)kSyncBits && a < 64u) {
                     c = code_at(ac, (window << u) & 0xFFFFu);
@@ -145,15 +144,17 @@ __device__ void build_tables(CodeTables& out, const HuffTable* pool, uint32_t dc
             }
             st.entry[i] = i + 1 < (uint32_t)SyncTab::kEntries ? e : 0u;
         }
+        if (tid == 0) { st.off = (int32_t)near - (int32_t)far; st.huff = side ? ac_id : dc_id; st.is_ac = side; }
+    } else {
+        ValueTab& vt = out.value[side];
+        uint32_t covered = 0;  // windows of kLutBits bits that start with a code
+        for (int k = 0; k < (1 << kLutBits); k += 32) covered += __popc(__ballot_sync(0xFFFFFFFFu, __ldg(t->lut + k + (tid & 31)) != 0u));
+        const uint32_t far = covered << (16 - kLutBits), near = far >> (16 - kValueBits);
         for (uint32_t i = tid; i < (uint32_t)ValueTab::kEntries; i += nthreads) {
-            const uint32_t c = code_at(t, i < vnear ? i << (16 - kValueBits) : min(vfar + (i - vnear), 0xFFFFu));
+            const uint32_t c = code_at(t, i < near ? i << (16 - kValueBits) : min(far + (i - near), 0xFFFFu));
             vt.entry[i] = i + 1 < (uint32_t)ValueTab::kEntries && !(c >> 31) ? value_entry(c, side != 0) : 0u;
         }
-        if (tid == 0) {
-            st.off = (int32_t)snear - (int32_t)sfar; vt.off = (int32_t)vnear - (int32_t)vfar;
-            st.huff = vt.huff = side ? ac_id : dc_id;
-            st.is_ac = vt.is_ac = side;
-        }
+        if (tid == 0) { vt.off = (int32_t)near - (int32_t)far; vt.huff = side ? ac_id : dc_id; vt.is_ac = side; }
     }
 }
 
@@ -226,8 +227,8 @@ __global__ void __launch_bounds__(kUnstuffThreads) k_unstuff_count(JpegWave w) {
     wait_for_previous();
     if (blockIdx.x >= w.us_tiles.total) {
         const uint32_t k = blockIdx.x - w.us_tiles.total;
-        const uint2 ids = w.table_pairs[k];
-        build_tables(reinterpret_cast<CodeTables*>(w.codes)[k], w.huff, ids.x, ids.y, threadIdx.x, kUnstuffThreads);
+        const uint2 ids = w.table_pairs[k / kTableParts];
+        build_table(reinterpret_cast<CodeTables*>(w.codes)[k / kTableParts], w.huff, ids.x, ids.y, k % kTableParts, threadIdx.x, kUnstuffThreads);
         return;
     }
     const uint32_t o = owner_of(w.us_tiles, blockIdx.x);
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(kUnstuffThreads) k_unstuff_write(JpegWave w) {
 
 void launch_unstuff(const JpegWave& w, cudaStream_t s) {
     if (!w.n) return;
-    launch_after(k_unstuff_count, w.us_tiles.total + w.n_pairs, kUnstuffThreads, 0, s, w);
+    launch_after(k_unstuff_count, w.us_tiles.total + w.n_pairs * kTableParts, kUnstuffThreads, 0, s, w);
     launch_after(k_unstuff_write, w.us_tiles.total, kUnstuffThreads, 0, s, w);
 }
 
