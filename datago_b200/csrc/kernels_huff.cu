@@ -1254,8 +1254,8 @@ void launch_restart(const JpegWave& w, cudaStream_t s) {
     launch_after(k_huff_restart<T>, w.restart_ctas.total, T, sizeof(ValueMisc<T>) + kRestartStage<T> + w.max_pairs * 2 * sizeof(ValueTab), s, w);
 }
 
-// CTAs per image: eight while they all run at once; with many images that only adds CTAs (1024 files: passes of 3170 us with two to four,
-// see the commit for one).
+// CTAs per image: eight while they all run at once; with many images that only adds CTAs (1024 files: passes of 3 200 us with two to
+// four, 3 189 with one).
 void launch_dc(const JpegWave& w, cudaStream_t s) {
     const uint32_t size = w.n_spec <= kSms / 4 ? 8 : w.n_spec <= kSms ? 2 : 1;
     cudaLaunchAttribute attrs[2];
