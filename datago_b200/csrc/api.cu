@@ -857,6 +857,24 @@ static void await_inputs(dg_batch* b) {
     b->in_flight = false;
 }
 
+// A caller may record the context's stream into a graph.  Copies under way outside it cannot be waited for from inside, so that
+// the host waits for them.
+static bool being_captured(cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    cudaGetLastError();  // (the legacy stream while another one is being captured: it cannot be itself)
+    return false;
+}
+static cudaError_t await_inputs_outside_capture(dg_batch* b) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // of this thread: it may wait for a stream that is not captured
+    cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return e;
+    e = cudaStreamSynchronize(b->ctx->up);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaSuccess) b->in_flight = false;
+    return e;
+}
+
 static int abandon(dg_batch* b, int rc) {
     dg_ctx* ctx = b->ctx;
     await_inputs(b);
@@ -1485,7 +1503,7 @@ extern "C" int dg_batch_upload(dg_batch* b) {
     // status zeros + compressed blob + raw pixel inputs (contiguous in the staging buffer and on the device), metadata
     const size_t head = b->off_rawin + align_up(b->rawin_bytes, 256);
     b->h2d = head + b->meta_total;
-    if (!b->queued) {
+    if (!b->queued || being_captured(ctx->stream)) {  // (a graph copies the inputs whenever it is launched)
         CU(cudaMemcpyAsync(b->d_persist, b->h_pin, head, cudaMemcpyHostToDevice, ctx->stream));
         CU(cudaMemcpyAsync(b->d_meta, b->h_meta, b->meta_total, cudaMemcpyHostToDevice, ctx->stream));
     }
@@ -1541,6 +1559,7 @@ static int batch_run_locked(dg_batch* b) {
         return cudaEventRecord(b->events[ev++].b, s);
     };
     b->launches = 0;
+    if (b->in_flight && being_captured(ctx->stream)) CU(await_inputs_outside_capture(b));
     if (b->ran) CU(cudaMemsetAsync(b->d_persist + b->off_status, 0, status_bytes(b->n), s));  // of the previous run
     if (two_lanes) {
         CU(cudaEventRecord(ctx->ev_fork, ctx->stream));

@@ -1,0 +1,57 @@
+"""The batch scheduler's host side (csrc/api.cu), built against a stand-in for the CUDA runtime and the kernels: what is copied and
+when, what a call returns, and what happens while the caller's stream is being captured."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import datago_b200 as dg
+from datago_b200 import synth
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "datago_b200", "csrc")
+CFG = dict(crop_and_resize=True, default_image_size=512, downsampling_ratio=16, min_aspect_ratio=0.5, max_aspect_ratio=2.0)
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("fake") / "libbatch.so")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    sources = [os.path.join(ROOT, "tests", "fake_device.cpp")] + [os.path.join(CSRC, f) for f in ("api.cu", "feeder.cpp", "host_blocks.cpp", "host_logic.cpp", "jpeg_header.cpp")]
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-pthread", "-Wl,-Bsymbolic", "-I", os.path.join(cuda, "include"), "-x", "c++", *sources, "-o", out], check=True)
+    return out
+
+
+@pytest.fixture
+def fake(library, monkeypatch):
+    monkeypatch.setattr(dg, "library_path", lambda: library)
+    monkeypatch.setattr(dg, "_lib", None)
+    monkeypatch.delenv("DATAGO_B200_REBUILD", raising=False)
+    L = dg.lib()
+    L.fake_capture.argtypes, L.fake_timeouts.argtypes = [C.c_void_p, C.c_int], [C.c_uint]
+    L.fake_to_device.restype = L.fake_to_host.restype = C.c_uint64
+    return L
+
+
+def raw(shape):
+    return np.zeros(shape, np.uint8)
+
+
+@pytest.mark.parametrize("n", [1, 3])  # 0.4 MB of inputs: copied by upload; 3.2: queued by the time the batch exists
+@pytest.mark.parametrize("upload_inside", [False, True])
+def test_a_captured_stream_waits_for_no_event_from_outside(fake, n, upload_inside):
+    c = dg.Context(0, CFG)
+    with c.batch([raw((300 * n, 400 * n, 3))]) as b:
+        if not upload_inside:
+            b.upload()
+        fake.fake_capture(c.stream, 1)
+        before = fake.fake_to_device()
+        if upload_inside:
+            b.upload()
+            assert fake.fake_to_device() - before == b.counters()["h2d_bytes"]  # a graph holds the copies
+        b.run()
+        fake.fake_capture(c.stream, 0)
+        b.sync()
+    c.close()

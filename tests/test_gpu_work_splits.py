@@ -163,3 +163,36 @@ def test_inputs_copied_while_they_are_staged(n, monkeypatch):
                 assert_same(outs[i], want[i % 3], str(i))
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("n", [1, 40])
+@pytest.mark.parametrize("upload_inside", [False, True])
+def test_calls_recorded_into_a_graph(n, upload_inside, monkeypatch):
+    # the caller's stream is being captured when a batch is run, or uploaded and run: also a batch whose inputs are still on
+    # their way, on a stream that is not captured
+    import torch
+    rng = np.random.default_rng(351)
+    items = [jpeg(rng, w, h, q=95, rst=rst, noise=8.0) for w, h, rst in [(640, 480, 0), (333, 222, 4), (480, 640, 0)]] * n
+    want = [oracle.jpeg_decode(d) for d in items[:3]]
+    monkeypatch.setenv("DATAGO_B200_WAVE_MB", "16")
+    stream = torch.cuda.Stream()
+    c = dg.Context(0, None, stream=stream.cuda_stream)
+    try:
+        with c.batch(items) as b:
+            if not upload_inside:
+                b.upload()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+                if upload_inside:
+                    b.upload()
+                b.run()
+            with torch.cuda.stream(stream):
+                graph.replay()
+                graph.replay()
+            outs = b.download(); b.sync()
+            for i, out in enumerate(outs):
+                assert b.result(i).status == 0, i
+                assert_same(out, want[i % 3], str(i))
+            del graph
+    finally:
+        c.close()
