@@ -565,16 +565,16 @@ class Batch:
         return dict(chunks=int(out[0]), rounds=int(out[1]), subsequence_decodes=int(out[2]))
 
     def debug_coefficients(self, i):
-        """int16 [blocks, 64] coefficients of JPEG item i in scan order (single-wave batches created with
-        BATCH_KEEP_COEFFICIENTS, after sync)."""
+        """int16 [blocks, 64] coefficients of JPEG item i in scan order (batches with less than 1 GiB of intermediates, created
+        with BATCH_KEEP_COEFFICIENTS, after sync)."""
         coef, nb = C.c_void_p(), C.c_uint64()
         _check(lib().dg_batch_debug(self._h, i, C.byref(coef), C.byref(nb), None))
         raw = self.ctx.copy_to_host(coef.value, int(nb.value) * 128)
         return raw.view(np.int16).reshape(int(nb.value), 64)
 
     def debug_decoded(self, i):
-        """The full-size decoded image of JPEG item i (single-wave batches, after sync).  When a resize reads it, its
-        rows are padded to 16 bytes in device memory; the padding is dropped here."""
+        """The full-size decoded image of JPEG item i (batches with less than 1 GiB of intermediates, after sync).  When a
+        resize reads it, its rows are padded to 16 bytes in device memory; the padding is dropped here."""
         r = self.result(i)
         dec = C.c_void_p()
         _check(lib().dg_batch_debug(self._h, i, None, None, C.byref(dec)))

@@ -442,6 +442,7 @@ struct dg_batch {
     uint64_t h2d = 0, d2h = 0;
     uint32_t launches = 0;
     bool uploaded = false, ran = false;
+    bool views = false;  // dg_batch_debug answers; the batch then has at most two waves, with a scratch block each
     // Inputs that dg_batch_create has queued on ctx->up already, and arrived[k]: those of wave k are on the device.
     bool queued = false, in_flight = false;
     std::vector<cudaEvent_t> arrived;
@@ -1020,8 +1021,10 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         // (one wave / two, us a pass: 48 files of 1 Mpixel, 150 MB of coefficients, decoded 394 / 357; 150 files 835 / 740; 100 files
         // into buckets 957 / 836; 8 pairs of 4:4:4 and mask, 290 MB, 686 / 641; 48 files into buckets, 133 MB, 502 / 515.  Three
         // and more: 790 for the pairs, 3 770 instead of 3 570 for 256 files of 5 Mbit.)
-        const bool kept = (flags & DG_BATCH_KEEP_COEFFICIENTS) != 0;  // dg_batch_debug looks into single waves
-        if (n_waves == 1 && (total_coef + total_big > ((size_t)1 << 30) || (total_coef > ((size_t)144 << 20) && !kept))) n_waves = 2;
+        if (n_waves == 1 && total_coef + total_big > ((size_t)1 << 30)) n_waves = 2;
+        b->views = n_waves == 1;
+        const bool kept = (flags & DG_BATCH_KEEP_COEFFICIENTS) != 0;
+        if (n_waves == 1 && total_coef > ((size_t)144 << 20) && !kept) n_waves = 2;
         const size_t coef_cap = total_coef / n_waves + 1, big_cap = total_big / n_waves + 1;
         WavePlan* wv = nullptr;
         size_t coef_bytes = 0, big_bytes = 0;
@@ -1919,12 +1922,13 @@ extern "C" int dg_batch_debug(const dg_batch* b, int i, const int16_t** coef, ui
     if (!b || i < 0 || i >= b->n) return fail(DG_E_INVALID, "bad index");
     const ItemPlan& it = b->items[i];
     if (it.status || !it.is_jpeg || it.wave < 0) return fail(DG_E_INVALID, "item has no JPEG intermediates");
-    if ((int)b->waves.size() != 1) return fail(DG_E_INVALID, "intermediates are only kept for single-wave batches");
+    if (!b->views && b->waves.size() != 1) return fail(DG_E_INVALID, "intermediates are only kept for batches with less than 1 GiB of them");
     const WavePlan& wv = b->waves[it.wave];
-    if (coef) *coef = (const int16_t*)(b->d_scratch + wv.off_coef) + it.coef_off_blocks * 64;
+    const uint8_t* const scratch = it.wave & 1 ? b->d_scratch2 : b->d_scratch;
+    if (coef) *coef = (const int16_t*)(scratch + wv.off_coef) + it.coef_off_blocks * 64;
     if (nblocks) *nblocks = it.nblocks;
     const bool transform = b->ctx->has_tfm && !(b->flags & DG_BATCH_DECODE_ONLY);
-    if (decoded) *decoded = transform ? b->d_scratch + wv.off_decoded + it.decoded_off : b->d_persist + b->off_out + it.pipe_off;
+    if (decoded) *decoded = transform ? scratch + wv.off_decoded + it.decoded_off : b->d_persist + b->off_out + it.pipe_off;
     return DG_OK;
 }
 

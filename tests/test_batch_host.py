@@ -55,3 +55,19 @@ def test_a_captured_stream_waits_for_no_event_from_outside(fake, n, upload_insid
         fake.fake_capture(c.stream, 0)
         b.sync()
     c.close()
+
+
+def test_intermediates_of_a_batch_in_two_waves(fake):
+    # 168 MiB of coefficients: two waves, which keep what they made in a scratch block each
+    data = synth.encode_jpeg(np.full((2048, 2048, 3), 90, np.uint8), 90, "4:4:4", 0)
+    c = dg.Context(0, CFG)
+    with c.batch([data] * 7) as b:
+        spans = []
+        for i in range(len(b)):
+            coef, blocks, decoded = C.c_void_p(), C.c_uint64(), C.c_void_p()
+            assert fake.dg_batch_debug(b._h, i, C.byref(coef), C.byref(blocks), C.byref(decoded)) == 0, i
+            assert blocks.value == 3 * 256 * 256
+            spans += [(coef.value, coef.value + blocks.value * 128), (decoded.value, decoded.value + 2048 * 2048 * 3)]
+        spans.sort()
+        assert all(a[1] <= b[0] for a, b in zip(spans, spans[1:]))
+    c.close()

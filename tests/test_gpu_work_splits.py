@@ -196,3 +196,14 @@ def test_calls_recorded_into_a_graph(n, upload_inside, monkeypatch):
             del graph
     finally:
         c.close()
+
+
+def test_intermediates_of_a_batch_in_two_waves():
+    # 168 MiB of coefficients: two waves
+    cfg = dict(crop_and_resize=True, default_image_size=512, downsampling_ratio=16, min_aspect_ratio=0.5, max_aspect_ratio=2.0)
+    rng = np.random.default_rng(352)
+    datas = [jpeg(rng, 2048, 2048, "4:4:4", noise=2.0)] * 4 + [jpeg(rng, 2041, 2047, "4:4:4", noise=2.0)] * 3
+    with ctx(cfg).batch(datas) as b:
+        b.upload(); b.run(); b.sync()
+        for i in (0, 6):
+            assert_same(b.debug_decoded(i), oracle.jpeg_decode(datas[i]), str(i))
