@@ -126,6 +126,9 @@ struct dg_ctx {
     // Three-component 4:2:0 images take the fused path (luma never leaves the SM); DATAGO_B200_FUSED=0 sends them through
     // the general IDCT and colour kernels instead (for measurements and for testing that path on the common sampling).
     bool fused_path = true;
+    // What dg_resize_device_static hands to the resize passes to count their time-outs in, page-locked, so that the host can read it
+    // after the synchronisation that the call ends with; always 0 between calls.
+    unsigned int* static_timeouts = nullptr;
     // Horizontal resize passes run on the tensor cores where their geometry fits; DATAGO_B200_HMMA=0 keeps them on the
     // dp2a kernel (measurements, and the test-suite's coverage of that kernel).
     bool hmma = true;
@@ -183,10 +186,12 @@ static int ctx_create(int device, const dg_image_config* cfg, void* stream, bool
         cudaEventCreateWithFlags(&c->ev_aux_go[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_aux_go[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_aux_done[0], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_aux_done[1], cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&c->ev_aux_done[1], cudaEventDisableTiming) != cudaSuccess ||
+        (c->has_tfm && cudaHostAlloc((void**)&c->static_timeouts, sizeof *c->static_timeouts, cudaHostAllocDefault) != cudaSuccess)) {
         delete c;
         return fail(DG_E_CUDA, "creating the second stream failed");
     }
+    if (c->static_timeouts) *c->static_timeouts = 0;
     if (const char* mb = getenv("DATAGO_B200_L2_GROUP_MB")) { long v = atol(mb); if (v >= 1) c->l2_group_bytes = (size_t)v << 20; }
     if (const char* mb = getenv("DATAGO_B200_TABLE_CACHE_MB")) { long v = atol(mb); if (v >= 0) c->table_cache_cap = (size_t)v << 20; }
     if (const char* v = getenv("DATAGO_B200_FUSED")) c->fused_path = atoi(v) != 0;
@@ -212,6 +217,7 @@ extern "C" void dg_ctx_destroy(dg_ctx* c) {
     cudaStreamDestroy(c->up);
     for (cudaEvent_t e : c->events) cudaEventDestroy(e);
     for (BlockCache* cache : {&c->dev, &c->pin, &c->dev_meta, &c->pin_meta}) cache->clear();
+    if (c->static_timeouts) cudaFreeHost(c->static_timeouts);
     cudaEventDestroy(c->ev_fork);
     cudaEventDestroy(c->ev_join);
     for (int i = 0; i < 2; ++i) {
@@ -1816,6 +1822,11 @@ static int device_status_to_code(uint32_t bits) {
     return DG_E_TRUNCATED;
 }
 
+// The tensor-core resize passes bound their waits for asynchronous copies; a wait that ran out left garbage behind.
+static int timed_out(unsigned int ctas) {
+    return fail(DG_E_CUDA, "resize: a copy into shared memory did not complete in time (%u CTAs gave up); the pixels are not valid", ctas);
+}
+
 extern "C" int dg_batch_sync(dg_batch* b) {
     if (!b) return fail(DG_E_INVALID, "NULL batch");
     dg_ctx* ctx = b->ctx;
@@ -1829,9 +1840,8 @@ extern "C" int dg_batch_sync(dg_batch* b) {
     await_inputs(b);
     landed(b);
     if (b->ran) {
-        // the tensor-core resize passes bound their waits for asynchronous copies; a wait that ran out left garbage behind
-        const unsigned int t = *(const unsigned int*)((const uint8_t*)b->h_status + timeouts_at(b->n));
-        if (t) return fail(DG_E_CUDA, "resize: a copy into shared memory did not complete in time (%u CTAs gave up); the batch's pixels are not valid", t);
+        const unsigned int gave_up = *(const unsigned int*)((const uint8_t*)b->h_status + timeouts_at(b->n));
+        if (gave_up) return timed_out(gave_up);
         for (int i = 0; i < b->n; ++i)
             if (b->items[i].status == DG_OK && b->h_status[i]) b->items[i].status = device_status_to_code(b->h_status[i]);
         if (!b->counted) {  // once per batch, however often it is run and synchronised
@@ -2096,8 +2106,6 @@ extern "C" int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, u
     }
     const size_t m_copies = m.put(wv.copies, 16);
     m_copy = put_owner_map(m, wv.copy_first);
-    const uint32_t no_timeouts = 0;
-    const size_t m_timeouts = m.put(&no_timeouts, sizeof no_timeouts);
     if (m.bytes.size() > meta_cap)
         return fail(DG_E_TOO_LARGE, "filter tables (%zu bytes) and intermediates (%zu bytes) exceed the %zu-byte static scratch",
                     m.bytes.size(), mid_bound, kStaticScratchBytes);
@@ -2118,12 +2126,13 @@ extern "C" int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, u
     for (int st = 0; st < 4; ++st) {
         if (wv.passes[st].empty()) continue;
         const ConvPass* passes = (const ConvPass*)(scratch + m_passes[st]);
-        unsigned int* const timeouts = (unsigned int*)(scratch + m_timeouts);
-        if (st & 1) launch_conv_v(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], timeouts, s);
-        else launch_conv_h(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], timeouts, s);
+        if (st & 1) launch_conv_v(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], ctx->static_timeouts, s);
+        else launch_conv_h(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], ctx->static_timeouts, s);
     }
     if (!copied && !wv.copies.empty()) launch_copy((const CopyJob*)(scratch + m_copies), map_at(m_copy), s);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(s));  // the host-side metadata image dies with this frame
-    return DG_OK;
+    const unsigned int gave_up = *(volatile unsigned int*)ctx->static_timeouts;
+    *ctx->static_timeouts = 0;
+    return gave_up ? timed_out(gave_up) : DG_OK;
 }

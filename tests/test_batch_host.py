@@ -71,3 +71,24 @@ def test_intermediates_of_a_batch_in_two_waves(fake):
         spans.sort()
         assert all(a[1] <= b[0] for a, b in zip(spans, spans[1:]))
     c.close()
+
+
+def test_a_resize_that_gave_up_waiting_is_reported(fake):
+    c = dg.Context(0, CFG)
+    x = raw((1104, 1408, 3))
+    dst = np.zeros((2048, 2048, 3), np.uint8)
+
+    def static():
+        c.resize_device_static(x.ctypes.data, x.shape[1], x.shape[0], 3, dst.ctypes.data)
+
+    static()
+    fake.fake_timeouts(2)
+    with pytest.raises(dg.DatagoB200Error, match="CTAs gave up"):
+        static()
+    with c.batch([x]) as b:
+        b.upload(); b.run()
+        with pytest.raises(dg.DatagoB200Error, match="CTAs gave up"):
+            b.sync()
+    fake.fake_timeouts(0)
+    static()
+    c.close()
