@@ -432,7 +432,7 @@ struct GlobalSource {
     struct Cursor { uint32_t at, w2; };
     const uint32_t* words;
     uint32_t n;
-    __device__ __forceinline__ uint32_t word(uint32_t i) const { return i < n ? __ldg(words + i) : 0u; }
+    __device__ __forceinline__ uint32_t word(uint32_t i) const { return i < n ? load_global(words + i) : 0u; }
     __device__ __forceinline__ Cursor start(uint32_t& w0, uint32_t& w1, uint32_t p) const {
         w0 = word(p >> 5); w1 = word((p >> 5) + 1);
         return Cursor{p >> 5, word((p >> 5) + 2)};
@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
                 if ((state & 0xFFFu) >= (uint32_t)CELL) next = state - CELL;  // no block starts in this cell
                 else {
                     const uint4* const c = cand + (k - kbeg) * cand_step;
-                    const uint4 a = __ldg(c), b = __ldg(c + piece), e = __ldg(c + 2 * piece);
+                    const uint4 a = load_global(c), b = load_global(c + piece), e = load_global(c + 2 * piece);
                     bool known = false;
                     auto look = [&](uint32_t x, uint32_t y) { if ((x & 0xFFFFu) == state) { next = x >> 16; n = y; known = true; } };
                     look(a.x, a.y); look(a.z, a.w); look(b.x, b.y); look(b.z, b.w); look(e.x, e.y); look(e.z, e.w);
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(T) k_huff_chain(JpegWave w) {
 
     uint32_t entry = 0;  // thread 0: bit 0, block 0
     if (active && tid) {
-        entry = __ldg(&cand->x) & 0xFFFFu;
+        entry = load_global(&cand->x) & 0xFFFFu;
         if (entry == kStDropped) entry = kStNone;
     }
     follow(active, kbeg, entry, false);

@@ -338,7 +338,7 @@ struct ChromaPlane {  // per-pixel path
     const uint8_t* p;
     uint32_t pitch;
     int dh, hs, vs;
-    __device__ __forceinline__ int px(int x, int y) const { return __ldg(p + (size_t)y * pitch + x); }
+    __device__ __forceinline__ int px(int x, int y) const { return (int)load_global(p + (size_t)y * pitch + x); }
     __device__ __forceinline__ int at(int x, int y) const {
         if (hs == 2) return px(x >> 1, vs == 2 ? y >> 1 : y);  // planes at most two samples wide: replicated
         const int cy = y >> 1, far = min(max((y & 1) ? cy + 1 : cy - 1, 0), dh - 1);  // 4:4:0: triangle filter down the column
@@ -374,12 +374,12 @@ __device__ __forceinline__ void chroma_tile_fetch(uint8_t (&s_c)[2][ROWS][kCTile
             uint32_t* sb = reinterpret_cast<uint32_t*>(s_c[0][r]);
             uint32_t* sr = reinterpret_cast<uint32_t*>(s_c[1][r]);
             const int g0 = min(max(w0 + lane, 0), wmax);
-            sb[lane] = __ldg(gb + g0);
-            sr[lane] = __ldg(gr + g0);
+            sb[lane] = load_global(gb + g0);
+            sr[lane] = load_global(gr + g0);
             if (lane < kWords - 32) {
                 const int g1 = min(max(w0 + 32 + lane, 0), wmax);
-                sb[32 + lane] = __ldg(gb + g1);
-                sr[32 + lane] = __ldg(gr + g1);
+                sb[32 + lane] = load_global(gb + g1);
+                sr[32 + lane] = load_global(gr + g1);
             }
         }
     }
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
         for (int k = 0; k < nsteps; ++k) {
             const int y = y_base + rowi + 8 * k;
             if (y >= H) break;
-            const uint2 v = __ldg(reinterpret_cast<const uint2*>(yp + (size_t)y * ypitch + x));
+            const uint2 v = load_global(reinterpret_cast<const uint2*>(yp + (size_t)y * ypitch + x));
             uint8_t* o = out + (size_t)y * d.out_pitch + x;
             if (npx == 8 && (reinterpret_cast<uintptr_t>(o) & 7u) == 0) __stcs(reinterpret_cast<uint2*>(o), v);
             else for (int i = 0; i < npx; ++i) o[i] = (uint8_t)((i < 4 ? v.x : v.y) >> (8 * (i & 3)));
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
         // pair at a time: the byte gathering is done once, the second row only swaps the weights.
         const int y_first = (int)ty * 8 * 2 * (int)kColorMcuRows - 1;
         auto luma = [&](int y) -> uint2 {
-            return (y >= 0 && y < H) ? __ldg(reinterpret_cast<const uint2*>(yp + (size_t)y * ypitch + x)) : make_uint2(0, 0);
+            return (y >= 0 && y < H) ? load_global(reinterpret_cast<const uint2*>(yp + (size_t)y * ypitch + x)) : make_uint2(0, 0);
         };
         uint2 nextA = luma(y_first + 2 * rowi), nextB = luma(y_first + 2 * rowi + 1);
 #pragma unroll 1
@@ -511,12 +511,12 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
         for (int k = 0; k < nsteps; ++k) {
             const int y = y_base + rowi + 8 * k;
             if (y >= H) break;
-            const uint2 b = __ldg(reinterpret_cast<const uint2*>(planes + d.plane_off[1] + (size_t)y * d.plane_pitch[1] + x));
-            const uint2 r = __ldg(reinterpret_cast<const uint2*>(planes + d.plane_off[2] + (size_t)y * d.plane_pitch[2] + x));
+            const uint2 b = load_global(reinterpret_cast<const uint2*>(planes + d.plane_off[1] + (size_t)y * d.plane_pitch[1] + x));
+            const uint2 r = load_global(reinterpret_cast<const uint2*>(planes + d.plane_off[2] + (size_t)y * d.plane_pitch[2] + x));
             const uint32_t b0 = b.x ^ 0x80808080u, b1 = b.y ^ 0x80808080u, r0 = r.x ^ 0x80808080u, r1 = r.y ^ 0x80808080u;
             const uint32_t c[8] = {chroma_word<0>(b0, r0), chroma_word<1>(b0, r0), chroma_word<2>(b0, r0), chroma_word<3>(b0, r0),
                                    chroma_word<0>(b1, r1), chroma_word<1>(b1, r1), chroma_word<2>(b1, r1), chroma_word<3>(b1, r1)};
-            const uint2 yv = __ldg(reinterpret_cast<const uint2*>(yp + (size_t)y * ypitch + x));
+            const uint2 yv = load_global(reinterpret_cast<const uint2*>(yp + (size_t)y * ypitch + x));
             uint32_t px[6];
             ycc_to_rgb8(yv.x, yv.y, c, px);
             store_rgb8(out + (size_t)y * d.out_pitch + x * 3, px, npx, lanes);
@@ -537,14 +537,14 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
 #pragma unroll
             for (int comp = 1; comp <= 2; ++comp) {
                 const uint8_t* row = planes + d.plane_off[comp] + (size_t)y * d.plane_pitch[comp];
-                const uint32_t q = __ldg(reinterpret_cast<const uint32_t*>(row + c0));
+                const uint32_t q = load_global(reinterpret_cast<const uint32_t*>(row + c0));
                 int32_t t[6];
-                t[0] = __ldg(row + max(c0 - 1, 0));
+                t[0] = (int32_t)load_global(row + max(c0 - 1, 0));
 #pragma unroll
                 for (int i = 0; i < 4; ++i) t[i + 1] = (int32_t)((q >> (8 * i)) & 255u);
-                if (inner) t[5] = __ldg(row + c0 + 4);
+                if (inner) t[5] = (int32_t)load_global(row + c0 + 4);
                 else {
-                    const int32_t last = __ldg(row + dw - 1);
+                    const int32_t last = (int32_t)load_global(row + dw - 1);
 #pragma unroll
                     for (int i = 1; i < 6; ++i) if (c0 + i - 1 >= dw) t[i] = last;
                 }
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
                     v[2 * i + 1] = ((3 * t[i + 1] + t[i + 2] + 2) >> 2) - 128;
                 }
             }
-            const uint2 yv = __ldg(reinterpret_cast<const uint2*>(yp + (size_t)y * ypitch + x));
+            const uint2 yv = load_global(reinterpret_cast<const uint2*>(yp + (size_t)y * ypitch + x));
             uint32_t px[6];
             uint32_t c[8];
 #pragma unroll
@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(kColorThreads, 4) k_color(JpegWave w, uint32_t
         if (y >= H) break;
 #pragma unroll 1
         for (int i = 0; i < npx; ++i) {
-            const int Y = __ldg(yp + (size_t)y * ypitch + x + i);
+            const int Y = (int)load_global(yp + (size_t)y * ypitch + x + i);
             const int cb = cbp.at(x + i, y) - 128, cr = crp.at(x + i, y) - 128;
             uint8_t* o = out + (size_t)y * d.out_pitch + (x + i) * 3;
             o[0] = (uint8_t)min(max(Y + ((91881 * cr + 32768) >> 16), 0), 255);

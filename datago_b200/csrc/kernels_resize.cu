@@ -72,13 +72,13 @@ constexpr int kConvHThreads = kConvTileW * 4;
 
 template <bool GUARD>
 __device__ __forceinline__ uint32_t load_word(const ConvPass& p, const uint32_t* w) {
-    if (!GUARD) return __ldg(w);
-    const uint8_t* b = reinterpret_cast<const uint8_t*>(w);
-    if (b >= p.guard_lo && b + 4 <= p.guard_hi) return __ldg(w);
+    if (!GUARD) return load_global(w);
+    const uint8_t* const caller = reinterpret_cast<const uint8_t*>(w);
+    if (caller >= p.guard_lo && caller + 4 <= p.guard_hi) return __ldg(reinterpret_cast<const uint32_t*>(caller));
     uint32_t v = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-        if (b + j >= p.guard_lo && b + j < p.guard_hi) v |= (uint32_t)__ldg(b + j) << (8 * j);
+        if (caller + j >= p.guard_lo && caller + j < p.guard_hi) v |= (uint32_t)__ldg(caller + j) << (8 * j);
     return v;
 }
 
@@ -440,7 +440,7 @@ __device__ void conv_h_rows_any(const ConvPass& p, const Table& tb, uint32_t x, 
         int32_t acc[4] = {1 << (p.precision - 1), 1 << (p.precision - 1), 1 << (p.precision - 1), 1 << (p.precision - 1)};
         for (int32_t i = 0; i < taps; ++i) {
             const int32_t wv = __ldg(k + (size_t)i * p.tab_n);
-            for (uint32_t c = 0; c < C; ++c) acc[c] += wv * (int32_t)__ldg(g + (size_t)i * C + c);
+            for (uint32_t c = 0; c < C; ++c) acc[c] += wv * (int32_t)load_global(g + (size_t)i * C + c);
         }
         uint8_t* o = p.dst + (size_t)(y0 + r) * p.dst_pitch + (size_t)x * C;
         for (uint32_t c = 0; c < C; ++c) o[c] = (uint8_t)clip8(acc[c], p.precision);
@@ -508,7 +508,7 @@ __device__ __forceinline__ void conv_v_plain(const ConvPass& p, const Table& tb,
     if (vec) {
         for (int32_t i = 0; i < taps; ++i) {
             const int32_t kv = __ldg(k + (size_t)i * p.tab_n);
-            const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(s + (size_t)i * p.src_pitch));
+            const uint32_t v = load_global(reinterpret_cast<const uint32_t*>(s + (size_t)i * p.src_pitch));
             a0 += kv * (int32_t)(v & 255u); a1 += kv * (int32_t)((v >> 8) & 255u);
             a2 += kv * (int32_t)((v >> 16) & 255u); a3 += kv * (int32_t)(v >> 24);
         }
@@ -516,10 +516,10 @@ __device__ __forceinline__ void conv_v_plain(const ConvPass& p, const Table& tb,
         for (int32_t i = 0; i < taps; ++i) {
             const int32_t kv = __ldg(k + (size_t)i * p.tab_n);
             const uint8_t* r = s + (size_t)i * p.src_pitch;
-            a0 += kv * (int32_t)__ldg(r);
-            if (nb > 1) a1 += kv * (int32_t)__ldg(r + 1);
-            if (nb > 2) a2 += kv * (int32_t)__ldg(r + 2);
-            if (nb > 3) a3 += kv * (int32_t)__ldg(r + 3);
+            a0 += kv * (int32_t)load_global(r);
+            if (nb > 1) a1 += kv * (int32_t)load_global(r + 1);
+            if (nb > 2) a2 += kv * (int32_t)load_global(r + 2);
+            if (nb > 3) a3 += kv * (int32_t)load_global(r + 3);
         }
     }
     uint8_t* o = p.dst + (size_t)y * p.dst_pitch + xb;
@@ -569,8 +569,8 @@ __device__ __forceinline__ void conv_v_vector(const ConvPass& p, const Table& tb
         for (int i = 0; i < 16; ++i) acc[i] = half;
         for (int32_t i = 0; i < taps; i += 2) {
             const uint32_t kp = s_k[r][i >> 1];  // the weight after the last tap of an odd window is zero
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(s + (size_t)i * p.src_pitch));
-            const uint4 b = __ldg(reinterpret_cast<const uint4*>(s + (size_t)min(i + 1, taps - 1) * p.src_pitch));
+            const uint4 a = load_global(reinterpret_cast<const uint4*>(s + (size_t)i * p.src_pitch));
+            const uint4 b = load_global(reinterpret_cast<const uint4*>(s + (size_t)min(i + 1, taps - 1) * p.src_pitch));
             const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
             for (int wq = 0; wq < 4; ++wq) {
@@ -841,11 +841,11 @@ __global__ void __launch_bounds__(256) k_copy(const CopyJob* jobs, OwnerMap map)
             const uint8_t* s = src + y * j.src_pitch + x;
             const uint32_t m = (uint32_t)(reinterpret_cast<uintptr_t>(s) & 15u);
             uint4 v;
-            if (m == 0) v = __ldg(reinterpret_cast<const uint4*>(s));
+            if (m == 0) v = load_global(reinterpret_cast<const uint4*>(s));
             else {
                 const uint32_t* w = reinterpret_cast<const uint32_t*>(s - (m & 3u));
                 const uint32_t sh = (m & 3u) * 8;
-                const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3), w4 = sh ? __ldg(w + 4) : 0u;
+                const uint32_t w0 = load_global(w), w1 = load_global(w + 1), w2 = load_global(w + 2), w3 = load_global(w + 3), w4 = sh ? load_global(w + 4) : 0u;
                 v = make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), __funnelshift_r(w2, w3, sh), __funnelshift_r(w3, w4, sh));
             }
             *reinterpret_cast<uint4*>(dst + b) = v;
@@ -854,7 +854,7 @@ __global__ void __launch_bounds__(256) k_copy(const CopyJob* jobs, OwnerMap map)
     }
     for (uint64_t b = at < lead ? 0 : at - lead; b < total && b + lead < at + 16; ++b) {
         const uint64_t y = b / j.row_bytes, x = b - y * j.row_bytes;
-        dst[b] = __ldg(src + y * j.src_pitch + x);
+        dst[b] = (uint8_t)load_global(src + y * j.src_pitch + x);
     }
 }
 
@@ -924,11 +924,11 @@ __global__ void __launch_bounds__(256) k_to_rgb8(const ToRgbJob* jobs, OwnerMap 
         if (i >= j.npx) break;
         uint8_t* d = j.dst + (size_t)i * 3;
         if (j.channels <= 2) {
-            const uint8_t v = __ldg(j.src + (size_t)i * j.channels);
+            const uint8_t v = (uint8_t)load_global(j.src + (size_t)i * j.channels);
             d[0] = v; d[1] = v; d[2] = v;
             continue;
         }
-        const uint32_t px = __ldg(reinterpret_cast<const uint32_t*>(j.src) + i);  // RGBA rows are 4-byte aligned
+        const uint32_t px = load_global(reinterpret_cast<const uint32_t*>(j.src) + i);  // RGBA rows are 4-byte aligned
         const uint32_t a = px >> 24;
         uint32_t c[3] = {px & 255u, (px >> 8) & 255u, (px >> 16) & 255u};
         if (a == 0) { c[0] = c[1] = c[2] = 128; }
