@@ -126,9 +126,6 @@ struct dg_ctx {
     // Three-component 4:2:0 images take the fused path (luma never leaves the SM); DATAGO_B200_FUSED=0 sends them through
     // the general IDCT and colour kernels instead (for measurements and for testing that path on the common sampling).
     bool fused_path = true;
-    // What dg_resize_device_static hands to the resize passes to count their time-outs in, page-locked, so that the host can read it
-    // after the synchronisation that the call ends with; always 0 between calls.
-    unsigned int* static_timeouts = nullptr;
     // Horizontal resize passes run on the tensor cores where their geometry fits; DATAGO_B200_HMMA=0 keeps them on the
     // dp2a kernel (measurements, and the test-suite's coverage of that kernel).
     bool hmma = true;
@@ -186,12 +183,10 @@ static int ctx_create(int device, const dg_image_config* cfg, void* stream, bool
         cudaEventCreateWithFlags(&c->ev_aux_go[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_aux_go[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_aux_done[0], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_aux_done[1], cudaEventDisableTiming) != cudaSuccess ||
-        (c->has_tfm && cudaHostAlloc((void**)&c->static_timeouts, sizeof *c->static_timeouts, cudaHostAllocDefault) != cudaSuccess)) {
+        cudaEventCreateWithFlags(&c->ev_aux_done[1], cudaEventDisableTiming) != cudaSuccess) {
         delete c;
         return fail(DG_E_CUDA, "creating the second stream failed");
     }
-    if (c->static_timeouts) *c->static_timeouts = 0;
     if (const char* mb = getenv("DATAGO_B200_L2_GROUP_MB")) { long v = atol(mb); if (v >= 1) c->l2_group_bytes = (size_t)v << 20; }
     if (const char* mb = getenv("DATAGO_B200_TABLE_CACHE_MB")) { long v = atol(mb); if (v >= 0) c->table_cache_cap = (size_t)v << 20; }
     if (const char* v = getenv("DATAGO_B200_FUSED")) c->fused_path = atoi(v) != 0;
@@ -217,7 +212,6 @@ extern "C" void dg_ctx_destroy(dg_ctx* c) {
     cudaStreamDestroy(c->up);
     for (cudaEvent_t e : c->events) cudaEventDestroy(e);
     for (BlockCache* cache : {&c->dev, &c->pin, &c->dev_meta, &c->pin_meta}) cache->clear();
-    if (c->static_timeouts) cudaFreeHost(c->static_timeouts);
     cudaEventDestroy(c->ev_fork);
     cudaEventDestroy(c->ev_join);
     for (int i = 0; i < 2; ++i) {
@@ -2008,17 +2002,26 @@ static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBy
 constexpr int kMaxDevices = 64;
 std::mutex g_static_mu;
 unsigned char* g_static_ptr[kMaxDevices] = {nullptr};
+// What the resize passes count their time-outs in: page-locked, so that the host can read it after the synchronisation that the
+// call ends with.  0 between calls; like the array, it stays until the process exits.
+unsigned int* g_static_timeouts[kMaxDevices] = {nullptr};
 
-int static_scratch_for(int device, unsigned char** out) {
+int static_scratch_for(int device, unsigned char** out, unsigned int** timeouts) {
     if (device < 0 || device >= kMaxDevices) return fail(DG_E_INVALID, "device ordinal %d not supported here", device);
     std::lock_guard<std::mutex> lock(g_static_mu);
     if (!g_static_ptr[device]) {
         void* p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_static_scratch);
         if (e != cudaSuccess || !p) return fail(DG_E_CUDA, "cudaGetSymbolAddress(static scratch): %s", cudaGetErrorString(e));
+        void* word = nullptr;
+        e = cudaHostAlloc(&word, sizeof(unsigned int), cudaHostAllocDefault);
+        if (e != cudaSuccess) return fail(DG_E_CUDA, "page-locking a word: %s", cudaGetErrorString(e));
+        *(unsigned int*)word = 0;
+        g_static_timeouts[device] = (unsigned int*)word;
         g_static_ptr[device] = (unsigned char*)p;
     }
     *out = g_static_ptr[device];
+    *timeouts = g_static_timeouts[device];
     return DG_OK;
 }
 
@@ -2038,7 +2041,8 @@ extern "C" int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, u
     std::lock_guard<std::mutex> lock(ctx->mu);
     CU(cudaSetDevice(ctx->device));
     unsigned char* scratch = nullptr;
-    rc = static_scratch_for(ctx->device, &scratch);  // first call on a device: symbol look-up
+    unsigned int* timeouts = nullptr;
+    rc = static_scratch_for(ctx->device, &scratch, &timeouts);  // first call on a device: symbol look-up
     if (rc) return rc;
 
     // intermediates go to the top part of the array, metadata to the bottom part
@@ -2126,13 +2130,13 @@ extern "C" int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, u
     for (int st = 0; st < 4; ++st) {
         if (wv.passes[st].empty()) continue;
         const ConvPass* passes = (const ConvPass*)(scratch + m_passes[st]);
-        if (st & 1) launch_conv_v(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], ctx->static_timeouts, s);
-        else launch_conv_h(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], ctx->static_timeouts, s);
+        if (st & 1) launch_conv_v(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], timeouts, s);
+        else launch_conv_h(passes, map_at(m_pass[st]), tables, wv.mma_tiles[st], timeouts, s);
     }
     if (!copied && !wv.copies.empty()) launch_copy((const CopyJob*)(scratch + m_copies), map_at(m_copy), s);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(s));  // the host-side metadata image dies with this frame
-    const unsigned int gave_up = *(volatile unsigned int*)ctx->static_timeouts;
-    *ctx->static_timeouts = 0;
+    const unsigned int gave_up = *(volatile unsigned int*)timeouts;
+    *timeouts = 0;
     return gave_up ? timed_out(gave_up) : DG_OK;
 }

@@ -312,7 +312,8 @@ DG_API void dg_feeder_destroy(dg_feeder* f);
  * Limit: intermediates + tables must fit those 32 MiB; the intermediates are bounded by
  * new_w * channels * (max(src_h, new_h) + 2 * new_h) bytes (new_w, new_h from dg_plan_geometry), e.g. a 4096 x 4096
  * RGB source into a 1024-class bucket needs about 19 MiB.  Larger inputs get DG_E_TOO_LARGE and nothing is launched.
- * The first call on a device looks up the array's device address; make that call before any stream capture.
+ * The first call on a device looks up the array's device address and page-locks a word of host memory; make that call before any
+ * stream capture.
  * All calls share the array and it keeps whatever the last call left (nothing in it needs clearing: every byte is
  * written before it is read), so two calls that overlap on the same GPU -- two contexts, two streams -- race; calls
  * on one ctx are serialised and the function returns after its work has completed. */

@@ -16,7 +16,7 @@ struct Event { bool captured = false; };
 std::mutex mu;
 unsigned long long to_device = 0, to_host = 0;
 unsigned int timeouts_per_pass = 0;
-int waits = 0;
+int host_allocations = 0;
 bool capturing(cudaStream_t s) { return s && reinterpret_cast<Stream*>(s)->capturing; }
 CUresult encode(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                 CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill) { return CUDA_SUCCESS; }
@@ -30,7 +30,7 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "?"; }
 cudaError_t cudaMalloc(void** p, size_t n) { *p = aligned_alloc(256, (n + 255) / 256 * 256); return *p ? cudaSuccess : cudaErrorMemoryAllocation; }
 cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned int) { return cudaMalloc(p, n); }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned int) { ++host_allocations; return cudaMalloc(p, n); }
 cudaError_t cudaFreeHost(void* p) { return cudaFree(p); }
 cudaError_t cudaHostRegister(void*, size_t, unsigned int) { return cudaSuccess; }
 cudaError_t cudaHostUnregister(void*) { return cudaSuccess; }
@@ -55,7 +55,6 @@ cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 0.
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { reinterpret_cast<Event*>(e)->captured = capturing(s); return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned int) {
     std::lock_guard<std::mutex> lock(mu);
-    ++waits;
     if (capturing(s) && !reinterpret_cast<Event*>(e)->captured) return cudaErrorStreamCaptureIsolation;
     if (reinterpret_cast<Event*>(e)->captured) reinterpret_cast<Stream*>(s)->capturing = true;  // joins the capture
     return cudaSuccess;
@@ -72,6 +71,7 @@ void fake_capture(void* s, int on) { reinterpret_cast<Stream*>(s)->capturing = o
 void fake_timeouts(unsigned int per_pass) { timeouts_per_pass = per_pass; }
 unsigned long long fake_to_device() { return to_device; }
 unsigned long long fake_to_host() { return to_host; }
+int fake_host_allocations() { return host_allocations; }
 }
 
 namespace dg {

@@ -92,3 +92,16 @@ def test_a_resize_that_gave_up_waiting_is_reported(fake):
     fake.fake_timeouts(0)
     static()
     c.close()
+
+
+def test_what_the_static_resize_needs_is_made_once_per_device(fake):
+    # page-locking takes longer than the rest of making a context
+    x, dst = raw((300, 400, 3)), np.zeros((2048, 2048, 3), np.uint8)
+    made = []
+    for _ in range(3):
+        c = dg.Context(0, CFG)
+        before = fake.fake_host_allocations()
+        c.resize_device_static(x.ctypes.data, 400, 300, 3, dst.ctypes.data)
+        made.append((before, fake.fake_host_allocations()))
+        c.close()
+    assert made[0][1] == made[1][0] == made[1][1] == made[2][0] == made[2][1]
