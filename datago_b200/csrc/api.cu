@@ -432,7 +432,7 @@ struct dg_batch {
     uint8_t* d_scratch2 = nullptr;  // scratch of the odd waves (same block when the batch has one wave)
     uint8_t* h_pin = nullptr;       // pinned image of [status zeros | blob | raw inputs]
     uint8_t* h_meta = nullptr;      // ... and of the metadata
-    uint32_t* h_status = nullptr;   // pinned, n words
+    uint32_t* h_status = nullptr;   // pinned, status_bytes(n)
     size_t off_status = 0, off_blob = 0, off_rawin = 0, off_out = 0;
     size_t blob_bytes = 0, rawin_bytes = 0, out_bytes = 0;
     size_t arena_bytes = 0;  // out_bytes plus the pre-conversion images of DG_ITEM_TO_RGB8 items (never downloaded)
@@ -1828,7 +1828,7 @@ extern "C" int dg_batch_sync(dg_batch* b) {
     CU(cudaSetDevice(ctx->device));
     if (b->ran) {
         CU(cudaMemcpyAsync(b->h_status, b->d_persist + b->off_status, status_bytes(b->n), cudaMemcpyDeviceToHost, ctx->stream));
-        b->d2h += (size_t)b->n * 4;
+        b->d2h += status_bytes(b->n);
     }
     CU(cudaStreamSynchronize(ctx->stream));
     await_inputs(b);

@@ -229,7 +229,8 @@ DG_API int dg_batch_bucket_count(const dg_batch* b);
 DG_API int dg_batch_bucket(const dg_batch* b, int k, dg_bucket* out);
 /* Milliseconds per stage of the last dg_batch_run of a DG_BATCH_TIMING batch (after dg_batch_sync). */
 DG_API int dg_batch_stage_ms(const dg_batch* b, float ms[DG_STAGE_COUNT]);
-/* Bytes copied host->device by upload, and kernels launched by one run. */
+/* Bytes copied to the device for the batch, bytes copied back since the last download was queued (the status words of
+ * dg_batch_sync included), kernels launched by one run. */
 DG_API int dg_batch_counters(const dg_batch* b, uint64_t* h2d_bytes, uint64_t* d2h_bytes, uint32_t* kernel_launches);
 /* Counters of the speculative entropy decoder over the last run: cells (of 512 or 1024 bits) that the restart-free streams
  * are cut into, rounds of linking them (added up over the images), decodes of a cell (by every candidate state, again where

@@ -105,3 +105,17 @@ def test_what_the_static_resize_needs_is_made_once_per_device(fake):
         made.append((before, fake.fake_host_allocations()))
         c.close()
     assert made[0][1] == made[1][0] == made[1][1] == made[2][0] == made[2][1]
+
+
+@pytest.mark.parametrize("n", [1, 4, 5])
+def test_counters_hold_what_was_copied(fake, n):
+    c = dg.Context(0, CFG)
+    with c.batch([raw((300, 400, 3))] * n) as b:
+        before = fake.fake_to_device(), fake.fake_to_host()
+        b.upload(); b.run()
+        b.download_packed(np.empty(b.packed_bytes(), np.uint8))
+        b.sync()
+        k = b.counters()
+        # (small batches: larger ones are copied before upload is called)
+        assert (k["h2d_bytes"], k["d2h_bytes"]) == (fake.fake_to_device() - before[0], fake.fake_to_host() - before[1])
+    c.close()
