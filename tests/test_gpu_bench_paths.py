@@ -143,7 +143,8 @@ def test_general_kernels_still_decode_420_images():
 
 def test_longest_images_take_the_widest_decoder_beside_the_others():
     # images of some hundred thousand bytes, whose linking threads (1024 of them here) own several cells each, beside small
-    # ones and one for the restart decoder on the lane's auxiliary stream; then alone in a batch
+    # ones and one for the restart decoder on the lane's auxiliary stream; then alone in a batch; then so often that cells
+    # are long ones, and in spans of four, while a linking thread still has more than four of them
     rng = np.random.default_rng(303)
     big = [synth.encode_jpeg(rng.integers(0, 256, (1024, 1024, 3), dtype=np.uint8), 97, "4:4:4", 0),
            synth.encode_jpeg(rng.integers(0, 256, (1400, 900, 3), dtype=np.uint8), 95, "4:2:0", 0)]
@@ -151,7 +152,11 @@ def test_longest_images_take_the_widest_decoder_beside_the_others():
     small = [jpeg(rng, 320, 200), jpeg(rng, 200, 320, rst=3), jpeg(rng, 640, 480, q=95, noise=20.0)]
     datas = [small[0], big[0], small[1], big[1], small[2]]
     want = _oracle_all(datas)
-    for batch in (datas, big, [big[1]]):
+    blocks = [3, 6]  # of an MCU: threads of the synchronising decoder per cell
+    threads = sum(len(b) * 8 * k for b, k in zip(big, blocks))  # times the bits of a cell
+    assert 2 * threads / 512 > 148 * 2048 > 2 * threads / 1024 and 4 * threads / 1024 > 148 * 2048
+    assert all(len(b) * 8 > 4 * 1024 * 1024 for b in big)
+    for batch in (datas, big, [big[1]], big * 2, big * 4):
         for (st, out, _), d in zip(ctx().process(batch), batch):
             assert st == 0
             assert_same(out, want[datas.index(d)], f"{len(d)} bytes")
