@@ -100,7 +100,7 @@ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct dg_ctx {
     int device = 0;
-    cudaStream_t stream = nullptr;   // everything the caller can observe is ordered on this stream
+    cudaStream_t stream = nullptr;   // kernels and downloads are ordered on this stream, and dg_batch_run orders it behind the inputs
     cudaStream_t stream2 = nullptr;  // odd waves of a batch run here, concurrently with the even ones
     cudaStream_t aux[2] = {nullptr, nullptr};  // per lane: the restart-interval decoder runs beside the speculative one
     cudaStream_t up = nullptr;                 // inputs of larger batches, copied while the rest is being staged (see dg_batch_create)
@@ -1018,9 +1018,11 @@ extern "C" int dg_batch_create(dg_ctx* ctx, const dg_item* items, int n, uint32_
         }
         size_t n_waves = std::max<size_t>(1, std::max((total_coef + ctx->wave_bytes - 1) / ctx->wave_bytes,
                                                       (total_big + 2 * ctx->wave_bytes - 1) / (2 * ctx->wave_bytes)));
-        // (one wave / two, us a pass: 48 files of 1 Mpixel, 150 MB of coefficients, decoded 394 / 357; 150 files 835 / 740; 100 files
-        // into buckets 957 / 836; 8 pairs of 4:4:4 and mask, 290 MB, 686 / 641; 48 files into buckets, 133 MB, 502 / 515.  Three
-        // and more: 790 for the pairs, 3 770 instead of 3 570 for 256 files of 5 Mbit.)
+        // (two waves over one, time of a pass.  4:2:0 files of 0.3 to 3 Mpixel, 150 MB of coefficients: decoded 0.85 to 0.89, into
+        // buckets 0.89 to 1.00; 200 MB 0.90 to 0.96 and 0.94 to 1.00; 300 and 450 MB 0.92 to 0.99 and 0.93 to 1.00; 60 and 100 MB 0.98 to
+        // 1.13 and 0.99 to 1.12.  4:4:4 of 8 Mpixel: 130 MB 0.98 to 1.00, 220 MB 0.92 to 0.96.  4:2:2 of 2 Mpixel loses at 147 MB, 1.05 to
+        // 1.06, and wins from 200 MB on, 0.91 to 0.92.  Three waves and more: pairs of 4:4:4 and mask 790 us instead of 640, 256 files of 5
+        // Mbit 3 770 instead of 3 570.)
         if (n_waves == 1 && total_coef + total_big > ((size_t)1 << 30)) n_waves = 2;
         b->views = n_waves == 1;
         const bool kept = (flags & DG_BATCH_KEEP_COEFFICIENTS) != 0;
@@ -2057,8 +2059,11 @@ extern "C" int dg_resize_device_static(dg_ctx* ctx, const uint8_t* device_src, u
     size_t mid_used = 0;
     // The tensor-core passes want rows that start on 16-byte boundaries.  Where the caller's do not, a copy with padded rows goes
     // into the array first, if there is room for it and the horizontal pass is long enough to pay for it: long windows on a large
-    // image (1 413 x 1 121 pixels to 512: a call 58 us without the copy, 48 with; 2 813 x 2 241: 89 and 76).  With shorter
-    // windows, or so much output that the plain pass has enough CTAs, it is the better one (to 1024: 58 and 61, 94 and 99).
+    // image.  A call without / with the copy, us, RGB: 1 229 x 1 229 pixels to 512 43 / 37, 2 049 x 2 049 59 / 46, 2 345 x 1 789 73 /
+    // 62; to 224, where the windows are too long for the tensor cores and the plain pass gains by needing no guard, 2 017 x 2 017
+    // 61 / 50, 2 913 x 2 913 168 / 137.  Reductions by 2.0 to 2.3 of 3 to 4 MB are on the line, from 15 us better to 4 worse; below
+    // that the copy loses (997 x 761 by 1.7: 44 / 47).  It would also pay for one channel from 0.5 MB on (1 229 x 1 229 to 512: 35 /
+    // 31) and for more output than kStaticCopyOut (2 457 x 2 457 to 1024: 80 / 61), where the plain pass is still taken.
     const size_t row = (size_t)w * channels, padded = align_up(row, 16), copy_bytes = align_up(padded * h, 256);
     // no less than what the descriptors and the filter tables take: 2 * (6 * in / out + 3) + 8 bytes per output of a resize to `out`,
     // 24 of a half-pixel shift

@@ -372,7 +372,8 @@ void launch_unstuff(const JpegWave& w, cudaStream_t s) {
 //  scheduler to hide it, or one where there is little work.  So a step is few instructions (SyncTab, ValueTab), none of them a
 //  jump (SyncLane::run_to, decode_blocks), and what it needs next is on its way before (Cursor, SyncLane::nx).  Before / after
 //  these three, us: values 43 / 21 (one thumbnail), 51 / 28 (one photo), 1 340 / 890 (256 files of 5 Mbit); candidates 19 / 15
-//  (thumbnail), 58 / 50 (8 files of 4:4:4), 789 / 624 (256 files); restart segments 732 / 530 (512 files of 0.4 Mbit).
+//  (thumbnail), 789 / 624 (256 files), 58 / 51 (8 files of 4:4:4, which now take twice the lead and 60, see kLead); restart segments
+//  732 / 530 (512 files of 0.4 Mbit).
 // ---------------------------------------------------------------------------------------------------------------
 namespace {
 
@@ -527,7 +528,7 @@ __device__ __forceinline__ uint32_t pack_state(uint32_t p, uint32_t cell_bit, ui
 // Where cell k of an image stands in w.cells and w.cand.  A thread of the linking kernel walks `run` consecutive cells.  Where
 // runs are long (`mixed`, see JpegWave), the cells that all threads read in the same step are neighbours instead: in order, a load
 // of a warp touched 32 lines, and the loads of a step queued for 2 900 cycles (8 images of 4:4:4, up to 17 cells a thread: 66 us
-// for the kernel, 50 like this).
+// for the kernel, 50 like this, and 39 with the longer lead on top).
 struct CellOrder {
     uint32_t run, threads;
     bool mixed;

@@ -164,7 +164,8 @@ DG_API int dg_ctx_create(int device, const dg_image_config* cfg, dg_ctx** out);
 /* Same, running on a caller-owned CUDA stream (a cudaStream_t passed as void*). */
 DG_API int dg_ctx_create_on_stream(int device, const dg_image_config* cfg, void* cuda_stream, dg_ctx** out);
 DG_API void dg_ctx_destroy(dg_ctx* ctx);
-/* The cudaStream_t all work of this ctx is queued on. */
+/* The cudaStream_t of this ctx.  A batch's kernels and downloads are ordered with it (some of them run on streams of the library
+ * that are joined to it); the copies of larger batches' inputs are not, see dg_batch_create. */
 DG_API void* dg_ctx_stream(dg_ctx* ctx);
 DG_API int dg_ctx_get_counters(dg_ctx* ctx, dg_ctx_counters* out);
 
@@ -195,9 +196,13 @@ DG_API uint64_t dg_key_rank(const char* key, uint64_t len, uint64_t world_size);
  * followed by image_to_payload (src/image_processing.rs:341-431).
  * create: parses headers, plans geometry, builds device descriptors and filter tables, copies the compressed
  *         (or raw) bytes into pinned staging.  Items whose header is bad keep a non-zero status and are skipped,
- *         as datago drops a sample whose decode fails (src/worker_files.rs:63-70).
- * upload: host -> device copies (async on the ctx stream).
- * run:    all kernels (async).  May be called repeatedly on an uploaded batch.
+ *         as datago drops a sample whose decode fails (src/worker_files.rs:63-70).  From 2 MB of inputs on it also queues
+ *         their host -> device copies, on a stream of the library while the rest is being staged: they go into memory that
+ *         only the batch uses and are ordered with nothing of the caller's.
+ * upload: host -> device copies (async on the ctx stream), unless create has queued them: then the first call queues nothing.
+ *         Inside a stream capture, and when called again, it always queues them on the ctx stream.
+ * run:    all kernels (async); orders the ctx stream behind the inputs, wherever their copies were queued.  May be called
+ *         repeatedly on an uploaded batch.
  * download: device -> host copy of every ok item into host_out[i] (entries may be NULL to skip).
  * sync:   waits for the stream and collects per-item device status words.
  */
