@@ -1919,6 +1919,7 @@ extern "C" int dg_batch_huffman_stats(dg_batch* b, uint64_t out[3]) {
     dg_ctx* ctx = b->ctx;
     std::lock_guard<std::mutex> lock(ctx->mu);
     CU(cudaSetDevice(ctx->device));
+    if (!b->ran) await_inputs(b);  // (zeros, which come with the inputs)
     CU(cudaMemcpyAsync(out, b->d_persist + b->off_status + stats_at(b->n), 24, cudaMemcpyDeviceToHost, ctx->stream));
     CU(cudaStreamSynchronize(ctx->stream));
     return DG_OK;

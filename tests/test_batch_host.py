@@ -119,3 +119,15 @@ def test_counters_hold_what_was_copied(fake, n):
         # (small batches: larger ones are copied before upload is called)
         assert (k["h2d_bytes"], k["d2h_bytes"]) == (fake.fake_to_device() - before[0], fake.fake_to_host() - before[1])
     c.close()
+
+
+@pytest.mark.parametrize("n", [1, 3])
+def test_decoder_counters_of_a_batch_that_has_not_run(fake, n):
+    # zeros, as uploaded, also while the inputs of a larger batch are on their way
+    c = dg.Context(0, CFG)
+    with c.batch([raw((300 * n, 400 * n, 3))]) as b:
+        b.upload()
+        assert set(b.huffman_stats().values()) == {0}
+        b.run()
+        b.sync()
+    c.close()
