@@ -84,6 +84,24 @@ def test_large_images_at_every_alignment(shape, lead):
         assert np.array_equal(dst.cpu().numpy(), want), sentinel
 
 
+@pytest.mark.parametrize("shape,lead", [((2403, 2403, 3), 1), ((2048, 2048, 3), 0), ((2048, 2048, 3), 5), ((2600, 2403, 1), 3), ((3300, 3401, 1), 2)])
+def test_reductions_beyond_what_the_tensor_cores_take(shape, lead):
+    # by 9 to 15: RGB windows are too long for a CTA of the tensor-core pass, in place and in the padded copy; gray ones still fit
+    # in the copy but the last
+    import torch
+    cfg = dict(crop_and_resize=True, default_image_size=224, downsampling_ratio=16, min_aspect_ratio=0.5, max_aspect_ratio=2.0)
+    ctx = dg.Context(0, cfg)
+    img = np.random.default_rng(44).integers(0, 256, shape, dtype=np.uint8)
+    (status, want, _), = ctx.process([img[:, :, 0] if shape[2] == 1 else img])
+    assert status == 0
+    big = torch.full((lead + img.size + 64,), 255, dtype=torch.uint8, device="cuda")
+    big[lead:lead + img.size] = torch.from_numpy(img.reshape(-1)).cuda()
+    dst = torch.zeros(want.shape, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    ctx.resize_device_static(big.data_ptr() + lead, shape[1], shape[0], shape[2], dst.data_ptr())
+    assert np.array_equal(dst.cpu().numpy(), want)
+
+
 def test_identity_and_copy_only_plans():
     ctx = dg.Context(0, CFG)
     rng = np.random.default_rng(42)
